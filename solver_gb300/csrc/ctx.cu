@@ -78,7 +78,8 @@ void launch_perm_gather(const c64*, const int32_t*, const double*, int, c64*, cu
 int sptrsv_grp_prepare(size_t smem_bytes);
 int launch_sptrsv(const GrpPlan&, cudaStream_t, cudaEvent_t, cudaEvent_t, const int32_t*, int,
                   int, const SfTri&, const SfTri&,
-                  const c64*, const int32_t*, const double*, c64*, c64*, int*, cudaStream_t);
+                  const c64*, const int32_t*, const double*, c64*, c64*, c64*, int*, cudaStream_t);
+int lu_lanes(int nr, int ne, bool shared);
 int red_blocks(size_t N);
 int launch_multidot(const c64*, size_t, const c64*, size_t, int, c64*, c64*, cudaStream_t);
 int launch_multidot(const cff*, size_t, const c64*, size_t, int, c64*, c64*, cudaStream_t);
@@ -134,6 +135,7 @@ struct LevelTri {  // triangular factor without its diagonal (CSR) and its level
   std::vector<int32_t> rows;     // rows sorted by level (host)
   std::vector<int> lvl_off;      // offsets into rows per level (host)
   std::vector<int32_t> hptr, hcol;  // host copy of the structure
+  bool unit = false;                // the diagonal is one
 };
 
 struct peec_ctx {
@@ -210,13 +212,14 @@ struct peec_ctx {
   // synchronisation-free triangular solves: claim order (L levels then U levels, each
   // padded with -1 to whole warps), its length, the L part's length, control words
   int32_t* sf_ord = nullptr;
-  // per-warp group solves (GrpPlan): components of at most comp_max rows; the device
+  // per-CTA group solves (GrpPlan): components of at most comp_max rows; the device
   // arrays of the plan (host-built with the factors' structure)
-  int comp_max = SF_COMP_MAX;  // largest component solved per warp (0: global scheme only)
+  int comp_max = SF_COMP_MAX;  // largest component solved per CTA (0: global scheme only)
   GrpPlan grp;
   int32_t *grp_goff = nullptr, *grp_seg = nullptr, *grp_segoff = nullptr, *grp_nsegL = nullptr;
+  int32_t *grp_eoff = nullptr, *grp_esrc = nullptr;
   GrpRow* grp_rows = nullptr;
-  int16_t *grp_uq = nullptr, *grp_lcolL = nullptr, *grp_lcolU = nullptr;
+  int16_t *grp_uq = nullptr, *grp_ecol = nullptr;
   c64 *ir_b = nullptr, *ir_x = nullptr, *ir_r = nullptr, *ir_d = nullptr;  // refinement vectors
   // the frequency w on the device (the row kernels read it there, so captured graphs of
   // the operator stay valid when only the frequency state changes) and the entries the
@@ -515,7 +518,7 @@ extern "C" void peec_ctx_destroy(peec_ctx* ctx) {
   cudaFree(ctx->rf_err);
   for (void* p : {(void*)ctx->grp_goff, (void*)ctx->grp_seg, (void*)ctx->grp_segoff,
                   (void*)ctx->grp_nsegL, (void*)ctx->grp_rows, (void*)ctx->grp_uq,
-                  (void*)ctx->grp_lcolL, (void*)ctx->grp_lcolU})
+                  (void*)ctx->grp_eoff, (void*)ctx->grp_esrc, (void*)ctx->grp_ecol})
     cudaFree(p);
   for (c64* p : {ctx->ir_b, ctx->ir_x, ctx->ir_r, ctx->ir_d, ctx->cc_x, ctx->cc_LpI, ctx->cc_PQ})
     cudaFree(p);
@@ -1438,6 +1441,7 @@ static int make_tri(peec_ctx* ctx, LevelTri& T, int64_t n, const int64_t* ptr, c
   c.reserve(ptr[n]);
   v.reserve(ptr[n]);
   std::vector<int> level(n, 0);
+  T.unit = true;
   for (int64_t r = 0; r < n; ++r) {
     cd diag(0.0, 0.0);
     for (int64_t q = ptr[r]; q < ptr[r + 1]; ++q) {
@@ -1454,6 +1458,7 @@ static int make_tri(peec_ctx* ctx, LevelTri& T, int64_t n, const int64_t* ptr, c
       }
     }
     if (diag == cd(0.0, 0.0)) return bad(ctx, PEEC_ERR_BADARG, "zero pivot in triangular factor");
+    T.unit = T.unit && diag == cd(1.0, 0.0);
     const cd di = 1.0 / diag;
     dinv[r] = mk<double>(di.real(), di.imag());
     p[r + 1] = (int32_t)c.size();
@@ -1499,11 +1504,10 @@ static int make_tri(peec_ctx* ctx, LevelTri& T, int64_t n, const int64_t* ptr, c
 
 // Work split of the LU solves. The rows of L and U fall into connected components
 // (rows linked by a factor entry); rows of different components never depend on one
-// another. Components of at most comp_max rows are solved per warp (k_sptrsv_grp): those
-// of at most 32 rows and SF_GRP_E entries packed into groups of at most 32 rows and
-// SF_GRP_E entries, in order of their level depth (so that a group's levels are mostly
-// full), larger ones one per group; the rows of components above comp_max (or too large
-// for a warp's shared memory) go to the synchronisation-free global scheme.
+// another. Components of at most comp_max rows are solved per CTA (k_sptrsv_grp): small
+// ones packed into groups in order of their level depth (so that a group's levels are
+// mostly full), larger ones one per group; the rows of components above comp_max (or too
+// large for a CTA's shared memory) go to the synchronisation-free global scheme.
 static int build_solve_plan(peec_ctx* ctx, int64_t n) {
   const LevelTri &L = ctx->Lf, &U = ctx->Uf;
   // union-find over the factor entries
@@ -1535,12 +1539,12 @@ static int build_solve_plan(peec_ctx* ctx, int64_t n) {
     cent[c] += (L.hptr[r + 1] - L.hptr[r]) + (U.hptr[r + 1] - U.hptr[r]);
     cdepth[c] = std::max(cdepth[c], lvL[r] + lvU[r] + 2);
   }
-  // largest groups a warp's shared memory takes (a large component alone)
+  // largest group a CTA's shared memory takes (a large component alone)
   const size_t smem_cap = 160 * 1024;
   std::vector<int32_t> big, small;
   for (int64_t r = 0; r < n; ++r) {
     if (comp[r] != r || csize[r] > ctx->comp_max) continue;
-    if (csize[r] <= 32 && cent[r] <= SF_GRP_E) small.push_back((int32_t)r);
+    if (csize[r] <= SF_PACK_COMP && cent[r] <= SF_PACK_E / 2) small.push_back((int32_t)r);
     else if (cent[r] < 32768 && grp_smem(csize[r], cent[r]) <= smem_cap) big.push_back((int32_t)r);
   }
   // large components, longest chains first; small ones by depth
@@ -1556,18 +1560,28 @@ static int build_solve_plan(peec_ctx* ctx, int64_t n) {
     eb = std::max(eb, cent[c]);
   }
   const int nbig = ng;
+  int rp = 0, ep = 0;
   {
+    // two groups per SM before they grow to SF_PACK_R rows: a small system's levels are
+    // latency, a large one's groups should be full
+    int64_t total = 0;
+    for (int32_t c : small) total += csize[c];
+    const int64_t slots = 2 * std::max(ctx->nsm, 1);
+    const int cap = (int)std::min<int64_t>(SF_PACK_R, std::max<int64_t>(32, (total + slots - 1) / slots));
     int rows = 0, ents = 0;
     for (int32_t c : small) {
-      if (ng == nbig || rows + csize[c] > 32 || ents + cent[c] > SF_GRP_E) {
+      if (ng == nbig || (rows && rows + csize[c] > cap) || ents + cent[c] > SF_PACK_E) {
         ++ng;
         rows = ents = 0;
       }
       gidx[c] = ng - 1;
       rows += csize[c];
       ents += cent[c];
+      rp = std::max(rp, rows);
+      ep = std::max(ep, ents);
     }
   }
+  const bool crowded = ng > 4 * std::max(ctx->nsm, 1);  // more groups than one per warp scheduler
   // the groups' rows, in L-level order within each group
   std::vector<int32_t> goff(ng + 1, 0);
   for (int64_t r = 0; r < n; ++r)
@@ -1578,45 +1592,63 @@ static int build_solve_plan(peec_ctx* ctx, int64_t n) {
     if (gidx[comp[r]] >= 0) rowsL[fill[gidx[comp[r]]]++] = (int32_t)r;
   std::vector<int32_t> rowsU(rowsL), local(n, -1), seg, segoff(ng + 1, 0), nsegL(ng, 0);
   std::vector<GrpRow> grows(goff[ng]);
-  std::vector<int16_t> uq(goff[ng]);
+  std::vector<int16_t> uq(goff[ng]), ecol;
+  std::vector<int32_t> eoff(ng + 1, 0), esrc;
+  // results straight through Pc when every row is in a group and Pc is a permutation
+  std::vector<int32_t> outp(n, -1);
+  bool direct = goff[ng] == n && (int64_t)ctx->h_gout.size() == n;
+  for (int64_t i = 0; direct && i < n; ++i) {
+    int32_t& t = outp[ctx->h_gout[i]];
+    direct = t < 0;
+    t = (int32_t)i;
+  }
   for (int g = 0; g < ng; ++g) {
     const auto b0 = rowsL.begin() + goff[g], e0 = rowsL.begin() + goff[g + 1];
     std::stable_sort(b0, e0, [&](int32_t x, int32_t y) { return lvL[x] < lvL[y]; });
     for (int32_t q = goff[g]; q < goff[g + 1]; ++q) local[rowsL[q]] = q - goff[g];
-    for (int32_t q = goff[g]; q < goff[g + 1]; ++q)
-      if (q + 1 == goff[g + 1] || lvL[rowsL[q + 1]] != lvL[rowsL[q]]) seg.push_back(q + 1 - goff[g]);
-    nsegL[g] = (int32_t)seg.size() - segoff[g];
     const auto bu = rowsU.begin() + goff[g], eu = rowsU.begin() + goff[g + 1];
     std::stable_sort(bu, eu, [&](int32_t x, int32_t y) { return lvU[x] < lvU[y]; });
-    for (int32_t q = goff[g]; q < goff[g + 1]; ++q) {
-      uq[q] = (int16_t)local[rowsU[q]];
-      if (q + 1 == goff[g + 1] || lvU[rowsU[q + 1]] != lvU[rowsU[q]]) seg.push_back(q + 1 - goff[g]);
+    for (int32_t q = goff[g]; q < goff[g + 1]; ++q) uq[q] = (int16_t)local[rowsU[q]];
+    for (const LevelTri* T : {&L, &U}) {
+      const std::vector<int32_t>&rows = T == &L ? rowsL : rowsU, &lv = T == &L ? lvL : lvU;
+      int first = goff[g], ne = 0;
+      for (int32_t q = goff[g]; q < goff[g + 1]; ++q) {
+        const int32_t r = rows[q];
+        ne = std::max(ne, T->hptr[r + 1] - T->hptr[r]);
+        if (q + 1 == goff[g + 1] || lv[rows[q + 1]] != lv[r]) {
+          const int lw = lu_lanes(q + 1 - first, ne, crowded && g >= nbig);
+          seg.push_back((q + 1 - goff[g]) | (lw << 16));
+          first = q + 1;
+          ne = 0;
+        }
+      }
+      if (T == &L) nsegL[g] = (int32_t)seg.size() - segoff[g];
     }
     segoff[g + 1] = (int32_t)seg.size();
-    int e = 0;
     for (int32_t q = goff[g]; q < goff[g + 1]; ++q) {
       const int32_t r = rowsL[q];
       GrpRow& gr = grows[q];
       gr.r = r;
-      gr.pL = L.hptr[r];
-      gr.pU = U.hptr[r];
       gr.j = ctx->h_gin.empty() ? r : ctx->h_gin[r];
+      gr.o = direct ? outp[r] : r;
       gr.nL = (int16_t)(L.hptr[r + 1] - L.hptr[r]);
       gr.nU = (int16_t)(U.hptr[r + 1] - U.hptr[r]);
-      gr.eL = (int16_t)e;
-      e += gr.nL;
-      gr.eU = (int16_t)e;
-      e += gr.nU;
+      gr.eL = (int16_t)((int32_t)esrc.size() - eoff[g]);
+      for (int32_t t = L.hptr[r]; t < L.hptr[r + 1]; ++t) {
+        esrc.push_back(t);
+        ecol.push_back((int16_t)local[L.hcol[t]]);
+      }
+      gr.eU = (int16_t)((int32_t)esrc.size() - eoff[g]);
+      for (int32_t t = U.hptr[r]; t < U.hptr[r + 1]; ++t) {
+        esrc.push_back(~t);
+        ecol.push_back((int16_t)local[U.hcol[t]]);
+      }
     }
+    eoff[g + 1] = (int32_t)esrc.size();
   }
-  // entry columns as positions in the row's group
-  std::vector<int16_t> lcolL(std::max<size_t>(L.hcol.size(), 1), -1),
-      lcolU(std::max<size_t>(U.hcol.size(), 1), -1);
-  for (const auto* T : {&L, &U}) {
-    std::vector<int16_t>& lc = T == &L ? lcolL : lcolU;
-    for (int64_t r = 0; r < n; ++r)
-      if (local[r] >= 0)
-        for (int32_t q = T->hptr[r]; q < T->hptr[r + 1]; ++q) lc[q] = (int16_t)local[T->hcol[q]];
+  if (esrc.empty()) {
+    esrc.push_back(0);
+    ecol.push_back(0);
   }
   if (ng == 0) {  // keep the arrays non-empty
     seg.push_back(0);
@@ -1631,8 +1663,9 @@ static int build_solve_plan(peec_ctx* ctx, int64_t n) {
   CTX_TRY(upload(&ctx->grp_seg, seg, ctx->st));
   CTX_TRY(upload(&ctx->grp_segoff, segoff, ctx->st));
   CTX_TRY(upload(&ctx->grp_nsegL, nsegL, ctx->st));
-  CTX_TRY(upload(&ctx->grp_lcolL, lcolL, ctx->st));
-  CTX_TRY(upload(&ctx->grp_lcolU, lcolU, ctx->st));
+  CTX_TRY(upload(&ctx->grp_eoff, eoff, ctx->st));
+  CTX_TRY(upload(&ctx->grp_esrc, esrc, ctx->st));
+  CTX_TRY(upload(&ctx->grp_ecol, ecol, ctx->st));
   GrpPlan& P = ctx->grp;
   P.goff = ctx->grp_goff;
   P.rows = ctx->grp_rows;
@@ -1640,13 +1673,18 @@ static int build_solve_plan(peec_ctx* ctx, int64_t n) {
   P.seg = ctx->grp_seg;
   P.segoff = ctx->grp_segoff;
   P.nsegL = ctx->grp_nsegL;
-  P.lcolL = ctx->grp_lcolL;
-  P.lcolU = ctx->grp_lcolU;
+  P.eoff = ctx->grp_eoff;
+  P.esrc = ctx->grp_esrc;
+  P.ecol = ctx->grp_ecol;
   P.nbig = nbig;
   P.ngroups = ng;
   P.rb = rb;
   P.eb = eb;
-  const size_t need = std::max(grp_smem(rb, eb), SF_GRP_WARPS * grp_smem(32, SF_GRP_E));
+  P.rp = rp;
+  P.ep = ep;
+  P.direct = direct;
+  P.unit_l = L.unit;
+  const size_t need = grp_smem(std::max(rb, rp), std::max(eb, ep));
   if (sptrsv_grp_prepare(need)) return PEEC_ERR_CUDA;
   std::vector<int32_t> cidx(n, -1);
   for (int64_t r = 0; r < n; ++r) cidx[r] = gidx[comp[r]];
@@ -2107,9 +2145,10 @@ static void lu_solve(peec_ctx* ctx, const c64* b, c64* x) {
   const int n = (int)ctx->n;
   const LevelTri &L = ctx->Lf, &U = ctx->Uf;
   ctx->launches += launch_sptrsv(
-      ctx->grp, ctx->st2, ctx->ev_fork, ctx->ev_join, ctx->sf_ord, ctx->sf_nL, ctx->sf_total, SfTri{L.ptr, L.col, L.val, L.dinv, L.flag},
-      SfTri{U.ptr, U.col, U.val, U.dinv, U.flag}, b, ctx->g_in, ctx->lu_rs, ctx->lutmp,
-      ctx->lutmp2, ctx->sf_ctl, ctx->st);
+      ctx->grp, ctx->st2, ctx->ev_fork, ctx->ev_join, ctx->sf_ord, ctx->sf_nL, ctx->sf_total,
+      SfTri{L.ptr, L.col, L.val, L.dinv, L.flag}, SfTri{U.ptr, U.col, U.val, U.dinv, U.flag}, b,
+      ctx->g_in, ctx->lu_rs, ctx->lutmp, ctx->lutmp2, x, ctx->sf_ctl, ctx->st);
+  if (ctx->grp.direct) return;
   launch_perm_gather(ctx->lutmp2, ctx->g_out, nullptr, n, x, ctx->st);
   ctx->launches += 1;
 }

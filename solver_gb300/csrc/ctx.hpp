@@ -27,18 +27,19 @@ constexpr int SF_TPB = 128;
 
 // Groups of the LU solves (sparse.cu, k_sptrsv_grp). The rows of L and U fall into
 // connected components (rows linked by a factor entry) that never depend on one another.
-// Components of at most 32 rows (and SF_GRP_E entries) are packed into groups of at most
-// 32 rows; larger ones (up to SF_COMP_MAX rows) form a group each. One warp solves a
-// group: it loads all of the group's rows, entries and right-hand sides into shared
-// memory with parallel loads, then runs the group's L levels and U levels there.
+// Components of at most SF_PACK_COMP rows and SF_PACK_E / 2 entries are packed, in order of
+// their depth, into groups of up to SF_PACK_R rows; larger ones (up to SF_COMP_MAX rows)
+// form a group each. One CTA solves a group: it loads all of the group's rows, entries and
+// right-hand sides into shared memory, then runs the group's L levels and U levels there.
 constexpr int SF_COMP_MAX = 512;
-constexpr int SF_GRP_E = 256;  // entries (L and U off-diagonal) of a packed group
-constexpr int SF_GRP_WARPS = 4;
-constexpr int SF_BIG_LANES = 4;  // lanes per row in the large components' level loops
+constexpr int SF_PACK_COMP = 64;  // rows of a component that may be packed with others
+constexpr int SF_PACK_R = 256;    // rows of a packed group
+constexpr int SF_PACK_E = 1024;   // its entries (L and U off-diagonal)
+constexpr int SF_GRP_TPB = 128;   // one warp per SM sub-partition, each with its FP64 pipe
 struct GrpRow {
   int32_t r;       // factor row
-  int32_t pL, pU;  // first entry of the row in L and in U (CSR)
   int32_t j;       // original row of its right-hand side (Pr)
+  int32_t o;       // where its result goes: the original column (Pc), or r (GrpPlan::direct)
   int16_t nL, nU;  // entries of the row in L and in U
   int16_t eL, eU;  // their offsets in the group's shared entry array
 };
@@ -46,20 +47,25 @@ struct GrpPlan {
   const int32_t* goff = nullptr;    // ngroups + 1 offsets into rows
   const GrpRow* rows = nullptr;     // per position: the group's rows in L-level order
   const int16_t* uq = nullptr;      // per position in U-level order: that row's L position
-  const int32_t* seg = nullptr;     // per group: ends of its L levels, then of its U levels
+  const int32_t* seg = nullptr;     // per group: its L levels, then its U levels; the end of
+                                    // the level, and above bit 16 log2 of the lanes per row
   const int32_t* segoff = nullptr;  // ngroups + 1 offsets into seg
-  const int32_t* nsegL = nullptr;   // per group: the number of its L level ends
-  const int16_t* lcolL = nullptr;   // per L entry (CSR order): its column's L position
-  const int16_t* lcolU = nullptr;   // per U entry
+  const int32_t* nsegL = nullptr;   // per group: the number of its L levels
+  const int32_t* eoff = nullptr;    // ngroups + 1 offsets into esrc / ecol
+  const int32_t* esrc = nullptr;    // per group entry: its index in L's values, or ~index in U's
+  const int16_t* ecol = nullptr;    // per group entry: its column's L position in the group
   int nbig = 0, ngroups = 0;        // groups [0, nbig) hold one large component each
   int rb = 0, eb = 0;               // the large groups' largest row and entry counts
+  int rp = 0, ep = 0;               // the packed groups' largest
+  bool direct = false;              // results go through Pc already (no global-scheme rows)
+  bool unit_l = false;              // L's diagonal is one
 };
-// shared memory of one group of R rows and E entries
+// shared memory of a group of R rows and E entries
 __host__ __device__ inline size_t grp_smem(int R, int E) {
   size_t o = 48 * (size_t)R + 16 * (size_t)E;  // x, 1/L(i,i), 1/U(i,i), entry values
   o += 8 * (size_t)R + 2 * (size_t)E + 2 * (size_t)R;  // row metadata, entry columns, U order
   o = (o + 3) & ~(size_t)3;
-  o += 8 * (size_t)R;  // level ends (at most 2R)
+  o += 8 * (size_t)R;  // levels (at most 2R)
   return (o + 15) & ~(size_t)15;
 }
 

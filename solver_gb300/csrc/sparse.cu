@@ -152,28 +152,38 @@ __global__ void k_sptrsv_begin(int* ctl) {
   ctl[3] = 0;
 }
 
-// One warp per group (GrpPlan): components of the factors, several small ones packed
-// together or one large one. The warp first brings everything the group's solve reads
-// into its slice of shared memory -- per row the right-hand side (gathered through Pr
-// and scaled by Rs), both inverse diagonals, its L and U entries with their columns as
-// positions in the group -- with every row's loads independent of the others', so the
-// whole group costs a few round trips to memory. Then the L levels, the U levels (in
-// place: a U row reads its own L value and the U values of rows of earlier U levels),
-// __syncwarp between levels, and the results go out to z. Per row the arithmetic is that
-// of k_sptrsv (right-hand side, entries subtracted in row order, times the inverse
-// diagonal). R, E: the shared-memory capacity of a warp's slice (rows, entries).
-// W lanes per row in the level loops: 1 for the packed groups (short rows, one lane each);
-// more for the large components, whose rows carry tens of entries on a chain of dozens
-// of levels: the lanes of a row split its entries and combine their partial sums with a
-// fixed shuffle tree (the same order on every run).
-template <int W>
-__global__ void k_sptrsv_grp(GrpPlan P, int g0, int g1, int R, int E, SfTri L, SfTri U,
-                             const c64* __restrict__ b, const double* __restrict__ rs, c64* z) {
+// One CTA per group (GrpPlan): components of the factors, several small ones packed
+// together or one large one. The CTA first brings everything the group's solve reads into
+// shared memory -- per row the right-hand side (gathered through Pr and scaled by Rs) and
+// both inverse diagonals, per entry its value and its column as a position in the group --
+// with all loads independent of one another. Then the L levels, the U levels (in place: a U
+// row reads its own L value and the U values of rows of earlier U levels), a barrier between
+// levels, and the results go out.
+//
+// What bounds it is the FP64 pipe's latency and issue: on GB300 a warp's FP64 instruction
+// holds its sub-partition's pipe for 64 cycles whatever the number of its active lanes
+// (19 cycles per instruction with all four sub-partitions busy). So a level's cost is the
+// number of FP64 instructions on its longest warp, not its flops, and the split keeps that
+// low: four warps per group, one per sub-partition; a row takes 2 to 32 lanes (chosen per
+// level on the host, lu_lanes), half of them for the real and half for the imaginary part,
+// so that a complex multiply-add is two instructions and the final product with the inverse
+// diagonal two more (none in L when its diagonal is one). The lanes' partial sums meet in a
+// fixed shuffle tree, so results do not depend on scheduling.
+// Measured, one solve on an idle GPU: 128x128x64 (183,490 rows, 60,943 components, depth 29)
+// 44.4 us, against 72.5 us beside 72.1 us on a second stream with one warp per group and a
+// row on one to four lanes; 96x96x48 copper (largest component 291 rows) 39.8 against
+// 128.1 us; the 20x20x4 crossbar (one component, 100 levels) 57.7 against 111.4 us.
+__global__ void __launch_bounds__(SF_GRP_TPB) k_sptrsv_grp(GrpPlan P, int g0, int R, int E,
+                                                           const c64* __restrict__ Lval,
+                                                           const c64* __restrict__ Uval,
+                                                           const c64* __restrict__ Ldinv,
+                                                           const c64* __restrict__ Udinv,
+                                                           const c64* __restrict__ b,
+                                                           const double* __restrict__ rs,
+                                                           c64* __restrict__ out) {
   extern __shared__ __align__(16) unsigned char grp_sm[];
-  const int lane = threadIdx.x & 31;
-  const int wib = threadIdx.x >> 5, wpb = blockDim.x >> 5;
-  unsigned char* base = grp_sm + (size_t)wib * grp_smem(R, E);
-  c64* xs = reinterpret_cast<c64*>(base);
+  const int tid = threadIdx.x;
+  c64* xs = reinterpret_cast<c64*>(grp_sm);
   c64* dl = xs + R;
   c64* du = dl + R;
   c64* ev = du + R;
@@ -182,84 +192,63 @@ __global__ void k_sptrsv_grp(GrpPlan P, int g0, int g1, int R, int E, SfTri L, S
   int16_t* uqs = ec + E;
   int32_t* segs = reinterpret_cast<int32_t*>(
       (reinterpret_cast<uintptr_t>(uqs + R) + 3) & ~(uintptr_t)3);
-  for (int g = g0 + blockIdx.x * wpb + wib; g < g1; g += gridDim.x * wpb) {
-    const int q0 = P.goff[g], nr = P.goff[g + 1] - q0;
-    const int s0 = P.segoff[g], ns = P.segoff[g + 1] - s0, nsl = P.nsegL[g];
-    for (int q = lane; q < nr; q += 32) {
-      const GrpRow pr = P.rows[q0 + q];
-      xs[q] = rs ? cscale(b[pr.j], rs[pr.j]) : b[pr.j];
-      dl[q] = L.dinv[pr.r];
-      du[q] = U.dinv[pr.r];
-      meta[q] = make_short4(pr.eL, pr.nL, pr.eU, pr.nU);
-      for (int t = 0; t < pr.nL; ++t) {
-        ev[pr.eL + t] = L.val[pr.pL + t];
-        ec[pr.eL + t] = P.lcolL[pr.pL + t];
-      }
-      for (int t = 0; t < pr.nU; ++t) {
-        ev[pr.eU + t] = U.val[pr.pU + t];
-        ec[pr.eU + t] = P.lcolU[pr.pU + t];
-      }
-      uqs[q] = P.uq[q0 + q];
-    }
-    for (int t = lane; t < ns; t += 32) segs[t] = P.seg[s0 + t];
-    __syncwarp();
-    if constexpr (W == 1) {
-      int prev = 0;
-      for (int s = 0; s < nsl; ++s) {
-        const int se = segs[s];
-        for (int q = prev + lane; q < se; q += 32) {
-          const short4 m = meta[q];
-          c64 acc = xs[q];
-          for (int t = 0; t < m.y; ++t) acc = acc - ev[m.x + t] * xs[ec[m.x + t]];
-          xs[q] = acc * dl[q];
-        }
-        __syncwarp();
-        prev = se;
-      }
-      prev = 0;
-      for (int s = nsl; s < ns; ++s) {
-        const int se = segs[s];
-        for (int t = prev + lane; t < se; t += 32) {
-          const int q = uqs[t];
-          const short4 m = meta[q];
-          c64 acc = xs[q];
-          for (int e = 0; e < m.w; ++e) acc = acc - ev[m.z + e] * xs[ec[m.z + e]];
-          xs[q] = acc * du[q];
-        }
-        __syncwarp();
-        prev = se;
-      }
-    } else {
-      constexpr int G = 32 / W;  // rows in flight per step
-      const int sub = lane % W, grp = lane / W;
-      int prev = 0;
-      for (int s = 0; s < ns; ++s) {
-        const bool upper = s >= nsl;
-        const int se = segs[s];
-        for (int t0 = prev; t0 < se; t0 += G) {  // warp-uniform: every lane shuffles
-          const int t = t0 + grp;
-          const bool valid = t < se;
-          const int q = valid ? (upper ? (int)uqs[t] : t) : 0;
-          c64 part = mk<double>(0, 0);
-          if (valid) {
-            const short4 m = meta[q];
-            const int e0 = upper ? m.z : m.x, ne = upper ? m.w : m.y;
-            for (int e = sub; e < ne; e += W) part = part + ev[e0 + e] * xs[ec[e0 + e]];
-          }
-#pragma unroll
-          for (int o = W / 2; o > 0; o >>= 1) {
-            part.x += __shfl_xor_sync(0xffffffffu, part.x, o, W);
-            part.y += __shfl_xor_sync(0xffffffffu, part.y, o, W);
-          }
-          if (valid && sub == 0) xs[q] = (xs[q] - part) * (upper ? du[q] : dl[q]);
-        }
-        __syncwarp();
-        prev = s + 1 == nsl ? 0 : se;
-      }
-    }
-    for (int q = lane; q < nr; q += 32) z[P.rows[q0 + q].r] = xs[q];
-    __syncwarp();
+  const int g = g0 + blockIdx.x;
+  const int q0 = P.goff[g], nr = P.goff[g + 1] - q0;
+  const int s0 = P.segoff[g], ns = P.segoff[g + 1] - s0, nsl = P.nsegL[g];
+  const int e0 = P.eoff[g], ne_g = P.eoff[g + 1] - e0;
+  const bool unit = P.unit_l;
+  for (int e = tid; e < ne_g; e += SF_GRP_TPB) {
+    const int src = P.esrc[e0 + e];
+    ec[e] = P.ecol[e0 + e];
+    ev[e] = src >= 0 ? Lval[src] : Uval[~src];
   }
+  for (int q = tid; q < nr; q += SF_GRP_TPB) {
+    const GrpRow pr = P.rows[q0 + q];
+    xs[q] = rs ? cscale(b[pr.j], rs[pr.j]) : b[pr.j];
+    if (!unit) dl[q] = Ldinv[pr.r];
+    du[q] = Udinv[pr.r];
+    meta[q] = make_short4(pr.eL, pr.nL, pr.eU, pr.nU);
+    uqs[q] = P.uq[q0 + q];
+  }
+  for (int t = tid; t < ns; t += SF_GRP_TPB) segs[t] = P.seg[s0 + t];
+  __syncthreads();
+  const int part = tid & 1;
+  const int warp0 = tid & ~31;
+  int prev = 0;
+  for (int s = 0; s < ns; ++s) {
+    const bool upper = s >= nsl;
+    const int sg = segs[s];
+    const int se = sg & 0xffff, lw = sg >> 16;
+    const int W = 1 << lw, H = W >> 1, slots = SF_GRP_TPB >> lw;
+    const int h = (tid & (W - 1)) >> 1;
+    // warp-uniform: every lane of a warp with rows left shuffles
+    for (int t0 = prev; t0 + (warp0 >> lw) < se; t0 += slots) {
+      const int t = t0 + (tid >> lw);
+      const bool valid = t < se;
+      const int q = valid ? (upper ? (int)uqs[t] : t) : 0;
+      double acc = 0.0;
+      if (valid) {
+        const short4 m = meta[q];
+        const int eb = upper ? m.z : m.x, n = upper ? m.w : m.y;
+        for (int e = h; e < n; e += H) {
+          const c64 v = ev[eb + e], x = xs[ec[eb + e]];
+          acc = fma(v.x, part ? x.y : x.x, acc);
+          acc = fma(v.y, part ? x.x : -x.y, acc);
+        }
+      }
+      for (int o = H; o >= 2; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+      double r = reinterpret_cast<const double*>(xs)[2 * q + part] - acc;
+      if (upper || !unit) {
+        const c64 d = upper ? du[q] : dl[q];
+        const double p = __shfl_xor_sync(0xffffffffu, r, 1);
+        r = part ? fma(p, d.y, r * d.x) : fma(-p, d.y, r * d.x);
+      }
+      if (valid && h == 0) reinterpret_cast<double*>(xs)[2 * q + part] = r;
+    }
+    __syncthreads();
+    prev = s + 1 == nsl ? 0 : se;
+  }
+  for (int q = tid; q < nr; q += SF_GRP_TPB) out[P.rows[q0 + q].o] = xs[q];
 }
 
 __device__ __forceinline__ void sf_wait(const int* f, int epoch, int* err, int limit) {
@@ -345,6 +334,8 @@ __global__ void __launch_bounds__(SF_TPB) k_sptrsv(const int32_t* __restrict__ o
   }
 }
 
+constexpr size_t SF_ONE_LAUNCH_SMEM = 56 * 1024;  // four resident CTAs per SM
+
 static inline unsigned grid_for(long long n, int tpb = 256) {
   long long g = (n + tpb - 1) / tpb;
   if (g < 1) g = 1;
@@ -394,43 +385,61 @@ int sptrsv_grp_prepare(size_t smem_bytes) {
   std::lock_guard<std::mutex> lock(mu);
   // set every time (a re-created context starts from the default again)
   const size_t v = std::max(smem_bytes, granted[dev]);
-  PEEC_CUDA_TRY(cudaFuncSetAttribute(k_sptrsv_grp<1>,
-                                     cudaFuncAttributeMaxDynamicSharedMemorySize, (int)v));
-  PEEC_CUDA_TRY(cudaFuncSetAttribute(k_sptrsv_grp<SF_BIG_LANES>,
-                                     cudaFuncAttributeMaxDynamicSharedMemorySize, (int)v));
+  PEEC_CUDA_TRY(cudaFuncSetAttribute(k_sptrsv_grp, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)v));
   granted[dev] = v;
   return 0;
 }
 
+// lanes per row (log2) of a level with nr rows of at most ne entries: the smallest product
+// of the level's passes over the CTA (alone) or over its warps (shared: the SM runs several
+// groups and its FP64 issue is what counts) and the FP64 instructions of one pass
+int lu_lanes(int nr, int ne, bool shared) {
+  int best = 1;
+  long cost = -1;
+  for (int lw = 1; lw <= 5; ++lw) {
+    const int H = 1 << (lw - 1);
+    const long unit = shared ? 32 : SF_GRP_TPB;
+    const long passes = ((long)nr * (1 << lw) + unit - 1) / unit;
+    const long c = passes * (2L * ((ne + H - 1) / H) + (lw - 1) + 3);
+    if (cost < 0 || c < cost) {
+      cost = c;
+      best = lw;
+    }
+  }
+  return best;
+}
+
 // returns the number of kernels launched
-// The large groups go to st2 (forked from st with ev_fork, joined back with ev_join) so
-// that they run beside the packed groups: the two launches are independent (different
-// rows), and each is set by its own deepest groups' chain of levels. Under stream capture
-// the fork and join become graph edges.
+// One launch over all groups when the large ones fit the shared memory of a few resident
+// CTAs; else the large groups go to st2 (forked from st with ev_fork, joined back with
+// ev_join; under stream capture the fork and join become graph edges) so that they run
+// beside the packed groups without widening these groups' shared memory.
 int launch_sptrsv(const GrpPlan& P, cudaStream_t st2, cudaEvent_t ev_fork, cudaEvent_t ev_join,
                   const int32_t* ord, int nL, int total, const SfTri& L, const SfTri& U,
-                  const c64* b, const int32_t* g_in, const double* rs, c64* y, c64* z, int* ctl,
-                  cudaStream_t st) {
+                  const c64* b, const int32_t* g_in, const double* rs, c64* y, c64* z, c64* x,
+                  int* ctl, cudaStream_t st) {
   int launches = 0;
-  const bool fork = st2 && P.nbig > 0 && P.ngroups > P.nbig;
-  if (fork) {
-    cudaEventRecord(ev_fork, st);
-    cudaStreamWaitEvent(st2, ev_fork, 0);
-  }
-  if (P.nbig > 0) {  // one warp per large component, shared memory sized for the largest
-    k_sptrsv_grp<SF_BIG_LANES><<<P.nbig, 32, grp_smem(P.rb, P.eb), fork ? st2 : st>>>(
-        P, 0, P.nbig, P.rb, P.eb, L, U, b, rs, z);
+  c64* out = P.direct ? x : z;
+  auto groups = [&](int a, int e, int R, int E, cudaStream_t s) {
+    if (e <= a) return;
+    k_sptrsv_grp<<<e - a, SF_GRP_TPB, grp_smem(R, E), s>>>(P, a, R, E, L.val, U.val, L.dinv,
+                                                           U.dinv, b, rs, out);
     ++launches;
+  };
+  const int R = std::max(P.rb, P.rp), E = std::max(P.eb, P.ep);
+  if (P.nbig == 0 || P.nbig == P.ngroups || grp_smem(R, E) <= SF_ONE_LAUNCH_SMEM) {
+    groups(0, P.ngroups, R, E, st);
+  } else {
+    if (st2) {
+      cudaEventRecord(ev_fork, st);
+      cudaStreamWaitEvent(st2, ev_fork, 0);
+    }
+    groups(0, P.nbig, P.rb, P.eb, st2 ? st2 : st);
+    if (st2) cudaEventRecord(ev_join, st2);
+    groups(P.nbig, P.ngroups, P.rp, P.ep, st);
+    if (st2) cudaStreamWaitEvent(st, ev_join, 0);
   }
-  if (fork) cudaEventRecord(ev_join, st2);
-  if (P.ngroups > P.nbig) {
-    const int nsmall = P.ngroups - P.nbig;
-    const int blocks = (nsmall + SF_GRP_WARPS - 1) / SF_GRP_WARPS;
-    k_sptrsv_grp<1><<<blocks, 32 * SF_GRP_WARPS, SF_GRP_WARPS * grp_smem(32, SF_GRP_E), st>>>(
-        P, P.nbig, P.ngroups, 32, SF_GRP_E, L, U, b, rs, z);
-    ++launches;
-  }
-  if (fork) cudaStreamWaitEvent(st, ev_join, 0);
   if (total <= 0) return launches;
   k_sptrsv_begin<<<1, 1, 0, st>>>(ctl);
   launches += 2;
