@@ -50,13 +50,14 @@ int fail_cuda(cudaError_t e, const char* expr, const char* file, int line) {
 }
 
 // launchers defined in the other translation units
-void launch_edge_rows(const c64*, const c64*, const c64*, const c64*, const int32_t*,
-                      const int32_t*, const double*, int, c64*, c64*, cudaStream_t);
-void launch_surf_rows(const c64*, const c64*, const int32_t*, const double*, int, c64*, c64*,
-                      cudaStream_t);
-void launch_node_rows(const c64*, const c64*, const c64*, const c64*, const c64*, const int32_t*,
-                      const int32_t*, const int32_t*, const int32_t*, const int32_t*,
-                      const int32_t*, const c64*, const double*, int, c64*, cudaStream_t);
+void launch_branch_rows(const c64*, const c64*, const c64*, const c64*, const c64*, const int32_t*,
+                        const int32_t*, const int32_t*, const double*, const double*, int, int,
+                        c64*, c64*, c64*, cudaStream_t);
+void launch_node_rows(const NodeSums&, const int32_t*, const int32_t*, const int32_t*,
+                      const int32_t*, int, c64*, cudaStream_t);
+void launch_inv_dz(const c64* DZ, int64_t m, c64* invZ, cudaStream_t st);
+void launch_scale_u(const int32_t* ptr, const c64* val, const c64* dinv, int64_t n, c64* sval,
+                    cudaStream_t st);
 void launch_set_scalar(double* p, double v, cudaStream_t st);
 void launch_edge_dz(int64_t m, const double* R4, const double* Cd4, const double* Lpd,
                     const double* Zs0, const uint8_t* surf, double escal_R, double sq, double w,
@@ -78,8 +79,8 @@ void launch_perm_gather(const c64*, const int32_t*, const double*, int, c64*, cu
 int sptrsv_grp_prepare(size_t smem_bytes);
 int launch_sptrsv(const GrpPlan&, cudaStream_t, cudaEvent_t, cudaEvent_t, const int32_t*, int,
                   int, const SfTri&, const SfTri&,
-                  const c64*, const int32_t*, const double*, c64*, c64*, c64*, int*, cudaStream_t);
-int lu_lanes(int nr, int ne, bool shared);
+                  const c64*, const NodeSums*, const int32_t*, const double*, c64*, c64*, c64*,
+                  int*, cudaStream_t);
 int red_blocks(size_t N);
 int launch_multidot(const c64*, size_t, const c64*, size_t, int, c64*, c64*, cudaStream_t);
 int launch_multidot(const cff*, size_t, const c64*, size_t, int, c64*, c64*, cudaStream_t);
@@ -131,6 +132,7 @@ using cd = std::complex<double>;
 struct LevelTri {  // triangular factor without its diagonal (CSR) and its level sets
   int32_t *ptr = nullptr, *col = nullptr, *flag = nullptr;
   c64 *val = nullptr, *dinv = nullptr;
+  c64* sval = nullptr;  // U: values times the row's inverse diagonal
   int64_t nflag = 0;
   std::vector<int32_t> rows;     // rows sorted by level (host)
   std::vector<int> lvl_off;      // offsets into rows per level (host)
@@ -216,10 +218,12 @@ struct peec_ctx {
   // arrays of the plan (host-built with the factors' structure)
   int comp_max = SF_COMP_MAX;  // largest component solved per CTA (0: global scheme only)
   GrpPlan grp;
-  int32_t *grp_goff = nullptr, *grp_seg = nullptr, *grp_segoff = nullptr, *grp_nsegL = nullptr;
-  int32_t *grp_eoff = nullptr, *grp_esrc = nullptr;
+  GrpHead* grp_head = nullptr;
+  int32_t *grp_rec = nullptr, *grp_esrc = nullptr, *grp_eij = nullptr, *grp_gsrc = nullptr;
+  // host copies of the node -> edge / surface lists, for the groups' gather lists
+  std::vector<int32_t> h_ne_ptr, h_ne_idx, h_nsn_ptr, h_nsn_idx;
+  std::vector<int32_t> h_yp;  // host copy of the installed Yle's row offsets
   GrpRow* grp_rows = nullptr;
-  int16_t *grp_uq = nullptr, *grp_ecol = nullptr;
   c64 *ir_b = nullptr, *ir_x = nullptr, *ir_r = nullptr, *ir_d = nullptr;  // refinement vectors
   // the frequency w on the device (the row kernels read it there, so captured graphs of
   // the operator stay valid when only the frequency state changes) and the entries the
@@ -247,7 +251,8 @@ struct peec_ctx {
   std::vector<int32_t> rf_yp, rf_yc;    // the Yle pattern (CSR) the plan was built for
   int* rf_err = nullptr;
   // matvec work
-  c64 *LpI = nullptr, *PQ = nullptr, *Y1 = nullptr, *U1 = nullptr, *Y2 = nullptr, *U2 = nullptr;
+  c64 *LpI = nullptr, *PQ = nullptr, *V1 = nullptr, *V2 = nullptr, *G = nullptr, *invZ = nullptr;
+  c64* xcopy = nullptr;  // input of an application whose output overlaps it
   c64 *tvec = nullptr, *Mvec = nullptr, *lutmp = nullptr, *lutmp2 = nullptr;
   // host staging
   c64 *hx = nullptr, *hy = nullptr;  // pinned N
@@ -464,6 +469,7 @@ static void free_refactor(RefactorPlan& r) {
 
 static void free_tri(LevelTri& t) {
   cudaFree(t.ptr); cudaFree(t.col); cudaFree(t.val); cudaFree(t.dinv); cudaFree(t.flag);
+  cudaFree(t.sval);
   t = LevelTri();
 }
 
@@ -475,8 +481,8 @@ extern "C" void peec_ctx_destroy(peec_ctx* ctx) {
   drop_graphs(ctx);
   void* ptrs[] = {ctx->tw64, ctx->tw32, ctx->twff, ctx->n1, ctx->n2, ctx->snode, ctx->invP, ctx->ne_ptr,
                   ctx->ne_idx, ctx->nsn_ptr, ctx->nsn_idx, ctx->DZ, ctx->yle_ptr, ctx->yle_col,
-                  ctx->yle_val, ctx->g_in, ctx->g_out, ctx->lu_rs, ctx->LpI, ctx->PQ, ctx->Y1, ctx->U1,
-                  ctx->Y2, ctx->U2, ctx->tvec, ctx->Mvec, ctx->lutmp, ctx->lutmp2, ctx->dx, ctx->dy, ctx->U, (c64*)ctx->U32,
+                  ctx->yle_val, ctx->g_in, ctx->g_out, ctx->lu_rs, ctx->LpI, ctx->PQ, ctx->V1, ctx->V2,
+                  ctx->G, ctx->invZ, ctx->xcopy, ctx->tvec, ctx->Mvec, ctx->lutmp, ctx->lutmp2, ctx->dx, ctx->dy, ctx->U, (c64*)ctx->U32,
                   ctx->gb, ctx->gx, ctx->gr, ctx->gv, ctx->gw, ctx->gxm, ctx->gxmin, ctx->gtmp,
                   ctx->gzero, ctx->dcoef, ctx->dcoef2, ctx->dpart, ctx->dred, ctx->dscal, ctx->dT,
                   ctx->mdpart, ctx->LpI2, ctx->PQ2, ctx->gm_block, ctx->d_w, ctx->dn_part,
@@ -516,9 +522,8 @@ extern "C" void peec_ctx_destroy(peec_ctx* ctx) {
   cudaFree(ctx->sf_ctl);
   free_refactor(ctx->rf);
   cudaFree(ctx->rf_err);
-  for (void* p : {(void*)ctx->grp_goff, (void*)ctx->grp_seg, (void*)ctx->grp_segoff,
-                  (void*)ctx->grp_nsegL, (void*)ctx->grp_rows, (void*)ctx->grp_uq,
-                  (void*)ctx->grp_eoff, (void*)ctx->grp_esrc, (void*)ctx->grp_ecol})
+  for (void* p : {(void*)ctx->grp_head, (void*)ctx->grp_rec, (void*)ctx->grp_rows,
+                  (void*)ctx->grp_esrc, (void*)ctx->grp_eij, (void*)ctx->grp_gsrc})
     cudaFree(p);
   for (c64* p : {ctx->ir_b, ctx->ir_x, ctx->ir_r, ctx->ir_d, ctx->cc_x, ctx->cc_LpI, ctx->cc_PQ})
     cudaFree(p);
@@ -613,6 +618,11 @@ static int set_incidence_lists(peec_ctx* ctx, int64_t m, int64_t ns, int64_t n,
   CTX_TRY(upload(&ctx->ne_idx, nei, ctx->st));
   CTX_TRY(upload(&ctx->nsn_ptr, sdeg, ctx->st));
   CTX_TRY(upload(&ctx->nsn_idx, nsi, ctx->st));
+  PEEC_CUDA_TRY(cudaStreamSynchronize(ctx->st));  // the uploads read the host lists
+  ctx->h_ne_ptr = std::move(deg);
+  ctx->h_ne_idx = std::move(nei);
+  ctx->h_nsn_ptr = std::move(sdeg);
+  ctx->h_nsn_idx = std::move(nsi);
   return PEEC_OK;
 }
 
@@ -623,10 +633,12 @@ static int alloc_work(peec_ctx* ctx) {
   CTX_TRY(dalloc(&ctx->PQ, ns));
   CTX_TRY(dalloc(&ctx->LpI2, m));
   CTX_TRY(dalloc(&ctx->PQ2, ns));
-  CTX_TRY(dalloc(&ctx->Y1, m));
-  CTX_TRY(dalloc(&ctx->U1, m));
-  CTX_TRY(dalloc(&ctx->Y2, ns));
-  CTX_TRY(dalloc(&ctx->U2, ns));
+  CTX_TRY(dalloc(&ctx->V1, m));
+  CTX_TRY(dalloc(&ctx->V2, ns));
+  CTX_TRY(dalloc(&ctx->G, m + ns));
+  CTX_TRY(dalloc(&ctx->invZ, m));
+  cudaFree(ctx->xcopy);
+  ctx->xcopy = nullptr;
   CTX_TRY(dalloc(&ctx->tvec, n));
   CTX_TRY(dalloc(&ctx->Mvec, n));
   CTX_TRY(dalloc(&ctx->lutmp, n));
@@ -1495,9 +1507,15 @@ static int make_tri(peec_ctx* ctx, LevelTri& T, int64_t n, const int64_t* ptr, c
   T.hcol = std::move(c);
   CTX_TRY(upload(&T.val, v, ctx->st));
   CTX_TRY(upload(&T.dinv, dinv, ctx->st));
+  if (!lower) {
+    CTX_TRY(dalloc(&T.sval, v.size()));
+    launch_scale_u(T.ptr, T.val, T.dinv, n, T.sval, ctx->st);
+    ctx->launches++;
+  }
   // ready flags start below every epoch the solve will use (epochs start at 1)
   CTX_TRY(dalloc(&T.flag, (size_t)n));
   PEEC_CUDA_TRY(cudaMemsetAsync(T.flag, 0, sizeof(int32_t) * n, ctx->st));
+  PEEC_CUDA_TRY(cudaStreamSynchronize(ctx->st));  // the uploads read v and dinv
   T.nflag = n;
   return PEEC_OK;
 }
@@ -1540,12 +1558,12 @@ static int build_solve_plan(peec_ctx* ctx, int64_t n) {
     cdepth[c] = std::max(cdepth[c], lvL[r] + lvU[r] + 2);
   }
   // largest group a CTA's shared memory takes (a large component alone)
-  const size_t smem_cap = 160 * 1024;
+  const size_t smem_cap = 200 * 1024;
   std::vector<int32_t> big, small;
   for (int64_t r = 0; r < n; ++r) {
     if (comp[r] != r || csize[r] > ctx->comp_max) continue;
     if (csize[r] <= SF_PACK_COMP && cent[r] <= SF_PACK_E / 2) small.push_back((int32_t)r);
-    else if (cent[r] < 32768 && grp_smem(csize[r], cent[r]) <= smem_cap) big.push_back((int32_t)r);
+    else if (grp_smem(csize[r], cent[r], cent[r], 0) <= smem_cap) big.push_back((int32_t)r);
   }
   // large components, longest chains first; small ones by depth
   std::stable_sort(big.begin(), big.end(),
@@ -1581,8 +1599,7 @@ static int build_solve_plan(peec_ctx* ctx, int64_t n) {
       ep = std::max(ep, ents);
     }
   }
-  const bool crowded = ng > 4 * std::max(ctx->nsm, 1);  // more groups than one per warp scheduler
-  // the groups' rows, in L-level order within each group
+  // the groups' rows
   std::vector<int32_t> goff(ng + 1, 0);
   for (int64_t r = 0; r < n; ++r)
     if (gidx[comp[r]] >= 0) goff[gidx[comp[r]] + 1]++;
@@ -1590,10 +1607,10 @@ static int build_solve_plan(peec_ctx* ctx, int64_t n) {
   std::vector<int32_t> rowsL(goff[ng]), fill(goff.begin(), goff.end() - 1);
   for (int64_t r = 0; r < n; ++r)
     if (gidx[comp[r]] >= 0) rowsL[fill[gidx[comp[r]]]++] = (int32_t)r;
-  std::vector<int32_t> rowsU(rowsL), local(n, -1), seg, segoff(ng + 1, 0), nsegL(ng, 0);
+  std::vector<int32_t> local(n, -1), rec, esrc, eij, gsrc;
   std::vector<GrpRow> grows(goff[ng]);
-  std::vector<int16_t> uq(goff[ng]), ecol;
-  std::vector<int32_t> eoff(ng + 1, 0), esrc;
+  std::vector<GrpHead> heads(ng);
+  int kb = 0, kp = 0, gb = 0, gp = 0;
   // results straight through Pc when every row is in a group and Pc is a permutation
   std::vector<int32_t> outp(n, -1);
   bool direct = goff[ng] == n && (int64_t)ctx->h_gout.size() == n;
@@ -1602,89 +1619,144 @@ static int build_solve_plan(peec_ctx* ctx, int64_t n) {
     direct = t < 0;
     t = (int32_t)i;
   }
+  // rows of equal node sums side by side: the lanes of a warp then run the same loops
+  auto shape = [&](int32_t r) {
+    const int32_t j = ctx->h_gin.empty() ? r : ctx->h_gin[r];
+    int minus = 0;
+    const int e0 = ctx->h_ne_ptr[j], e1 = ctx->h_ne_ptr[j + 1];
+    for (int t = e0; t < e1; ++t) minus += (ctx->h_ne_idx[t] & 1) == 0;
+    return std::make_tuple(ctx->h_nsn_ptr[j + 1] - ctx->h_nsn_ptr[j], e1 - e0, minus);
+  };
+  std::vector<std::pair<std::tuple<int, int, int>, int32_t>> order;
   for (int g = 0; g < ng; ++g) {
-    const auto b0 = rowsL.begin() + goff[g], e0 = rowsL.begin() + goff[g + 1];
-    std::stable_sort(b0, e0, [&](int32_t x, int32_t y) { return lvL[x] < lvL[y]; });
-    for (int32_t q = goff[g]; q < goff[g + 1]; ++q) local[rowsL[q]] = q - goff[g];
-    const auto bu = rowsU.begin() + goff[g], eu = rowsU.begin() + goff[g + 1];
-    std::stable_sort(bu, eu, [&](int32_t x, int32_t y) { return lvU[x] < lvU[y]; });
-    for (int32_t q = goff[g]; q < goff[g + 1]; ++q) uq[q] = (int16_t)local[rowsU[q]];
-    for (const LevelTri* T : {&L, &U}) {
-      const std::vector<int32_t>&rows = T == &L ? rowsL : rowsU, &lv = T == &L ? lvL : lvU;
-      int first = goff[g], ne = 0;
-      for (int32_t q = goff[g]; q < goff[g + 1]; ++q) {
-        const int32_t r = rows[q];
-        ne = std::max(ne, T->hptr[r + 1] - T->hptr[r]);
-        if (q + 1 == goff[g + 1] || lv[rows[q + 1]] != lv[r]) {
-          const int lw = lu_lanes(q + 1 - first, ne, crowded && g >= nbig);
-          seg.push_back((q + 1 - goff[g]) | (lw << 16));
-          first = q + 1;
-          ne = 0;
-        }
-      }
-      if (T == &L) nsegL[g] = (int32_t)seg.size() - segoff[g];
+    order.clear();
+    for (int32_t q = goff[g]; q < goff[g + 1]; ++q) order.push_back({shape(rowsL[q]), rowsL[q]});
+    std::sort(order.begin(), order.end());
+    for (int32_t q = goff[g]; q < goff[g + 1]; ++q) {
+      rowsL[q] = order[q - goff[g]].second;
+      local[rowsL[q]] = q - goff[g];
     }
-    segoff[g + 1] = (int32_t)seg.size();
+  }
+  // a group's update passes: the entries by the level of their column; within a level a row
+  // with k entries takes its first in the first pass, its second in the second, ..., rows in
+  // the order of falling k, so that a row keeps its place (its lane) through the passes
+  struct Upd {
+    int32_t lev, row, src;
+  };
+  std::vector<Upd> upd;
+  std::vector<std::pair<int32_t, int32_t>> first;  // (entries, first entry in upd) per row
+  for (int g = 0; g < ng; ++g) {
+    GrpHead& h = heads[g];
+    h = GrpHead{};
+    h.q0 = goff[g];
+    h.nr = goff[g + 1] - goff[g];
+    h.r0 = (int32_t)rec.size();
+    h.e0 = (int32_t)esrc.size();
+    h.t0 = (int32_t)gsrc.size();
+    for (const LevelTri* T : {&L, &U}) {
+      const std::vector<int32_t>& lv = T == &L ? lvL : lvU;
+      upd.clear();
+      for (int32_t q = goff[g]; q < goff[g + 1]; ++q)
+        for (int32_t t = T->hptr[rowsL[q]]; t < T->hptr[rowsL[q] + 1]; ++t)
+          upd.push_back({lv[T->hcol[t]], q - goff[g], t});
+      std::stable_sort(upd.begin(), upd.end(), [](const Upd& a, const Upd& b) {
+        return a.lev != b.lev ? a.lev < b.lev : a.row < b.row;
+      });
+      for (size_t a = 0; a < upd.size();) {
+        size_t e = a;
+        first.clear();
+        for (; e < upd.size() && upd[e].lev == upd[a].lev; ++e) {
+          if (e == a || upd[e].row != upd[e - 1].row) first.push_back({0, (int32_t)e});
+          first.back().first++;
+        }
+        std::stable_sort(first.begin(), first.end(),
+                         [](const std::pair<int32_t, int32_t>& x, const std::pair<int32_t, int32_t>& y) {
+                           return x.first > y.first;
+                         });
+        for (int32_t k = 0; k < first[0].first; ++k) {
+          int32_t cnt = 0;
+          for (const auto& f : first) {
+            if (f.first <= k) break;
+            const Upd& u = upd[f.second + k];
+            esrc.push_back(T == &L ? u.src : ~u.src);
+            eij.push_back(u.row | (local[T->hcol[u.src]] << 16));
+            ++cnt;
+          }
+          rec.push_back(k + 1 == first[0].first ? ~cnt : cnt);
+        }
+        a = e;
+      }
+      if (T == &L) {
+        h.nrl = (int32_t)rec.size() - h.r0;
+        h.nl = (int32_t)esrc.size() - h.e0;
+      }
+    }
+    h.nrec = (int32_t)rec.size() - h.r0;
+    h.ne = (int32_t)esrc.size() - h.e0;
     for (int32_t q = goff[g]; q < goff[g + 1]; ++q) {
       const int32_t r = rowsL[q];
       GrpRow& gr = grows[q];
+      gr = GrpRow{};
       gr.r = r;
       gr.j = ctx->h_gin.empty() ? r : ctx->h_gin[r];
       gr.o = direct ? outp[r] : r;
-      gr.nL = (int16_t)(L.hptr[r + 1] - L.hptr[r]);
-      gr.nU = (int16_t)(U.hptr[r + 1] - U.hptr[r]);
-      gr.eL = (int16_t)((int32_t)esrc.size() - eoff[g]);
-      for (int32_t t = L.hptr[r]; t < L.hptr[r + 1]; ++t) {
-        esrc.push_back(t);
-        ecol.push_back((int16_t)local[L.hcol[t]]);
+      auto at = [&] { return (int16_t)((int32_t)gsrc.size() - h.t0); };
+      gr.g0 = at();
+      for (int plus = 0; plus < 2; ++plus) {
+        for (int32_t t = ctx->h_ne_ptr[gr.j]; t < ctx->h_ne_ptr[gr.j + 1]; ++t)
+          if ((ctx->h_ne_idx[t] & 1) == plus) gsrc.push_back(ctx->h_ne_idx[t] >> 1);
+        (plus ? gr.g2 : gr.g1) = at();
       }
-      gr.eU = (int16_t)((int32_t)esrc.size() - eoff[g]);
-      for (int32_t t = U.hptr[r]; t < U.hptr[r + 1]; ++t) {
-        esrc.push_back(~t);
-        ecol.push_back((int16_t)local[U.hcol[t]]);
-      }
+      for (int32_t t = ctx->h_nsn_ptr[gr.j]; t < ctx->h_nsn_ptr[gr.j + 1]; ++t)
+        gsrc.push_back(~ctx->h_nsn_idx[t]);
+      gr.g3 = at();
+      gr.y0 = ctx->h_yp[gr.j];
+      gr.y1 = ctx->h_yp[gr.j + 1];
     }
-    eoff[g + 1] = (int32_t)esrc.size();
+    h.nt = (int32_t)gsrc.size() - h.t0;
+    int &km = g < nbig ? kb : kp, &gm = g < nbig ? gb : gp;
+    km = std::max(km, h.nrec);
+    gm = std::max(gm, h.nt);
   }
   if (esrc.empty()) {
     esrc.push_back(0);
-    ecol.push_back(0);
+    eij.push_back(0);
   }
+  if (rec.empty()) rec.push_back(0);
+  if (gsrc.empty()) gsrc.push_back(0);
   if (ng == 0) {  // keep the arrays non-empty
-    seg.push_back(0);
-    rowsL.push_back(0);
     grows.push_back(GrpRow());
-    uq.push_back(0);
-    nsegL.push_back(0);
+    heads.push_back(GrpHead());
   }
-  CTX_TRY(upload(&ctx->grp_goff, goff, ctx->st));
+  CTX_TRY(upload(&ctx->grp_head, heads, ctx->st));
   CTX_TRY(upload(&ctx->grp_rows, grows, ctx->st));
-  CTX_TRY(upload(&ctx->grp_uq, uq, ctx->st));
-  CTX_TRY(upload(&ctx->grp_seg, seg, ctx->st));
-  CTX_TRY(upload(&ctx->grp_segoff, segoff, ctx->st));
-  CTX_TRY(upload(&ctx->grp_nsegL, nsegL, ctx->st));
-  CTX_TRY(upload(&ctx->grp_eoff, eoff, ctx->st));
+  CTX_TRY(upload(&ctx->grp_rec, rec, ctx->st));
   CTX_TRY(upload(&ctx->grp_esrc, esrc, ctx->st));
-  CTX_TRY(upload(&ctx->grp_ecol, ecol, ctx->st));
+  CTX_TRY(upload(&ctx->grp_eij, eij, ctx->st));
+  CTX_TRY(upload(&ctx->grp_gsrc, gsrc, ctx->st));
   GrpPlan& P = ctx->grp;
-  P.goff = ctx->grp_goff;
+  P.head = ctx->grp_head;
   P.rows = ctx->grp_rows;
-  P.uq = ctx->grp_uq;
-  P.seg = ctx->grp_seg;
-  P.segoff = ctx->grp_segoff;
-  P.nsegL = ctx->grp_nsegL;
-  P.eoff = ctx->grp_eoff;
+  P.rec = ctx->grp_rec;
   P.esrc = ctx->grp_esrc;
-  P.ecol = ctx->grp_ecol;
+  P.eij = ctx->grp_eij;
+  P.gsrc = ctx->grp_gsrc;
+  P.gb = gb;
+  P.gp = gp;
   P.nbig = nbig;
   P.ngroups = ng;
   P.rb = rb;
   P.eb = eb;
+  P.kb = kb;
   P.rp = rp;
   P.ep = ep;
+  P.kp = kp;
   P.direct = direct;
   P.unit_l = L.unit;
-  const size_t need = grp_smem(std::max(rb, rp), std::max(eb, ep));
+  P.sums = direct && std::max(gb, gp) <= SF_GATHER_MAX &&
+           std::max(grp_smem(rb, eb, kb, gb), grp_smem(rp, ep, kp, gp)) <= smem_cap;
+  const size_t need = std::max({grp_smem(rb, eb, kb, P.sums ? gb : 0),
+                                grp_smem(rp, ep, kp, P.sums ? gp : 0), SF_ONE_LAUNCH_SMEM});
   if (sptrsv_grp_prepare(need)) return PEEC_ERR_CUDA;
   std::vector<int32_t> cidx(n, -1);
   for (int64_t r = 0; r < n; ++r) cidx[r] = gidx[comp[r]];
@@ -1766,11 +1838,14 @@ static int peec_set_frequency_body(peec_ctx* ctx, double w, const double* DZ, in
   std::vector<c64> dz(m);
   for (int64_t e = 0; e < m; ++e) dz[e] = mk<double>(DZ[2 * e], DZ[2 * e + 1]);
   CTX_TRY(upload(&ctx->DZ, dz, ctx->st));
+  launch_inv_dz(ctx->DZ, m, ctx->invZ, ctx->st);
+  ctx->launches++;
   // Yle COO -> CSR (duplicates summed, as sparse() does)
   std::vector<int32_t> yp, yc;
   std::vector<c64> yv;
   CTX_TRY(yle_csr(ctx, n, yle_nnz, yle_row, yle_col, yle_val, yp, yc, yv));
   CTX_TRY(upload(&ctx->yle_ptr, yp, ctx->st));
+  ctx->h_yp = yp;
   CTX_TRY(upload(&ctx->yle_col, yc, ctx->st));
   CTX_TRY(upload(&ctx->yle_val, yv, ctx->st));
   ctx->yle_cap = yv.size();
@@ -2009,11 +2084,13 @@ static int refactor_run(peec_ctx* ctx) {
   ctx->have_freq = false;
   PEEC_CUDA_TRY(cudaMemsetAsync(ctx->rf_err, 0, sizeof(int), ctx->st));
   const LevelTri &L = ctx->Lf, &U = ctx->Uf;
+  launch_inv_dz(ctx->DZ, ctx->m, ctx->invZ, ctx->st);
   const int nl = refactor_launch(ctx->rf, SfTri{L.ptr, L.col, L.val, L.dinv, L.flag},
-                                 SfTri{U.ptr, U.col, U.val, U.dinv, U.flag}, L.val, U.val, ctx->DZ,
+                                 SfTri{U.ptr, U.col, U.val, U.dinv, U.flag}, L.val, U.val, ctx->invZ,
                                  ctx->invP, ctx->yle_val, ctx->w, ctx->rf_err, ctx->st);
   if (nl < 0) return nl;
-  ctx->launches += nl;
+  launch_scale_u(U.ptr, U.val, U.dinv, ctx->n, U.sval, ctx->st);
+  ctx->launches += nl + 2;
   int herr = 0;
   cudaMemcpyAsync(&herr, ctx->rf_err, sizeof(int), cudaMemcpyDeviceToHost, ctx->st);
   PEEC_CUDA_TRY(cudaStreamSynchronize(ctx->st));
@@ -2141,13 +2218,15 @@ static int peec_set_frequency_device_body(peec_ctx* ctx, double w, int64_t yle_n
 // operator
 // ------------------------------------------------------------------------------------
 
-static void lu_solve(peec_ctx* ctx, const c64* b, c64* x) {
+// x = F\b, or with S (and every row in a group) F\ the node sums
+static void lu_solve(peec_ctx* ctx, const c64* b, const NodeSums* S, c64* x) {
   const int n = (int)ctx->n;
   const LevelTri &L = ctx->Lf, &U = ctx->Uf;
   ctx->launches += launch_sptrsv(
       ctx->grp, ctx->st2, ctx->ev_fork, ctx->ev_join, ctx->sf_ord, ctx->sf_nL, ctx->sf_total,
-      SfTri{L.ptr, L.col, L.val, L.dinv, L.flag}, SfTri{U.ptr, U.col, U.val, U.dinv, U.flag}, b,
-      ctx->g_in, ctx->lu_rs, ctx->lutmp, ctx->lutmp2, x, ctx->sf_ctl, ctx->st);
+      SfTri{L.ptr, L.col, L.val, L.dinv, L.flag},
+      SfTri{U.ptr, U.col, U.val, U.dinv, U.flag, U.sval}, b, S, ctx->g_in, ctx->lu_rs, ctx->lutmp,
+      ctx->lutmp2, x, ctx->sf_ctl, ctx->st);
   if (ctx->grp.direct) return;
   launch_perm_gather(ctx->lutmp2, ctx->g_out, nullptr, n, x, ctx->st);
   ctx->launches += 1;
@@ -2174,29 +2253,39 @@ static int check_solve_errors(peec_ctx* ctx) {
 }
 
 // enqueue the sparse half of an operator application y = M^-1 K x (block rows, the LU
-// solve of the preconditioner), given the convolutions LpI = Lp*I and PQ = P*Q of x
+// solve of the preconditioner), given the convolutions LpI = Lp*I and PQ = P*Q of x:
+// the edge and surface rows, the LU groups (which form their own nodes' sums and write
+// y's node block), the final rows. x and y do not overlap.
 static void sparse_enqueue(peec_ctx* ctx, const c64* x, c64* y, const c64* LpI, const c64* PQ) {
   const int64_t m = ctx->m, ns = ctx->ns, n = ctx->n;
   cudaStream_t st = ctx->st;
   const c64* I = x;
   const c64* Q = x + m;
   const c64* Phi = x + m + ns;
-  launch_edge_rows(I, Phi, LpI, ctx->DZ, ctx->n1, ctx->n2, ctx->d_w, (int)m, ctx->Y1, ctx->U1, st);
-  launch_surf_rows(PQ, Phi, ctx->snode, ctx->invP, (int)ns, ctx->Y2, ctx->U2, st);
-  launch_node_rows(I, Q, Phi, ctx->U1, ctx->U2, ctx->ne_ptr, ctx->ne_idx, ctx->nsn_ptr,
-                   ctx->nsn_idx, ctx->yle_ptr, ctx->yle_col, ctx->yle_val, ctx->d_w, (int)n,
-                   ctx->tvec, st);
-  ctx->launches += 3;
-  lu_solve(ctx, ctx->tvec, ctx->Mvec);
-  launch_final_rows(ctx->Y1, ctx->Y2, ctx->Mvec, ctx->DZ, ctx->n1, ctx->n2, ctx->snode, ctx->invP,
+  c64* M = y + m + ns;
+  launch_branch_rows(Q, Phi, LpI, PQ, ctx->invZ, ctx->n1, ctx->n2, ctx->snode, ctx->invP, ctx->d_w,
+                     (int)m, (int)ns, ctx->V1, ctx->V2, ctx->G, st);
+  const NodeSums S{ctx->V1, ctx->V2, Phi, ctx->yle_ptr, ctx->yle_col, ctx->yle_val, ctx->d_w};
+  if (ctx->grp.sums) {
+    lu_solve(ctx, nullptr, &S, M);
+  } else {
+    launch_node_rows(S, ctx->ne_ptr, ctx->ne_idx, ctx->nsn_ptr, ctx->nsn_idx, (int)n, ctx->tvec, st);
+    ctx->launches++;
+    lu_solve(ctx, ctx->tvec, nullptr, M);
+  }
+  launch_final_rows(I, ctx->G, M, ctx->invZ, ctx->n1, ctx->n2, ctx->snode, ctx->invP,
                     (int)m, (int)ns, (int)n, y, st);
-  ctx->launches++;
+  ctx->launches += 2;
 }
 
 // enqueue one operator application y = M^-1 K x on the context stream
 static int matvec_enqueue(peec_ctx* ctx, const c64* x, c64* y, int prec, bool events) {
   cudaStream_t st = ctx->st;
   if (events) cudaEventRecord(ctx->ev[0], st);
+  if (x < y + ctx->N && y < x + ctx->N) {  // a caller's output over its input
+    PEEC_CUDA_TRY(cudaMemcpyAsync(ctx->xcopy, x, sizeof(c64) * ctx->N, cudaMemcpyDeviceToDevice, st));
+    x = ctx->xcopy;
+  }
   if (ctx->dense) {
     // Lp blocks (without their diagonals) and P: FP32 copies for the FP32 operator, FP64
     // for the others (more accurate than float-float, at FP64 speed). The pass events of
@@ -2272,6 +2361,7 @@ static int matvec_enqueue(peec_ctx* ctx, const c64* x, c64* y, int prec, bool ev
 static int matvec_dev(peec_ctx* ctx, const c64* x, c64* y, int prec, bool timed) {
   if (!ctx->have_topo || !ctx->have_spec || !ctx->have_freq || !ctx->have_pdiag)
     return bad(ctx, PEEC_ERR_STATE, "operator incomplete (topology, pdiag, rows, frequency)");
+  if (x < y + ctx->N && y < x + ctx->N && !ctx->xcopy) CTX_TRY(dalloc(&ctx->xcopy, (size_t)ctx->N));
   if (timed || ctx->prof || !ctx->use_graphs) {
     CTX_TRY(matvec_enqueue(ctx, x, y, prec, timed));
   } else {
@@ -2449,12 +2539,10 @@ static int peec_port_rhs_body(peec_ctx* ctx, int64_t n1, int64_t n2, double Is, 
   is[n1] = mk<double>(Is, 0);
   is[n2] = mk<double>(-Is, 0);
   PEEC_CUDA_TRY(cudaMemcpyAsync(ctx->tvec, is.data(), sizeof(c64) * n, cudaMemcpyHostToDevice, ctx->st));
-  lu_solve(ctx, ctx->tvec, ctx->Mvec);
+  lu_solve(ctx, ctx->tvec, nullptr, ctx->Mvec);
   // Y1 = Y2 = 0 gives y1 = -invZ*A*M, y2 = invP*Gamma'*M, y3 = M
-  PEEC_CUDA_TRY(cudaMemsetAsync(ctx->Y1, 0, sizeof(c64) * (m > 0 ? m : 1), ctx->st));
-  PEEC_CUDA_TRY(cudaMemsetAsync(ctx->Y2, 0, sizeof(c64) * (ns > 0 ? ns : 1), ctx->st));
-  launch_final_rows(ctx->Y1, ctx->Y2, ctx->Mvec, ctx->DZ, ctx->n1, ctx->n2, ctx->snode, ctx->invP,
-                    (int)m, (int)ns, (int)n, ctx->dy, ctx->st);
+  launch_final_rows(nullptr, nullptr, ctx->Mvec, ctx->invZ, ctx->n1, ctx->n2, ctx->snode,
+                    ctx->invP, (int)m, (int)ns, (int)n, ctx->dy, ctx->st);
   ctx->launches++;
   PEEC_CUDA_TRY(cudaMemcpyAsync(tn, ctx->dy, sizeof(c64) * ctx->N, cudaMemcpyDeviceToHost, ctx->st));
   PEEC_CUDA_TRY(cudaStreamSynchronize(ctx->st));

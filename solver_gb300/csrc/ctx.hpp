@@ -22,8 +22,18 @@ struct SfTri {
   const c64* val;
   const c64* dinv;
   int* flag;  // per row: the epoch of the solve that last finished the row
+  const c64* sval = nullptr;  // U: each row's entries times the row's inverse diagonal
 };
 constexpr int SF_TPB = 128;
+
+// The operands of the node sums t = sum_e A(e, node) V1[e] + jw sum_s V2[s] + (Yle Phi)[node]
+// (sparse.cu, branch_rows), which the group solves form for their own rows
+struct NodeSums {
+  const c64 *V1 = nullptr, *V2 = nullptr, *Phi = nullptr;
+  const int32_t *yle_ptr = nullptr, *yle_col = nullptr;  // (the groups know their rows of Yle)
+  const c64* yle_val = nullptr;
+  const double* w = nullptr;
+};
 
 // Groups of the LU solves (sparse.cu, k_sptrsv_grp). The rows of L and U fall into
 // connected components (rows linked by a factor entry) that never depend on one another.
@@ -36,37 +46,47 @@ constexpr int SF_PACK_COMP = 64;  // rows of a component that may be packed with
 constexpr int SF_PACK_R = 256;    // rows of a packed group
 constexpr int SF_PACK_E = 1024;   // its entries (L and U off-diagonal)
 constexpr int SF_GRP_TPB = 128;   // one warp per SM sub-partition, each with its FP64 pipe
-struct GrpRow {
-  int32_t r;       // factor row
-  int32_t j;       // original row of its right-hand side (Pr)
-  int32_t o;       // where its result goes: the original column (Pc), or r (GrpPlan::direct)
-  int16_t nL, nU;  // entries of the row in L and in U
-  int16_t eL, eU;  // their offsets in the group's shared entry array
+struct alignas(16) GrpRow {
+  int32_t r;           // factor row
+  int32_t j;           // original row of its right-hand side (Pr)
+  int32_t o;           // where its result goes: the original column (Pc), or r (GrpPlan::direct)
+  int16_t g0, g1, g2, g3;  // node j's sum in the group's gather list: edges with A = -1
+                           // [g0, g1), with A = +1 [g1, g2), surfaces [g2, g3)
+  int32_t y0, y1;      // its row of Yle
+  int32_t pad;
+};
+struct alignas(16) GrpHead {
+  int32_t q0, nr;            // its rows
+  int32_t r0, nrec, nrl;     // its update passes, the first nrl of them L's
+  int32_t e0, ne, nl;        // its entries, the first nl of them L's
+  int32_t t0, nt;            // its gather list
+  int32_t pad0, pad1;
 };
 struct GrpPlan {
-  const int32_t* goff = nullptr;    // ngroups + 1 offsets into rows
-  const GrpRow* rows = nullptr;     // per position: the group's rows in L-level order
-  const int16_t* uq = nullptr;      // per position in U-level order: that row's L position
-  const int32_t* seg = nullptr;     // per group: its L levels, then its U levels; the end of
-                                    // the level, and above bit 16 log2 of the lanes per row
-  const int32_t* segoff = nullptr;  // ngroups + 1 offsets into seg
-  const int32_t* nsegL = nullptr;   // per group: the number of its L levels
-  const int32_t* eoff = nullptr;    // ngroups + 1 offsets into esrc / ecol
-  const int32_t* esrc = nullptr;    // per group entry: its index in L's values, or ~index in U's
-  const int16_t* ecol = nullptr;    // per group entry: its column's L position in the group
-  int nbig = 0, ngroups = 0;        // groups [0, nbig) hold one large component each
-  int rb = 0, eb = 0;               // the large groups' largest row and entry counts
-  int rp = 0, ep = 0;               // the packed groups' largest
-  bool direct = false;              // results go through Pc already (no global-scheme rows)
-  bool unit_l = false;              // L's diagonal is one
+  const GrpHead* head = nullptr;  // per group
+  const GrpRow* rows = nullptr;   // the groups' rows
+  const int32_t* rec = nullptr;   // update passes of the L levels, then of the U levels: the
+                                  // number of entries, < 0 (~number) when a barrier follows
+                                  // (the level's last pass)
+  const int32_t* esrc = nullptr;  // per entry, in pass order: its index in L's values, or
+                                  // ~index in U's
+  const int32_t* eij = nullptr;   // its row (low 16 bits) and column as positions in the group
+  const int32_t* gsrc = nullptr;  // gather lists: edge, or ~surface
+  int nbig = 0, ngroups = 0;      // groups [0, nbig) hold one large component each
+  // the large groups' largest row, entry, pass and gather counts, and the packed groups'
+  int rb = 0, eb = 0, kb = 0, gb = 0;
+  int rp = 0, ep = 0, kp = 0, gp = 0;
+  bool direct = false;            // results go through Pc already (no global-scheme rows)
+  bool sums = false;              // the groups can form their nodes' sums
+  bool unit_l = false;            // L's diagonal is one
 };
-// shared memory of a group of R rows and E entries
-__host__ __device__ inline size_t grp_smem(int R, int E) {
-  size_t o = 48 * (size_t)R + 16 * (size_t)E;  // x, 1/L(i,i), 1/U(i,i), entry values
-  o += 8 * (size_t)R + 2 * (size_t)E + 2 * (size_t)R;  // row metadata, entry columns, U order
-  o = (o + 3) & ~(size_t)3;
-  o += 8 * (size_t)R;  // levels (at most 2R)
-  return (o + 15) & ~(size_t)15;
+constexpr size_t SF_ONE_LAUNCH_SMEM = 56 * 1024;  // four resident CTAs per SM
+constexpr int SF_GATHER_MAX = 2048;  // a group's gather list, above which node sums run apart
+// shared memory of a group of R rows, E entries, K passes and G gathered values: the vector,
+// 1/U(i,i) and the node sums' ranges, the entries' values and positions, the passes, the node
+// sums' terms
+__host__ __device__ inline size_t grp_smem(int R, int E, int K, int G) {
+  return (48 * (size_t)R + 20 * (size_t)E + 4 * (size_t)K + 16 * (size_t)G + 15) & ~(size_t)15;
 }
 
 // Device refactorisation of SS in a fixed pattern (refactor.cu): slots are the off-diagonal
@@ -82,7 +102,7 @@ struct RefactorPlan {
   c64* D = nullptr;              // diagonal of U
 };
 int refactor_launch(const RefactorPlan& R, const SfTri& L, const SfTri& U, c64* Lval, c64* Uval,
-                    const c64* DZ, const double* invP, const c64* yle, double w, int* err,
+                    const c64* invZ, const double* invP, const c64* yle, double w, int* err,
                     cudaStream_t st);
 
 // Device-resident state of one Householder GMRES cycle (the Arnoldi loop's scalar work

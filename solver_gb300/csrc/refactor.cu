@@ -23,7 +23,7 @@ namespace peec {
 constexpr uint32_t RF_EDGE_DIAG = 0u, RF_EDGE_OFF = 1u, RF_SURF = 2u, RF_YLE = 3u;
 
 __global__ void k_rf_assemble(int64_t nslot, const int64_t* __restrict__ ptr,
-                              const uint32_t* __restrict__ src, const c64* __restrict__ DZ,
+                              const uint32_t* __restrict__ src, const c64* __restrict__ invZ,
                               const double* __restrict__ invP, const c64* __restrict__ yle,
                               double w, int64_t nL, int64_t n, c64* Lval, c64* D, c64* Uval) {
   for (int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; s < nslot;
@@ -33,9 +33,7 @@ __global__ void k_rf_assemble(int64_t nslot, const int64_t* __restrict__ ptr,
       const uint32_t code = src[q];
       const uint32_t t = code >> 30, i = code & 0x3fffffffu;
       if (t == RF_EDGE_DIAG || t == RF_EDGE_OFF) {
-        const c64 d = DZ[i];
-        const double den = d.x * d.x + d.y * d.y;
-        const c64 iz = mk<double>(d.x / den, -d.y / den);
+        const c64 iz = invZ[i];
         acc = t == RF_EDGE_DIAG ? acc + iz : acc - iz;
       } else if (t == RF_SURF) {
         acc = acc + mk<double>(0.0, w * invP[i]);
@@ -83,13 +81,13 @@ __global__ void k_rf_rows(const int32_t* __restrict__ rows, int nrows, SfTri L, 
 }
 
 int refactor_launch(const RefactorPlan& R, const SfTri& L, const SfTri& U, c64* Lval, c64* Uval,
-                    const c64* DZ, const double* invP, const c64* yle, double w, int* err,
+                    const c64* invZ, const double* invP, const c64* yle, double w, int* err,
                     cudaStream_t st) {
   const int64_t nslot = R.nL + R.n + R.nU;
   int64_t blocks = (nslot + 255) / 256;
   if (blocks > 152 * 16) blocks = 152 * 16;
   if (blocks < 1) blocks = 1;
-  k_rf_assemble<<<(unsigned)blocks, 256, 0, st>>>(nslot, R.asm_ptr, R.asm_src, DZ, invP, yle, w,
+  k_rf_assemble<<<(unsigned)blocks, 256, 0, st>>>(nslot, R.asm_ptr, R.asm_src, invZ, invP, yle, w,
                                                   R.nL, R.n, Lval, R.D, Uval);
   int launches = 1;
   for (size_t l = 0; l + 1 < R.lvl_off.size(); ++l) {

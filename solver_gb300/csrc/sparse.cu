@@ -17,88 +17,99 @@
 
 namespace peec {
 
-__global__ void k_edge_rows(const c64* __restrict__ I, const c64* __restrict__ Phi,
-                            const c64* __restrict__ LpI, const c64* __restrict__ DZ,
-                            const int32_t* __restrict__ n1, const int32_t* __restrict__ n2,
-                            const double* __restrict__ wp, int m, c64* Y1, c64* U1) {
+// The operator rows of edges and surfaces that the preconditioner's node sums and the final
+// rows need, in one launch. With g = jw*LpI + A*Phi the edge rows are Y1 = DZ.*I + g, so
+// invZ.*Y1 = I + V1 with V1 = invZ.*g, and the node sums take A'*(invZ*Y1 - I) = A'*V1: the
+// currents cancel before any rounding, and 1/DZ (formed once per frequency) replaces two
+// divisions per edge. Surfaces: h = PQ - Phi, V2 = Q - invP.*h.
+// Bound by the FP64 pipe (about ten instructions an edge, six a surface) and the gathers: 9.8 us
+// at 128x128x64, 17.5 us as two kernels with the divisions.
+__global__ void __launch_bounds__(256) k_branch_rows(
+    const c64* __restrict__ Q, const c64* __restrict__ Phi, const c64* __restrict__ LpI,
+    const c64* __restrict__ PQ, const c64* __restrict__ invZ, const int32_t* __restrict__ n1,
+    const int32_t* __restrict__ n2, const int32_t* __restrict__ snode,
+    const double* __restrict__ invP, const double* __restrict__ wp, int m, int ns, c64* V1,
+    c64* V2, c64* G) {
   const double w = *wp;
-  for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < m; e += gridDim.x * blockDim.x) {
-    const c64 l = LpI[e], d = DZ[e], i = I[e];
-    const c64 a = Phi[n2[e]] - Phi[n1[e]];
-    // jw*l + d*i + a
-    c64 y = mk<double>(-w * l.y, w * l.x) + d * i + a;
-    Y1[e] = y;
-    // y / d
-    const double den = d.x * d.x + d.y * d.y;
-    U1[e] = mk<double>((y.x * d.x + y.y * d.y) / den, (y.y * d.x - y.x * d.y) / den);
-  }
-}
-
-__global__ void k_surf_rows(const c64* __restrict__ PQ, const c64* __restrict__ Phi,
-                            const int32_t* __restrict__ snode, const double* __restrict__ invP,
-                            int ns, c64* Y2, c64* U2) {
-  for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < ns; s += gridDim.x * blockDim.x) {
-    const c64 y = PQ[s] - Phi[snode[s]];
-    Y2[s] = y;
-    U2[s] = cscale(y, invP[s]);
-  }
-}
-
-// t[node] = sum_e A(e,node)*U1[e] - jw*sum_s U2[s] + Y3[node]
-// Y3[node] = -sum_e A(e,node)*I[e] + (Yle*Phi)[node] + jw*sum_s Q[s]
-__global__ void k_node_rows(const c64* __restrict__ I, const c64* __restrict__ Q,
-                            const c64* __restrict__ Phi, const c64* __restrict__ U1,
-                            const c64* __restrict__ U2, const int32_t* __restrict__ ne_ptr,
-                            const int32_t* __restrict__ ne_idx, const int32_t* __restrict__ ns_ptr,
-                            const int32_t* __restrict__ ns_idx, const int32_t* __restrict__ yle_ptr,
-                            const int32_t* __restrict__ yle_col, const c64* __restrict__ yle_val,
-                            const double* __restrict__ wp, int n, c64* t) {
-  const double w = *wp;
-  for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x) {
-    c64 au = mk<double>(0, 0), ai = mk<double>(0, 0);
-    for (int p = ne_ptr[v]; p < ne_ptr[v + 1]; ++p) {
-      const int code = ne_idx[p];  // edge index * 2 + (1 if A = +1 else 0)
-      const int e = code >> 1;
-      if (code & 1) {
-        au = au + U1[e];
-        ai = ai + I[e];
-      } else {
-        au = au - U1[e];
-        ai = ai - I[e];
-      }
-    }
-    c64 su = mk<double>(0, 0), sq = mk<double>(0, 0);
-    for (int p = ns_ptr[v]; p < ns_ptr[v + 1]; ++p) {
-      const int s = ns_idx[p];
-      su = su + U2[s];
-      sq = sq + Q[s];
-    }
-    c64 yp = mk<double>(0, 0);
-    for (int p = yle_ptr[v]; p < yle_ptr[v + 1]; ++p) yp = yp + yle_val[p] * Phi[yle_col[p]];
-    // jw*(sq - su)
-    const c64 d = sq - su;
-    t[v] = au - ai + yp + mk<double>(-w * d.y, w * d.x);
-  }
-}
-
-__global__ void k_final_rows(const c64* __restrict__ Y1, const c64* __restrict__ Y2,
-                             const c64* __restrict__ M, const c64* __restrict__ DZ,
-                             const int32_t* __restrict__ n1, const int32_t* __restrict__ n2,
-                             const int32_t* __restrict__ snode, const double* __restrict__ invP,
-                             int m, int ns, int n, c64* y) {
-  const int total = m + ns + n;
+  const int total = m + ns;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
     if (i < m) {
-      const c64 v = Y1[i] - (M[n2[i]] - M[n1[i]]);
-      const c64 d = DZ[i];
-      const double den = d.x * d.x + d.y * d.y;
-      y[i] = mk<double>((v.x * d.x + v.y * d.y) / den, (v.y * d.x - v.x * d.y) / den);
+      const c64 l = LpI[i], a = Phi[n2[i]] - Phi[n1[i]];
+      const c64 g = mk<double>(fma(-w, l.y, a.x), fma(w, l.x, a.y));
+      G[i] = g;
+      V1[i] = g * invZ[i];
+    } else {
+      const int s = i - m;
+      const c64 h = PQ[s] - Phi[snode[s]], q = Q[s];
+      const double p = invP[s];
+      G[i] = h;
+      V2[s] = mk<double>(fma(-p, h.x, q.x), fma(-p, h.y, q.y));
+    }
+  }
+}
+
+// the node sums (NodeSums) as a vector, for solves that are not all in groups
+__global__ void k_node_rows(NodeSums S, const int32_t* __restrict__ ne_ptr,
+                            const int32_t* __restrict__ ne_idx, const int32_t* __restrict__ ns_ptr,
+                            const int32_t* __restrict__ ns_idx, int n, c64* out) {
+  const double w = *S.w;
+  for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x) {
+    c64 t = mk<double>(0, 0), q = mk<double>(0, 0);
+    for (int p = ne_ptr[v]; p < ne_ptr[v + 1]; ++p) {
+      const int code = ne_idx[p];  // 2 * edge + (A = +1)
+      const c64 x = S.V1[code >> 1];
+      t = (code & 1) ? t + x : t - x;
+    }
+    for (int p = ns_ptr[v]; p < ns_ptr[v + 1]; ++p) q = q + S.V2[ns_idx[p]];
+    // Yle*Phi by itself: a large admittance between two nodes at almost the same potential
+    // cancels to a few digits, which a running sum would take from the other terms
+    c64 yp = mk<double>(0, 0);
+    for (int p = S.yle_ptr[v], e = S.yle_ptr[v + 1]; p < e; ++p)
+      yp = yp + S.yle_val[p] * S.Phi[S.yle_col[p]];
+    out[v] = mk<double>(fma(-w, q.y, t.x), fma(w, q.x, t.y)) + yp;
+  }
+}
+
+// y1 = invZ.*(Y1 - A*M) = I + invZ.*(g - A*M), y2 = invP.*(h + Gamma'*M), y3 = M (skipped
+// where M already is y's node block); G: g per edge, then h per surface. I and G null: zero.
+__global__ void __launch_bounds__(256) k_final_rows(
+    const c64* __restrict__ I, const c64* __restrict__ G, const c64* M,
+    const c64* __restrict__ invZ, const int32_t* __restrict__ n1, const int32_t* __restrict__ n2,
+    const int32_t* __restrict__ snode, const double* __restrict__ invP, int m, int ns, int n,
+    c64* y) {
+  const int total = M == y + m + ns ? m + ns : m + ns + n;
+  const c64 zero = mk<double>(0, 0);
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
+    if (i < m) {
+      const c64 d = (G ? G[i] : zero) - (M[n2[i]] - M[n1[i]]), z = invZ[i];
+      const c64 b = I ? I[i] : zero;
+      y[i] = mk<double>(b.x + (d.x * z.x - d.y * z.y), b.y + (d.x * z.y + d.y * z.x));
     } else if (i < m + ns) {
       const int s = i - m;
-      y[i] = cscale(Y2[s] + M[snode[s]], invP[s]);
+      y[i] = cscale((G ? G[i] : zero) + M[snode[s]], invP[s]);
     } else {
       y[i] = M[i - m - ns];
     }
+  }
+}
+
+// 1/DZ
+__global__ void k_inv_dz(const c64* __restrict__ DZ, int64_t m, c64* invZ) {
+  for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < m;
+       e += (int64_t)gridDim.x * blockDim.x) {
+    const c64 d = DZ[e];
+    const double den = d.x * d.x + d.y * d.y;
+    invZ[e] = mk<double>(d.x / den, -d.y / den);
+  }
+}
+
+// U's rows times their inverse diagonals (SfTri::sval), one row per thread
+__global__ void k_scale_u(const int32_t* __restrict__ ptr, const c64* __restrict__ val,
+                          const c64* __restrict__ dinv, int64_t n, c64* sval) {
+  for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r < n;
+       r += (int64_t)gridDim.x * blockDim.x) {
+    const c64 d = dinv[r];
+    for (int p = ptr[r], e = ptr[r + 1]; p < e; ++p) sval[p] = val[p] * d;
   }
 }
 
@@ -154,101 +165,187 @@ __global__ void k_sptrsv_begin(int* ctl) {
 
 // One CTA per group (GrpPlan): components of the factors, several small ones packed
 // together or one large one. The CTA first brings everything the group's solve reads into
-// shared memory -- per row the right-hand side (gathered through Pr and scaled by Rs) and
-// both inverse diagonals, per entry its value and its column as a position in the group --
-// with all loads independent of one another. Then the L levels, the U levels (in place: a U
-// row reads its own L value and the U values of rows of earlier U levels), a barrier between
-// levels, and the results go out.
+// shared memory -- per row the right-hand side (the terms of its node's sum, one thread a
+// term, or b gathered through Pr; scaled by Rs) and the inverse diagonal, per entry its value
+// and positions -- by asynchronous copies, all in flight at once. Then the levels of L and of U by
+// columns: once a level's values are final, every row with entries in that level's columns
+// takes its update, x_i -= a_ij x_j, a barrier, the next level.
 //
 // What bounds it is the FP64 pipe's latency and issue: on GB300 a warp's FP64 instruction
 // holds its sub-partition's pipe for 64 cycles whatever the number of its active lanes
-// (19 cycles per instruction with all four sub-partitions busy). So a level's cost is the
-// number of FP64 instructions on its longest warp, not its flops, and the split keeps that
-// low: four warps per group, one per sub-partition; a row takes 2 to 32 lanes (chosen per
-// level on the host, lu_lanes), half of them for the real and half for the imaginary part,
-// so that a complex multiply-add is two instructions and the final product with the inverse
-// diagonal two more (none in L when its diagonal is one). The lanes' partial sums meet in a
-// fixed shuffle tree, so results do not depend on scheduling.
-// Measured, one solve on an idle GPU: 128x128x64 (183,490 rows, 60,943 components, depth 29)
-// 44.4 us, against 72.5 us beside 72.1 us on a second stream with one warp per group and a
-// row on one to four lanes; 96x96x48 copper (largest component 291 rows) 39.8 against
-// 128.1 us; the 20x20x4 crossbar (one component, 100 levels) 57.7 against 111.4 us.
-__global__ void __launch_bounds__(SF_GRP_TPB) k_sptrsv_grp(GrpPlan P, int g0, int R, int E,
+// (19 cycles per instruction with all four sub-partitions busy). By rows, a level's chain is
+// a row's whole sum: its products and a tree over the lanes that share it. By columns it is
+// the entries in the one level before, mostly one: two instructions, as the real and the
+// imaginary part of a product go to two lanes. A lane keeps its row through the level's
+// passes (a row with k entries in the level's columns takes k), so that only levels need
+// barriers. U's rows come divided by their diagonals (SfTri::sval), which leaves one product
+// per row before the U levels; L's columns are divided by theirs while they are staged
+// (skipped when L's diagonal is one). The next pass's entries are loaded before the barrier.
+// Every row's updates come in a fixed order, so results do not depend on scheduling.
+// Measured, one solve with its node sums on an idle GPU: 128x128x64 (183,490 rows, 60,943
+// components, 29 levels of L and U in the deepest) 37.8 us; 96x96x48 copper (largest component
+// 291 rows) 34.4 us; the 20x20x4 crossbar (one component, 100 levels) 30.0 us. By rows with a
+// tree over each row's lanes: 44.4, 39.8 and 57.7 us, and the node sums 46.8, 20.2 and 6.8 us
+// in a kernel of their own; one warp per group 72.5 (beside 72.1), 128.1 and 111.4 us.
+__device__ __forceinline__ void grp_passes(c64* xs, const c64* ev, const int32_t* eij,
+                                           const int32_t* rec, int nrec) {
+  const int slot = threadIdx.x >> 1;
+  const bool im = threadIdx.x & 1;
+  constexpr int SLOTS = SF_GRP_TPB / 2;
+  double* xd = reinterpret_cast<double*>(xs) + (im ? 1 : 0);
+  auto cnt = [](int r) { return r < 0 ? ~r : r; };
+  // an update a = a - c1 x.x + c2 x.y: its row's part, its column, and the coefficients
+  // (re -= v.x x.x - v.y x.y, im -= v.y x.x + v.x x.y; the sign by its bit, as a negation
+  // may cost an FP64 instruction)
+  struct Upd {
+    double* a;
+    const double2* x;
+    double c1, c2;
+  };
+  const int flip = im ? (int)0x80000000 : 0;
+  auto fetch = [&](int e) {
+    const int ij = eij[e];
+    const c64 v = ev[e];
+    return Upd{xd + 2 * (ij & 0xffff), reinterpret_cast<const double2*>(xs + (ij >> 16)),
+               im ? v.y : v.x,
+               __hiloint2double(__double2hiint(im ? v.x : v.y) ^ flip,
+                                __double2loint(im ? v.x : v.y))};
+  };
+  int off = 0;
+  int cur = nrec > 0 ? rec[0] : 0;
+  int nxt = nrec > 1 ? rec[1] : 0;
+  Upd u = {};
+  if (slot < cnt(cur)) u = fetch(slot);
+  for (int k = 0; k < nrec; ++k) {
+    const int n = cnt(cur);
+    const bool bar = cur < 0;
+    const int nn = k + 2 < nrec ? rec[k + 2] : 0;
+    Upd un = {};
+    if (slot < n) {
+      const double2 x = *u.x;
+      const double a = *u.a;
+      // the next pass's first entry, while this one's operands and products are under way
+      if (slot < cnt(nxt)) un = fetch(off + n + slot);
+      *u.a = fma(u.c2, x.y, fma(-u.c1, x.x, a));
+      for (int t = slot + SLOTS; t < n; t += SLOTS) {
+        const Upd v = fetch(off + t);
+        const double2 y = *v.x;
+        *v.a = fma(v.c2, y.y, fma(-v.c1, y.x, *v.a));
+      }
+    } else if (slot < cnt(nxt)) {
+      un = fetch(off + n + slot);
+    }
+    off += n;
+    cur = nxt;
+    nxt = nn;
+    u = un;
+    if (bar) __syncthreads();
+  }
+}
+
+__device__ __forceinline__ void cp_async16(void* dst, const void* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"(
+                   (uint32_t)__cvta_generic_to_shared(dst)),
+               "l"(src)
+               : "memory");
+}
+__device__ __forceinline__ void cp_async_wait_all() {
+  asm volatile("cp.async.wait_all;" ::: "memory");
+}
+
+template <bool NODE>
+__global__ void __launch_bounds__(SF_GRP_TPB) k_sptrsv_grp(GrpPlan P, int g0, int R, int E, int G,
                                                            const c64* __restrict__ Lval,
                                                            const c64* __restrict__ Uval,
                                                            const c64* __restrict__ Ldinv,
                                                            const c64* __restrict__ Udinv,
-                                                           const c64* __restrict__ b,
+                                                           const c64* __restrict__ b, NodeSums S,
                                                            const double* __restrict__ rs,
                                                            c64* __restrict__ out) {
   extern __shared__ __align__(16) unsigned char grp_sm[];
   const int tid = threadIdx.x;
   c64* xs = reinterpret_cast<c64*>(grp_sm);
-  c64* dl = xs + R;
-  c64* du = dl + R;
-  c64* ev = du + R;
-  short4* meta = reinterpret_cast<short4*>(ev + E);  // (eL, nL, eU, nU)
-  int16_t* ec = reinterpret_cast<int16_t*>(meta + R);
-  int16_t* uqs = ec + E;
-  int32_t* segs = reinterpret_cast<int32_t*>(
-      (reinterpret_cast<uintptr_t>(uqs + R) + 3) & ~(uintptr_t)3);
-  const int g = g0 + blockIdx.x;
-  const int q0 = P.goff[g], nr = P.goff[g + 1] - q0;
-  const int s0 = P.segoff[g], ns = P.segoff[g + 1] - s0, nsl = P.nsegL[g];
-  const int e0 = P.eoff[g], ne_g = P.eoff[g + 1] - e0;
-  const bool unit = P.unit_l;
-  for (int e = tid; e < ne_g; e += SF_GRP_TPB) {
-    const int src = P.esrc[e0 + e];
-    ec[e] = P.ecol[e0 + e];
-    ev[e] = src >= 0 ? Lval[src] : Uval[~src];
-  }
-  for (int q = tid; q < nr; q += SF_GRP_TPB) {
-    const GrpRow pr = P.rows[q0 + q];
-    xs[q] = rs ? cscale(b[pr.j], rs[pr.j]) : b[pr.j];
-    if (!unit) dl[q] = Ldinv[pr.r];
-    du[q] = Udinv[pr.r];
-    meta[q] = make_short4(pr.eL, pr.nL, pr.eU, pr.nU);
-    uqs[q] = P.uq[q0 + q];
-  }
-  for (int t = tid; t < ns; t += SF_GRP_TPB) segs[t] = P.seg[s0 + t];
-  __syncthreads();
-  const int part = tid & 1;
-  const int warp0 = tid & ~31;
-  int prev = 0;
-  for (int s = 0; s < ns; ++s) {
-    const bool upper = s >= nsl;
-    const int sg = segs[s];
-    const int se = sg & 0xffff, lw = sg >> 16;
-    const int W = 1 << lw, H = W >> 1, slots = SF_GRP_TPB >> lw;
-    const int h = (tid & (W - 1)) >> 1;
-    // warp-uniform: every lane of a warp with rows left shuffles
-    for (int t0 = prev; t0 + (warp0 >> lw) < se; t0 += slots) {
-      const int t = t0 + (tid >> lw);
-      const bool valid = t < se;
-      const int q = valid ? (upper ? (int)uqs[t] : t) : 0;
-      double acc = 0.0;
-      if (valid) {
-        const short4 m = meta[q];
-        const int eb = upper ? m.z : m.x, n = upper ? m.w : m.y;
-        for (int e = h; e < n; e += H) {
-          const c64 v = ev[eb + e], x = xs[ec[eb + e]];
-          acc = fma(v.x, part ? x.y : x.x, acc);
-          acc = fma(v.y, part ? x.x : -x.y, acc);
-        }
+  c64* du = xs + R;
+  short4* gi = reinterpret_cast<short4*>(du + R);
+  int2* yy = reinterpret_cast<int2*>(gi + R);
+  c64* ev = reinterpret_cast<c64*>(yy + R);
+  c64* gat = ev + E;
+  int32_t* eij = reinterpret_cast<int32_t*>(gat + (NODE ? G : 0));
+  int32_t* rec = eij + E;
+  const GrpHead h = P.head[g0 + blockIdx.x];
+  // indices into registers, then every value straight into shared memory, all in flight
+  constexpr int B = 8;
+  GrpRow row = {};
+  if (tid < h.nr) row = P.rows[h.q0 + tid];
+  const int nmax = NODE && h.nt > h.ne ? h.nt : h.ne;
+  for (int t0 = tid; t0 < nmax; t0 += B * SF_GRP_TPB) {
+    int gi[B], es[B], ej[B];
+#pragma unroll
+    for (int u = 0; u < B; ++u) {
+      const int t = t0 + u * SF_GRP_TPB;
+      if (NODE && t < h.nt) gi[u] = P.gsrc[h.t0 + t];
+      if (t < h.ne) {
+        es[u] = P.esrc[h.e0 + t];
+        ej[u] = P.eij[h.e0 + t];
       }
-      for (int o = H; o >= 2; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-      double r = reinterpret_cast<const double*>(xs)[2 * q + part] - acc;
-      if (upper || !unit) {
-        const c64 d = upper ? du[q] : dl[q];
-        const double p = __shfl_xor_sync(0xffffffffu, r, 1);
-        r = part ? fma(p, d.y, r * d.x) : fma(-p, d.y, r * d.x);
-      }
-      if (valid && h == 0) reinterpret_cast<double*>(xs)[2 * q + part] = r;
     }
-    __syncthreads();
-    prev = s + 1 == nsl ? 0 : se;
+#pragma unroll
+    for (int u = 0; u < B; ++u) {
+      const int t = t0 + u * SF_GRP_TPB;
+      if (NODE && t < h.nt) cp_async16(gat + t, gi[u] >= 0 ? S.V1 + gi[u] : S.V2 + ~gi[u]);
+      if (t < h.ne) {
+        cp_async16(ev + t, es[u] >= 0 ? Lval + es[u] : Uval + ~es[u]);
+        eij[t] = ej[u];
+      }
+    }
   }
-  for (int q = tid; q < nr; q += SF_GRP_TPB) out[P.rows[q0 + q].o] = xs[q];
+  for (int t = tid; t < h.nrec; t += SF_GRP_TPB) rec[t] = P.rec[h.r0 + t];
+  for (int q = tid; q < h.nr; q += SF_GRP_TPB) {
+    const GrpRow pr = q == tid ? row : P.rows[h.q0 + q];
+    cp_async16(du + q, Udinv + pr.r);
+    if (!NODE) cp_async16(xs + q, b + pr.j);
+    gi[q] = make_short4(pr.g0, pr.g1, pr.g2, pr.g3);
+    yy[q] = make_int2(pr.y0, pr.y1);
+  }
+  const double w = NODE ? *S.w : 0.0;
+  cp_async_wait_all();
+  __syncthreads();
+  if constexpr (NODE) {
+    // two lanes a row: the parts of its node's sum, t + jw s
+    const int part = tid & 1;
+    const double ws = part ? w : -w;
+    double* xd = reinterpret_cast<double*>(xs);
+    const double* gt = reinterpret_cast<const double*>(gat) + part;
+    const double* gs = reinterpret_cast<const double*>(gat) + 1 - part;
+    for (int q = tid >> 1; q < h.nr; q += SF_GRP_TPB / 2) {
+      const short4 g = gi[q];
+      const int2 y = yy[q];
+      double t = 0.0, s = 0.0;
+      for (int p = g.x; p < g.y; ++p) t -= gt[2 * p];
+      for (int p = g.y; p < g.z; ++p) t += gt[2 * p];
+      for (int p = g.z; p < g.w; ++p) s += gs[2 * p];
+      t = fma(ws, s, t);
+      if (y.x < y.y) {  // Yle*Phi by itself, as in k_node_rows
+        c64 yp = mk<double>(0, 0);
+        for (int p = y.x; p < y.y; ++p) yp = yp + S.yle_val[p] * S.Phi[S.yle_col[p]];
+        t += part ? yp.y : yp.x;
+      }
+      xd[2 * q + part] = rs ? t * rs[P.rows[h.q0 + q].j] : t;
+    }
+  } else if (rs) {
+    for (int q = tid; q < h.nr; q += SF_GRP_TPB) xs[q] = cscale(xs[q], rs[P.rows[h.q0 + q].j]);
+  }
+  if (!P.unit_l) {  // L's columns over their diagonals; its rows take theirs with U's
+    for (int e = tid; e < h.nl; e += SF_GRP_TPB)
+      ev[e] = ev[e] * Ldinv[P.rows[h.q0 + (eij[e] >> 16)].r];
+    for (int q = tid; q < h.nr; q += SF_GRP_TPB) du[q] = du[q] * Ldinv[P.rows[h.q0 + q].r];
+  }
+  __syncthreads();
+  grp_passes(xs, ev, eij, rec, h.nrl);
+  for (int q = tid; q < h.nr; q += SF_GRP_TPB) xs[q] = xs[q] * du[q];
+  __syncthreads();
+  grp_passes(xs, ev + h.nl, eij + h.nl, rec + h.nrl, h.nrec - h.nrl);
+  for (int q = tid; q < h.nr; q += SF_GRP_TPB) out[q == tid ? row.o : P.rows[h.q0 + q].o] = xs[q];
 }
 
 __device__ __forceinline__ void sf_wait(const int* f, int epoch, int* err, int limit) {
@@ -334,8 +431,6 @@ __global__ void __launch_bounds__(SF_TPB) k_sptrsv(const int32_t* __restrict__ o
   }
 }
 
-constexpr size_t SF_ONE_LAUNCH_SMEM = 56 * 1024;  // four resident CTAs per SM
-
 static inline unsigned grid_for(long long n, int tpb = 256) {
   long long g = (n + tpb - 1) / tpb;
   if (g < 1) g = 1;
@@ -343,27 +438,31 @@ static inline unsigned grid_for(long long n, int tpb = 256) {
   return (unsigned)g;
 }
 
-void launch_edge_rows(const c64* I, const c64* Phi, const c64* LpI, const c64* DZ,
-                      const int32_t* n1, const int32_t* n2, const double* w, int m, c64* Y1,
-                      c64* U1, cudaStream_t st) {
-  if (m > 0) k_edge_rows<<<grid_for(m), 256, 0, st>>>(I, Phi, LpI, DZ, n1, n2, w, m, Y1, U1);
+void launch_branch_rows(const c64* Q, const c64* Phi, const c64* LpI, const c64* PQ,
+                        const c64* invZ, const int32_t* n1, const int32_t* n2,
+                        const int32_t* snode, const double* invP, const double* w, int m, int ns,
+                        c64* V1, c64* V2, c64* G, cudaStream_t st) {
+  if (m + ns > 0)
+    k_branch_rows<<<grid_for((long long)m + ns), 256, 0, st>>>(Q, Phi, LpI, PQ, invZ, n1, n2, snode,
+                                                              invP, w, m, ns, V1, V2, G);
 }
-void launch_surf_rows(const c64* PQ, const c64* Phi, const int32_t* snode, const double* invP,
-                      int ns, c64* Y2, c64* U2, cudaStream_t st) {
-  if (ns > 0) k_surf_rows<<<grid_for(ns), 256, 0, st>>>(PQ, Phi, snode, invP, ns, Y2, U2);
+void launch_node_rows(const NodeSums& S, const int32_t* ne_ptr, const int32_t* ne_idx,
+                      const int32_t* ns_ptr, const int32_t* ns_idx, int n, c64* t,
+                      cudaStream_t st) {
+  k_node_rows<<<grid_for(n), 256, 0, st>>>(S, ne_ptr, ne_idx, ns_ptr, ns_idx, n, t);
 }
-void launch_node_rows(const c64* I, const c64* Q, const c64* Phi, const c64* U1, const c64* U2,
-                      const int32_t* ne_ptr, const int32_t* ne_idx, const int32_t* ns_ptr,
-                      const int32_t* ns_idx, const int32_t* yle_ptr, const int32_t* yle_col,
-                      const c64* yle_val, const double* w, int n, c64* t, cudaStream_t st) {
-  k_node_rows<<<grid_for(n), 256, 0, st>>>(I, Q, Phi, U1, U2, ne_ptr, ne_idx, ns_ptr, ns_idx,
-                                           yle_ptr, yle_col, yle_val, w, n, t);
-}
-void launch_final_rows(const c64* Y1, const c64* Y2, const c64* M, const c64* DZ,
+void launch_final_rows(const c64* I, const c64* G, const c64* M, const c64* invZ,
                        const int32_t* n1, const int32_t* n2, const int32_t* snode,
                        const double* invP, int m, int ns, int n, c64* y, cudaStream_t st) {
-  k_final_rows<<<grid_for((long long)m + ns + n), 256, 0, st>>>(Y1, Y2, M, DZ, n1, n2, snode,
+  k_final_rows<<<grid_for((long long)m + ns + n), 256, 0, st>>>(I, G, M, invZ, n1, n2, snode,
                                                                invP, m, ns, n, y);
+}
+void launch_inv_dz(const c64* DZ, int64_t m, c64* invZ, cudaStream_t st) {
+  if (m > 0) k_inv_dz<<<grid_for(m), 256, 0, st>>>(DZ, m, invZ);
+}
+void launch_scale_u(const int32_t* ptr, const c64* val, const c64* dinv, int64_t n, c64* sval,
+                    cudaStream_t st) {
+  k_scale_u<<<grid_for(n, 128), 128, 0, st>>>(ptr, val, dinv, n, sval);
 }
 void launch_perm_gather(const c64* b, const int32_t* perm, const double* rs, int n, c64* out,
                         cudaStream_t st) {
@@ -385,59 +484,48 @@ int sptrsv_grp_prepare(size_t smem_bytes) {
   std::lock_guard<std::mutex> lock(mu);
   // set every time (a re-created context starts from the default again)
   const size_t v = std::max(smem_bytes, granted[dev]);
-  PEEC_CUDA_TRY(cudaFuncSetAttribute(k_sptrsv_grp, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)v));
+  PEEC_CUDA_TRY(cudaFuncSetAttribute(k_sptrsv_grp<false>,
+                                     cudaFuncAttributeMaxDynamicSharedMemorySize, (int)v));
+  PEEC_CUDA_TRY(cudaFuncSetAttribute(k_sptrsv_grp<true>,
+                                     cudaFuncAttributeMaxDynamicSharedMemorySize, (int)v));
   granted[dev] = v;
   return 0;
 }
 
-// lanes per row (log2) of a level with nr rows of at most ne entries: the smallest product
-// of the level's passes over the CTA (alone) or over its warps (shared: the SM runs several
-// groups and its FP64 issue is what counts) and the FP64 instructions of one pass
-int lu_lanes(int nr, int ne, bool shared) {
-  int best = 1;
-  long cost = -1;
-  for (int lw = 1; lw <= 5; ++lw) {
-    const int H = 1 << (lw - 1);
-    const long unit = shared ? 32 : SF_GRP_TPB;
-    const long passes = ((long)nr * (1 << lw) + unit - 1) / unit;
-    const long c = passes * (2L * ((ne + H - 1) / H) + (lw - 1) + 3);
-    if (cost < 0 || c < cost) {
-      cost = c;
-      best = lw;
-    }
-  }
-  return best;
-}
-
-// returns the number of kernels launched
+// returns the number of kernels launched. S: the right-hand side is the node sums, formed by
+// the groups themselves (only when every row is in a group, GrpPlan::direct); else b.
 // One launch over all groups when the large ones fit the shared memory of a few resident
 // CTAs; else the large groups go to st2 (forked from st with ev_fork, joined back with
 // ev_join; under stream capture the fork and join become graph edges) so that they run
 // beside the packed groups without widening these groups' shared memory.
 int launch_sptrsv(const GrpPlan& P, cudaStream_t st2, cudaEvent_t ev_fork, cudaEvent_t ev_join,
                   const int32_t* ord, int nL, int total, const SfTri& L, const SfTri& U,
-                  const c64* b, const int32_t* g_in, const double* rs, c64* y, c64* z, c64* x,
-                  int* ctl, cudaStream_t st) {
+                  const c64* b, const NodeSums* S, const int32_t* g_in, const double* rs, c64* y,
+                  c64* z, c64* x, int* ctl, cudaStream_t st) {
   int launches = 0;
   c64* out = P.direct ? x : z;
-  auto groups = [&](int a, int e, int R, int E, cudaStream_t s) {
+  auto groups = [&](int a, int e, int R, int E, int K, int G, cudaStream_t s) {
     if (e <= a) return;
-    k_sptrsv_grp<<<e - a, SF_GRP_TPB, grp_smem(R, E), s>>>(P, a, R, E, L.val, U.val, L.dinv,
-                                                           U.dinv, b, rs, out);
+    if (S)
+      k_sptrsv_grp<true><<<e - a, SF_GRP_TPB, grp_smem(R, E, K, G), s>>>(
+          P, a, R, E, G, L.val, U.sval, L.dinv, U.dinv, nullptr, *S, rs, out);
+    else
+      k_sptrsv_grp<false><<<e - a, SF_GRP_TPB, grp_smem(R, E, K, 0), s>>>(
+          P, a, R, E, 0, L.val, U.sval, L.dinv, U.dinv, b, NodeSums(), rs, out);
     ++launches;
   };
-  const int R = std::max(P.rb, P.rp), E = std::max(P.eb, P.ep);
-  if (P.nbig == 0 || P.nbig == P.ngroups || grp_smem(R, E) <= SF_ONE_LAUNCH_SMEM) {
-    groups(0, P.ngroups, R, E, st);
+  const int R = std::max(P.rb, P.rp), E = std::max(P.eb, P.ep), K = std::max(P.kb, P.kp),
+            G = std::max(P.gb, P.gp);
+  if (P.nbig == 0 || P.nbig == P.ngroups || grp_smem(R, E, K, S ? G : 0) <= SF_ONE_LAUNCH_SMEM) {
+    groups(0, P.ngroups, R, E, K, G, st);
   } else {
     if (st2) {
       cudaEventRecord(ev_fork, st);
       cudaStreamWaitEvent(st2, ev_fork, 0);
     }
-    groups(0, P.nbig, P.rb, P.eb, st2 ? st2 : st);
+    groups(0, P.nbig, P.rb, P.eb, P.kb, P.gb, st2 ? st2 : st);
     if (st2) cudaEventRecord(ev_join, st2);
-    groups(P.nbig, P.ngroups, P.rp, P.ep, st);
+    groups(P.nbig, P.ngroups, P.rp, P.ep, P.kp, P.gp, st);
     if (st2) cudaStreamWaitEvent(st, ev_join, 0);
   }
   if (total <= 0) return launches;
