@@ -1,6 +1,7 @@
 // GPU fill of the nine generating rows of the voxel Lp / P circulant blocks
-// (compute_FFT_mutual_coupling_mats with QS_Rcc_FW == 1), one thread per lattice
-// entry, FP64 throughout (the near-field closed forms cancel ~R^5 terms down to ~s^6/R).
+// (compute_FFT_mutual_coupling_mats with QS_Rcc_FW == 1), FP64 throughout (the near-field
+// closed forms cancel ~R^5 terms down to ~s^6/R). The near field sums corner terms that
+// neighbouring entries share; they are evaluated once into a table (see "corner tables").
 //
 // Lp rows: compute_Lp_Voxels.jl:40-60 with round_ud_fft(.,14) coordinates (:807-815) and
 // the Integ_vol_vol_fft dispatch (:65-435): the volume-volume closed form
@@ -45,6 +46,19 @@ __device__ __forceinline__ double sgn(int k) { return (k & 1) ? -1.0 : 1.0; }
 // i.e. (-1)^(sum0 + n [+1]) with the 0-based corner bits used here
 // ---------------------------------------------------------------------------------
 
+__device__ __forceinline__ double vol_corner(double X, double Y, double Z) {
+  const double X2 = X * X, Y2 = Y * Y, Z2 = Z * Z;
+  const double R = sqrt(X2 + Y2 + Z2);
+  const double t1 = (X2 * X2 + Y2 * Y2 + Z2 * Z2 - 3 * X2 * Y2 - 3 * Y2 * Z2 - 3 * X2 * Z2) * R / 60;
+  const double t2 = fin((Y2 * Z2 / 4 - Y2 * Y2 / 24 - Z2 * Z2 / 24) * X * lgc(X + R));
+  const double t3 = fin((Y2 * X2 / 4 - Y2 * Y2 / 24 - X2 * X2 / 24) * Z * lgc(Z + R));
+  const double t4 = fin((Z2 * X2 / 4 - Z2 * Z2 / 24 - X2 * X2 / 24) * Y * lgc(Y + R));
+  const double t5 = -fabs(X) * X2 * Y * Z / 6 * atan2(Y * Z, fabs(X) * R);
+  const double t6 = -X * fabs(Y) * Y2 * Z / 6 * atan2(X * Z, fabs(Y) * R);
+  const double t7 = -X * Y * fabs(Z) * Z2 / 6 * atan2(X * Y, fabs(Z) * R);
+  return t1 + t2 + t3 + t4 + t5 + t6 + t7;
+}
+
 __device__ double vol_vol(const double* x1v, const double* y1v, const double* z1v,
                           const double* x2v, const double* y2v, const double* z2v) {
   double sol = 0.0;
@@ -52,65 +66,60 @@ __device__ double vol_vol(const double* x1v, const double* y1v, const double* z1
   for (int c = 0; c < 64; ++c) {
     const int c1 = (c >> 5) & 1, c2 = (c >> 4) & 1, c3 = (c >> 3) & 1, c4 = (c >> 2) & 1,
               c5 = (c >> 1) & 1, c6 = c & 1;
-    const double X = x1v[c1] - x2v[c4], Y = y1v[c2] - y2v[c5], Z = z1v[c3] - z2v[c6];
-    const double X2 = X * X, Y2 = Y * Y, Z2 = Z * Z;
-    const double R = sqrt(X2 + Y2 + Z2);
-    const double t1 = (X2 * X2 + Y2 * Y2 + Z2 * Z2 - 3 * X2 * Y2 - 3 * Y2 * Z2 - 3 * X2 * Z2) * R / 60;
-    const double t2 = fin((Y2 * Z2 / 4 - Y2 * Y2 / 24 - Z2 * Z2 / 24) * X * lgc(X + R));
-    const double t3 = fin((Y2 * X2 / 4 - Y2 * Y2 / 24 - X2 * X2 / 24) * Z * lgc(Z + R));
-    const double t4 = fin((Z2 * X2 / 4 - Z2 * Z2 / 24 - X2 * X2 / 24) * Y * lgc(Y + R));
-    const double t5 = -fabs(X) * X2 * Y * Z / 6 * atan2(Y * Z, fabs(X) * R);
-    const double t6 = -X * fabs(Y) * Y2 * Z / 6 * atan2(X * Z, fabs(Y) * R);
-    const double t7 = -X * Y * fabs(Z) * Z2 / 6 * atan2(X * Y, fabs(Z) * R);
-    sol += sgn(c1 + c2 + c3 + c4 + c5 + c6 + 1) * (t1 + t2 + t3 + t4 + t5 + t6 + t7);
+    sol += sgn(c1 + c2 + c3 + c4 + c5 + c6 + 1) *
+           vol_corner(x1v[c1] - x2v[c4], y1v[c2] - y2v[c5], z1v[c3] - z2v[c6]);
   }
   return sol;
 }
 
 // surfaces in (x, y) planes at heights z1, z2
+__device__ __forceinline__ double para_corner(double X, double Y, double Z) {
+  const double R = sqrt(X * X + Y * Y + Z * Z);
+  const double t1 = -1.0 / 6 * (X * X + Y * Y - 2 * Z * Z) * R;
+  const double t2 = -X * Y * fabs(Z) * atan2(X * Y, fabs(Z) * R);
+  const double t3 = fin(0.5 * (X * X - Z * Z) * Y * lgc(Y + R));
+  const double t4 = fin(0.5 * (Y * Y - Z * Z) * X * lgc(X + R));
+  return t1 + t2 + t3 + t4;
+}
+
 __device__ double ss_para(const double* x1v, const double* y1v, double z1, const double* x2v,
                           const double* y2v, double z2) {
   double sol = 0.0;
-#pragma unroll
+#pragma unroll 1
   for (int c = 0; c < 16; ++c) {
     const int c1 = (c >> 3) & 1, c2 = (c >> 2) & 1, c3 = (c >> 1) & 1, c4 = c & 1;
-    const double X = x1v[c1] - x2v[c4], Y = y1v[c2] - y2v[c3], Z = z1 - z2;
-    const double R = sqrt(X * X + Y * Y + Z * Z);
-    const double t1 = -1.0 / 6 * (X * X + Y * Y - 2 * Z * Z) * R;
-    const double t2 = -X * Y * fabs(Z) * atan2(X * Y, fabs(Z) * R);
-    const double t3 = fin(0.5 * (X * X - Z * Z) * Y * lgc(Y + R));
-    const double t4 = fin(0.5 * (Y * Y - Z * Z) * X * lgc(X + R));
-    sol += sgn(c1 + c2 + c3 + c4) * (t1 + t2 + t3 + t4);
+    sol += sgn(c1 + c2 + c3 + c4) * para_corner(x1v[c1] - x2v[c4], y1v[c2] - y2v[c3], z1 - z2);
   }
   return sol;
 }
 
 // surface in the (x, y) plane at z1 against one in the (x, z) plane at y2; pform selects
 // the seven-term integ_surf_surf_ortho_P over the four-term integ_surf_surf_ortho_fft
+__device__ __forceinline__ double ortho_corner(double X, double Y, double Z, int pform) {
+  const double R = sqrt(X * X + Y * Y + Z * Z);
+  const double t1 = -1.0 / 3 * Y * Z * R;
+  const double t2 = -0.5 * X * fabs(Z) * Z * atan2(X * Y, fabs(Z) * R);
+  if (pform) {
+    const double t3 = -0.5 * X * fabs(Y) * Y * atan2(X * Z, fabs(Y) * R);
+    const double t4 = -1.0 / 6 * fabs(X) * X * X * atan2(Y * Z, fabs(X) * R);
+    const double t5 = fin(X * Y * Z * lgc(X + R));
+    const double t6 = fin((0.5 * X * X - 1.0 / 6 * Z * Z) * Z * lgc(Y + R));
+    const double t7 = fin((0.5 * X * X - 1.0 / 6 * Y * Y) * Y * lgc(Z + R));
+    return t1 + t2 + t3 + t4 + t5 + t6 + t7;
+  }
+  const double t3 = fin(0.5 * (X * X - Z * Z) * Y * lgc(Y + R));
+  const double t4 = fin(0.5 * (X * X - Y * Y) * X * lgc(X + R));
+  return t1 + t2 + t3 + t4;
+}
+
 __device__ double ss_ortho(const double* x1v, const double* y1v, double z1, const double* x2v,
                            double y2, const double* z2v, int pform) {
   double sol = 0.0;
 #pragma unroll 1
   for (int c = 0; c < 16; ++c) {
     const int c1 = (c >> 3) & 1, c2 = (c >> 2) & 1, c3 = (c >> 1) & 1, c4 = c & 1;
-    const double X = x1v[c1] - x2v[c4], Y = y1v[c2] - y2, Z = z1 - z2v[c3];
-    const double R = sqrt(X * X + Y * Y + Z * Z);
-    const double t1 = -1.0 / 3 * Y * Z * R;
-    const double t2 = -0.5 * X * fabs(Z) * Z * atan2(X * Y, fabs(Z) * R);
-    double s;
-    if (pform) {
-      const double t3 = -0.5 * X * fabs(Y) * Y * atan2(X * Z, fabs(Y) * R);
-      const double t4 = -1.0 / 6 * fabs(X) * X * X * atan2(Y * Z, fabs(X) * R);
-      const double t5 = fin(X * Y * Z * lgc(X + R));
-      const double t6 = fin((0.5 * X * X - 1.0 / 6 * Z * Z) * Z * lgc(Y + R));
-      const double t7 = fin((0.5 * X * X - 1.0 / 6 * Y * Y) * Y * lgc(Z + R));
-      s = t1 + t2 + t3 + t4 + t5 + t6 + t7;
-    } else {
-      const double t3 = fin(0.5 * (X * X - Z * Z) * Y * lgc(Y + R));
-      const double t4 = fin(0.5 * (X * X - Y * Y) * X * lgc(X + R));
-      s = t1 + t2 + t3 + t4;
-    }
-    sol += sgn(c1 + c2 + c3 + c4) * s;
+    sol += sgn(c1 + c2 + c3 + c4) *
+           ortho_corner(x1v[c1] - x2v[c4], y1v[c2] - y2, z1 - z2v[c3], pform);
   }
   return sol;
 }
@@ -513,32 +522,6 @@ __device__ __forceinline__ void lp_box(Box& b, const double c[3], const double s
   }
 }
 
-__global__ void k_fill_lp(LpRowArgs a, double* row, int64_t N, int* bad) {
-  const double sx = a.s[0], sy = a.s[1], sz = a.s[2];
-  double S = sy * sz * sy * sz;
-  if (a.dir == 1) S = sx * sz * sx * sz;
-  else if (a.dir == 2) S = sx * sy * sx * sy;
-  const double c1[3] = {lp_center(a, 0, 0), lp_center(a, 1, 0), lp_center(a, 2, 0)};
-  Box A;
-  lp_box(A, c1, a.s);
-  for (int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p < N;
-       p += (int64_t)gridDim.x * blockDim.x) {
-    const int i = (int)(p % a.M[0]);
-    const int j = (int)((p / a.M[0]) % a.M[1]);
-    const int k = (int)(p / ((int64_t)a.M[0] * a.M[1]));
-    const double c2[3] = {lp_center(a, 0, i), lp_center(a, 1, j), lp_center(a, 2, k)};
-    Box B;
-    lp_box(B, c2, a.s);
-    lp_flags(A, B);
-    const double v = (A.n + B.n == 0)
-                         ? vol_vol(A.iv[0], A.iv[1], A.iv[2], B.iv[0], B.iv[1], B.iv[2])
-                         : integ_boxes(A, B, a.form);
-    const double e = (p == 0) ? 0.0 : a.escal * (1e-7 / S * v);
-    if (!isfinite(e)) atomicOr(bad, a.form == 2 ? 2 : 1);
-    row[p] = e;
-  }
-}
-
 // ---------------------------------------------------------------------------------
 // P rows
 // ---------------------------------------------------------------------------------
@@ -571,10 +554,9 @@ __device__ __forceinline__ int face_box(Box& b, const double fc[3], const double
   return nrm;
 }
 
-// Integ_sup_sup_P (compute_row_P_sup.jl:106-381) over two face boxes with normals p1, p2
-// (pform 1); pform 4: Song_P_improved_Ivana_strategy (Song_P_improved_Ivana_strategy.jl:
-// 1-256), the same tree over the dense RIS surfaces
-__device__ double sup_sup_boxes(Box& A, Box& B, int p1, int p2, int pform) {
+// suppression flags of Integ_sup_sup_P (compute_row_P_sup.jl:106-170) over two face boxes
+// with normals p1, p2
+__device__ __forceinline__ void sup_flags(Box& A, Box& B, int p1, int p2) {
   const double s1 = A.len[0] * A.len[1] * A.len[2], s2 = B.len[0] * B.len[1] * B.len[2];
   double mxd[3];
   const double min_R = box_gaps(A, B, mxd);
@@ -588,6 +570,13 @@ __device__ double sup_sup_boxes(Box& A, Box& B, int p1, int p2, int pform) {
   B.s[p2] = 1;
   A.n = A.s[0] + A.s[1] + A.s[2];
   B.n = B.s[0] + B.s[1] + B.s[2];
+}
+
+// Integ_sup_sup_P (compute_row_P_sup.jl:106-381) over two face boxes with normals p1, p2;
+// pform 4: Song_P_improved_Ivana_strategy (Song_P_improved_Ivana_strategy.jl:1-256), the same
+// tree over the dense RIS surfaces
+__device__ double sup_sup_boxes(Box& A, Box& B, int p1, int p2, int pform) {
+  sup_flags(A, B, p1, p2);
   if (A.n + B.n == 2) {  // face - face, the near field
     const double w = A.len[p1] * B.len[p2];
     if (p1 == p2) {
@@ -599,13 +588,6 @@ __device__ double sup_sup_boxes(Box& A, Box& B, int p1, int p2, int pform) {
     return w * ss_ortho(A.iv[a], A.iv[p2], A.c[p1], B.iv[a], B.c[p2], B.iv[p1], pform);
   }
   return integ_boxes(A, B, pform);
-}
-
-__device__ double sup_sup(const double f1[3], const double e1[3], const double f2[3],
-                          const double e2[3]) {
-  Box A, B;
-  const int p1 = face_box(A, f1, e1), p2 = face_box(B, f2, e2);
-  return sup_sup_boxes(A, B, p1, p2, 1);
 }
 
 struct PRowArgs {
@@ -629,27 +611,271 @@ __device__ __forceinline__ void face(int caser, double cx, double cy, double cz,
   }
 }
 
-__global__ void k_fill_p(PRowArgs a, double* row, int64_t N, int* bad) {
-  const double pi = 3.141592653589793;
-  const double eps0 = 8.854187816997944e-12;
-  const double sx = a.s[0], sy = a.s[1], sz = a.s[2];
-  double f1[3], e1[3], d1[2];
-  face(a.caser, ctr(a.o[0], sx, 0, a.half[0]), ctr(a.o[1], sy, 0, a.half[1]),
-       ctr(a.o[2], sz, 0, a.half[2]), sx, sy, sz, f1, e1, d1);
-  const double A1 = d1[0] * d1[1];
-  for (int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p < N;
+// ---------------------------------------------------------------------------------
+// Corner tables of the near field
+//
+// A near-field entry is a signed sum over the corners of its two bodies -- 64 for two
+// voxels, 16 for two faces -- of a function f(X, Y, Z) of the corner differences along the
+// axes, three logarithms and three arctangents each. What bounds the fill is the FP64 pipe,
+// and neighbouring entries share most of their corners: along an axis of M cells the 4 M
+// differences (two corners of the generating body, two of each cell) hold only about 1.1 M
+// to 2 M distinct doubles (the rounding of the coordinates makes some of the equal
+// differences differ in their last bits). So per row and axis the distinct differences are
+// listed (k_fill_lists, compared by their bits), the f of the triples that some near-field
+// entry takes are evaluated once (k_fill_mark, k_fill_eval), and every entry sums its own
+// corners from the table in the closed form's order (k_fill_sum): the same terms in the same
+// order, bit for bit, and 3 to 5 evaluations an entry in place of 64 or 16. The cross P rows
+// repeat every cell two or four times over their interleaved axes; each cell is summed once.
+// Entries in the far field are evaluated directly, as before.
+// Measured at 128x128x64 (19.0 M entries): peec_fill 288.7 ms with one thread per entry
+// evaluating its own corners (rows 264 ms), 44.5 ms from the tables.
+// ---------------------------------------------------------------------------------
+
+struct RowSpec {
+  int lp;
+  LpRowArgs l;
+  PRowArgs p;
+  int kind;      // 0 volumes, 1 parallel faces, 2 orthogonal faces
+  int p1, p2;    // the faces' normals (P rows)
+  int role[3];   // the physical axis of X, Y, Z
+  int ns[3], nt[3];  // per role: corners (2) or the centre (1) of the generating body / a cell
+  int D[3];      // distinct cells per physical axis
+  int rep[3];    // how often a distinct cell occurs along the axis (1 or 2)
+  int M[3];      // lattice extents
+};
+constexpr int kFillRows = 9;
+struct RowSet {
+  RowSpec r[kFillRows];
+  double* row[kFillRows];
+  double* val[kFillRows][3];   // distinct differences per role
+  int32_t* map[kFillRows][3];  // difference (source corner, cell corner, cell) -> its index
+  int n;
+  int k0, k1;                  // cells of the physical z axis in this slab
+};
+
+// the generating body (cell 0) or cell i of a row
+__device__ __forceinline__ void row_box(const RowSpec& s, const int i[3], bool source, Box& b) {
+  if (s.lp) {
+    const double c[3] = {lp_center(s.l, 0, i[0]), lp_center(s.l, 1, i[1]), lp_center(s.l, 2, i[2])};
+    lp_box(b, c, s.l.s);
+  } else {
+    // centre index of the distinct cell: the interleaved axes' ceil(i/2) lattice is its own
+    const PRowArgs& a = s.p;
+    double fc[3], e[3], d[2];
+    face(source ? a.caser : a.caser2, ctr(a.o[0], a.s[0], i[0], 0), ctr(a.o[1], a.s[1], i[1], 0),
+         ctr(a.o[2], a.s[2], i[2], 0), a.s[0], a.s[1], a.s[2], fc, e, d);
+    face_box(b, fc, e);
+  }
+}
+
+// cells of a role's axis in this slab
+__device__ __forceinline__ int role_cells(const RowSet& S, const RowSpec& s, int q, int* first) {
+  const int ax = s.role[q];
+  *first = ax == 2 ? S.k0 : 0;
+  return ax == 2 ? min(S.k1, s.D[2]) - S.k0 : s.D[ax];
+}
+
+// One CTA per (role, row): the distinct differences of the axis, in order of first occurrence,
+// and every difference's index. scr: scratch of 2 * 4 M entries per CTA (differences, ranks).
+__global__ void __launch_bounds__(1024) k_fill_lists(RowSet S, double* scr, int32_t* rank,
+                                                     int stride, int* count) {
+  __shared__ int wsum[32];
+  __shared__ int base;
+  const int q = blockIdx.x, r = blockIdx.y;
+  const RowSpec& s = S.r[r];
+  int first;
+  const int M = role_cells(S, s, q, &first);
+  const int ax = s.role[q], ns = s.ns[q], nt = s.nt[q], n = M > 0 ? ns * nt * M : 0;
+  double* x = scr + (size_t)(r * 3 + q) * stride;
+  int32_t* rk = rank + (size_t)(r * 3 + q) * stride;
+  const int zero[3] = {0, 0, 0};
+  Box A;
+  row_box(s, zero, true, A);
+  for (int e = threadIdx.x; e < n; e += blockDim.x) {
+    const int i = e % M, ct = (e / M) % nt, cs = e / (M * nt);
+    int at[3] = {0, 0, 0};
+    at[ax] = first + i;
+    Box B;
+    row_box(s, at, false, B);
+    x[e] = (ns == 2 ? A.iv[ax][cs] : A.c[ax]) - (nt == 2 ? B.iv[ax][ct] : B.c[ax]);
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) base = 0;
+  // an entry's first equal; the first ones take consecutive indices
+  for (int e0 = 0; e0 < n; e0 += blockDim.x) {
+    const int e = e0 + threadIdx.x;
+    int f = e;
+    if (e < n) {
+      const long long b = __double_as_longlong(x[e]);
+      for (int t = 0; t < e; ++t)
+        if (__double_as_longlong(x[t]) == b) {
+          f = t;
+          break;
+        }
+    }
+    const bool own = e < n && f == e;
+    const unsigned m = __ballot_sync(0xffffffffu, own);
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    __syncthreads();
+    if (lane == 0) wsum[w] = __popc(m);
+    __syncthreads();
+    int before = base + __popc(m & ((1u << lane) - 1));
+    for (int t = 0; t < w; ++t) before += wsum[t];
+    if (own) {
+      rk[e] = before;
+      S.val[r][q][before] = x[e];
+    } else if (e < n) {
+      rk[e] = ~f;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0)
+      for (int t = 0; t < 32; ++t) base += wsum[t];
+    __syncthreads();
+  }
+  for (int e = threadIdx.x; e < n; e += blockDim.x)
+    S.map[r][q][e] = rk[e] >= 0 ? rk[e] : rk[~rk[e]];
+  if (threadIdx.x == 0) count[r * 3 + q] = base;
+}
+
+// table index of a corner from its per-role indices
+__device__ __forceinline__ size_t corner_at(const int U[3], int x, int y, int z) {
+  return ((size_t)z * U[1] + y) * U[0] + x;
+}
+
+// calls f(sign, index) for a near-field cell's corners in the closed form's order
+template <typename F>
+__device__ __forceinline__ void each_corner(const RowSet& S, const RowSpec& s, int r, const int U[3],
+                                            const int i[3], F&& f) {
+  int id[3][4], M[3], c[3];
+  for (int q = 0; q < 3; ++q) {
+    int first;
+    M[q] = role_cells(S, s, q, &first);
+    c[q] = i[s.role[q]] - first;
+    for (int t = 0; t < s.ns[q] * s.nt[q]; ++t) id[q][t] = S.map[r][q][t * M[q] + c[q]];
+  }
+  if (s.kind == 0) {
+#pragma unroll 4
+    for (int k = 0; k < 64; ++k) {
+      const int c1 = (k >> 5) & 1, c2 = (k >> 4) & 1, c3 = (k >> 3) & 1, c4 = (k >> 2) & 1,
+                c5 = (k >> 1) & 1, c6 = k & 1;
+      f(sgn(c1 + c2 + c3 + c4 + c5 + c6 + 1),
+        corner_at(U, id[0][2 * c1 + c4], id[1][2 * c2 + c5], id[2][2 * c3 + c6]));
+    }
+  } else {
+#pragma unroll 4
+    for (int k = 0; k < 16; ++k) {
+      const int c1 = (k >> 3) & 1, c2 = (k >> 2) & 1, c3 = (k >> 1) & 1, c4 = k & 1;
+      const size_t at = s.kind == 1 ? corner_at(U, id[0][2 * c1 + c4], id[1][2 * c2 + c3], id[2][0])
+                                    : corner_at(U, id[0][2 * c1 + c4], id[1][c2], id[2][c3]);
+      f(sgn(c1 + c2 + c3 + c4), at);
+    }
+  }
+}
+
+// cell of flat index p in the slab; near: whether no dimension collapses beyond the faces'
+// normals
+__device__ __forceinline__ bool slab_cell(const RowSet& S, const RowSpec& s, int64_t p, int i[3],
+                                          Box& A, Box& B) {
+  const int64_t plane = (int64_t)s.D[0] * s.D[1];
+  i[0] = (int)(p % s.D[0]);
+  i[1] = (int)((p / s.D[0]) % s.D[1]);
+  i[2] = S.k0 + (int)(p / plane);
+  const int zero[3] = {0, 0, 0};
+  row_box(s, zero, true, A);
+  row_box(s, i, false, B);
+  if (s.lp) {
+    lp_flags(A, B);
+    return A.n + B.n == 0;
+  }
+  sup_flags(A, B, s.p1, s.p2);
+  return A.n + B.n == 2;
+}
+
+__device__ __forceinline__ int64_t slab_cells(const RowSet& S, const RowSpec& s) {
+  return (int64_t)s.D[0] * s.D[1] * max(0, min(S.k1, s.D[2]) - S.k0);
+}
+
+// marks the corners the row's near-field cells take
+__global__ void k_fill_mark(RowSet S, int r, int U0, int U1, int U2, uint8_t* need, uint8_t* near) {
+  const RowSpec& s = S.r[r];
+  const int U[3] = {U0, U1, U2};
+  const int64_t n = slab_cells(S, s);
+  for (int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p < n;
        p += (int64_t)gridDim.x * blockDim.x) {
-    const int i = (int)(p % a.M[0]);
-    const int j = (int)((p / a.M[0]) % a.M[1]);
-    const int k = (int)(p / ((int64_t)a.M[0] * a.M[1]));
-    double f2[3], e2[3], d2[2];
-    face(a.caser2, ctr(a.o[0], sx, i, a.half[0]), ctr(a.o[1], sy, j, a.half[1]),
-         ctr(a.o[2], sz, k, a.half[2]), sx, sy, sz, f2, e2, d2);
-    const double v = sup_sup(f1, e1, f2, e2);
-    const double pref = 1.0 / (4 * pi * eps0 * A1 * d2[0] * d2[1]);
-    const double e = a.escal * (pref * v);
-    if (!isfinite(e)) atomicOr(bad, 1);
-    row[p] = e;
+    int i[3];
+    Box A, B;
+    const bool nr = slab_cell(S, s, p, i, A, B);
+    near[p] = nr;
+    if (nr) each_corner(S, s, r, U, i, [&](double, size_t at) { need[at] = 1; });
+  }
+}
+
+template <int KIND>
+__global__ void __launch_bounds__(128) k_fill_eval(const double* __restrict__ X,
+                                                   const double* __restrict__ Y,
+                                                   const double* __restrict__ Z, int U0, int U1,
+                                                   int64_t n, const uint8_t* __restrict__ need,
+                                                   double* __restrict__ tab) {
+  for (int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p < n;
+       p += (int64_t)gridDim.x * blockDim.x) {
+    if (!need[p]) continue;
+    const double x = X[p % U0], y = Y[(p / U0) % U1], z = Z[p / ((int64_t)U0 * U1)];
+    tab[p] = KIND == 0 ? vol_corner(x, y, z) : (KIND == 1 ? para_corner(x, y, z) : ortho_corner(x, y, z, 1));
+  }
+}
+
+// the row's entries: near-field cells from the table, the others by their closed forms
+__global__ void __launch_bounds__(128) k_fill_sum(RowSet S, int r, int U0, int U1, int U2,
+                                                  const double* __restrict__ tab,
+                                                  const uint8_t* __restrict__ near, int* bad) {
+  const RowSpec& s = S.r[r];
+  const int U[3] = {U0, U1, U2};
+  const int64_t n = slab_cells(S, s);
+  double* row = S.row[r];
+  for (int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p < n;
+       p += (int64_t)gridDim.x * blockDim.x) {
+    int i[3];
+    double v;
+    if (near[p]) {
+      i[0] = (int)(p % s.D[0]);
+      i[1] = (int)((p / s.D[0]) % s.D[1]);
+      i[2] = S.k0 + (int)(p / ((int64_t)s.D[0] * s.D[1]));
+      double sol = 0.0;
+      each_corner(S, s, r, U, i, [&](double sg, size_t at) { sol += sg * tab[at]; });
+      v = sol;  // the faces' normal lengths, a factor of the closed form, are one
+    } else {
+      Box A, B;
+      slab_cell(S, s, p, i, A, B);
+      v = integ_boxes(A, B, s.lp ? s.l.form : 1);
+    }
+    double e;
+    int flag = 1;
+    if (s.lp) {
+      const double sx = s.l.s[0], sy = s.l.s[1], sz = s.l.s[2];
+      double S4 = sy * sz * sy * sz;
+      if (s.l.dir == 1) S4 = sx * sz * sx * sz;
+      else if (s.l.dir == 2) S4 = sx * sy * sx * sy;
+      e = (i[0] | i[1] | i[2]) == 0 ? 0.0 : s.l.escal * (1e-7 / S4 * v);
+      if (s.l.form == 2) flag = 2;
+    } else {
+      const double pi = 3.141592653589793;
+      const double eps0 = 8.854187816997944e-12;
+      const PRowArgs& a = s.p;
+      double fc[3], ex[3], d1[2], d2[2];
+      face(a.caser, 0, 0, 0, a.s[0], a.s[1], a.s[2], fc, ex, d1);
+      face(a.caser2, 0, 0, 0, a.s[0], a.s[1], a.s[2], fc, ex, d2);
+      const double A1 = d1[0] * d1[1];
+      const double pref = 1.0 / (4 * pi * eps0 * A1 * d2[0] * d2[1]);
+      e = a.escal * (pref * v);
+    }
+    if (!isfinite(e)) atomicOr(bad, flag);
+    for (int cz = 0; cz < s.rep[2]; ++cz)
+      for (int cy = 0; cy < s.rep[1]; ++cy)
+        for (int cx = 0; cx < s.rep[0]; ++cx) {
+          const int x = i[0] * s.rep[0] + cx, y = i[1] * s.rep[1] + cy, z = i[2] * s.rep[2] + cz;
+          if (x < s.M[0] && y < s.M[1] && z < s.M[2])
+            row[((size_t)z * s.M[1] + y) * s.M[0] + x] = e;
+        }
   }
 }
 
@@ -668,6 +894,15 @@ static void p_defs(int Nx, int Ny, int Nz, PDef pd[6]) {
   for (int r = 0; r < 6; ++r) pd[r] = d[r];
 }
 
+static int face_axis(int caser) { return caser <= 2 ? 1 : (caser <= 4 ? 0 : 2); }
+
+// normal of a face as face_box finds it: the smallest extent
+static int face_normal(int caser, const double s[3]) {
+  double e[3] = {s[0], s[1], s[2]};
+  e[face_axis(caser)] = 0;
+  return (e[0] <= e[1] && e[0] <= e[2]) ? 0 : ((e[1] <= e[0] && e[1] <= e[2]) ? 1 : 2);
+}
+
 // rcc = 0: the QS rows (compute_FFT_mutual_coupling_mats.jl:36-128); rcc = 1: the QS parts
 // of the Rcc rows (compute_rows_Rcc_Lp.jl:20-35 over compute_Lp_Voxels_QS,
 // compute_rows_Rcc_P.jl:47-52), escaled, Lp self entries zero
@@ -675,39 +910,142 @@ static int fill_rows_any(const double origin[3], double sx, double sy, double sz
                          double escal_Lp, double escal_P, int Nx, int Ny, int Nz,
                          double* const d_rows[9], const int64_t row_len[9], int* d_bad,
                          cudaStream_t st, int rcc) {
-  const int grid = 152 * 8, tpb = 128;
+  RowSet S{};
+  int maxM = 1, maxz = 1;
   const int lpM[3][3] = {{Nx - 1, Ny, Nz}, {Nx, Ny - 1, Nz}, {Nx, Ny, Nz - 1}};
-  for (int d = 0; d < 3; ++d) {
-    if (!d_rows[d] || row_len[d] == 0) continue;
-    LpRowArgs a;
-    a.dir = d;
-    for (int q = 0; q < 3; ++q) {
-      a.M[q] = lpM[d][q];
-      a.o[q] = origin[q];
-    }
-    a.s[0] = sx; a.s[1] = sy; a.s[2] = sz;
-    a.escal = escal_Lp;
-    a.form = rcc ? 2 : 0;
-    k_fill_lp<<<grid, tpb, 0, st>>>(a, d_rows[d], row_len[d], d_bad);
-  }
   PDef pd[6];
   p_defs(Nx, Ny, Nz, pd);
-  for (int r = 0; r < 6; ++r) {
-    if (!d_rows[3 + r] || row_len[3 + r] == 0) continue;
-    PRowArgs a;
-    a.caser = rcc ? pd[r].r1 : pd[r].c1;
-    a.caser2 = rcc ? pd[r].r2 : pd[r].c2;
+  const double sc[3] = {sx, sy, sz};
+  for (int r = 0; r < 9; ++r) {
+    if (!d_rows[r] || row_len[r] == 0) continue;
+    RowSpec& s = S.r[S.n];
+    S.row[S.n++] = d_rows[r];
+    s.lp = r < 3;
     for (int q = 0; q < 3; ++q) {
-      a.M[q] = pd[r].M[q];
-      a.half[q] = pd[r].half[q];
-      a.o[q] = origin[q];
+      s.M[q] = s.lp ? lpM[r][q] : pd[r - 3].M[q];
+      s.l.o[q] = s.p.o[q] = origin[q];
+      s.l.s[q] = s.p.s[q] = sc[q];
+      s.l.M[q] = s.p.M[q] = s.M[q];
+      s.rep[q] = 1;
     }
-    a.s[0] = sx; a.s[1] = sy; a.s[2] = sz;
-    a.escal = escal_P;
-    k_fill_p<<<grid, tpb, 0, st>>>(a, d_rows[3 + r], row_len[3 + r], d_bad);
+    if (s.lp) {
+      s.l.dir = r;
+      s.l.escal = escal_Lp;
+      s.l.form = rcc ? 2 : 0;
+      s.kind = 0;
+      for (int q = 0; q < 3; ++q) {
+        s.role[q] = q;
+        s.ns[q] = s.nt[q] = 2;
+      }
+    } else {
+      const PDef& d = pd[r - 3];
+      s.p.caser = rcc ? d.r1 : d.c1;
+      s.p.caser2 = rcc ? d.r2 : d.c2;
+      s.p.escal = escal_P;
+      for (int q = 0; q < 3; ++q) {
+        s.p.half[q] = d.half[q];
+        s.rep[q] = d.half[q] ? 2 : 1;
+      }
+      s.p1 = face_normal(s.p.caser, sc);
+      s.p2 = face_normal(s.p.caser2, sc);
+      if (s.p1 == s.p2) {
+        s.kind = 1;
+        s.role[0] = s.p1 == 0 ? 1 : 0;
+        s.role[1] = s.p1 == 2 ? 1 : 2;
+        s.role[2] = s.p1;
+        for (int q = 0; q < 3; ++q) s.ns[q] = s.nt[q] = q < 2 ? 2 : 1;
+      } else {
+        s.kind = 2;
+        s.role[0] = 3 - s.p1 - s.p2;
+        s.role[1] = s.p2;
+        s.role[2] = s.p1;
+        s.ns[0] = s.nt[0] = 2;
+        s.ns[1] = 2; s.nt[1] = 1;
+        s.ns[2] = 1; s.nt[2] = 2;
+      }
+    }
+    for (int q = 0; q < 3; ++q) {
+      s.D[q] = (s.M[q] + s.rep[q] - 1) / s.rep[q];
+      maxM = std::max(maxM, s.D[q]);
+    }
+    maxz = std::max(maxz, s.D[2]);
   }
-  PEEC_CUDA_TRY(cudaGetLastError());
-  return 0;
+  if (S.n == 0) return 0;
+  // slabs of cells along z, so that a row's table stays below FILL_TABLE entries (16 MB: the
+  // entries' corner reads come from L2; a slab's extra plane of corners is a few percent)
+  constexpr int64_t FILL_TABLE = (int64_t)1 << 21;
+  const int stride = 4 * maxM;
+  const size_t lists = (size_t)S.n * 3 * stride;
+  double *val = nullptr, *scr = nullptr;
+  int32_t *map = nullptr, *rank = nullptr;
+  int* cnt = nullptr;
+  const size_t list_bytes = lists * (2 * sizeof(double) + 2 * sizeof(int32_t)) + 27 * sizeof(int);
+  PEEC_CUDA_TRY(cudaMallocAsync((void**)&val, list_bytes, st));
+  scr = val + lists;
+  map = reinterpret_cast<int32_t*>(scr + lists);
+  rank = map + lists;
+  cnt = rank + lists;
+  for (int r = 0; r < S.n; ++r)
+    for (int q = 0; q < 3; ++q) {
+      S.val[r][q] = val + (size_t)(r * 3 + q) * stride;
+      S.map[r][q] = map + (size_t)(r * 3 + q) * stride;
+    }
+  double* tab = nullptr;
+  uint8_t *need = nullptr, *near = nullptr;
+  int64_t tab_cap = 0, near_cap = 0;
+  auto run = [&]() -> int {
+    int cz = maxz;
+    for (int k0 = 0; k0 < maxz;) {
+      S.k0 = k0;
+      S.k1 = std::min(k0 + cz, maxz);
+      k_fill_lists<<<dim3(3, S.n), 1024, 0, st>>>(S, scr, rank, stride, cnt);
+      int U[27];
+      PEEC_CUDA_TRY(cudaMemcpyAsync(U, cnt, sizeof(U[0]) * 3 * S.n, cudaMemcpyDeviceToHost, st));
+      PEEC_CUDA_TRY(cudaStreamSynchronize(st));
+      int64_t most = 1, cells = 1;
+      for (int r = 0; r < S.n; ++r) {
+        most = std::max(most, (int64_t)U[3 * r] * U[3 * r + 1] * U[3 * r + 2]);
+        cells = std::max(cells, (int64_t)S.r[r].D[0] * S.r[r].D[1] *
+                                    std::max(0, std::min(S.k1, S.r[r].D[2]) - k0));
+      }
+      if (most > FILL_TABLE && S.k1 - k0 > 1) {
+        cz = (int)std::max<int64_t>(1, std::min<int64_t>(S.k1 - k0 - 1, (S.k1 - k0) * FILL_TABLE / most));
+        continue;
+      }
+      if (most > tab_cap || cells > near_cap) {
+        if (tab) PEEC_CUDA_TRY(cudaFreeAsync(tab, st));
+        tab = nullptr;
+        tab_cap = std::max(tab_cap, most);
+        near_cap = std::max(near_cap, cells);
+        PEEC_CUDA_TRY(cudaMallocAsync((void**)&tab, tab_cap * (sizeof(double) + 1) + near_cap, st));
+        need = reinterpret_cast<uint8_t*>(tab + tab_cap);
+        near = need + tab_cap;
+      }
+      for (int r = 0; r < S.n; ++r) {
+        const RowSpec& s = S.r[r];
+        const int U0 = U[3 * r], U1 = U[3 * r + 1], U2 = U[3 * r + 2];
+        const int64_t nt = (int64_t)U0 * U1 * U2;
+        const int64_t nc = (int64_t)s.D[0] * s.D[1] * std::max(0, std::min(S.k1, s.D[2]) - k0);
+        if (nc <= 0 || nt <= 0) continue;
+        auto blocks = [](int64_t n, int tpb) {
+          return (unsigned)std::min<int64_t>((n + tpb - 1) / tpb, 152 * 64);
+        };
+        PEEC_CUDA_TRY(cudaMemsetAsync(need, 0, nt, st));
+        k_fill_mark<<<blocks(nc, 128), 128, 0, st>>>(S, r, U0, U1, U2, need, near);
+        auto eval = s.kind == 0 ? k_fill_eval<0> : (s.kind == 1 ? k_fill_eval<1> : k_fill_eval<2>);
+        eval<<<blocks(nt, 128), 128, 0, st>>>(S.val[r][0], S.val[r][1], S.val[r][2], U0, U1, nt,
+                                              need, tab);
+        k_fill_sum<<<blocks(nc, 128), 128, 0, st>>>(S, r, U0, U1, U2, tab, near, d_bad);
+      }
+      k0 = S.k1;
+    }
+    PEEC_CUDA_TRY(cudaGetLastError());
+    return 0;
+  };
+  const int rc = run();
+  if (tab) cudaFreeAsync(tab, st);
+  cudaFreeAsync(val, st);
+  return rc;
 }
 
 int fill_rows_gpu(const double origin[3], double sx, double sy, double sz, double escal_Lp,
