@@ -33,7 +33,7 @@ CUDA_SOURCES = ["ctx.cu", "fftconv.cu", "fftconv_f32.cu", "fftconv_f64.cu", "fft
                 "mesher_gpu.cu", "dense.cu"]
 # the fill keeps the reference's scalar rounding: no FMA contraction
 FILE_FLAGS = {"fill.cu": ["-fmad=false"]}
-CUDA_HEADERS = ["common.cuh", "fft.cuh", "fft_reg.cuh", "fftconv_impl.cuh",
+CUDA_HEADERS = ["common.cuh", "fft_reg.cuh", "fftconv_impl.cuh", "tma.cuh",
                 "ctx.hpp"]
 
 

@@ -1200,15 +1200,17 @@ static int build_spectrum_set(peec_ctx* ctx, Spectrum* dst, double* const d_rows
                                  {2, 1, 2}, {1, 1, 1}, {1, 1, 1}, {1, 1, 1}};
   static const int odim[9][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}, {1, -1, 0}, {0, -1, 1},
                                  {-1, 0, 1}, {0, 0, 0}, {0, 0, 0}, {0, 0, 0}};
+  SpecJob jobs[9];
+  int nj = 0;
   for (int i = 0; i < 9; ++i) {
     if (!ctx->fam[fout[i]].active || !ctx->fam[fin[i]].active) continue;
     if (!d_rows[srow[i]]) return bad(ctx, PEEC_ERR_BADARG, "missing generating row");
     const bool sym = i < 3 || i >= 6;
-    CTX_TRY(spectrum_build(dst[i], d_rows[srow[i]], ctx->row_dims[srow[i]],
-                           ctx->fam[fout[i]].dims, ctx->fam[fin[i]].dims, sdim[i], odim[i],
-                           sym ? 1 : 0, ctx->tw64, ctx->twmax, ctx->st));
-    ctx->launches += 6;
+    jobs[nj++] = SpecJob{&dst[i], d_rows[srow[i]], ctx->row_dims[srow[i]], ctx->fam[fout[i]].dims,
+                         ctx->fam[fin[i]].dims, sdim[i], odim[i], sym ? 1 : 0};
   }
+  CTX_TRY(spectra_build(jobs, nj, ctx->tw64, ctx->twmax, ctx->ph64, ctx->st));
+  ctx->launches += nj ? 3 + 2 * nj : 0;
   return PEEC_OK;
 }
 

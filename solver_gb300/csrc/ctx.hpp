@@ -220,8 +220,16 @@ int phase_tables(const int L[3], void* e64[3], void* e32[3], cudaStream_t st);
 // tiles, enough z points; the edge families on one shared grid)
 bool zpass_yz_faces(const Family* F, int nfam);
 bool zpass_yz_edges(const Family* F, int nfam);
-int spectrum_build(Spectrum& S, const double* d_row, const int M[3], const int na[3],
-                   const int nb[3], const int sdim[3], const int odim[3], int symmetric,
-                   const void* twiddles64, int twmax, cudaStream_t st);
+// A spectrum to build from a generating row on the device: the row's extents, the output and
+// input family extents, stride and offset per axis (K(e) = row[|sdim e + odim|])
+struct SpecJob {
+  Spectrum* S;
+  const double* row;
+  const int *M, *na, *nb, *sdim, *odim;
+  int symmetric;
+};
+// ph: the face grid's FP64 phase tables (x, y, z)
+int spectra_build(const SpecJob* jobs, int njobs, const void* tw64, int twmax,
+                  const void* const ph[3], cudaStream_t st);
 
 }  // namespace peec

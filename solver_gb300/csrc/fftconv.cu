@@ -33,8 +33,10 @@
 #include <set>
 #include <utility>
 
+#include <algorithm>
+
 #include "ctx.hpp"
-#include "fft.cuh"
+#include "fft_reg.cuh"
 
 namespace peec {
 
@@ -44,13 +46,6 @@ int conv_all_f64(const Family*, int, const Spectrum*, const void* const*, const 
                  c64*, int64_t, const void*, int, cudaStream_t, cudaEvent_t*, const ZTune*);
 int conv_all_ff(const Family*, int, const Spectrum*, const void* const*, const c64*, c64*,
                 c64*, int64_t, const void*, int, cudaStream_t, cudaEvent_t*, const ZTune*);
-
-// copy W_L[e] = exp(-2 pi i e / L) for e < n from the master table of length twmax
-template <typename R>
-__device__ void load_tw(cx<R>* dst, const cx<R>* __restrict__ master, int twmax, int L, int n) {
-  const int step = twmax / L;
-  for (int e = threadIdx.x; e < n; e += blockDim.x) dst[e] = master[e * step];
-}
 
 // prec: PEEC_PREC_FP64 (0), PEEC_PREC_FP32 (1), PEEC_PREC_FF (2); tw[prec] the matching
 // master twiddle table
@@ -91,15 +86,27 @@ bool zpass_yz_edges(const Family* F, int nfam) {
 }
 
 // --------------------------------------------------------------------------- spectra
-// spectra: embed the generating row as a (possibly non-symmetric) circulant kernel,
-// forward-FFT it with the same DIF transforms, fold the 1/(Lx*Ly*Lz) scale
+// The spectrum of a generating row: along each axis the embedded kernel
+// K(e) = row[|s e + o|] is even (s = 1, o = 0) or even about a half-sample shift
+// (s = 2, o = +-1, c = -o), so its transform is exp(-i pi c f / L) times a real, even R(f)
+// and the three axes are three real transforms of the row's own octant:
+//   x: (uz, uy, t) -> (uz, uy, fx)   y: -> (uz, fy, fx)   z: -> (fy, fz, fx) = R,
+// u the used entries of an axis (every one, or the odd ones of an interleaved axis) and
+// f = 0 .. L/2. A complex FFT of length L transforms two lines at once, one as the real and
+// one as the imaginary part: after the shift's phase they separate by themselves. An eighth
+// of the lines of the embedded complex transform, half of them again by the pairing; all
+// rows of a set share each pass's launch. FP64 pipe bound. Measured at 128x128x64 (nine
+// spectra): transforms 1.65 ms and the full forms 0.97 ms, against 13.3 and 1.3 ms as complex
+// transforms of the embedded kernels; a retarded frequency at 48x48x24 (eighteen spectra)
+// 0.40 against 3.2 ms.
 // ------------------------------------------------------------------------------------
 
-struct EmbedDim {
-  int L, na, nb, s, o, M;
+struct SpecAxis {
+  int L, n, na, nb, s, o, c;
+  int M, U;  // entries of the row along the axis, and those used
 };
 
-__device__ __forceinline__ int embed_index(int j, const EmbedDim& d) {
+__device__ __forceinline__ int embed_index(int j, const SpecAxis& d) {
   // offset e of circulant slot j: e = j for j < na, e = j - L for j > L - nb
   int e;
   if (j < d.na) e = j;
@@ -110,112 +117,118 @@ __device__ __forceinline__ int embed_index(int j, const EmbedDim& d) {
   return t < d.M ? t : -1;
 }
 
-__global__ void k_embed(const double* __restrict__ row, c64* out, EmbedDim dx, EmbedDim dy,
-                        EmbedDim dz) {
-  const size_t total = (size_t)dx.L * dy.L * dz.L;
-  for (size_t p = blockIdx.x * (size_t)blockDim.x + threadIdx.x; p < total;
-       p += (size_t)gridDim.x * blockDim.x) {
-    const int jz = p % dz.L;
-    const int jy = (p / dz.L) % dy.L;
-    const int jx = p / ((size_t)dz.L * dy.L);
-    const int ix = embed_index(jx, dx), iy = embed_index(jy, dy), iz = embed_index(jz, dz);
-    double v = 0.0;
-    if (ix >= 0 && iy >= 0 && iz >= 0) v = row[((size_t)iz * dy.M + iy) * dx.M + ix];
-    out[p] = mk<double>(v, 0.0);
-  }
-}
+struct SpecRow {
+  SpecAxis ax[3];
+  const double* row;
+  double *A, *B, *oct;  // after the x and the y pass; R
+  double scale;
+};
+constexpr int kSpecRows = 9;
+struct SpecSet {
+  SpecRow r[kSpecRows];
+  int cta0[kSpecRows + 1];  // first CTA of each row in this pass
+  int n;
+};
 
-// forward DIF along one axis of a (Lx,Ly,Lz) array with z fastest. For axis 2 the
-// pencils are contiguous; for axes 0/1 a CTA takes TZ consecutive pencils.
-template <int TZ>
-__global__ void k_fft_axis(c64* data, int Lx, int Ly, int Lz, int axis, int logL,
-                           const c64* __restrict__ twm, int twmax) {
-  extern __shared__ unsigned char smem_raw[];
-  const int L = axis == 0 ? Lx : (axis == 1 ? Ly : Lz);
+// One pass along axis AX: 2^LC pairs of lines per CTA, tile element (pos, pair) at
+// buf[pos * (C + 1) + pair].
+template <int AX, int LC>
+__global__ void __launch_bounds__(256) k_spec_pass(SpecSet S, const c64* __restrict__ twm,
+                                                   int twmax) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  constexpr int C = 1 << LC, RS = C + 1;
+  int ri = 0;
+#pragma unroll
+  for (int i = 1; i < kSpecRows; ++i)
+    if (i < S.n && (int)blockIdx.x >= S.cta0[i]) ri = i;
+  const SpecRow& R = S.r[ri];
+  const SpecAxis& d = R.ax[AX];
+  const int ox = R.ax[0].L / 2 + 1, oy = R.ax[1].L / 2 + 1, oz = R.ax[2].L / 2 + 1;
+  const int Uy = R.ax[1].U, Uz = R.ax[2].U;
+  const int64_t lines = AX == 0 ? (int64_t)Uz * Uy : (AX == 1 ? (int64_t)Uz * ox : (int64_t)oy * ox);
+  const int64_t l0 = (int64_t)((int)blockIdx.x - S.cta0[ri]) * (2 * C);
+  const int L = d.L, half = L / 2 + 1;
   c64* W = reinterpret_cast<c64*>(smem_raw);
-  c64* buf = W + (L / 2 > 0 ? L / 2 : 1);
-  load_tw<double>(W, twm, twmax, L, L / 2);
-  if (axis == 2) {
-    // TZ pencils: rows of length Lz
-    const size_t row0 = (size_t)blockIdx.x * TZ;
-    const size_t nrows = (size_t)Lx * Ly;
-    const int sst = L + 1;
-    for (int p = threadIdx.x; p < TZ * L; p += blockDim.x) {
-      const int rr = p / L, z = p - rr * L;
-      buf[rr * sst + z] = (row0 + rr < nrows) ? data[(row0 + rr) * L + z] : mk<double>(0, 0);
+  c64* buf = W + L;
+  load_twiddles<double>(W, twm, twmax, L);
+  auto in = [&](int64_t l, int t) -> double {  // entry t of line l
+    if (l >= lines) return 0.0;
+    if (AX == 0) {
+      const int uz = (int)(l / Uy), uy = (int)(l % Uy);
+      const int tz = R.ax[2].s == 2 ? 2 * uz + 1 : uz, ty = R.ax[1].s == 2 ? 2 * uy + 1 : uy;
+      return R.row[((size_t)tz * R.ax[1].M + ty) * d.M + t];
     }
+    const int u = d.s == 2 ? t >> 1 : t;
+    if (AX == 1) return R.A[((l / ox) * Uy + u) * ox + l % ox];
+    return R.B[(int64_t)u * oy * ox + l];
+  };
+  // the lanes run along the axis where that is contiguous, else along the lines
+  for (int q = threadIdx.x; q < L << LC; q += blockDim.x) {
+    const int j = AX == 0 ? q & (L - 1) : q >> LC, col = AX == 0 ? q >> d.n : q & (C - 1);
+    const int t = embed_index(j, d);
+    c64 v = mk<double>(0, 0);
+    if (t >= 0) v = mk<double>(in(l0 + 2 * col, t), in(l0 + 2 * col + 1, t));
+    buf[j * RS + col] = v;
+  }
+  __syncthreads();
+  for (int s = 0; s < d.n;) {
+    const int q = min(3, d.n - s);
+    smem_group_q<double, false, LC>(buf, RS, q, d.n, s, W);
+    s += q;
     __syncthreads();
-    block_fft<double, false, false>(buf, TZ, sst, 1, logL, W);
-    for (int p = threadIdx.x; p < TZ * L; p += blockDim.x) {
-      const int rr = p / L, z = p - rr * L;
-      if (row0 + rr < nrows) data[(row0 + rr) * L + z] = buf[rr * sst + z];
+  }
+  for (int q = threadIdx.x; q < half << LC; q += blockDim.x) {
+    const int f = AX == 0 ? q % half : q >> LC, col = AX == 0 ? q / half : q & (C - 1);
+    c64 v = buf[(d.n ? brev(f & (L - 1), d.n) : 0) * RS + col];
+    if (d.c) {
+      double sn, cs;
+      sincospi((double)d.c * f / L, &sn, &cs);
+      v = mk<double>(v.x * cs - v.y * sn, v.x * sn + v.y * cs);
     }
-  } else {
-    // pencils along x or y: take TZ consecutive z at fixed (other index)
-    const int nzb = (Lz + TZ - 1) / TZ;
-    const int zb = blockIdx.x % nzb;
-    const int other = blockIdx.x / nzb;  // y (axis 0) or x (axis 1)
-    const size_t stride = axis == 0 ? (size_t)Ly * Lz : (size_t)Lz;
-    const size_t base = axis == 0 ? (size_t)other * Lz : (size_t)other * Ly * Lz;
-    for (int p = threadIdx.x; p < TZ * L; p += blockDim.x) {
-      const int j = p / TZ, zz = p - j * TZ;
-      const int z = zb * TZ + zz;
-      buf[zz + j * TZ] = (z < Lz) ? data[base + j * stride + z] : mk<double>(0, 0);
-    }
-    __syncthreads();
-    block_fft<double, false, true>(buf, TZ, 1, TZ, logL, W);
-    for (int p = threadIdx.x; p < TZ * L; p += blockDim.x) {
-      const int j = p / TZ, zz = p - j * TZ;
-      const int z = zb * TZ + zz;
-      if (z < Lz) data[base + j * stride + z] = buf[zz + j * TZ];
+    if (AX == 2) v = cscale(v, R.scale);
+    double* out = AX == 0 ? R.A : (AX == 1 ? R.B : R.oct);
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int64_t l = l0 + 2 * col + h;
+      if (l >= lines) break;
+      int64_t at;
+      if (AX == 0) at = l * ox + f;
+      else if (AX == 1) at = ((l / ox) * oy + f) * ox + l % ox;
+      else at = ((l / ox) * oz + f) * ox + l % ox;
+      out[at] = h ? v.y : v.x;
     }
   }
 }
 
-// full (x,y,z; z fastest) -> stored (ky, kz, kx; kx fastest), scaled, real part only for
-// symmetric kernels, FP64 and FP32 copies
-__global__ void k_spec_store(const c64* __restrict__ full, void* d64, void* d32, int Lx, int Ly,
-                             int Lz, int is_complex, double scale) {
-  const size_t n = (size_t)Lx * Ly * Lz;
-  for (size_t o = blockIdx.x * (size_t)blockDim.x + threadIdx.x; o < n;
-       o += (size_t)gridDim.x * blockDim.x) {
-    const int kx = (int)(o % Lx);
-    const size_t r = o / Lx;
-    const int kz = (int)(r % Lz), ky = (int)(r / Lz);
-    const c64 v = full[((size_t)kx * Ly + ky) * Lz + kz];
-    if (is_complex) {
-      reinterpret_cast<c64*>(d64)[o] = mk<double>(v.x * scale, v.y * scale);
-      reinterpret_cast<c32*>(d32)[o] = mk<float>((float)(v.x * scale), (float)(v.y * scale));
-    } else {
-      reinterpret_cast<double*>(d64)[o] = v.x * scale;
-      reinterpret_cast<float*>(d32)[o] = (float)(v.x * scale);
-    }
-  }
-}
-
-// full (x,y,z; z fastest, DIF bit-reversed positions along each axis) -> octant R of the
-// half-sample-shift form (see Spectrum), scaled, FP64
-__global__ void k_spec_octant(const c64* __restrict__ full, double* o64, int Lx, int Ly, int Lz,
-                              int cx, int cy, int cz, double scale) {
-  const int ox = Lx / 2 + 1, oy = Ly / 2 + 1, oz = Lz / 2 + 1;
+// octant R -> the full form (ky, kz, kx) in the transforms' position order, kx fastest: R
+// itself for symmetric kernels, R prod_a E_a (shift +1) or conj(E_a) (shift -1) for the cross
+// blocks, E the phase tables of the face grid; FP64 and FP32
+__global__ void k_spec_full(const double* __restrict__ oct, void* d64, void* d32, int Lx, int Ly,
+                            int Lz, int cx_, int cy_, int cz_, const c64* __restrict__ ex,
+                            const c64* __restrict__ ey, const c64* __restrict__ ez,
+                            int is_complex) {
   const int nx = ilog2(Lx), ny = ilog2(Ly), nz = ilog2(Lz);
-  const size_t n = (size_t)ox * oy * oz;
+  const int ox = Lx / 2 + 1, oz = Lz / 2 + 1;
+  const size_t n = (size_t)Lx * Ly * Lz;
+  auto fold = [](int p, int n_) {
+    const int k = n_ ? (int)(__brev((unsigned)p) >> (32 - n_)) : 0, L = 1 << n_;
+    return k <= (L >> 1) ? k : L - k;
+  };
   for (size_t o = blockIdx.x * (size_t)blockDim.x + threadIdx.x; o < n;
        o += (size_t)gridDim.x * blockDim.x) {
-    const int fx = (int)(o % ox);
-    const size_t rr = o / ox;
-    const int fz = (int)(rr % oz), fy = (int)(rr / oz);
-    const int px = brev(fx & (Lx - 1), nx), py = brev(fy & (Ly - 1), ny),
-              pz = brev(fz & (Lz - 1), nz);
-    const c64 v = full[((size_t)px * Ly + py) * Lz + pz];
-    // R = Re(S * prod exp(+i*pi*c*f/L)); the phase angle sum is exact in double
-    double ph = 0.0;
-    if (cx) ph += (double)cx * fx / Lx;
-    if (cy) ph += (double)cy * fy / Ly;
-    if (cz) ph += (double)cz * fz / Lz;
-    double sn, cs;
-    sincospi(ph, &sn, &cs);
-    o64[o] = (v.x * cs - v.y * sn) * scale;
+    const int px = (int)(o & (Lx - 1)), pz = (int)((o >> nx) & (Lz - 1)), py = (int)(o >> (nx + nz));
+    const double r = oct[((size_t)fold(py, ny) * oz + fold(pz, nz)) * ox + fold(px, nx)];
+    if (is_complex) {
+      c64 f = mk<double>(r, 0);
+      if (cx_) f = cx_ > 0 ? f * ex[px] : cmulc(f, ex[px]);
+      if (cy_) f = cy_ > 0 ? f * ey[py] : cmulc(f, ey[py]);
+      if (cz_) f = cz_ > 0 ? f * ez[pz] : cmulc(f, ez[pz]);
+      reinterpret_cast<c64*>(d64)[o] = f;
+      reinterpret_cast<c32*>(d32)[o] = ccast<float>(f);
+    } else {
+      reinterpret_cast<double*>(d64)[o] = r;
+      reinterpret_cast<float*>(d32)[o] = (float)r;
+    }
   }
 }
 
@@ -262,50 +275,99 @@ int phase_tables(const int L[3], void* e64[3], void* e32[3], cudaStream_t st) {
   return 0;
 }
 
-int spectrum_build(Spectrum& S, const double* d_row, const int M[3], const int na[3],
-                   const int nb[3], const int sdim[3], const int odim[3], int symmetric,
-                   const void* tw64, int twmax, cudaStream_t st) {
-  // the kernel embedding of a generating row at S.L, forward-transformed in place
-  const size_t n = (size_t)S.L[0] * S.L[1] * S.L[2];
-  c64* full = nullptr;
-  PEEC_CUDA_TRY(cudaMallocAsync(&full, n * sizeof(c64), st));
-  EmbedDim d[3];
-  for (int i = 0; i < 3; ++i) d[i] = EmbedDim{S.L[i], na[i], nb[i], sdim[i], odim[i], M[i]};
-  k_embed<<<1184, 256, 0, st>>>(d_row, full, d[0], d[1], d[2]);
-  const c64* tw = reinterpret_cast<const c64*>(tw64);
-  constexpr int TZ = 8;
-  for (int axis = 2; axis >= 0; --axis) {
-    const int L = S.L[axis];
-    const int logL = ilog2(L);
-    if (logL == 0) continue;
-    size_t sm = sizeof(c64) * ((L / 2) + (size_t)TZ * (L + 1));
-    unsigned grid = axis == 2 ? (unsigned)((S.L[0] * (size_t)S.L[1] + TZ - 1) / TZ)
-                              : (unsigned)(((S.L[2] + TZ - 1) / TZ) * (axis == 0 ? S.L[1] : S.L[0]));
-    if (sm > 48 * 1024)
-      PEEC_CUDA_TRY(cudaFuncSetAttribute(k_fft_axis<TZ>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)sm));
-    k_fft_axis<TZ><<<grid, 256, sm, st>>>(full, S.L[0], S.L[1], S.L[2], axis, logL, tw, twmax);
+template <int AX, int LC>
+static int spec_pass(SpecSet& S, int ctas, const c64* tw, int twmax, cudaStream_t st) {
+  size_t sm = 0;
+  for (int i = 0; i < S.n; ++i)
+    sm = std::max(sm, sizeof(c64) * (size_t)S.r[i].ax[AX].L * ((1 << LC) + 2));
+  if (sm > 48 * 1024)
+    PEEC_CUDA_TRY(cudaFuncSetAttribute(k_spec_pass<AX, LC>,
+                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+  k_spec_pass<AX, LC><<<ctas, 256, sm, st>>>(S, tw, twmax);
+  return 0;
+}
+
+template <int AX>
+static int spec_axis(SpecSet& S, const c64* tw, int twmax, cudaStream_t st) {
+  int Lmax = 1;
+  for (int i = 0; i < S.n; ++i) Lmax = std::max(Lmax, S.r[i].ax[AX].L);
+  // pairs of lines per CTA: sixteen while the tile leaves room for two CTAs per SM
+  int lc = 4;
+  while (lc > 0 && sizeof(c64) * (size_t)Lmax * ((1 << lc) + 2) > 110 * 1024) lc -= 2;
+  int ctas = 0;
+  for (int i = 0; i < S.n; ++i) {
+    const SpecRow& R = S.r[i];
+    const int64_t ox = R.ax[0].L / 2 + 1, oy = R.ax[1].L / 2 + 1;
+    const int64_t lines = AX == 0 ? (int64_t)R.ax[2].U * R.ax[1].U
+                                  : (AX == 1 ? R.ax[2].U * ox : oy * ox);
+    S.cta0[i] = ctas;
+    ctas += (int)((lines + (2 << lc) - 1) / (2 << lc));
   }
-  // half-sample shift per axis: |2e + o| is even about e = -o/2 (the embedding window is
-  // symmetric about the same point because na - nb = -o there)
-  for (int a = 0; a < 3; ++a) S.c[a] = (!symmetric && sdim[a] == 2) ? -odim[a] : 0;
-  S.is_complex = symmetric ? 0 : 1;
-  const size_t es64 = S.is_complex ? sizeof(c64) : sizeof(double);
-  const size_t es32 = S.is_complex ? sizeof(c32) : sizeof(float);
-  if (!S.d[0]) PEEC_CUDA_TRY(cudaMalloc(&S.d[0], n * es64));
-  if (!S.d[1]) PEEC_CUDA_TRY(cudaMalloc(&S.d[1], n * es32));
-  k_spec_store<<<1184, 256, 0, st>>>(full, S.d[0], S.d[1], S.L[0], S.L[1], S.L[2], S.is_complex,
-                                     1.0 / (double)n);
-  const size_t no = (size_t)(S.L[0] / 2 + 1) * (S.L[1] / 2 + 1) * (S.L[2] / 2 + 1);
-  if (!S.oct) PEEC_CUDA_TRY(cudaMalloc(&S.oct, no * sizeof(double)));
-  k_spec_octant<<<1184, 256, 0, st>>>(full, (double*)S.oct, S.L[0], S.L[1], S.L[2], S.c[0],
-                                      S.c[1], S.c[2], 1.0 / (double)n);
-  const size_t ny32 = (size_t)S.L[0] * (S.L[1] / 2 + 1) * (S.L[2] / 2 + 1);
-  if (!S.yz32) PEEC_CUDA_TRY(cudaMalloc(&S.yz32, ny32 * sizeof(float)));
-  k_spec_yzfold<<<1184, 256, 0, st>>>((const double*)S.oct, (float*)S.yz32, S.L[0], S.L[1],
-                                      S.L[2]);
+  S.cta0[S.n] = ctas;
+  if (lc == 4) return spec_pass<AX, 4>(S, ctas, tw, twmax, st);
+  if (lc == 2) return spec_pass<AX, 2>(S, ctas, tw, twmax, st);
+  return spec_pass<AX, 0>(S, ctas, tw, twmax, st);
+}
+
+int spectra_build(const SpecJob* jobs, int njobs, const void* tw64, int twmax,
+                  const void* const ph[3], cudaStream_t st) {
+  if (njobs <= 0) return 0;
+  if (njobs > kSpecRows) return set_error("too many spectra"), PEEC_ERR_UNSUPPORTED_INTERNAL;
+  SpecSet set{};
+  set.n = njobs;
+  size_t na = 0, nb = 0;
+  for (int i = 0; i < njobs; ++i) {
+    const SpecJob& J = jobs[i];
+    Spectrum& S = *J.S;
+    SpecRow& R = set.r[i];
+    for (int a = 0; a < 3; ++a) {
+      // half-sample shift per axis: |2e + o| is even about e = -o/2 (the embedding window is
+      // symmetric about the same point because na - nb = -o there)
+      S.c[a] = (!J.symmetric && J.sdim[a] == 2) ? -J.odim[a] : 0;
+      R.ax[a] = SpecAxis{S.L[a], ilog2(S.L[a]), J.na[a], J.nb[a], J.sdim[a], J.odim[a], S.c[a],
+                         J.M[a], J.sdim[a] == 2 ? J.M[a] / 2 : J.M[a]};
+    }
+    S.is_complex = J.symmetric ? 0 : 1;
+    const size_t n = (size_t)S.L[0] * S.L[1] * S.L[2];
+    if (!S.d[0]) PEEC_CUDA_TRY(cudaMalloc(&S.d[0], n * (S.is_complex ? sizeof(c64) : sizeof(double))));
+    if (!S.d[1]) PEEC_CUDA_TRY(cudaMalloc(&S.d[1], n * (S.is_complex ? sizeof(c32) : sizeof(float))));
+    const size_t no = (size_t)(S.L[0] / 2 + 1) * (S.L[1] / 2 + 1) * (S.L[2] / 2 + 1);
+    if (!S.oct) PEEC_CUDA_TRY(cudaMalloc(&S.oct, no * sizeof(double)));
+    const size_t ny32 = (size_t)S.L[0] * (S.L[1] / 2 + 1) * (S.L[2] / 2 + 1);
+    if (!S.yz32) PEEC_CUDA_TRY(cudaMalloc(&S.yz32, ny32 * sizeof(float)));
+    R.row = J.row;
+    R.oct = (double*)S.oct;
+    R.scale = 1.0 / (double)n;
+    na += (size_t)R.ax[2].U * R.ax[1].U * (S.L[0] / 2 + 1);
+    nb += (size_t)R.ax[2].U * (S.L[1] / 2 + 1) * (S.L[0] / 2 + 1);
+  }
+  double* scr = nullptr;
+  PEEC_CUDA_TRY(cudaMallocAsync(&scr, (na + nb + 1) * sizeof(double), st));
+  size_t oa = 0, ob = na;
+  for (int i = 0; i < njobs; ++i) {
+    SpecRow& R = set.r[i];
+    R.A = scr + oa;
+    R.B = scr + ob;
+    oa += (size_t)R.ax[2].U * R.ax[1].U * (R.ax[0].L / 2 + 1);
+    ob += (size_t)R.ax[2].U * (R.ax[1].L / 2 + 1) * (R.ax[0].L / 2 + 1);
+  }
+  const c64* tw = reinterpret_cast<const c64*>(tw64);
+  CTX_CHECK(spec_axis<0>(set, tw, twmax, st));
+  CTX_CHECK(spec_axis<1>(set, tw, twmax, st));
+  CTX_CHECK(spec_axis<2>(set, tw, twmax, st));
+  for (int i = 0; i < njobs; ++i) {
+    Spectrum& S = *jobs[i].S;
+    const size_t n = (size_t)S.L[0] * S.L[1] * S.L[2];
+    const unsigned grid = (unsigned)std::min<size_t>((n + 255) / 256, 152 * 16);
+    k_spec_full<<<grid, 256, 0, st>>>((const double*)S.oct, S.d[0], S.d[1], S.L[0], S.L[1], S.L[2],
+                                      S.c[0], S.c[1], S.c[2], (const c64*)ph[0], (const c64*)ph[1],
+                                      (const c64*)ph[2], S.is_complex);
+    const size_t ny32 = (size_t)S.L[0] * (S.L[1] / 2 + 1) * (S.L[2] / 2 + 1);
+    k_spec_yzfold<<<(unsigned)std::min<size_t>((ny32 + 255) / 256, 152 * 16), 256, 0, st>>>(
+        (const double*)S.oct, (float*)S.yz32, S.L[0], S.L[1], S.L[2]);
+  }
   PEEC_CUDA_TRY(cudaGetLastError());
-  PEEC_CUDA_TRY(cudaFreeAsync(full, st));
+  PEEC_CUDA_TRY(cudaFreeAsync(scr, st));
   return 0;
 }
 
