@@ -177,7 +177,7 @@ class Clocks:
                 "samples": len(rows)}
 
 
-def conv_bytes(info, prec, staged=None):
+def conv_bytes(info, prec):
     """Algorithmic bytes of the convolution passes per operator application: every
     per-family intermediate written once and read once by the next pass, each
     spectrum read once, lattice maps (int32) once, compact vectors (complex128) read
@@ -201,13 +201,11 @@ def conv_bytes(info, prec, staged=None):
         b["z"] += 2 * t_y
         b["yinv"] += t_y + t_x
         b["xinv"] += t_x + cells * 4 + cells * 16
-        G = Lx * Ly * Lz
-        folded = Lx * (Ly // 2 + 1) * (Lz // 2 + 1) * 4
-        if prec == 1 and staged["edges" if f["edge"] else "faces"]:
-            b["z"] += folded if f["edge"] else 2 * folded  # per face family: 2 of the 6 tables
-        else:
-            b["z"] += (G * c // 2) if f["edge"] else (G * c // 2 + G * c)  # per face family: 1 real + 1 complex
+        folded = Lx * (Ly // 2 + 1) * (Lz // 2 + 1) * c // 2
+        b["z"] += folded if f["edge"] else 2 * folded  # per face family: 2 of the 6 tables
     return b
+
+
 def reference_model_bytes(grid, c):
     """Bytes per operator application under the pruned three-pass pencil model counted at
     the reference's own circulant extents (4.25 complex elements per padded point per
@@ -229,10 +227,10 @@ def conv_gbs(b, prof):
 
 
 # the FP32 z-pass kernels of each tuner form
-ZKERNEL = {"face": {"direct": "k_zconv3<float>", "direct_yz": "k_zconv3_yz",
-                    "staged": "k_zconv3_staged"},
-           "edge": {"direct": "k_zconv1<float> x3", "direct_yz": "k_zconv1_yz x3",
-                    "staged": "k_zedge_staged"}}
+ZKERNEL = {"face": {"direct": "k_zconv3<float>", "direct_yz": "k_zconv3<float>",
+                    "staged": "k_zconv3_staged", "pair": "k_zpair<float>"},
+           "edge": {"direct": "k_zconv1<float> x3", "direct_yz": "k_zconv1<float> x3",
+                    "staged": "k_zedge_staged", "pair": "k_zpair<float>"}}
 
 
 def z_traffic(grid, tuning):
@@ -971,8 +969,7 @@ def main():
     prof64 = op.profile_matvec(0, max(3, args.profile_iters // 4))
     profff = op.profile_matvec(2, max(3, args.profile_iters // 4))
     tuning = op.zpass_tuning()
-    staged = {"faces": tuning["face"] != "direct", "edges": tuning["edge"] != "direct"}
-    b32, b64 = conv_bytes(info, 1, staged), conv_bytes(info, 0)
+    b32, b64 = conv_bytes(info, 1), conv_bytes(info, 0)
     peak, peak_kind = load_peaks()
     if args.profile_only:
         # operator applications only (a few hundred launches): the command ncu captures run
@@ -1184,7 +1181,7 @@ def main():
                      "peak_kind": peak_kind, "unit": "GB/s",
                      "frac": b32["z"] / (prof32["z"] * 1e-3) / 1e9 / peak,
                      "traffic": z_traffic(P["grid"], tuning), "bytes_per_matvec": b32["z"],
-                     "launches_per_matvec": 2 if tuning["edge"] == "staged" else 4},
+                     "launches_per_matvec": 4 if tuning["edge"].startswith("direct") else 2},
     }
     line["fill"] = fill_report(P, rank == 0 and ws == 1 and not args.no_cpu_baseline)
     if rank == 0 and ws == 1 and not args.no_cpu_baseline:

@@ -186,7 +186,7 @@ struct peec_ctx {
   int32_t *ne_ptr = nullptr, *ne_idx = nullptr, *nsn_ptr = nullptr, *nsn_idx = nullptr;
   Family fam[6];
   Spectrum spec[9];
-  void* ph64[3] = {nullptr, nullptr, nullptr};  // face-grid phase tables (octant spectra)
+  void* ph64[3] = {nullptr, nullptr, nullptr};  // face-grid phase tables
   void* ph32[3] = {nullptr, nullptr, nullptr};  // their FP32 rounding (FP32 z passes)
   int* zerr = nullptr;  // set by a staged z pass whose copy wait ran into its limit
   int nsm = 0;          // SM count of the device
@@ -507,9 +507,7 @@ extern "C" void peec_ctx_destroy(peec_ctx* ctx) {
     for (int i = 0; i < 9; ++i) {
       Spectrum& s = set[i];
       for (int p = 0; p < 2; ++p)
-        if (s.d[p]) cudaFree(s.d[p]);
-      if (s.oct) cudaFree(s.oct);
-      if (s.yz32) cudaFree(s.yz32);
+        if (s.yz[p]) cudaFree(s.yz[p]);
     }
   for (int a = 0; a < 3; ++a) {
     if (ctx->ph64[a]) cudaFree(ctx->ph64[a]);
@@ -745,13 +743,9 @@ static int peec_set_topology_body(peec_ctx* ctx, int Nx, int Ny, int Nz, int64_t
     for (int i = 0; i < 9; ++i) {
       Spectrum& sp = set[i];
       for (int p = 0; p < 2; ++p) {
-        if (sp.d[p]) cudaFree(sp.d[p]);
-        sp.d[p] = nullptr;
+        if (sp.yz[p]) cudaFree(sp.yz[p]);
+        sp.yz[p] = nullptr;
       }
-      if (sp.oct) cudaFree(sp.oct);
-      sp.oct = nullptr;
-      if (sp.yz32) cudaFree(sp.yz32);
-      sp.yz32 = nullptr;
       std::memcpy(sp.L, i < 6 ? LP : ctx->fam[i - 3].L, sizeof(LP));
     }
   for (double*& p : ctx->rcc_qs) {
@@ -1162,6 +1156,12 @@ static int tune_zpass(peec_ctx* ctx) {
       CTX_TRY(timed(z, 0, &c.fms[form]));
       if (c.fms[form] < c.fms[c.face]) c.face = form;
     }
+    if (zpair_ok(ctx->fam[0])) {
+      double ms = 0;
+      z.face = 3;
+      CTX_TRY(timed(z, 0, &ms));
+      if (ms < c.fms[c.face]) c.face = 3;
+    }
   }
   if (edges) {
     const int nform = zpass_yz_edges(ctx->fam, 6) ? 3 : 1;
@@ -1179,6 +1179,11 @@ static int tune_zpass(peec_ctx* ctx) {
         }
       }
     }
+    double ms = 0;
+    z.edge = 3;
+    z.edge_plan = c.plan;
+    CTX_TRY(timed(z, 1, &ms));
+    if (ms < best) c.edge = 3;
   }
   CTX_TRY(check_solve_errors(ctx));
   {
@@ -1209,8 +1214,8 @@ static int build_spectrum_set(peec_ctx* ctx, Spectrum* dst, double* const d_rows
     jobs[nj++] = SpecJob{&dst[i], d_rows[srow[i]], ctx->row_dims[srow[i]], ctx->fam[fout[i]].dims,
                          ctx->fam[fin[i]].dims, sdim[i], odim[i], sym ? 1 : 0};
   }
-  CTX_TRY(spectra_build(jobs, nj, ctx->tw64, ctx->twmax, ctx->ph64, ctx->st));
-  ctx->launches += nj ? 3 + 2 * nj : 0;
+  CTX_TRY(spectra_build(jobs, nj, ctx->tw64, ctx->twmax, ctx->st));
+  ctx->launches += nj ? 3 + nj : 0;
   return PEEC_OK;
 }
 
@@ -2350,10 +2355,7 @@ static int matvec_enqueue(peec_ctx* ctx, const c64* x, c64* y, int prec, bool ev
   // one launch per x / y pass over all families, the shared z pass of the face
   // families, and the edge families' z passes: one launch over all of them in the staged
   // FP32 form (ZTune form 2), else one per family
-  int nedge = 0;
-  for (const auto& F : ctx->fam) nedge += (F.active && F.lp) ? 1 : 0;
-  const bool edge_one = prec == PEEC_PREC_FP32 && ctx->zt.edge == 2 && zpass_yz_edges(ctx->fam, 6);
-  ctx->launches += (5 + (edge_one ? (nedge > 0) : nedge)) * (ctx->rcc ? 2 : 1);
+  ctx->launches += (5 + zedge_launches(ctx->fam, 6, prec, ctx->zt)) * (ctx->rcc ? 2 : 1);
   if (events) cudaEventRecord(ctx->ev[1], st);
   sparse_enqueue(ctx, x, y, ctx->LpI, ctx->PQ);
   if (events) cudaEventRecord(ctx->ev[2], st);
@@ -2430,8 +2432,8 @@ extern "C" int peec_conv_count(const peec_ctx* ctx) { return ctx ? 6 : 0; }
 
 extern "C" int peec_set_zpass_forms(peec_ctx* ctx, int face, int edge, int edge_plan) {
   if (!ctx) return badarg(__func__);
-  if (face < 0 || face > 2 || edge < 0 || edge > 2 || edge_plan < 0 || edge_plan > 1)
-    return bad(ctx, PEEC_ERR_BADARG, "z-pass forms are 0..2 and edge plans 0..1");
+  if (face < 0 || face > 3 || edge < 0 || edge > 3 || edge_plan < 0 || edge_plan > 1)
+    return bad(ctx, PEEC_ERR_BADARG, "z-pass forms are 0..3 and edge plans 0..1");
   drop_graphs(ctx);
   ctx->zt.face = face;
   ctx->zt.edge = edge;
@@ -2443,8 +2445,11 @@ extern "C" int peec_zpass_tuning(const peec_ctx* ctx, int choice[3], double face
                                  double edge_ms[6]) {
   if (!ctx) return badarg(__func__);
   if (choice) {
-    choice[0] = zpass_yz_faces(ctx->fam, 6) ? ctx->zt.face : 0;
-    choice[1] = zpass_yz_edges(ctx->fam, 6) ? ctx->zt.edge : 0;
+    const bool pf = ctx->zt.face == 3 ? zpair_ok(ctx->fam[0]) : zpass_yz_faces(ctx->fam, 6);
+    bool pe = ctx->zt.edge == 3 ? false : zpass_yz_edges(ctx->fam, 6);
+    for (int f = 3; f < 6 && ctx->zt.edge == 3; ++f) pe |= zpair_ok(ctx->fam[f]);
+    choice[0] = pf ? ctx->zt.face : 0;
+    choice[1] = pe ? ctx->zt.edge : 0;
     choice[2] = ctx->zt.edge_plan;
   }
   if (face_ms) std::memcpy(face_ms, ctx->zface_ms, sizeof(ctx->zface_ms));

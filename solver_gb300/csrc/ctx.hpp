@@ -167,27 +167,17 @@ struct Family {
   void* T[2] = {nullptr, nullptr};  // work buffer per precision: [z < dims[2]][y < Ly][kx < Lx]
 };
 
-// A block spectrum, scaled by 1/(Lx*Ly*Lz), in two forms.
-// Full: every position, layout (ky, kz, kx), kx fastest, in the transforms' bit-reversed
-//   position order; real for symmetric kernels; FP64 and FP32 copies (coalesced reads for
-//   the FP32 and FP64 passes).
-// Octant: along each axis the kernel is even (c = 0) or even about a half-sample shift
-//   (c = +-1), so S(k) = R(|k_x|, |k_y|, |k_z|) * prod_a exp(-i*pi*c_a*k_a/L_a) with
-//   k_a in (-L_a/2, L_a/2] and R real; the (L_x/2+1)(L_y/2+1)(L_z/2+1) values of R are kept
-//   in FP64, layout (fy, fz, fx), fx fastest. The float-float passes read this form: an
-//   eighth (a sixteenth for cross blocks) of the FP64 bytes.
-// y/z-folded FP32 form (the FP32 z passes): R at the folded y and z frequencies but at
-//   every x position, layout (fy, fz, px), px the DIF position, so a z-pass tile's 16
-//   consecutive columns read 64 contiguous bytes; Lx(Ly/2+1)(Lz/2+1) floats, about a
-//   quarter of the full FP32 form. Cross blocks take their half-sample phases at run time
-//   from the FP32 phase tables.
+// A block spectrum, scaled by 1/(Lx*Ly*Lz). Along each axis the kernel is even (c = 0) or even
+// about a half-sample shift (c = +-1), so S(k) = R(|k_x|, |k_y|, |k_z|) *
+// prod_a exp(-i*pi*c_a*k_a/L_a) with k_a in (-L_a/2, L_a/2] and R real. Kept y/z-folded: R at
+// the folded y and z frequencies but at every x position, layout (fy, fz, px), px the DIF
+// position, so that consecutive columns of a z pass read contiguous values;
+// Lx(Ly/2+1)(Lz/2+1) values in FP64 (FP64 and float-float passes) and FP32 (FP32 passes), a
+// quarter of the positions. Cross blocks take their phases from the phase tables.
 struct Spectrum {
   int L[3] = {1, 1, 1};
   int c[3] = {0, 0, 0};
-  int is_complex = 0;
-  void* d[2] = {nullptr, nullptr};  // full: [0] fp64, [1] fp32
-  void* oct = nullptr;              // octant R, fp64
-  void* yz32 = nullptr;             // y/z-folded R, fp32
+  void* yz[2] = {nullptr, nullptr};  // [0] fp64, [1] fp32
 };
 
 // Launchers (fftconv.cu). prec: 0 = fp64, 1 = fp32, 2 = float-float; tw[prec] the master
@@ -195,9 +185,9 @@ struct Spectrum {
 // 0..2 are the face families, 3..5 the edge families; spectra 0..5 = P blocks
 // (00, 11, 22, 01, 02, 12), 6..8 = Lp blocks of families 3..5.
 // FP32 z-pass forms, chosen per grid by measurement (tune_zpass in ctx.cu). Face / edge
-// form 0: register-direct kernels on the full-form spectra; 1: register-direct kernels on
-// the y/z-folded spectra; 2: staged kernels (persistent CTAs, bulk-copied tiles, y/z-folded
-// spectra; the edge families in one launch). edge_plan: the edge families' z radix plan
+// form 0 (and 1, kept as a name): register-direct kernels; 2: staged kernels (persistent CTAs,
+// bulk-copied tiles; the edge families in one launch); 3: pair kernels (half-length transforms
+// of the even and odd frequencies). edge_plan: the edge families' z radix plan of forms 0 to 2
 // (0: make_plan(n, 4, 4, 4), 1: make_plan(n, 4, 4, 3); 8 x 16 and 16 x 8 at Lz = 128).
 struct ZTune {
   int* err = nullptr;  // error word set by a staged kernel whose copy wait ran into its limit
@@ -220,6 +210,13 @@ int phase_tables(const int L[3], void* e64[3], void* e32[3], cudaStream_t st);
 // tiles, enough z points; the edge families on one shared grid)
 bool zpass_yz_faces(const Family* F, int nfam);
 bool zpass_yz_edges(const Family* F, int nfam);
+// launches of the edge families' z passes in a precision (0 fp64, 1 fp32, 2 float-float)
+int zedge_launches(const Family* F, int nfam, int prec, const ZTune& zt);
+// z extents the pair passes take: a circulant of 2 to 128 points (half of it in registers)
+inline bool zpair_ok(const Family& f) {
+  return f.active && f.L[2] >= 2 && f.L[2] <= 128 && f.dims[2] <= f.L[2] / 2 + 1 &&
+         (int64_t)f.L[0] * f.L[1] < ((int64_t)1 << 30);
+}
 // A spectrum to build from a generating row on the device: the row's extents, the output and
 // input family extents, stride and offset per axis (K(e) = row[|sdim e + odim|])
 struct SpecJob {
@@ -228,8 +225,6 @@ struct SpecJob {
   const int *M, *na, *nb, *sdim, *odim;
   int symmetric;
 };
-// ph: the face grid's FP64 phase tables (x, y, z)
-int spectra_build(const SpecJob* jobs, int njobs, const void* tw64, int twmax,
-                  const void* const ph[3], cudaStream_t st);
+int spectra_build(const SpecJob* jobs, int njobs, const void* tw64, int twmax, cudaStream_t st);
 
 }  // namespace peec

@@ -27,8 +27,7 @@
 // group, the spectral product and the first inverse group run back to back in
 // registers. Shared-memory tiles keep sequences contiguous (element (pos, seq) at
 // pos*rs + seq), so the middle groups are bank-conflict free.
-// Spectra carry the 1/(Lx*Ly*Lz) normalisation and are stored (ky, kz, kx), kx fastest,
-// in the transforms' bit-reversed position order.
+// Spectra carry the 1/(Lx*Ly*Lz) normalisation (Spectrum).
 #include <mutex>
 #include <set>
 #include <utility>
@@ -57,7 +56,7 @@ int conv_all(const Family* F, int nfam, const Spectrum* spec, const void* const*
   return conv_all_f32(F, nfam, spec, ph, x, LpI, PQ, m, tw[1], twmax, st, ev, zt);
 }
 
-// The y/z-folded and staged FP32 z passes need whole 16-column tiles (Lx a multiple of 16, so every
+// The staged FP32 z passes need whole 16-column tiles (Lx a multiple of 16, so every
 // staged row is 128 bytes at a 128-byte offset), at least two radix groups along z, and
 // tiles that fit three (faces) / one (edges) per shared-memory budget; the edge families
 // must share one circulant grid to share a launch.
@@ -85,6 +84,20 @@ bool zpass_yz_edges(const Family* F, int nfam) {
   return f0 != nullptr;
 }
 
+int zedge_launches(const Family* F, int nfam, int prec, const ZTune& zt) {
+  if (prec == 1 && zt.edge == 2 && zpass_yz_edges(F, nfam)) return 1;
+  const bool pair = prec == 2 || (prec == 1 && zt.edge == 3);
+  int n = 0;
+  for (int f = 3; f < nfam; ++f) {
+    if (!F[f].active) continue;
+    bool first = true;  // of the families that share a pair launch
+    for (int g = 3; g < f && pair && zpair_ok(F[f]); ++g)
+      first = first && !(zpair_ok(F[g]) && F[g].L[2] == F[f].L[2]);
+    n += first ? 1 : 0;
+  }
+  return n;
+}
+
 // --------------------------------------------------------------------------- spectra
 // The spectrum of a generating row: along each axis the embedded kernel
 // K(e) = row[|s e + o|] is even (s = 1, o = 0) or even about a half-sample shift
@@ -96,9 +109,8 @@ bool zpass_yz_edges(const Family* F, int nfam) {
 // one as the imaginary part: after the shift's phase they separate by themselves. An eighth
 // of the lines of the embedded complex transform, half of them again by the pairing; all
 // rows of a set share each pass's launch. FP64 pipe bound. Measured at 128x128x64 (nine
-// spectra): transforms 1.65 ms and the full forms 0.97 ms, against 13.3 and 1.3 ms as complex
-// transforms of the embedded kernels; a retarded frequency at 48x48x24 (eighteen spectra)
-// 0.40 against 3.2 ms.
+// spectra): 1.65 ms, against 13.3 ms as complex transforms of the embedded kernels; a retarded
+// frequency at 48x48x24 (eighteen spectra) 0.40 against 3.2 ms.
 // ------------------------------------------------------------------------------------
 
 struct SpecAxis {
@@ -200,51 +212,22 @@ __global__ void __launch_bounds__(256) k_spec_pass(SpecSet S, const c64* __restr
   }
 }
 
-// octant R -> the full form (ky, kz, kx) in the transforms' position order, kx fastest: R
-// itself for symmetric kernels, R prod_a E_a (shift +1) or conj(E_a) (shift -1) for the cross
-// blocks, E the phase tables of the face grid; FP64 and FP32
-__global__ void k_spec_full(const double* __restrict__ oct, void* d64, void* d32, int Lx, int Ly,
-                            int Lz, int cx_, int cy_, int cz_, const c64* __restrict__ ex,
-                            const c64* __restrict__ ey, const c64* __restrict__ ez,
-                            int is_complex) {
-  const int nx = ilog2(Lx), ny = ilog2(Ly), nz = ilog2(Lz);
-  const int ox = Lx / 2 + 1, oz = Lz / 2 + 1;
-  const size_t n = (size_t)Lx * Ly * Lz;
-  auto fold = [](int p, int n_) {
-    const int k = n_ ? (int)(__brev((unsigned)p) >> (32 - n_)) : 0, L = 1 << n_;
-    return k <= (L >> 1) ? k : L - k;
-  };
-  for (size_t o = blockIdx.x * (size_t)blockDim.x + threadIdx.x; o < n;
-       o += (size_t)gridDim.x * blockDim.x) {
-    const int px = (int)(o & (Lx - 1)), pz = (int)((o >> nx) & (Lz - 1)), py = (int)(o >> (nx + nz));
-    const double r = oct[((size_t)fold(py, ny) * oz + fold(pz, nz)) * ox + fold(px, nx)];
-    if (is_complex) {
-      c64 f = mk<double>(r, 0);
-      if (cx_) f = cx_ > 0 ? f * ex[px] : cmulc(f, ex[px]);
-      if (cy_) f = cy_ > 0 ? f * ey[py] : cmulc(f, ey[py]);
-      if (cz_) f = cz_ > 0 ? f * ez[pz] : cmulc(f, ez[pz]);
-      reinterpret_cast<c64*>(d64)[o] = f;
-      reinterpret_cast<c32*>(d32)[o] = ccast<float>(f);
-    } else {
-      reinterpret_cast<double*>(d64)[o] = r;
-      reinterpret_cast<float*>(d32)[o] = (float)r;
-    }
-  }
-}
-
-// octant R (FP64, (fy, fz, fx)) -> y/z-folded FP32 R ((fy, fz, px), px every DIF x position)
-__global__ void k_spec_yzfold(const double* __restrict__ o64, float* y32, int Lx, int Ly,
-                              int Lz) {
+// octant R (FP64, (fy, fz, fx)) -> the y/z-folded form ((fy, fz, px), px every DIF x position)
+// in FP64 and FP32
+__global__ void k_spec_yzfold(const double* __restrict__ o64, double* y64, float* y32, int Lx,
+                              int Ly, int Lz) {
   const int ox = Lx / 2 + 1, oy = Ly / 2 + 1, oz = Lz / 2 + 1;
   const int nx = ilog2(Lx);
   const size_t n = (size_t)Lx * oy * oz;
   for (size_t o = blockIdx.x * (size_t)blockDim.x + threadIdx.x; o < n;
        o += (size_t)gridDim.x * blockDim.x) {
-    const int px = (int)(o % Lx);
-    const size_t rr = o / Lx;  // fy * oz + fz
-    int k = brev(px, nx);
+    const int px = (int)(o & (Lx - 1));
+    const size_t rr = o >> nx;  // fy * oz + fz
+    const int k = nx ? (int)(__brev((unsigned)px) >> (32 - nx)) : 0;
     const int fx = k <= Lx / 2 ? k : Lx - k;
-    y32[o] = (float)o64[rr * ox + fx];
+    const double v = o64[rr * ox + fx];
+    y64[o] = v;
+    y32[o] = (float)v;
   }
 }
 
@@ -309,13 +292,12 @@ static int spec_axis(SpecSet& S, const c64* tw, int twmax, cudaStream_t st) {
   return spec_pass<AX, 0>(S, ctas, tw, twmax, st);
 }
 
-int spectra_build(const SpecJob* jobs, int njobs, const void* tw64, int twmax,
-                  const void* const ph[3], cudaStream_t st) {
+int spectra_build(const SpecJob* jobs, int njobs, const void* tw64, int twmax, cudaStream_t st) {
   if (njobs <= 0) return 0;
   if (njobs > kSpecRows) return set_error("too many spectra"), PEEC_ERR_UNSUPPORTED_INTERNAL;
   SpecSet set{};
   set.n = njobs;
-  size_t na = 0, nb = 0;
+  size_t na = 0, nb = 0, no = 0;
   for (int i = 0; i < njobs; ++i) {
     const SpecJob& J = jobs[i];
     Spectrum& S = *J.S;
@@ -327,29 +309,26 @@ int spectra_build(const SpecJob* jobs, int njobs, const void* tw64, int twmax,
       R.ax[a] = SpecAxis{S.L[a], ilog2(S.L[a]), J.na[a], J.nb[a], J.sdim[a], J.odim[a], S.c[a],
                          J.M[a], J.sdim[a] == 2 ? J.M[a] / 2 : J.M[a]};
     }
-    S.is_complex = J.symmetric ? 0 : 1;
-    const size_t n = (size_t)S.L[0] * S.L[1] * S.L[2];
-    if (!S.d[0]) PEEC_CUDA_TRY(cudaMalloc(&S.d[0], n * (S.is_complex ? sizeof(c64) : sizeof(double))));
-    if (!S.d[1]) PEEC_CUDA_TRY(cudaMalloc(&S.d[1], n * (S.is_complex ? sizeof(c32) : sizeof(float))));
-    const size_t no = (size_t)(S.L[0] / 2 + 1) * (S.L[1] / 2 + 1) * (S.L[2] / 2 + 1);
-    if (!S.oct) PEEC_CUDA_TRY(cudaMalloc(&S.oct, no * sizeof(double)));
-    const size_t ny32 = (size_t)S.L[0] * (S.L[1] / 2 + 1) * (S.L[2] / 2 + 1);
-    if (!S.yz32) PEEC_CUDA_TRY(cudaMalloc(&S.yz32, ny32 * sizeof(float)));
+    const size_t ny = (size_t)S.L[0] * (S.L[1] / 2 + 1) * (S.L[2] / 2 + 1);
+    if (!S.yz[0]) PEEC_CUDA_TRY(cudaMalloc(&S.yz[0], ny * sizeof(double)));
+    if (!S.yz[1]) PEEC_CUDA_TRY(cudaMalloc(&S.yz[1], ny * sizeof(float)));
     R.row = J.row;
-    R.oct = (double*)S.oct;
-    R.scale = 1.0 / (double)n;
+    R.scale = 1.0 / ((double)S.L[0] * S.L[1] * S.L[2]);
     na += (size_t)R.ax[2].U * R.ax[1].U * (S.L[0] / 2 + 1);
     nb += (size_t)R.ax[2].U * (S.L[1] / 2 + 1) * (S.L[0] / 2 + 1);
+    no += (size_t)(S.L[0] / 2 + 1) * (S.L[1] / 2 + 1) * (S.L[2] / 2 + 1);
   }
   double* scr = nullptr;
-  PEEC_CUDA_TRY(cudaMallocAsync(&scr, (na + nb + 1) * sizeof(double), st));
-  size_t oa = 0, ob = na;
+  PEEC_CUDA_TRY(cudaMallocAsync(&scr, (na + nb + no + 1) * sizeof(double), st));
+  size_t oa = 0, ob = na, oo = na + nb;
   for (int i = 0; i < njobs; ++i) {
     SpecRow& R = set.r[i];
     R.A = scr + oa;
     R.B = scr + ob;
+    R.oct = scr + oo;
     oa += (size_t)R.ax[2].U * R.ax[1].U * (R.ax[0].L / 2 + 1);
     ob += (size_t)R.ax[2].U * (R.ax[1].L / 2 + 1) * (R.ax[0].L / 2 + 1);
+    oo += (size_t)(R.ax[2].L / 2 + 1) * (R.ax[1].L / 2 + 1) * (R.ax[0].L / 2 + 1);
   }
   const c64* tw = reinterpret_cast<const c64*>(tw64);
   CTX_CHECK(spec_axis<0>(set, tw, twmax, st));
@@ -357,14 +336,9 @@ int spectra_build(const SpecJob* jobs, int njobs, const void* tw64, int twmax,
   CTX_CHECK(spec_axis<2>(set, tw, twmax, st));
   for (int i = 0; i < njobs; ++i) {
     Spectrum& S = *jobs[i].S;
-    const size_t n = (size_t)S.L[0] * S.L[1] * S.L[2];
-    const unsigned grid = (unsigned)std::min<size_t>((n + 255) / 256, 152 * 16);
-    k_spec_full<<<grid, 256, 0, st>>>((const double*)S.oct, S.d[0], S.d[1], S.L[0], S.L[1], S.L[2],
-                                      S.c[0], S.c[1], S.c[2], (const c64*)ph[0], (const c64*)ph[1],
-                                      (const c64*)ph[2], S.is_complex);
-    const size_t ny32 = (size_t)S.L[0] * (S.L[1] / 2 + 1) * (S.L[2] / 2 + 1);
-    k_spec_yzfold<<<(unsigned)std::min<size_t>((ny32 + 255) / 256, 152 * 16), 256, 0, st>>>(
-        (const double*)S.oct, (float*)S.yz32, S.L[0], S.L[1], S.L[2]);
+    const size_t ny = (size_t)S.L[0] * (S.L[1] / 2 + 1) * (S.L[2] / 2 + 1);
+    k_spec_yzfold<<<(unsigned)std::min<size_t>((ny + 255) / 256, 152 * 16), 256, 0, st>>>(
+        set.r[i].oct, (double*)S.yz[0], (float*)S.yz[1], S.L[0], S.L[1], S.L[2]);
   }
   PEEC_CUDA_TRY(cudaGetLastError());
   PEEC_CUDA_TRY(cudaFreeAsync(scr, st));

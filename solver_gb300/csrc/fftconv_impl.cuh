@@ -401,44 +401,20 @@ __global__ void __launch_bounds__(TPB) k_ypass(PassSet<R> s, const cx<R>* __rest
 
 // --------------------------------------------------------------------------- z passes
 
-// The six P spectra: full form (diagonal blocks real, cross blocks complex, in the pass's
-// storage precision) and octant form (real R, FP64) with the cross blocks' half-sample
-// shifts and the face grid's phase tables E_a[p] = exp(-i*pi*k/L_a), k the signed
-// frequency of position p. In octant form a cross spectrum is R times the product of
-// E_a (shift +1) or conj(E_a) (shift -1) over its shifted axes. The FP32 and FP64 passes
-// read the full form (coalesced); the float-float passes read the octant (an eighth of
-// the FP64 bytes, and FP32-pipe arithmetic for the phases).
+// The six P spectra (blocks 00, 11, 22, 01, 02, 12) in the y/z-folded form (Spectrum::yz) and
+// the face grid's phase tables E_a[p] = exp(-i*pi*k/L_a), k the signed frequency of position
+// p. The cross blocks' half-sample shifts pair up: block fg carries E of family f's axis
+// (y, x, z for f = 0, 1, 2) and conj(E) of family g's. FP32 passes read the FP32
+// tables, FP64 and float-float passes the FP64 ones.
 struct PSpec {
-  const void* f00;
-  const void* f11;
-  const void* f22;
-  const void* f01;
-  const void* f02;
-  const void* f12;
-  const void* o00;
-  const void* o11;
-  const void* o22;
-  const void* o01;
-  const void* o02;
-  const void* o12;
+  const void* y[6];
   const void* ex;
   const void* ey;
   const void* ez;
-  int c01[3], c02[3], c12[3];
-  // staged FP32 z pass: y/z-folded R (00, 11, 22, 01, 02, 12) and FP32 phase tables
-  const float* y[6];
-  const c32* ex32;
-  const c32* ey32;
-  const c32* ez32;
 };
 
-template <typename R>
-constexpr bool octant_spectra() {
-  return std::is_same<R, ff>::value;
-}
-
-// storage type of the spectra a pass of arithmetic type R reads: the float-float
-// passes split the FP64 spectra on load
+// storage type of the spectra and phase tables a pass of arithmetic type R reads: the
+// float-float passes split the FP64 ones on load
 template <typename R>
 struct SpecOf {
   using T = R;
@@ -460,99 +436,57 @@ __device__ __forceinline__ cx<R> spec_cx(const void* p, size_t i) {
 __device__ __forceinline__ int brevn(int v, int n) {
   return n ? (int)(__brev((unsigned)v) >> (32 - n)) : 0;
 }
-// octant index of the frequency at DIF position p of a length-2^n axis
+// folded frequency at DIF position p of a length-2^n axis
 __device__ __forceinline__ int fold_pos(int p, int n) {
   const int k = brevn(p, n), L = 1 << n;
   return k <= (L >> 1) ? k : L - k;
 }
 
-// Spectrum addressing of one z-pass CTA (fixed ky, kx tile). Full form: (ky, kz, kx0+col)
-// at sbase + kz*Lx + col. Octant form: entry (fy, fz, fx) at (fy*oz + fz)*ox + fx with
-// o_a = L_a/2 + 1.
-struct OctIdx {
-  size_t rowbase;  // fy * oz * ox
-  size_t sbase;    // ky * Lz * Lx + kx0
-  int Lx, ox, nx, nz, kx0;
+// spectrum index of a tile's column col at z position pz in the y/z-folded tables
+struct YzIdx {
+  size_t rowbase;  // fold(ky) * (Lz/2 + 1) * Lx + kx0
+  int Lx, nz;
   __device__ __forceinline__ size_t at(int col, int pz) const {
-    return rowbase + (size_t)fold_pos(pz, nz) * ox + fold_pos(kx0 + col, nx);
-  }
-  __device__ __forceinline__ size_t full(int col, int pz) const {
-    return sbase + (size_t)pz * Lx + col;
+    return rowbase + (size_t)fold_pos(pz, nz) * Lx + col;
   }
 };
 
-__device__ __forceinline__ OctIdx make_octidx(int Lx, int Ly, int Lz, int kx0, int ky) {
-  OctIdx o;
-  o.Lx = Lx;
-  o.nx = ilog2(Lx);
-  o.nz = ilog2(Lz);
-  o.ox = Lx / 2 + 1;
-  o.kx0 = kx0;
-  o.rowbase = (size_t)fold_pos(ky, ilog2(Ly)) * (Lz / 2 + 1) * o.ox;
-  o.sbase = (size_t)ky * Lz * Lx + kx0;
-  return o;
+__device__ __forceinline__ YzIdx make_yzidx(int Lx, int Ly, int Lz, int kx0, int ky) {
+  YzIdx y;
+  y.Lx = Lx;
+  y.nz = ilog2(Lz);
+  y.rowbase = (size_t)fold_pos(ky, ilog2(Ly)) * (Lz / 2 + 1) * Lx + kx0;
+  return y;
 }
 
+// The phases of a frequency relative to family 0: S_fg = phi_f conj(phi_g) R_fg with phi =
+// (E_y, E_x, E_z), so with psi_1 = E_x conj(E_y) (constant along a column) and psi_2 =
+// E_z conj(E_y) the product is psi_f sum_g R_fg conj(psi_g) X_g, R real and symmetric.
+// Y_f = sum_g S_fg X_g at the frequency of (column col, z position pz) of the CTA; p1 = psi_1,
+// ey the CTA's y phase
 template <typename R>
-__device__ __forceinline__ cx<R> shift_phase(const int c[3], const cx<R>& ex, const cx<R>& ey,
-                                             const cx<R>& ez) {
-  cx<R> f = mk<R>(1, 0);
-  if (c[0]) f = c[0] > 0 ? f * ex : cmulc(f, ex);
-  if (c[1]) f = c[1] > 0 ? f * ey : cmulc(f, ey);
-  if (c[2]) f = c[2] > 0 ? f * ez : cmulc(f, ez);
-  return f;
-}
-
-// Y_f = sum_g S_fg X_g with S_gf = conj(S_fg), at the frequency of (column col, z
-// position pz) of the CTA; ex / ey the CTA's x (per column) and y phases
-template <typename R>
-__device__ __forceinline__ void pspec_apply(const PSpec& S, const OctIdx& O, int col, int pz,
-                                            const cx<R>& ex, const cx<R>& ey, cx<R>& a0,
+__device__ __forceinline__ void pspec_apply(const PSpec& S, const YzIdx& Y, int col, int pz,
+                                            const cx<R>& p1, const cx<R>& ey, cx<R>& a0,
                                             cx<R>& a1, cx<R>& a2) {
-  cx<R> c01, c02, c12;
-  R d00, d11, d22;
-  if constexpr (octant_spectra<R>()) {
-    const size_t oi = O.at(col, pz);
-    const cx<R> ez = spec_cx<R>(S.ez, pz);
-    c01 = cscale(shift_phase<R>(S.c01, ex, ey, ez), spec_re<R>(S.o01, oi));
-    c02 = cscale(shift_phase<R>(S.c02, ex, ey, ez), spec_re<R>(S.o02, oi));
-    c12 = cscale(shift_phase<R>(S.c12, ex, ey, ez), spec_re<R>(S.o12, oi));
-    d00 = spec_re<R>(S.o00, oi);
-    d11 = spec_re<R>(S.o11, oi);
-    d22 = spec_re<R>(S.o22, oi);
-  } else {
-    const size_t si = O.full(col, pz);
-    c01 = spec_cx<R>(S.f01, si);
-    c02 = spec_cx<R>(S.f02, si);
-    c12 = spec_cx<R>(S.f12, si);
-    d00 = spec_re<R>(S.f00, si);
-    d11 = spec_re<R>(S.f11, si);
-    d22 = spec_re<R>(S.f22, si);
-  }
-  const cx<R> b0 = cscale(a0, d00) + c01 * a1 + c02 * a2;
-  const cx<R> b1 = cmulc(a0, c01) + cscale(a1, d11) + c12 * a2;
-  const cx<R> b2 = cmulc(a0, c02) + cmulc(a1, c12) + cscale(a2, d22);
-  a0 = b0;
-  a1 = b1;
-  a2 = b2;
-}
-
-// the x and y phases of a column / the CTA (octant form only)
-template <typename R>
-__device__ __forceinline__ cx<R> phase_at(const void* table, int p) {
-  if constexpr (octant_spectra<R>()) return spec_cx<R>(table, p);
-  else return mk<R>(1, 0);
+  const size_t i = Y.at(col, pz);
+  const cx<R> p2 = cmulc(spec_cx<R>(S.ez, pz), ey);
+  const R r00 = spec_re<R>(S.y[0], i), r11 = spec_re<R>(S.y[1], i), r22 = spec_re<R>(S.y[2], i);
+  const R r01 = spec_re<R>(S.y[3], i), r02 = spec_re<R>(S.y[4], i), r12 = spec_re<R>(S.y[5], i);
+  const cx<R> x0 = a0, x1 = cmulc(a1, p1), x2 = cmulc(a2, p2);
+  a0 = cscale(x0, r00) + cscale(x1, r01) + cscale(x2, r02);
+  a1 = (cscale(x0, r01) + cscale(x1, r11) + cscale(x2, r12)) * p1;
+  a2 = (cscale(x0, r02) + cscale(x1, r12) + cscale(x2, r22)) * p2;
 }
 
 // single-group z transform of all three face families in registers
 template <typename R, int Q>
 __device__ __forceinline__ void z3_single(cx<R>* T0, cx<R>* T1, cx<R>* T2, int nz0, int nz1,
                                           int nz2, size_t pl, int ncols, const PSpec& S,
-                                          const OctIdx& O, const cx<R>& ey) {
+                                          const YzIdx& O, int kx0, const cx<R>& ey) {
   constexpr int N = 1 << Q;
   for (int col = threadIdx.x; col < TX; col += blockDim.x) {
     if (col >= ncols) continue;
-    const cx<R> ex = phase_at<R>(S.ex, O.kx0 + col);
+    const cx<R> p1 = cmulc(spec_cx<R>(S.ex, kx0 + col), ey);
     cx<R> v[3][N];
 #pragma unroll
     for (int r = 0; r < N; ++r) {
@@ -563,7 +497,7 @@ __device__ __forceinline__ void z3_single(cx<R>* T0, cx<R>* T1, cx<R>* T2, int n
 #pragma unroll
     for (int f = 0; f < 3; ++f) dft_dif<R, Q>(v[f]);
 #pragma unroll
-    for (int r = 0; r < N; ++r) pspec_apply<R>(S, O, col, r, ex, ey, v[0][r], v[1][r], v[2][r]);
+    for (int r = 0; r < N; ++r) pspec_apply<R>(S, O, col, r, p1, ey, v[0][r], v[1][r], v[2][r]);
 #pragma unroll
     for (int f = 0; f < 3; ++f) dft_dit<R, Q>(v[f]);
 #pragma unroll
@@ -580,7 +514,7 @@ __device__ __forceinline__ void z3_single(cx<R>* T0, cx<R>* T1, cx<R>* T2, int n
 // buf + f*tsz)
 template <typename R, int Q>
 __device__ __forceinline__ void z3_fused(cx<R>* buf, size_t tsz, const AxPlan& p, int ncols,
-                                         const PSpec& S, const OctIdx& O, const cx<R>& ey) {
+                                         const PSpec& S, const YzIdx& O, int kx0, const cx<R>& ey) {
   constexpr int N = 1 << Q;
   const int tasks = TX << (p.n - Q);
   for (int t = threadIdx.x; t < tasks; t += blockDim.x) {
@@ -594,10 +528,10 @@ __device__ __forceinline__ void z3_fused(cx<R>* buf, size_t tsz, const AxPlan& p
       dft_dif<R, Q>(v[f]);
     }
     if (col < ncols) {
-      const cx<R> ex = phase_at<R>(S.ex, O.kx0 + col);
+      const cx<R> p1 = cmulc(spec_cx<R>(S.ex, kx0 + col), ey);
 #pragma unroll
       for (int r = 0; r < N; ++r)
-        pspec_apply<R>(S, O, col, start + r, ex, ey, v[0][r], v[1][r], v[2][r]);
+        pspec_apply<R>(S, O, col, start + r, p1, ey, v[0][r], v[1][r], v[2][r]);
     }
 #pragma unroll
     for (int f = 0; f < 3; ++f) {
@@ -634,13 +568,13 @@ __global__ void __launch_bounds__(ZTPB, 4) k_zconv3(cx<R>* T0, cx<R>* T1, cx<R>*
   T0 += off;
   T1 += off;
   T2 += off;
-  const OctIdx O = make_octidx(Lx, Ly, Lz, kx0, ky);
-  const cx<R> ey = phase_at<R>(S.ey, ky);
+  const YzIdx O = make_yzidx(Lx, Ly, Lz, kx0, ky);
+  const cx<R> ey = spec_cx<R>(S.ey, ky);
   load_twiddles<R>(W, twm, twmax, Lz);
   __syncthreads();
   if constexpr (Q0 == 0) {
     if (p.ng == 1) {
-      qswitch<QCap<R>::Z3>(p.q[0], [&](auto QC) { z3_single<R, decltype(QC)::value>(T0, T1, T2, nz0, nz1, nz2, pl, ncols, S, O, ey); });
+      qswitch<QCap<R>::Z3>(p.q[0], [&](auto QC) { z3_single<R, decltype(QC)::value>(T0, T1, T2, nz0, nz1, nz2, pl, ncols, S, O, kx0, ey); });
       return;
     }
   }
@@ -658,7 +592,7 @@ __global__ void __launch_bounds__(ZTPB, 4) k_zconv3(cx<R>* T0, cx<R>* T1, cx<R>*
       __syncthreads();
     }
   }
-  qpick<QL, QCap<R>::Z3>(p.q[p.ng - 1], [&](auto QC) { z3_fused<R, decltype(QC)::value>(buf, tsz, p, ncols, S, O, ey); });
+  qpick<QL, QCap<R>::Z3>(p.q[p.ng - 1], [&](auto QC) { z3_fused<R, decltype(QC)::value>(buf, tsz, p, ncols, S, O, kx0, ey); });
   __syncthreads();
   {
     int s = p.n - p.q[p.ng - 1];
@@ -678,7 +612,7 @@ __global__ void __launch_bounds__(ZTPB, 4) k_zconv3(cx<R>* T0, cx<R>* T1, cx<R>*
 // one edge family with its real spectrum
 template <typename R, int Q>
 __device__ __forceinline__ void z1_single(cx<R>* Tg, int nz, size_t pl, int ncols,
-                                          const void* __restrict__ s, const OctIdx& O) {
+                                          const void* __restrict__ s, const YzIdx& O) {
   constexpr int N = 1 << Q;
   for (int col = threadIdx.x; col < TX; col += blockDim.x) {
     if (col >= ncols) continue;
@@ -688,7 +622,7 @@ __device__ __forceinline__ void z1_single(cx<R>* Tg, int nz, size_t pl, int ncol
     dft_dif<R, Q>(v);
 #pragma unroll
     for (int r = 0; r < N; ++r)
-      v[r] = cscale(v[r], spec_re<R>(s, octant_spectra<R>() ? O.at(col, r) : O.full(col, r)));
+      v[r] = cscale(v[r], spec_re<R>(s, O.at(col, r)));
     dft_dit<R, Q>(v);
 #pragma unroll
     for (int r = 0; r < N; ++r)
@@ -698,7 +632,7 @@ __device__ __forceinline__ void z1_single(cx<R>* Tg, int nz, size_t pl, int ncol
 
 template <typename R, int Q>
 __device__ __forceinline__ void z1_fused(cx<R>* buf, const AxPlan& p, int ncols,
-                                         const void* __restrict__ s, const OctIdx& O) {
+                                         const void* __restrict__ s, const YzIdx& O) {
   constexpr int N = 1 << Q;
   const int tasks = TX << (p.n - Q);
   for (int t = threadIdx.x; t < tasks; t += blockDim.x) {
@@ -711,8 +645,7 @@ __device__ __forceinline__ void z1_fused(cx<R>* buf, const AxPlan& p, int ncols,
     if (col < ncols) {
 #pragma unroll
       for (int r = 0; r < N; ++r)
-        v[r] = cscale(v[r], spec_re<R>(s, octant_spectra<R>() ? O.at(col, start + r)
-                                                              : O.full(col, start + r)));
+        v[r] = cscale(v[r], spec_re<R>(s, O.at(col, start + r)));
     }
     dft_dit<R, Q>(v);
 #pragma unroll
@@ -732,7 +665,7 @@ __global__ void __launch_bounds__(ZTPB, 4) k_zconv1(cx<R>* T0, int nz0, const vo
   const int ncols = min(TX, Lx - kx0);
   const size_t pl = (size_t)Ly * Lx;
   cx<R>* Tg = T0 + (size_t)ky * Lx + kx0;
-  const OctIdx O = make_octidx(Lx, Ly, Lz, kx0, ky);
+  const YzIdx O = make_yzidx(Lx, Ly, Lz, kx0, ky);
   load_twiddles<R>(W, twm, twmax, Lz);
   __syncthreads();
   if constexpr (Q0 == 0) {
@@ -762,40 +695,6 @@ __global__ void __launch_bounds__(ZTPB, 4) k_zconv1(cx<R>* T0, int nz0, const vo
 // copies in flight and ends the CTA.
 
 constexpr int ZWAIT_LIMIT = 1 << 20;
-
-// spectrum index of the tile's column col at z position pz in the y/z-folded tables
-struct YzIdx {
-  size_t rowbase;  // fold(ky) * (Lz/2 + 1) * Lx + kx0
-  int Lx, nz;
-  __device__ __forceinline__ size_t at(int col, int pz) const {
-    return rowbase + (size_t)fold_pos(pz, nz) * Lx + col;
-  }
-};
-
-__device__ __forceinline__ YzIdx make_yzidx(int Lx, int Ly, int Lz, int kx0, int ky) {
-  YzIdx y;
-  y.Lx = Lx;
-  y.nz = ilog2(Lz);
-  y.rowbase = (size_t)fold_pos(ky, ilog2(Ly)) * (Lz / 2 + 1) * Lx + kx0;
-  return y;
-}
-
-__device__ __forceinline__ void pspec_apply_yz(const PSpec& S, const YzIdx& Y, int col, int pz,
-                                               const c32& ex, const c32& ey, c32& a0, c32& a1,
-                                               c32& a2) {
-  const size_t i = Y.at(col, pz);
-  const c32 ez = S.ez32[pz];
-  const c32 c01 = cscale(shift_phase<float>(S.c01, ex, ey, ez), __ldg(S.y[3] + i));
-  const c32 c02 = cscale(shift_phase<float>(S.c02, ex, ey, ez), __ldg(S.y[4] + i));
-  const c32 c12 = cscale(shift_phase<float>(S.c12, ex, ey, ez), __ldg(S.y[5] + i));
-  const float d00 = __ldg(S.y[0] + i), d11 = __ldg(S.y[1] + i), d22 = __ldg(S.y[2] + i);
-  const c32 b0 = cscale(a0, d00) + c01 * a1 + c02 * a2;
-  const c32 b1 = cmulc(a0, c01) + cscale(a1, d11) + c12 * a2;
-  const c32 b2 = cmulc(a0, c02) + cmulc(a1, c12) + cscale(a2, d22);
-  a0 = b0;
-  a1 = b1;
-  a2 = b2;
-}
 
 // forward first group from the staged rows (row < nz; zero beyond) into the tile
 template <int Q>
@@ -837,9 +736,9 @@ __device__ __forceinline__ void z3_fused_yz(c32* buf, size_t tsz, const AxPlan& 
       for (int r = 0; r < N; ++r) v[f][r] = buf[f * tsz + ((start + r) << LTX) + col];
       dft_dif<float, Q>(v[f]);
     }
-    const c32 ex = S.ex32[kx0 + col];
+    const c32 p1 = cmulc(spec_cx<float>(S.ex, kx0 + col), ey);
 #pragma unroll
-    for (int r = 0; r < N; ++r) pspec_apply_yz(S, Y, col, start + r, ex, ey, v[0][r], v[1][r], v[2][r]);
+    for (int r = 0; r < N; ++r) pspec_apply<float>(S, Y, col, start + r, p1, ey, v[0][r], v[1][r], v[2][r]);
 #pragma unroll
     for (int f = 0; f < 3; ++f) {
       dft_dit<float, Q>(v[f]);
@@ -964,7 +863,7 @@ __global__ void __launch_bounds__(ZTPB, 3) k_zconv3_staged(c32* T0, c32* T1, c32
       }
     }
     const YzIdx Y = make_yzidx(Lx, Ly, Lz, kx0, ky);
-    const c32 ey = S.ey32[ky];
+    const c32 ey = spec_cx<float>(S.ey, ky);
     qpick<QL, QCap<float>::Z3>(p.q[p.ng - 1], [&](auto QC) {
       z3_fused_yz<decltype(QC)::value>(buf, tsz, p, S, Y, kx0, ey);
     });
@@ -1062,92 +961,437 @@ __global__ void __launch_bounds__(ZTPB, 4) k_zedge_staged(EdgeSet E, int nzs, in
   }
 }
 
-// Register-direct FP32 z passes on the y/z-folded spectra (ZTune form 1): k_zconv3 /
-// k_zconv1 with the spectral step of the staged kernels; whole 16-column tiles.
-template <int Q0, int QL>
-__global__ void __launch_bounds__(ZTPB, 4) k_zconv3_yz(c32* T0, c32* T1, c32* T2, int nz0,
-                                                       int nz1, int nz2, PSpec S, int Lx, int Ly,
-                                                       AxPlan p, const c32* __restrict__ twm,
-                                                       int twmax) {
-  extern __shared__ unsigned char smem_raw[];
-  const int Lz = 1 << p.n;
-  const size_t tsz = (size_t)Lz << LTX;
-  c32* W = reinterpret_cast<c32*>(smem_raw);
-  c32* buf = W + Lz;
-  const int kx0 = blockIdx.x * TX, ky = blockIdx.y;
-  const size_t pl = (size_t)Ly * Lx;
-  const size_t off = (size_t)ky * Lx + kx0;
-  T0 += off;
-  T1 += off;
-  T2 += off;
-  load_twiddles<float>(W, twm, twmax, Lz);
-  __syncthreads();
-  qpick<Q0, QCap<float>::XY>(p.q[0], [&](auto QC) {
-    col_first_fwd<float, decltype(QC)::value>(T0, pl, TX, nz0, buf, p, W, T0);
-    col_first_fwd<float, decltype(QC)::value>(T1, pl, TX, nz1, buf + tsz, p, W, T1);
-    col_first_fwd<float, decltype(QC)::value>(T2, pl, TX, nz2, buf + 2 * tsz, p, W, T2);
-  });
-  __syncthreads();
-  {
-    int s = p.q[0];
-    for (int g = 1; g + 1 < p.ng; ++g) {
-      smem_group_q<float, false, LTX>(buf, TX, p.q[g], p.n, s, W);
-      smem_group_q<float, false, LTX>(buf + tsz, TX, p.q[g], p.n, s, W);
-      smem_group_q<float, false, LTX>(buf + 2 * tsz, TX, p.q[g], p.n, s, W);
-      s += p.q[g];
-      __syncthreads();
+// --------------------------------------------------------------------------- pair z passes
+// z pass of columns whose occupied rows fill at most half the circulant (nz <= Lz/2 + 1, always
+// so here): the even and the odd frequencies are two transforms of half the length h = Lz/2,
+//   X(2f)   = FFT_h(x_j + x_{j+h}),      X(2f+1) = FFT_h((x_j - x_{j+h}) w^j),
+//   y_j     = E_j + conj(w)^j O_j,       y_{j+h} = E_j - conj(w)^j O_j,
+// with only j + h = h ever occupied, so no padding zero is loaded, transformed or multiplied
+// and each half's inverse gives just the rows kept. A column's h points sit in the registers of
+// G threads, V each (h = V G; V-point transforms over the rows k + G r of thread k, twiddles, a
+// transpose through shared memory, G-point transforms); the transform, the spectral product and
+// the inverse of a half run between two barriers. The three face families share the threads.
+// Spectra: the y/z-folded tables of the half's frequencies go to shared memory by asynchronous
+// copies while the rows load and the forward transform runs; both kz and Lz - kz read them.
+// The cross blocks' phases factor, S_fg = phi_f conj(phi_g) R_fg with R real: the phases of x
+// and y are constant along a column and multiply the rows before and after, those of z
+// multiply one family's points (relative to family 0), and the product is a real 3 x 3.
+// FP32 keeps the rows in registers for the second half; the wider types read them again and
+// leave the odd half's rows in their place until the even half's are there.
+// What bounds them: FP32 instruction issue and loads, float-float the FP32 pipes; the pruning
+// halves the arithmetic of the padded transforms. z passes of an operator application at
+// 128x128x64, faces + edges: FP32 267 us in the direct and staged forms, 169 here (93 + 72);
+// float-float 2541 us direct, 1491 here. FP64 stays direct (see conv_all_t).
+template <typename R>
+struct ZPairJob {
+  cx<R>* T[3];        // face families (edges: T[0] only)
+  int nz[3];
+  const void* S[6];   // the folded tables (edges: S[0] only)
+  const void *ex, *ey, *ez;
+  int lx, ly;         // log2 Lx, log2 Ly
+  int cta0;
+};
+template <typename R, int NJ>
+struct ZPairSet {
+  ZPairJob<R> j[NJ];
+  int n;
+};
+
+__device__ __forceinline__ void zp_cp_async16(void* dst, const void* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"(smem_addr(dst)), "l"(src)
+               : "memory");
+}
+__device__ __forceinline__ void zp_cp_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
+constexpr int ZP_TPB = 128;
+template <typename R, int A, int B, int NF>
+struct ZPairShape {
+  using ST = typename SpecOf<R>::T;
+  static constexpr int V = 1 << A, G = 1 << B, H = V * G, L = 2 * H, C = ZP_TPB / G;
+  static constexpr int NT = NF == 3 ? 6 : 1, NS = H / 2 + 1;
+  static constexpr bool KEEP = sizeof(R) == 4;
+  static constexpr size_t w = 0, ez = w + sizeof(cx<R>) * L,
+                          xch = ez + (NF == 3 ? sizeof(cx<R>) * L : 0),
+                          spec = xch + (B || !KEEP ? sizeof(cx<R>) * NF * H * C : 0),
+                          bytes = spec + sizeof(ST) * NT * NS * C;
+};
+
+// one CTA's columns of a pair pass
+template <typename R, int A, int B, int NF>
+struct ZPairCta {
+  using Sh = ZPairShape<R, A, B, NF>;
+  using ST = typename Sh::ST;
+  static constexpr int V = Sh::V, G = Sh::G, H = Sh::H, L = Sh::L, C = Sh::C, NT = Sh::NT,
+                       NS = Sh::NS;
+  struct Rows {  // a thread's rows k + G r of every family, and row H (thread k = 0)
+    cx<R> d[NF][V];
+  };
+  const ZPairJob<R>* P;
+  cx<R>*W, *Ez, *xch;
+  ST* sp;
+  int c, k, col0, px, py;
+  bool on;
+  size_t pl, at0;
+  cx<R> ph1, ph2, xh[NF];
+
+  // the CTA's job and columns; shared memory, the twiddles and the first spectra on their way
+  template <typename Set>
+  __device__ __forceinline__ void setup(const Set& J, unsigned char* sm, const cx<R>* twm,
+                                        int twmax) {
+    W = reinterpret_cast<cx<R>*>(sm + Sh::w);
+    Ez = reinterpret_cast<cx<R>*>(sm + Sh::ez);
+    xch = reinterpret_cast<cx<R>*>(sm + Sh::xch);
+    sp = reinterpret_cast<ST*>(sm + Sh::spec);
+    int ji = 0;
+    if (NF == 1) {
+#pragma unroll
+      for (int i = 1; i < 3; ++i)
+        if (i < J.n && (int)blockIdx.x >= J.j[i].cta0) ji = i;
+    }
+    P = &J.j[ji];
+    const int tid = threadIdx.x, lx = P->lx;
+    c = tid % C;
+    k = tid / C;
+    col0 = ((int)blockIdx.x - P->cta0) * C;
+    const int col = col0 + c;
+    on = col < (1 << (lx + P->ly));
+    px = col & ((1 << lx) - 1);
+    py = on ? col >> lx : 0;
+    pl = (size_t)1 << (lx + P->ly);
+    at0 = ((size_t)py << lx) + px;
+    stage(1);
+    for (int e = tid; e < L; e += ZP_TPB) {
+      W[e] = twm[e * (twmax / L)];
+      if (NF == 3) Ez[e] = spec_cx<R>(P->ez, brevn(e, A + B + 1));
+    }
+    // the columns' x and y phases of families 1 and 2 (relative to family 0)
+    ph1 = ph2 = mk<R>(1, 0);
+    if (NF == 3 && on) {
+      const cx<R> ex = spec_cx<R>(P->ex, px), ey = spec_cx<R>(P->ey, py);
+      ph1 = cmulc(ex, ey);  // psi_1; psi_2 = ez conj(ey)
+      ph2 = cconj(ey);
     }
   }
-  const YzIdx Y = make_yzidx(Lx, Ly, Lz, kx0, ky);
-  const c32 ey = S.ey32[ky];
-  qpick<QL, QCap<float>::Z3>(p.q[p.ng - 1], [&](auto QC) {
-    z3_fused_yz<decltype(QC)::value>(buf, tsz, p, S, Y, kx0, ey);
-  });
-  __syncthreads();
-  {
-    int s = p.n - p.q[p.ng - 1];
-    for (int g = p.ng - 2; g >= 1; --g) {
-      s -= p.q[g];
-      smem_group_q<float, true, LTX>(buf, TX, p.q[g], p.n, s, W);
-      smem_group_q<float, true, LTX>(buf + tsz, TX, p.q[g], p.n, s, W);
-      smem_group_q<float, true, LTX>(buf + 2 * tsz, TX, p.q[g], p.n, s, W);
-      __syncthreads();
+
+  // the half's spectra: odd (par 1) or even folded z frequencies of the CTA's columns
+  __device__ __forceinline__ void stage(int par) const {
+    const int cnt = par ? (H + 1) / 2 : NS, lx = P->lx;
+    constexpr int E16 = 16 / sizeof(ST);
+    if ((1 << lx) >= C) {
+      constexpr int CH = C / E16;  // 16-byte pieces of a row of C columns
+      const size_t base =
+          (((size_t)fold_pos(col0 >> lx, P->ly) * (H + 1)) << lx) + (col0 & ((1 << lx) - 1));
+      for (int e = threadIdx.x; e < NT * cnt * CH; e += ZP_TPB) {
+        const int ch = e % CH, i = (e / CH) % cnt, t = e / (CH * cnt);
+        zp_cp_async16(sp + ((size_t)t * NS + i) * C + ch * E16,
+                      reinterpret_cast<const ST*>(P->S[t]) + base + ((size_t)(2 * i + par) << lx) +
+                          ch * E16);
+      }
+    } else {
+      for (int e = threadIdx.x; e < NT * cnt * C; e += ZP_TPB) {
+        const int cc = e % C, i = (e / C) % cnt, t = e / (C * cnt);
+        const int q = col0 + cc, y = min(q >> lx, (1 << P->ly) - 1);
+        sp[((size_t)t * NS + i) * C + cc] = reinterpret_cast<const ST*>(
+            P->S[t])[(((size_t)fold_pos(y, P->ly) * (H + 1) + 2 * i + par) << lx) +
+                     (q & ((1 << lx) - 1))];
+      }
     }
   }
-  qpick<Q0, QCap<float>::XY>(p.q[0], [&](auto QC) {
-    col_last_inv<float, decltype(QC)::value>(buf, T0, pl, TX, nz0, p, W);
-    col_last_inv<float, decltype(QC)::value>(buf + tsz, T1, pl, TX, nz1, p, W);
-    col_last_inv<float, decltype(QC)::value>(buf + 2 * tsz, T2, pl, TX, nz2, p, W);
-  });
+
+  __device__ __forceinline__ void load(Rows& x) {
+#pragma unroll
+    for (int f = 0; f < NF; ++f) {
+      const cx<R>* T = P->T[f] + at0;
+      const int nz = P->nz[f];
+#pragma unroll
+      for (int r = 0; r < V; ++r) {
+        const int n = k + G * r;
+        x.d[f][r] = on && n < nz ? ld_stream(T + n * pl) : mk<R>(0, 0);
+      }
+      xh[f] = on && k == 0 && nz > H ? ld_stream(T + H * pl) : mk<R>(0, 0);
+    }
+    if constexpr (NF == 3) {
+#pragma unroll
+      for (int r = 0; r < V; ++r) {
+        x.d[1][r] = cmulc(x.d[1][r], ph1);
+        x.d[2][r] = cmulc(x.d[2][r], ph2);
+      }
+      xh[1] = cmulc(xh[1], ph1);
+      xh[2] = cmulc(xh[2], ph2);
+    }
+  }
+
+  // one half: transform, spectral product, inverse of the rows in place
+  __device__ __forceinline__ void half(Rows& x, int par) const {
+#pragma unroll
+    for (int f = 0; f < NF; ++f) dft_dif<R, A>(x.d[f]);
+    if constexpr (B > 0) {
+#pragma unroll
+      for (int r = 0; r < V; ++r) {
+        const int j = brevq(r, A);
+        const cx<R> w = W[2 * j * k];
+#pragma unroll
+        for (int f = 0; f < NF; ++f)
+          xch[((size_t)f * H + j * G + k) * C + c] = j ? x.d[f][r] * w : x.d[f][r];
+      }
+    }
+    zp_cp_wait();
+    __syncthreads();
+    if constexpr (B > 0) {
+#pragma unroll
+      for (int f = 0; f < NF; ++f) {
+#pragma unroll
+        for (int q = 0; q < V / G; ++q) {
+#pragma unroll
+          for (int t = 0; t < G; ++t)
+            x.d[f][q * G + t] = xch[((size_t)f * H + (k + G * q) * G + t) * C + c];
+          dft_dif<R, B>(x.d[f] + q * G);
+        }
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < V; ++i) {
+      // frequency j + V m of the half: j the thread's, m the register's (B = 0: j = register)
+      const int fr = B > 0 ? (k + G * (i / G)) + V * brevq(i % G, B) : brevq(i, A);
+      const int kz = 2 * fr + par, fz = kz <= H ? kz : L - kz;
+      const ST* s = sp + (size_t)(fz >> 1) * C + c;
+      if constexpr (NF == 1) {
+        x.d[0][i] = cscale(x.d[0][i], R(s[0]));
+      } else {
+        constexpr size_t TS = (size_t)NS * C;
+        const cx<R> e = Ez[kz];
+        const cx<R> x0 = x.d[0][i], x1 = x.d[1][i], x2 = cmulc(x.d[2][i], e);
+        const R r00 = R(s[0]), r11 = R(s[TS]), r22 = R(s[2 * TS]);
+        const R r01 = R(s[3 * TS]), r02 = R(s[4 * TS]), r12 = R(s[5 * TS]);
+        x.d[0][i] = cscale(x0, r00) + cscale(x1, r01) + cscale(x2, r02);
+        x.d[1][i] = cscale(x0, r01) + cscale(x1, r11) + cscale(x2, r12);
+        x.d[2][i] = (cscale(x0, r02) + cscale(x1, r12) + cscale(x2, r22)) * e;
+      }
+    }
+    if constexpr (B > 0) {
+      // back through the cells this thread read itself: no barrier before the writes
+#pragma unroll
+      for (int f = 0; f < NF; ++f) {
+#pragma unroll
+        for (int q = 0; q < V / G; ++q) dft_dit<R, B>(x.d[f] + q * G);
+      }
+#pragma unroll
+      for (int i = 0; i < V; ++i) {
+        const int j = k + G * (i / G), t = i % G;
+        const cx<R> w = W[2 * j * t];
+#pragma unroll
+        for (int f = 0; f < NF; ++f)
+          xch[((size_t)f * H + j * G + t) * C + c] = t ? cmulc(x.d[f][i], w) : x.d[f][i];
+      }
+    }
+    __syncthreads();
+    if (par) stage(0);
+    if constexpr (B > 0) {
+#pragma unroll
+      for (int f = 0; f < NF; ++f) {
+#pragma unroll
+        for (int r = 0; r < V; ++r)
+          x.d[f][r] = xch[((size_t)f * H + brevq(r, A) * G + k) * C + c];
+      }
+    }
+#pragma unroll
+    for (int f = 0; f < NF; ++f) dft_dit<R, A>(x.d[f]);
+  }
+
+  // rows of family f from its even half e and odd half o (rotated back)
+  __device__ __forceinline__ void store(int f, int r, const cx<R>& e, const cx<R>& o) const {
+    const int n = k + G * r;
+    cx<R>* T = P->T[f] + at0;
+    cx<R> y = e + o;
+    if (NF == 3 && f > 0) y = y * (f == 1 ? ph1 : ph2);
+    if (on && n < P->nz[f]) st_stream(T + n * pl, y);
+    if (r == 0 && on && k == 0 && P->nz[f] > H) {
+      cx<R> yh = e - o;
+      if (NF == 3 && f > 0) yh = yh * (f == 1 ? ph1 : ph2);
+      st_stream(T + H * pl, yh);
+    }
+  }
+};
+
+template <typename R, int A, int B, int NF, int MINB>
+__global__ void __launch_bounds__(ZP_TPB, MINB) k_zpair(ZPairSet<R, NF == 3 ? 1 : 3> J,
+                                                        const cx<R>* __restrict__ twm, int twmax) {
+  using Cta = ZPairCta<R, A, B, NF>;
+  using Sh = typename Cta::Sh;
+  constexpr int V = Cta::V, G = Cta::G;
+  extern __shared__ __align__(128) unsigned char smem_raw[];
+  Cta t;
+  t.setup(J, smem_raw, twm, twmax);
+  // x: the rows, then the odd half's rows; d: the half at work. One copy of the half's code (a
+  // loop of two), which stays in the instruction cache.
+  typename Cta::Rows x, d;
+  t.load(x);
+  __syncthreads();  // twiddles and phases are in place
+#pragma unroll
+  for (int r = 0; r < V; ++r) {
+    const cx<R> w = t.W[t.k + G * r];
+#pragma unroll
+    for (int f = 0; f < NF; ++f) d.d[f][r] = (r == 0 ? x.d[f][r] - t.xh[f] : x.d[f][r]) * w;
+  }
+#pragma unroll 1
+  for (int par = 1;; par = 0) {
+    t.half(d, par);
+    if (par == 0) break;
+#pragma unroll
+    for (int r = 0; r < V; ++r) {
+      const cx<R> w = t.W[t.k + G * r];
+#pragma unroll
+      for (int f = 0; f < NF; ++f) {
+        const cx<R> o = cmulc(d.d[f][r], w);
+        d.d[f][r] = r == 0 ? x.d[f][r] + t.xh[f] : x.d[f][r];
+        x.d[f][r] = o;
+      }
+    }
+  }
+#pragma unroll
+  for (int f = 0; f < NF; ++f) {
+#pragma unroll
+    for (int r = 0; r < V; ++r) t.store(f, r, d.d[f][r], x.d[f][r]);
+  }
 }
 
-template <int Q0, int QL>
-__global__ void __launch_bounds__(ZTPB, 4) k_zconv1_yz(c32* T0, int nz0, const float* __restrict__ sy,
-                                                       int Lx, int Ly, AxPlan p,
-                                                       const c32* __restrict__ twm, int twmax) {
-  extern __shared__ unsigned char smem_raw[];
-  const int Lz = 1 << p.n;
-  c32* W = reinterpret_cast<c32*>(smem_raw);
-  c32* buf = W + Lz;
-  const int kx0 = blockIdx.x * TX, ky = blockIdx.y;
-  const size_t pl = (size_t)Ly * Lx;
-  c32* Tg = T0 + (size_t)ky * Lx + kx0;
-  load_twiddles<float>(W, twm, twmax, Lz);
-  __syncthreads();
-  qpick<Q0, QCap<float>::XY>(p.q[0], [&](auto QC) {
-    col_first_fwd<float, decltype(QC)::value>(Tg, pl, TX, nz0, buf, p, W, Tg);
-  });
-  __syncthreads();
-  middle_groups<float, false, LTX>(buf, TX, p, W);
-  const YzIdx Y = make_yzidx(Lx, Ly, Lz, kx0, ky);
-  qpick<QL, QCap<float>::Z1>(p.q[p.ng - 1], [&](auto QC) {
-    z1_fused_yz<decltype(QC)::value>(buf, p, sy, Y);
-  });
-  __syncthreads();
-  middle_groups<float, true, LTX>(buf, TX, p, W);
-  qpick<Q0, QCap<float>::XY>(p.q[0], [&](auto QC) {
-    col_last_inv<float, decltype(QC)::value>(buf, Tg, pl, TX, nz0, p, W);
-  });
+// The pair pass of the wider types: one family's rows in registers at a time, the others in
+// shared memory, so that the code of a transform is there once (float-float's two copies of
+// three families each ran to some 30,000 instructions, bound by their fetch) and half the
+// registers do. Stage 0 starts the odd half, stage 1 ends it and starts the even one, stage 2
+// ends that; the odd half's rows wait in the place of the rows read.
+template <typename R, int A, int B, int NF, int MINB>
+__global__ void __launch_bounds__(ZP_TPB, MINB) k_zpair_wide(ZPairSet<R, NF == 3 ? 1 : 3> J,
+                                                             const cx<R>* __restrict__ twm,
+                                                             int twmax) {
+  using Cta = ZPairCta<R, A, B, NF>;
+  using Sh = typename Cta::Sh;
+  constexpr int V = Cta::V, G = Cta::G, H = Cta::H, L = Cta::L, C = Cta::C, NS = Cta::NS;
+  extern __shared__ __align__(128) unsigned char smem_raw[];
+  Cta t;
+  t.setup(J, smem_raw, twm, twmax);
+  const int c = t.c, k = t.k;
+  __syncthreads();  // twiddles and phases are in place
+#pragma unroll 1
+  for (int stage = 0; stage < 3; ++stage) {
+#pragma unroll 1
+    for (int f = 0; f < NF; ++f) {
+      cx<R>* T = t.P->T[f] + t.at0;
+      const int nz = t.P->nz[f];
+      cx<R>* xf = t.xch + (size_t)f * H * C + c;
+      const cx<R> ph = f == 1 ? t.ph1 : t.ph2;
+      cx<R> d[V], x[V], xh = mk<R>(0, 0);
+      if (stage < 2 && t.on && k == 0 && nz > H) xh = ld_stream(T + H * t.pl);
+      if (stage > 0) {
+#pragma unroll
+        for (int r = 0; r < V; ++r) d[r] = xf[(brevq(r, A) * G + k) * C];
+        dft_dit<R, A>(d);
+      }
+      // the rows as they were, or (stage 2) the odd half's
+#pragma unroll
+      for (int r = 0; r < V; ++r) {
+        const int n = k + G * r;
+        x[r] = t.on && n < nz ? ld_stream(T + n * t.pl) : mk<R>(0, 0);
+      }
+      if (stage == 2) {
+#pragma unroll
+        for (int r = 0; r < V; ++r) {
+          const int n = k + G * r;
+          cx<R> y = d[r] + x[r];
+          if (NF == 3 && f > 0) y = y * ph;
+          if (t.on && n < nz) st_stream(T + n * t.pl, y);
+          if (r == 0 && t.on && k == 0 && nz > H) {
+            cx<R> yh = d[0] - x[0];
+            if (NF == 3 && f > 0) yh = yh * ph;
+            st_stream(T + H * t.pl, yh);
+          }
+        }
+        continue;
+      }
+      if (stage == 1) {
+#pragma unroll
+        for (int r = 0; r < V; ++r) {
+          const int n = k + G * r;
+          const cx<R> o = cmulc(d[r], t.W[n]);
+          if (t.on && n < nz) st_stream(T + n * t.pl, o);
+        }
+      }
+      if (NF == 3 && f > 0) {
+#pragma unroll
+        for (int r = 0; r < V; ++r) x[r] = cmulc(x[r], ph);
+        xh = cmulc(xh, ph);
+      }
+      x[0] = stage == 0 ? x[0] - xh : x[0] + xh;
+      if (stage == 0) {
+#pragma unroll
+        for (int r = 0; r < V; ++r) x[r] = x[r] * t.W[k + G * r];
+      }
+      dft_dif<R, A>(x);
+#pragma unroll
+      for (int r = 0; r < V; ++r) {
+        const int j = brevq(r, A);
+        xf[(j * G + k) * C] = (B > 0 && j) ? x[r] * t.W[2 * j * k] : x[r];
+      }
+    }
+    if (stage == 2) break;
+    const int par = stage == 0 ? 1 : 0;
+    zp_cp_wait();
+    __syncthreads();
+    // this thread's cells: the rows j = k + G q of the half, every family
+    if constexpr (B > 0) {
+#pragma unroll 1
+      for (int f = 0; f < NF; ++f) {
+        cx<R>* xf = t.xch + ((size_t)f * H + k * G) * C + c;
+#pragma unroll
+        for (int q = 0; q < V / G; ++q) {
+          cx<R> d[G];
+#pragma unroll
+          for (int u = 0; u < G; ++u) d[u] = xf[(q * G * G + u) * C];
+          dft_dif<R, B>(d);
+#pragma unroll
+          for (int u = 0; u < G; ++u) xf[(q * G * G + brevq(u, B)) * C] = d[u];
+        }
+      }
+    }
+#pragma unroll 1
+    for (int i = 0; i < V; ++i) {
+      // B > 0: frequency j + V m at the cell (j, m); B = 0: j at the cell (brev j)
+      const int j = B > 0 ? k + G * (i / G) : i, m = B > 0 ? i % G : 0;
+      const int fr = j + V * m, kz = 2 * fr + par, fz = kz <= H ? kz : L - kz;
+      const typename Cta::ST* s = t.sp + (size_t)(fz >> 1) * C + c;
+      cx<R>* x = t.xch + (size_t)(j * G + m) * C + c;
+      if constexpr (NF == 1) {
+        *x = cscale(*x, R(s[0]));
+      } else {
+        constexpr size_t TS = (size_t)NS * C, XS = (size_t)H * C;
+        const cx<R> e = t.Ez[kz];
+        const cx<R> x0 = x[0], x1 = x[XS], x2 = cmulc(x[2 * XS], e);
+        const R r00 = R(s[0]), r11 = R(s[TS]), r22 = R(s[2 * TS]);
+        const R r01 = R(s[3 * TS]), r02 = R(s[4 * TS]), r12 = R(s[5 * TS]);
+        x[0] = cscale(x0, r00) + cscale(x1, r01) + cscale(x2, r02);
+        x[XS] = cscale(x0, r01) + cscale(x1, r11) + cscale(x2, r12);
+        x[2 * XS] = (cscale(x0, r02) + cscale(x1, r12) + cscale(x2, r22)) * e;
+      }
+    }
+    if constexpr (B > 0) {
+#pragma unroll 1
+      for (int f = 0; f < NF; ++f) {
+        cx<R>* xf = t.xch + ((size_t)f * H + k * G) * C + c;
+#pragma unroll
+        for (int q = 0; q < V / G; ++q) {
+          cx<R> d[G];
+#pragma unroll
+          for (int u = 0; u < G; ++u) d[u] = xf[(q * G * G + brevq(u, B)) * C];
+          dft_dit<R, B>(d);
+#pragma unroll
+          for (int u = 0; u < G; ++u)
+            xf[(q * G * G + u) * C] = u ? cmulc(d[u], t.W[2 * (k + G * q) * u]) : d[u];
+        }
+      }
+    }
+    __syncthreads();
+    if (par) t.stage(0);
+  }
 }
 
 // --------------------------------------------------------------------------- host side
@@ -1285,33 +1529,95 @@ struct Launch {
   }
 };
 
-// The FP32 z-pass forms (ZTune): direct on full-form spectra, direct on y/z-folded
-// spectra, staged. Templates, so that only the float instantiation compiles their kernels.
+template <typename R>
+struct ZPair {
+  template <int A, int B, int NF>
+  static int launch(ZPairSet<R, NF == 3 ? 1 : 3>& J, const cx<R>* tw, int twmax, cudaStream_t st) {
+    using Sh = ZPairShape<R, A, B, NF>;
+    int ctas = 0;
+    for (int i = 0; i < J.n; ++i) {
+      J.j[i].cta0 = ctas;
+      ctas += (int)((((int64_t)1 << (J.j[i].lx + J.j[i].ly)) + Sh::C - 1) / Sh::C);
+    }
+    constexpr int MINB = sizeof(R) == 4 ? (NF == 3 ? 4 : 6) : 4;
+    void (*kern)(ZPairSet<R, NF == 3 ? 1 : 3>, const cx<R>*, int);
+    if constexpr (Sh::KEEP) kern = k_zpair<R, A, B, NF, MINB>;
+    else kern = k_zpair_wide<R, A, B, NF, MINB>;
+    CTX_CHECK(smem_optin(kern, Sh::bytes));
+    kern<<<ctas, ZP_TPB, Sh::bytes, st>>>(J, tw, twmax);
+    return 0;
+  }
+  // h = V G: up to eight points a thread, sixteen or more points over several threads
+  template <int NF>
+  static int by_length(int logh, ZPairSet<R, NF == 3 ? 1 : 3>& J, const cx<R>* tw, int twmax,
+                       cudaStream_t st) {
+    switch (logh) {
+      case 0: return launch<0, 0, NF>(J, tw, twmax, st);
+      case 1: return launch<1, 0, NF>(J, tw, twmax, st);
+      case 2: return launch<2, 0, NF>(J, tw, twmax, st);
+      case 3: return launch<2, 1, NF>(J, tw, twmax, st);
+      case 4: return launch<2, 2, NF>(J, tw, twmax, st);
+      case 5: return launch<3, 2, NF>(J, tw, twmax, st);
+      default: return launch<3, 3, NF>(J, tw, twmax, st);
+    }
+  }
+  static int faces(const Family* F, const PSpec& S, const cx<R>* tw, int twmax, cudaStream_t st) {
+    ZPairSet<R, 1> J{};
+    J.n = 1;
+    ZPairJob<R>& j = J.j[0];
+    for (int f = 0; f < 3; ++f) {
+      j.T[f] = Launch<R>::buf(F[f]);
+      j.nz[f] = F[f].dims[2];
+    }
+    for (int i = 0; i < 6; ++i) j.S[i] = S.y[i];
+    j.ex = S.ex;
+    j.ey = S.ey;
+    j.ez = S.ez;
+    j.lx = F[0].logL[0];
+    j.ly = F[0].logL[1];
+    return by_length<3>(F[0].logL[2] - 1, J, tw, twmax, st);
+  }
+  // the edge families, one launch per circulant length; done[f]: taken here
+  static int edges(const Family* F, int nfam, const Spectrum* spec, const cx<R>* tw, int twmax,
+                   cudaStream_t st, bool* done) {
+    for (int f = 3; f < nfam; ++f) {
+      if (done[f] || !zpair_ok(F[f])) continue;
+      ZPairSet<R, 3> J{};
+      for (int g = f; g < nfam; ++g) {
+        if (done[g] || !zpair_ok(F[g]) || F[g].L[2] != F[f].L[2]) continue;
+        ZPairJob<R>& j = J.j[J.n++];
+        j.T[0] = Launch<R>::buf(F[g]);
+        j.nz[0] = F[g].dims[2];
+        j.S[0] = spec[3 + g].yz[slot_of<R>()];
+        j.lx = F[g].logL[0];
+        j.ly = F[g].logL[1];
+        done[g] = true;
+      }
+      CTX_CHECK(by_length<1>(F[f].logL[2] - 1, J, tw, twmax, st));
+    }
+    return 0;
+  }
+};
+
 template <typename R>
 static PSpec pspec_of(const Spectrum* spec, const void* const* ph) {
   const int p = slot_of<R>();
-  PSpec S{spec[0].d[p], spec[1].d[p], spec[2].d[p], spec[3].d[p], spec[4].d[p], spec[5].d[p],
-          spec[0].oct,  spec[1].oct,  spec[2].oct,  spec[3].oct,  spec[4].oct,  spec[5].oct,
-          ph[0],        ph[1],        ph[2],        {},           {},           {}};
-  for (int a = 0; a < 3; ++a) {
-    S.c01[a] = spec[3].c[a];
-    S.c02[a] = spec[4].c[a];
-    S.c12[a] = spec[5].c[a];
-  }
-  if (std::is_same<R, float>::value) {
-    for (int i = 0; i < 6; ++i) S.y[i] = (const float*)spec[i].yz32;
-    S.ex32 = (const c32*)ph[3];
-    S.ey32 = (const c32*)ph[4];
-    S.ez32 = (const c32*)ph[5];
-  }
+  PSpec S{};
+  for (int i = 0; i < 6; ++i) S.y[i] = spec[i].yz[p];
+  S.ex = ph[3 * p];
+  S.ey = ph[3 * p + 1];
+  S.ez = ph[3 * p + 2];
   return S;
 }
 
+// The FP32 z-pass forms (ZTune): pairs (k_zpair), direct (k_zconv3 / k_zconv1), staged.
+// Templates, so that only the float instantiation compiles their kernels.
 template <int UNUSED = 0>
 static int zface_f32(const Family* F, int nfam, const PSpec& S, const c32* tw, int twmax,
                      const ZTune& zt, cudaStream_t st) {
-  const int form = zpass_yz_faces(F, nfam) ? zt.face : 0;
-  if (form == 0) return Launch<float>::zconv3(F, S, tw, twmax, st);
+  int form = zt.face;
+  if (form == 3 && zpair_ok(F[0])) return ZPair<float>::faces(F, S, tw, twmax, st);
+  if (form != 2 || !zpass_yz_faces(F, nfam)) return Launch<float>::zconv3(F, S, tw, twmax, st);
   const int Lz = F[0].L[2], Lx = F[0].L[0], Ly = F[0].L[1];
   const AxPlan p = Plans<float>::z3(F[0].logL[2]);
   constexpr int QL = QCap<float>::Z3;
@@ -1319,15 +1625,6 @@ static int zface_f32(const Family* F, int nfam, const PSpec& S, const c32* tw, i
   c32* T0 = Launch<float>::buf(F[0]);
   c32* T1 = Launch<float>::buf(F[1]);
   c32* T2 = Launch<float>::buf(F[2]);
-  if (form == 1) {
-    const size_t sm = sizeof(c32) * (Lz + 3 * ((size_t)Lz << LTX));
-    auto kern = spec ? k_zconv3_yz<4, QL> : k_zconv3_yz<0, 0>;
-    CTX_CHECK(smem_optin(kern, sm));
-    dim3 g(Lx >> LTX, Ly);
-    kern<<<g, ZTPB, sm, st>>>(T0, T1, T2, F[0].dims[2], F[1].dims[2], F[2].dims[2], S, Lx, Ly,
-                              p, tw, twmax);
-    return 0;
-  }
   const int nzs = std::max(F[0].dims[2], std::max(F[1].dims[2], F[2].dims[2]));
   const size_t sm = 128 + sizeof(c32) * (Lz + 3 * ((size_t)Lz << LTX) + 3 * (size_t)nzs * TX);
   auto kern = spec ? k_zconv3_staged<4, QL> : k_zconv3_staged<0, 0>;
@@ -1343,28 +1640,12 @@ static int zface_f32(const Family* F, int nfam, const PSpec& S, const c32* tw, i
 template <int UNUSED = 0>
 static int zedge_f32(const Family* F, int nfam, const Spectrum* spec, const c32* tw, int twmax,
                      const ZTune& zt, cudaStream_t st) {
-  const int form = zpass_yz_edges(F, nfam) ? zt.edge : 0;
-  if (form < 2) {
-    for (int f = 3; f < nfam; ++f) {
-      if (!F[f].active) continue;
-      if (form == 0) {
-        CTX_CHECK(Launch<float>::zconv1(F[f], spec[3 + f].d[1], tw, twmax, st, zt.edge_plan));
-        continue;
-      }
-      const Family& fam = F[f];
-      const int Lz = fam.L[2];
-      const AxPlan p = Plans<float>::z1(fam.logL[2], zt.edge_plan);
-      const int q0 = p.q[0], ql = p.q[p.ng - 1];
-      auto kern = (q0 == 4 && ql == 3) ? k_zconv1_yz<4, 3>
-                  : (q0 == 3 && ql == 4) ? k_zconv1_yz<3, 4>
-                                         : k_zconv1_yz<0, 0>;
-      const size_t sm = sizeof(c32) * (Lz + ((size_t)Lz << LTX));
-      CTX_CHECK(smem_optin(kern, sm));
-      dim3 g(fam.L[0] >> LTX, fam.L[1]);
-      kern<<<g, ZTPB, sm, st>>>(Launch<float>::buf(fam), fam.dims[2],
-                                (const float*)spec[3 + f].yz32, fam.L[0], fam.L[1], p, tw,
-                                twmax);
-    }
+  if (zt.edge != 2 || !zpass_yz_edges(F, nfam)) {
+    bool done[kMaxFam] = {};
+    if (zt.edge == 3) CTX_CHECK(ZPair<float>::edges(F, nfam, spec, tw, twmax, st, done));
+    for (int f = 3; f < nfam; ++f)
+      if (F[f].active && !done[f])
+        CTX_CHECK(Launch<float>::zconv1(F[f], spec[3 + f].yz[1], tw, twmax, st, zt.edge_plan));
     return 0;
   }
   EdgeSet E{};
@@ -1375,7 +1656,7 @@ static int zedge_f32(const Family* F, int nfam, const Spectrum* spec, const c32*
     if (!f0) f0 = &F[f];
     E.T[E.nf] = Launch<float>::buf(F[f]);
     E.nz[E.nf] = F[f].dims[2];
-    E.sy[E.nf] = (const float*)spec[3 + f].yz32;
+    E.sy[E.nf] = (const float*)spec[3 + f].yz[1];
     nzs = std::max(nzs, F[f].dims[2]);
     ++E.nf;
   }
@@ -1423,11 +1704,19 @@ int conv_all_t(const Family* F, int nfam, const Spectrum* spec, const void* cons
     CTX_CHECK(zface_f32(F, nfam, S, tw, twmax, z, st));
     CTX_CHECK(zedge_f32(F, nfam, spec, tw, twmax, z, st));
   } else {
-    CTX_CHECK(Lc::zconv3(F, S, tw, twmax, st));
+    // float-float takes the pair passes; FP64 is bound by its pipe and the two forms' counts
+    // of operations are alike (128x128x64: 4.42 against 4.57 ms, 57x57x13: 0.25 against 0.22)
+    bool done[kMaxFam] = {};
+    bool pair = false;
+    if constexpr (std::is_same<R, ff>::value) {
+      pair = zpair_ok(F[0]);
+      if (pair) CTX_CHECK(ZPair<R>::faces(F, S, tw, twmax, st));
+      CTX_CHECK(ZPair<R>::edges(F, nfam, spec, tw, twmax, st, done));
+    }
+    if (!pair) CTX_CHECK(Lc::zconv3(F, S, tw, twmax, st));
     for (int f = 3; f < nfam; ++f)
-      if (F[f].active)
-        CTX_CHECK(Lc::zconv1(F[f], octant_spectra<R>() ? spec[3 + f].oct : spec[3 + f].d[p], tw,
-                             twmax, st));
+      if (F[f].active && !done[f])
+        CTX_CHECK(Lc::zconv1(F[f], spec[3 + f].yz[p], tw, twmax, st));
   }
   if (ev) cudaEventRecord(ev[3], st);
   CTX_CHECK(Lc::pass(3, F, nfam, nullptr, tw, twmax, st));

@@ -381,7 +381,7 @@ class GpuOperator:
                         "edge": bool(kind.value)})
         return out
 
-    FORMS = ("direct", "direct_yz", "staged")
+    FORMS = ("direct", "direct_yz", "staged", "pair")
 
     def zpass_tuning(self):
         """The FP32 z-pass forms the autotuner picked (face, edge, edge radix plan) and the
@@ -398,7 +398,7 @@ class GpuOperator:
                             for p_ in range(2) for i in range(3)}}
 
     def set_zpass_forms(self, face, edge, edge_plan=0):
-        """Pins the FP32 z-pass forms ("direct", "direct_yz", "staged" or 0..2) in place of
+        """Pins the FP32 z-pass forms ("direct", "direct_yz", "staged", "pair" or 0..3) in place of
         the tuner's choice until the next fill / set_rows."""
         f = self.FORMS.index(face) if isinstance(face, str) else int(face)
         e = self.FORMS.index(edge) if isinstance(edge, str) else int(edge)
