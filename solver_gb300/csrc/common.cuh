@@ -120,4 +120,35 @@ __host__ __device__ __forceinline__ ff operator*(ff a, ff b) {
   e = PEEC_FMA(a.lo, b.hi, e);
   return ff_fast_two_sum(p, e);
 }
+// Double to float-float and back by integer operations: a conversion instruction holds the FP64
+// pipe as long as a double multiply (64 cycles a warp and sub-partition), and the constructor
+// and cast above take four and three such instructions. Same roundings (to nearest but for ties
+// of the high part, which only move half a unit between the parts); values outside the range
+// handled here, and sums that leave the high part's binade, take the plain forms.
+__device__ __forceinline__ ff ff_split(double d) {
+  const int h = __double2hiint(d), l = __double2loint(d);
+  const int e = (h >> 20) & 0x7ff;
+  if (e < 950 || e >= 1150) return d == 0.0 ? ff(0.f, 0.f) : ff(d);
+  const int r = (int)((unsigned)l << 3) >> 3;  // the low 29 bits, signed
+  const unsigned m = (((unsigned)(h & 0x7fffffff) - (896u << 20)) << 3 | (unsigned)l >> 29) +
+                     (r < 0 ? 1u : 0u);
+  const unsigned sg = (unsigned)h & 0x80000000u;
+  const float lo = __fmul_rn((float)r, __uint_as_float((unsigned)(e - 948) << 23));
+  return ff(__uint_as_float(m | sg), __uint_as_float(__float_as_uint(lo) ^ sg));
+}
+__device__ __forceinline__ double ff_join(ff a) {
+  const unsigned h = __float_as_uint(a.hi);
+  const int e = (int)(h >> 23) & 0xff;
+  if (e >= 60 && e < 255) {
+    // the low part in units of the double's last place
+    const float u = __fmul_rn(a.lo, __uint_as_float((unsigned)(306 - e) << 23));
+    int r = __float2int_rn(u);
+    if ((int)h < 0) r = -r;
+    if (fabsf(u) <= 268435456.f && ((h & 0x7fffffu) != 0 || r >= 0)) {
+      const long long b = (((long long)(h & 0x7fffffffu) + (896ll << 23)) << 29) + r;
+      return __longlong_as_double(b | (long long)((unsigned long long)(h & 0x80000000u) << 32));
+    }
+  }
+  return (double)a;
+}
 using cff = cx<ff>;

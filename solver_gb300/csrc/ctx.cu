@@ -83,15 +83,7 @@ int launch_sptrsv(const GrpPlan&, cudaStream_t, cudaEvent_t, cudaEvent_t, const 
                   int*, cudaStream_t);
 int red_blocks(size_t N);
 int launch_multidot(const c64*, size_t, const c64*, size_t, int, c64*, c64*, cudaStream_t);
-int launch_multidot(const cff*, size_t, const c64*, size_t, int, c64*, c64*, cudaStream_t);
-int launch_multidot(const cff*, size_t, const cff*, size_t, int, c64*, c64*, cudaStream_t);
-void launch_multiaxpy(const c64*, size_t, const c64*, int, const c64*, int, size_t, c64*, size_t,
-                      double*, cudaStream_t);
-void launch_multiaxpy(const cff*, size_t, const c64*, int, const c64*, int, size_t, c64*, size_t,
-                      double*, cudaStream_t);
 void launch_norm2(const c64*, size_t, size_t, double*, double*, cudaStream_t);
-void launch_sum_parts(const double*, int, double*, cudaStream_t);
-void launch_scale_rnorm(c64*, size_t, const double*, cudaStream_t);
 void launch_make_reflector(const c64*, size_t, int, c64, double, c64*, cudaStream_t);
 void launch_make_reflector(const c64*, size_t, int, c64, double, cff*, cudaStream_t);
 void launch_sub(const c64*, const c64*, size_t, c64*, cudaStream_t);
@@ -264,8 +256,8 @@ struct peec_ctx {
   int kcap_u = 0, kcap_u32 = 0;
   c64 *gb = nullptr, *gx = nullptr, *gr = nullptr, *gv = nullptr, *gw = nullptr, *gxm = nullptr,
       *gxmin = nullptr, *gtmp = nullptr, *gzero = nullptr;
-  c64 *dcoef = nullptr, *dcoef2 = nullptr, *dpart = nullptr, *dT = nullptr;
-  double *dred = nullptr, *dscal = nullptr;
+  c64 *dcoef = nullptr, *dcoef2 = nullptr, *dT = nullptr;
+  double *dpart = nullptr, *dred = nullptr, *dscal = nullptr;
   c64* hsmall = nullptr;  // pinned staging ring for host -> device coefficients
   c64* hread = nullptr;   // pinned staging for device -> host reads
   double* hscal = nullptr;
@@ -2642,9 +2634,8 @@ static int ensure_krylov(peec_ctx* ctx, int k, int prec) {
   CTX_TRY(dalloc(&ctx->dcoef, 2 * (size_t)k + 16));  // xupdate stages 2k coefficients
   CTX_TRY(dalloc(&ctx->dcoef2, 2 * (size_t)k + 16));
   CTX_TRY(dalloc(&ctx->dT, (size_t)k * k));            // compact-WY T, ld = k
-  const int nb = red_blocks(N);
-  CTX_TRY(dalloc(&ctx->dpart, (size_t)nb * (k + 8)));
-  CTX_TRY(dalloc(&ctx->dred, nb + 8));
+  CTX_TRY(dalloc(&ctx->dpart, gm_part_doubles(N, k)));
+  CTX_TRY(dalloc(&ctx->dred, red_blocks(N) + 8));
   CTX_TRY(dalloc(&ctx->dscal, 16));
   ctx->kcap = k;
   return PEEC_OK;
@@ -2652,7 +2643,7 @@ static int ensure_krylov(peec_ctx* ctx, int k, int prec) {
 
 // byte offsets of the arrays of a cycle state with `inner` iterations (16-byte aligned)
 struct GmLayout {
-  size_t res, wv, J, Utop, R, total;
+  size_t res, wv, J, Utop, R, cvec, cpart, head, scr, total;
 };
 static GmLayout gm_layout(int inner) {
   auto up16 = [](size_t x) { return (x + 15) & ~(size_t)15; };
@@ -2668,6 +2659,12 @@ static GmLayout gm_layout(int inner) {
   o += sizeof(c64) * ((size_t)inner + 1) * ((size_t)inner + 1);
   L.R = o;
   o += sizeof(c64) * (size_t)inner * inner;
+  for (size_t* p : {&L.cvec, &L.cpart, &L.head}) {
+    *p = o;
+    o += sizeof(c64) * ((size_t)inner + 1);
+  }
+  L.scr = o;
+  o += sizeof(c64) * (4 * ((size_t)inner + 1) + 4);
   L.total = o;
   return L;
 }
@@ -2777,7 +2774,7 @@ namespace {
 // Host side of the Householder GMRES. Vectors of length N live on the device; the
 // compact-WY matrix T (reflector products P1..Pk = I - U T U^H) lives on the device
 // and is only touched by small kernels; so does the scalar work of an iteration
-// (k_gm_step: reflector heads, Givens rotations, R, w, the residual estimate). The host
+// (gm_step, krylov.cu: reflector heads, Givens rotations, R, w, the residual estimate). The host
 // runs the reference's control flow around it: the convergence checks on the true
 // residual, stagnation, restarts. Host -> device coefficient vectors go through a ring
 // of pinned slots.
@@ -2964,6 +2961,10 @@ static int gmres_run(peec_ctx* ctx, const c64* b_dev, c64* x_dev, double tol, in
   hdr.J = (c64*)(gblk + GL.J);
   hdr.Utop = (c64*)(gblk + GL.Utop);
   hdr.R = (c64*)(gblk + GL.R);
+  hdr.cvec = (c64*)(gblk + GL.cvec);
+  hdr.cpart = (c64*)(gblk + GL.cpart);
+  hdr.head = (c64*)(gblk + GL.head);
+  hdr.scr = (c64*)(gblk + GL.scr);
   GmBody B;
   if (f32) B.U32 = ctx->U32;
   else B.U = ctx->U;
@@ -2975,9 +2976,7 @@ static int gmres_run(peec_ctx* ctx, const c64* b_dev, c64* x_dev, double tol, in
   B.v = v;
   B.w = add;
   B.coef = ctx->dcoef;
-  B.coef2 = ctx->dcoef2;
   B.part = ctx->dpart;
-  B.red = ctx->dred;
   B.scal = ctx->dscal;
   B.st = ctx->st;
   // the first k columns of R and Utop, read back for the host's least-squares solves
@@ -3015,6 +3014,7 @@ static int gmres_run(peec_ctx* ctx, const c64* b_dev, c64* x_dev, double tol, in
       wv[0] = -beta;
       g.to_dev(hdr.Utop, std::vector<cd>(Utop.begin(), Utop.begin() + headlen));
       g.to_dev(hdr.wv, wv);
+      g.to_dev(hdr.cvec, {2.0 * std::conj(Utop[0])});  // T conj(Utop(0, :)), T(0,0) = 2
     }
     initercount = 0;
     int jdone = 0;       // iterations of this cycle done on the device

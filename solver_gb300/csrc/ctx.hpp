@@ -106,7 +106,7 @@ int refactor_launch(const RefactorPlan& R, const SfTri& L, const SfTri& U, c64* 
                     cudaStream_t st);
 
 // Device-resident state of one Householder GMRES cycle (the Arnoldi loop's scalar work
-// runs in k_gm_step, krylov.cu). The host writes the header before a run of iterations
+// runs in gm_step, krylov.cu). The host writes the header before a run of iterations
 // and reads back the header, res and wv after it; Utop and R only when its convergence
 // check needs them. All arrays live in one allocation after the header.
 struct GmDev {
@@ -116,18 +116,18 @@ struct GmDev {
   int headlen;    // min(N, inner + 1): rows of the reflectors kept in Utop
   int ld;         // inner + 1, leading dimension of Utop
   int exit_now;   // host: leave the loop after the next iteration
-  int refl_on;    // the last iteration appended a reflector (alpha != 0)
-  int pad_;
+  unsigned tick[32];  // CTAs done of each group of a reduction, and groups done (zero between)
   double tolb;    // tol * |b|: the loop continues while |w(j+1)| > tolb
   double normr;   // |w(j+1)| after the last iteration
-  double refl_scale;
-  double pad2_;
-  c64 refl_add;   // the new reflector: u = (v with rows < j zeroed, v(j) += add) * scale
   double* res;    // [inner + 2] residual estimates, res[initer] = |w(initer)|
   c64* wv;        // [inner + 1] Givens-rotated right-hand side w
   c64* J;         // [2 * inner] Givens rotations (c, s) per column
   c64* Utop;      // [ld * ld] leading rows of the reflectors, column-major
   c64* R;         // [inner * inner] upper-triangular R, column-major, ld = inner
+  c64* cvec;      // [ld] coefficients of the next iteration's v: T conj(Utop(j, :))
+  c64* cpart;     // [ld] their part from the columns before the newest
+  c64* head;      // [ld] leading rows of the orthogonalised vector
+  c64* scr;       // [4 * ld + 4] scratch of the reductions' last CTAs
 };
 
 // Buffers of the device loop's Arnoldi body (krylov.cu): the basis is U (complex double)
@@ -140,12 +140,13 @@ struct GmBody {
   c64* T = nullptr;
   int ldT = 0, kmax = 0;
   GmDev* gs = nullptr;
-  c64 *v = nullptr, *w = nullptr, *coef = nullptr, *coef2 = nullptr, *part = nullptr;
-  double *red = nullptr, *scal = nullptr;
+  c64 *v = nullptr, *w = nullptr, *coef = nullptr;
+  double *part = nullptr, *scal = nullptr;  // partial sums: gm_part_doubles(N, kmax + 1)
   cudaGraphConditionalHandle cond = 0;
   int use_cond = 0;  // 1 inside the WHILE node's body graph, 0 for a single eager iteration
   cudaStream_t st = nullptr;
 };
+size_t gm_part_doubles(size_t N, int k);
 int gm_pre(const GmBody& B);   // returns the kernels launched
 int gm_post(const GmBody& B);
 
