@@ -2347,7 +2347,8 @@ static int matvec_enqueue(peec_ctx* ctx, const c64* x, c64* y, int prec, bool ev
   // one launch per x / y pass over all families, the shared z pass of the face
   // families, and the edge families' z passes: one launch over all of them in the staged
   // FP32 form (ZTune form 2), else one per family
-  ctx->launches += (5 + zedge_launches(ctx->fam, 6, prec, ctx->zt)) * (ctx->rcc ? 2 : 1);
+  const int lines = line_launches(ctx->fam, 6, prec, 0) + line_launches(ctx->fam, 6, prec, 1);
+  ctx->launches += (1 + 2 * lines + zedge_launches(ctx->fam, 6, prec, ctx->zt)) * (ctx->rcc ? 2 : 1);
   if (events) cudaEventRecord(ctx->ev[1], st);
   sparse_enqueue(ctx, x, y, ctx->LpI, ctx->PQ);
   if (events) cudaEventRecord(ctx->ev[2], st);

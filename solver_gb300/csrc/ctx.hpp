@@ -211,6 +211,14 @@ int phase_tables(const int L[3], void* e64[3], void* e32[3], cudaStream_t st);
 // tiles, enough z points; the edge families on one shared grid)
 bool zpass_yz_faces(const Family* F, int nfam);
 bool zpass_yz_edges(const Family* F, int nfam);
+// lines along axis ax (x, y) the pair passes take: a circulant of 2 to 512 points
+inline bool line_pair_ok(const Family& f, int ax) {
+  return f.active && f.L[ax] >= 2 && f.L[ax] <= 512 && f.dims[ax] <= f.L[ax] / 2 + 1 &&
+         ((int64_t)f.dims[2] << f.logL[0]) < ((int64_t)1 << 30) &&
+         (int64_t)f.dims[1] * f.dims[2] < ((int64_t)1 << 30);
+}
+// launches of the x (ax 0) or y passes' one direction in a precision
+int line_launches(const Family* F, int nfam, int prec, int ax);
 // launches of the edge families' z passes in a precision (0 fp64, 1 fp32, 2 float-float)
 int zedge_launches(const Family* F, int nfam, int prec, const ZTune& zt);
 // z extents the pair passes take: a circulant of 2 to 128 points (half of it in registers)

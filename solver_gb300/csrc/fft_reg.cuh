@@ -59,7 +59,7 @@ __device__ __forceinline__ cx<R> rot16(const cx<R>& v, int a) {
   if (a == 12) return INV ? mk<R>(v.y, -v.x) : mk<R>(-v.y, v.x);
   const R c = (R)cospi8(a);
   const R s = INV ? (R)sinpi8(a) : (R)(-sinpi8(a));
-  return mk<R>(v.x * c - v.y * s, v.x * s + v.y * c);
+  return v * mk<R>(c, s);
 }
 
 // forward DFT of 2^Q registers: natural order in, register r holds output brev_Q(r)

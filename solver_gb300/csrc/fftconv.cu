@@ -84,6 +84,22 @@ bool zpass_yz_edges(const Family* F, int nfam) {
   return f0 != nullptr;
 }
 
+int line_launches(const Family* F, int nfam, int prec, int ax) {
+  int n = 0;
+  bool direct = false;
+  for (int f = 0; f < nfam; ++f) {
+    if (!F[f].active) continue;
+    if (prec == 0 || !line_pair_ok(F[f], ax)) {
+      direct = true;
+      continue;
+    }
+    bool first = true;  // of the families that share a launch
+    for (int g = 0; g < f; ++g) first = first && !(line_pair_ok(F[g], ax) && F[g].L[ax] == F[f].L[ax]);
+    n += first ? 1 : 0;
+  }
+  return n + (direct ? 1 : 0);
+}
+
 int zedge_launches(const Family* F, int nfam, int prec, const ZTune& zt) {
   if (prec == 1 && zt.edge == 2 && zpass_yz_edges(F, nfam)) return 1;
   const bool pair = prec == 2 || (prec == 1 && zt.edge == 3);

@@ -399,6 +399,365 @@ __global__ void __launch_bounds__(TPB) k_ypass(PassSet<R> s, const cx<R>* __rest
   }
 }
 
+// --------------------------------------------------------------------------- pair x and y passes
+// Lines whose occupied entries fill at most half the circulant (n <= L/2 + 1, always so here), as
+// two transforms of half the length H = L/2, the even and the odd frequencies:
+//   X(2f) = FFT_H(x_j + x_{j+H}),   X(2f+1) = FFT_H((x_j - x_{j+H}) w^j),   w = exp(-2 pi i / L),
+// only j + H = H ever occupied, and mirrored for the inverse. The padding is neither loaded nor
+// transformed. A line's H points sit in the registers of G threads, V = H/G each: V-point
+// transforms over the entries k + G r of thread k, twiddles, a transpose through shared memory,
+// G-point transforms; a thread then holds G consecutive positions of the bit-reversed order. y:
+// a CTA takes 128 / G consecutive columns, whose rows are contiguous across the lanes. x: a
+// line's threads are neighbouring lanes (no CTA barrier after the twiddles are there), its G
+// positions leave in 32-byte stores and the lattice map's and the vectors' entries come in lane
+// order, all of a thread's loads in flight at once.
+// What bounds them: FP32 the memory (about 1.3 times the family buffers' bytes in DRAM) and the
+// gathers' latency, float-float the FP32 pipes. The direct kernels (k_xfwd and so on) ran 37M and
+// 52M warp instructions in x and y at 128x128x64, on padding and through three transposes in
+// shared memory with CTA barriers. Operator application at 128x128x64, x / y / inverse y / inverse
+// x: FP32 70 / 78 / 70 / 87 -> 50 / 52 / 67 / 49 us, float-float 262 / 291 / 311 / 258 -> 186 / 234
+// / 252 / 158 us; FP32 at 64x64x32 13.9 / 16.3 / 14.9 / 15.5 -> 8.3 / 6.9 / 8.1 / 8.8 us. FP64
+// stays direct, like its z passes (its pipe is the bound in either form).
+__device__ __forceinline__ int brevn(int v, int n) {
+  return n ? (int)(__brev((unsigned)v) >> (32 - n)) : 0;
+}
+
+constexpr int XP_TPB = 128;
+template <typename R>
+struct LineFam {
+  cx<R>* T;
+  const int32_t* map;  // x: lattice map
+  c64* io;             // x: compact vector
+  int lx, ly;          // log2 of the circulant's x and y lengths
+  int n;               // occupied entries of a line
+  int ny;              // x: lines of a z plane
+  int lines;           // x: ny nz; y: nz << lx
+  int cta0;
+};
+template <typename R>
+struct LineSet {
+  LineFam<R> f[kMaxFam];
+  int nf;
+};
+
+__device__ __forceinline__ c32 line_swap(const c32& v, int m) {
+  return mk<float>(__shfl_xor_sync(0xffffffffu, v.x, m), __shfl_xor_sync(0xffffffffu, v.y, m));
+}
+__device__ __forceinline__ cff line_swap(const cff& v, int m) {
+  return mk<ff>(ff(__shfl_xor_sync(0xffffffffu, v.x.hi, m), __shfl_xor_sync(0xffffffffu, v.x.lo, m)),
+                ff(__shfl_xor_sync(0xffffffffu, v.y.hi, m), __shfl_xor_sync(0xffffffffu, v.y.lo, m)));
+}
+
+template <typename R>
+__device__ __forceinline__ cx<R> line_sel(bool t, cx<R> a, cx<R> b) {  // by value: no addresses
+  return t ? a : b;
+}
+
+// G <= V: a thread takes V/G of the second transforms whole. G = 2 V: two neighbouring threads
+// take one, as V points each (even and odd) and a last pair step in which they swap half.
+template <typename R, int A, int B>
+struct HalfLine {
+  static constexpr int V = 1 << A, G = 1 << B, H = V * G, L = 2 * H;
+  // lines of a CTA: x 128 threads; y at least 16 columns (128 bytes of FP32 rows)
+  static constexpr int CX = XP_TPB / G, CY = CX < 16 ? 16 : CX;
+  static constexpr bool SPLIT = G > V;
+  static_assert(!SPLIT || G == 2 * V, "at most two threads a second transform");
+  // x: exchange strides of a frequency group and of a line (bank-disjoint)
+  static constexpr int SJ = SPLIT ? G + 2 : G + 1, LS = V * SJ + 8;
+  static constexpr int RUN = B == 0 || SPLIT ? V : G, NRUN = V / RUN;
+  static constexpr size_t smem(bool x) {
+    return sizeof(cx<R>) * (L + (B == 0 ? 0 : x ? LS * CX : 2 * H * CY));
+  }
+  template <bool WARP>
+  static __device__ __forceinline__ void sync() {
+    if (WARP) __syncwarp();
+    else __syncthreads();
+  }
+  // run q of thread k after a forward half (registers q RUN ..): position within the half
+  static __device__ __forceinline__ int pos(int q, int k) {
+    if (SPLIT) return brevn(k >> 1, A) * G + (k & 1) * V;
+    return B > 0 ? brevn(k + G * q, A) * G : 0;
+  }
+  // entries k + G r -> positions in runs; the exchange cell of frequency group j, point t is
+  // xc[j * sj + t * st], the neighbour k ^ 1 is lane ^ nb
+  template <bool WARP>
+  static __device__ __forceinline__ void fwd(cx<R>* d, const cx<R>* W, int k, cx<R>* xc, int sj,
+                                             int st, int nb) {
+    dft_dif<R, A>(d);
+    if constexpr (B > 0) {
+      if (WARP) __syncwarp();
+#pragma unroll
+      for (int r = 0; r < V; ++r) {
+        const int j = brevq(r, A);
+        xc[j * sj + k * st] = j ? d[r] * W[2 * j * k] : d[r];
+      }
+      sync<WARP>();
+      if constexpr (SPLIT) {
+        const int j = k >> 1, t = k & 1;
+#pragma unroll
+        for (int i = 0; i < V; ++i) d[i] = xc[j * sj + (t + 2 * i) * st];
+        dft_dif<R, A>(d);
+#pragma unroll
+        for (int i = 1; i < V; ++i) d[i] = d[i] * W[t * brevq(i, A) * (L / G)];
+        cx<R> e[V];
+#pragma unroll
+        for (int i = 0; i < V / 2; ++i) {
+          const cx<R> o = line_swap(line_sel<R>(t, d[i], d[i + V / 2]), nb);
+          const cx<R> a = line_sel<R>(t, o, d[i]), b = line_sel<R>(t, d[i + V / 2], o);
+          e[2 * i] = a + b;
+          e[2 * i + 1] = a - b;
+        }
+#pragma unroll
+        for (int i = 0; i < V; ++i) d[i] = e[i];
+      } else {
+#pragma unroll
+        for (int q = 0; q < V / G; ++q) {
+#pragma unroll
+          for (int t = 0; t < G; ++t) d[q * G + t] = xc[(k + G * q) * sj + t * st];
+          dft_dif<R, B>(d + q * G);
+        }
+      }
+    }
+  }
+  // the conjugate transpose
+  template <bool WARP>
+  static __device__ __forceinline__ void inv(cx<R>* d, const cx<R>* W, int k, cx<R>* xc, int sj,
+                                             int st, int nb) {
+    if constexpr (B > 0) {
+      if (WARP) __syncwarp();
+      if constexpr (SPLIT) {
+        const int j = k >> 1, t = k & 1;
+        cx<R> e[V];
+#pragma unroll
+        for (int i = 0; i < V / 2; ++i) {
+          const cx<R> a = d[2 * i] + d[2 * i + 1], b = d[2 * i] - d[2 * i + 1];
+          const cx<R> o = line_swap(line_sel<R>(t, a, b), nb);
+          e[i] = line_sel<R>(t, o, a);
+          e[i + V / 2] = line_sel<R>(t, b, o);
+        }
+#pragma unroll
+        for (int i = 0; i < V; ++i) d[i] = i ? cmulc(e[i], W[t * brevq(i, A) * (L / G)]) : e[i];
+        dft_dit<R, A>(d);
+#pragma unroll
+        for (int i = 0; i < V; ++i)
+          xc[j * sj + (t + 2 * i) * st] = cmulc(d[i], W[2 * j * (t + 2 * i)]);
+      } else {
+#pragma unroll
+        for (int q = 0; q < V / G; ++q) {
+          dft_dit<R, B>(d + q * G);
+          const int j = k + G * q;
+#pragma unroll
+          for (int t = 0; t < G; ++t)
+            xc[j * sj + t * st] = t ? cmulc(d[q * G + t], W[2 * j * t]) : d[q * G + t];
+        }
+      }
+      sync<WARP>();
+#pragma unroll
+      for (int r = 0; r < V; ++r) d[r] = xc[brevq(r, A) * sj + k * st];
+    }
+    dft_dit<R, A>(d);
+  }
+};
+
+// this CTA's family
+template <typename R>
+__device__ __forceinline__ const LineFam<R>& line_family(const LineSet<R>& S) {
+  int f = 0;
+#pragma unroll
+  for (int i = 1; i < kMaxFam; ++i)
+    if (i < S.nf && (int)blockIdx.x >= S.f[i].cta0) f = i;
+  return S.f[f];
+}
+
+// N consecutive elements, 32 bytes at a time where they fill that
+template <typename R, int N>
+__device__ __forceinline__ void st_run(cx<R>* p, const cx<R>* d) {
+  if constexpr (sizeof(R) == 4 && N % 4 == 0) {
+#pragma unroll
+    for (int i = 0; i < N; i += 4)
+      asm volatile("st.global.cs.v8.f32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(p + i),
+                   "f"(d[i].x), "f"(d[i].y), "f"(d[i + 1].x), "f"(d[i + 1].y), "f"(d[i + 2].x),
+                   "f"(d[i + 2].y), "f"(d[i + 3].x), "f"(d[i + 3].y)
+                   : "memory");
+  } else if constexpr (std::is_same<R, ff>::value && N % 2 == 0) {
+#pragma unroll
+    for (int i = 0; i < N; i += 2)
+      asm volatile("st.global.cs.v8.f32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(p + i),
+                   "f"(d[i].x.hi), "f"(d[i].x.lo), "f"(d[i].y.hi), "f"(d[i].y.lo),
+                   "f"(d[i + 1].x.hi), "f"(d[i + 1].x.lo), "f"(d[i + 1].y.hi), "f"(d[i + 1].y.lo)
+                   : "memory");
+  } else {
+#pragma unroll
+    for (int i = 0; i < N; ++i) st_stream(p + i, d[i]);
+  }
+}
+template <typename R, int N>
+__device__ __forceinline__ void ld_run(const cx<R>* p, cx<R>* d) {
+  if constexpr (sizeof(R) == 4 && N % 4 == 0) {
+#pragma unroll
+    for (int i = 0; i < N; i += 4)
+      asm volatile("ld.global.cs.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                   : "=f"(d[i].x), "=f"(d[i].y), "=f"(d[i + 1].x), "=f"(d[i + 1].y),
+                     "=f"(d[i + 2].x), "=f"(d[i + 2].y), "=f"(d[i + 3].x), "=f"(d[i + 3].y)
+                   : "l"(p + i)
+                   : "memory");
+  } else if constexpr (std::is_same<R, ff>::value && N % 2 == 0) {
+#pragma unroll
+    for (int i = 0; i < N; i += 2)
+      asm volatile("ld.global.cs.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                   : "=f"(d[i].x.hi), "=f"(d[i].x.lo), "=f"(d[i].y.hi), "=f"(d[i].y.lo),
+                     "=f"(d[i + 1].x.hi), "=f"(d[i + 1].x.lo), "=f"(d[i + 1].y.hi),
+                     "=f"(d[i + 1].y.lo)
+                   : "l"(p + i)
+                   : "memory");
+  } else {
+#pragma unroll
+    for (int i = 0; i < N; ++i) d[i] = ld_stream(p + i);
+  }
+}
+__device__ __forceinline__ c32 line_in(const c64& v, float) { return ccast<float>(v); }
+__device__ __forceinline__ cff line_in(const c64& v, ff) {
+  return mk<ff>(ff_split(v.x), ff_split(v.y));
+}
+__device__ __forceinline__ c64 line_out(const c32& v) { return mk<double>((double)v.x, (double)v.y); }
+__device__ __forceinline__ c64 line_out(const cff& v) {
+  return mk<double>(ff_join(v.x), ff_join(v.y));
+}
+
+// half par of a forward line: the entries x (xh: entry H) combined and rotated
+template <typename R, int V, int G>
+__device__ __forceinline__ void line_half(const cx<R>* x, const cx<R>& xh, const cx<R>* W, int k,
+                                          int par, cx<R>* d) {
+#pragma unroll
+  for (int r = 0; r < V; ++r) d[r] = x[r];
+  d[0] = par ? x[0] - xh : x[0] + xh;
+  if (par) {
+#pragma unroll
+    for (int r = 0; r < V; ++r) d[r] = d[r] * W[k + G * r];
+  }
+}
+
+template <typename R, int A, int B, bool INV, int MINB>
+__global__ void __launch_bounds__(HalfLine<R, A, B>::CY << B, MINB)
+k_ypair(LineSet<R> S, const cx<R>* __restrict__ twm, int twmax) {
+  using HL = HalfLine<R, A, B>;
+  constexpr int V = HL::V, G = HL::G, H = HL::H, L = HL::L, C = HL::CY;
+  extern __shared__ __align__(128) unsigned char smem_raw[];
+  cx<R>* W = reinterpret_cast<cx<R>*>(smem_raw);
+  const LineFam<R>& F = line_family(S);
+  const int c = threadIdx.x % C, k = threadIdx.x / C;
+  cx<R>* xc = W + L + c;
+  for (int e = threadIdx.x; e < L; e += C * G) W[e] = twm[e * (twmax / L)];
+  const int line = ((int)blockIdx.x - F.cta0) * C + c, lx = F.lx, n = F.n;
+  const bool on = line < F.lines;
+  const size_t rs = (size_t)1 << lx;
+  cx<R>* T = F.T + (on ? (((size_t)(line >> lx) << (A + B + 1 + lx)) + (line & ((1 << lx) - 1))) : 0);
+  cx<R> x[V], d[V], xh = mk<R>(0, 0);
+  if (!INV) {
+#pragma unroll
+    for (int r = 0; r < V; ++r)
+      x[r] = on && k + G * r < n ? ld_stream(T + (k + G * r) * rs) : mk<R>(0, 0);
+    if (on && k == 0 && n > H) xh = ld_stream(T + H * rs);
+  }
+  __syncthreads();
+#pragma unroll 1
+  for (int h = 0; h < 2; ++h) {
+    // forward: even, odd; inverse: odd, even
+    const int par = INV ? 1 - h : h;
+    cx<R>* xb = xc + h * (H * C);
+    if (!INV) {
+      line_half<R, V, G>(x, xh, W, k, par, d);
+      HL::template fwd<false>(d, W, k, xb, G * C, C, C & 31);
+    }
+#pragma unroll
+    for (int q = 0; q < HL::NRUN; ++q) {
+      constexpr int RUN = HL::RUN;
+      cx<R>* p = T + (par * H + HL::pos(q, k)) * rs;
+#pragma unroll
+      for (int t = 0; t < RUN; ++t) {
+        if (!INV) {
+          if (on) st_stream(p + t * rs, d[q * RUN + t]);
+        } else {
+          d[q * RUN + t] = on ? ld_stream(p + t * rs) : mk<R>(0, 0);
+        }
+      }
+    }
+    if (INV) {
+      HL::template inv<false>(d, W, k, xb, G * C, C, C & 31);
+      if (h == 0) {
+#pragma unroll
+        for (int r = 0; r < V; ++r) x[r] = cmulc(d[r], W[k + G * r]);
+      }
+    }
+  }
+  if (INV && on) {
+#pragma unroll
+    for (int r = 0; r < V; ++r)
+      if (k + G * r < n) st_stream(T + (k + G * r) * rs, d[r] + x[r]);
+    if (k == 0 && n > H) st_stream(T + H * rs, d[0] - x[0]);
+  }
+}
+
+template <typename R, int A, int B, bool INV, int MINB>
+__global__ void __launch_bounds__(XP_TPB, MINB) k_xpair(LineSet<R> S, const cx<R>* __restrict__ twm,
+                                                        int twmax) {
+  using HL = HalfLine<R, A, B>;
+  constexpr int V = HL::V, G = HL::G, H = HL::H, L = HL::L, C = HL::CX;
+  extern __shared__ __align__(128) unsigned char smem_raw[];
+  cx<R>* W = reinterpret_cast<cx<R>*>(smem_raw);
+  const LineFam<R>& F = line_family(S);
+  const int c = threadIdx.x / G, k = threadIdx.x % G;
+  cx<R>* xc = W + L + c * HL::LS;
+  for (int e = threadIdx.x; e < L; e += XP_TPB) W[e] = twm[e * (twmax / L)];
+  const int line = ((int)blockIdx.x - F.cta0) * C + c, n = F.n;
+  const bool on = line < F.lines;
+  const int z = on ? line / F.ny : 0, y = on ? line - z * F.ny : 0;
+  cx<R>* T = F.T + ((((size_t)z << F.ly) + y) << (A + B + 1));
+  const int32_t* map = F.map + (size_t)(on ? line : 0) * n;
+  int id[V], ih = -1;
+#pragma unroll
+  for (int r = 0; r < V; ++r) id[r] = on && k + G * r < n ? map[k + G * r] : -1;
+  if (on && k == 0 && n > H) ih = map[H];
+  cx<R> x[V], d[V], xh = mk<R>(0, 0);
+  if (!INV) {
+#pragma unroll
+    for (int r = 0; r < V; ++r) x[r] = id[r] >= 0 ? line_in(F.io[id[r]], R()) : mk<R>(0, 0);
+    if (ih >= 0) xh = line_in(F.io[ih], R());
+  }
+  __syncthreads();
+#pragma unroll 1
+  for (int h = 0; h < 2; ++h) {
+    const int par = INV ? 1 - h : h;
+    if (!INV) {
+      line_half<R, V, G>(x, xh, W, k, par, d);
+      HL::template fwd<true>(d, W, k, xc, HL::SJ, 1, 1);
+    }
+#pragma unroll
+    for (int q = 0; q < HL::NRUN; ++q) {
+      constexpr int RUN = HL::RUN;
+      cx<R>* p = T + par * H + HL::pos(q, k);
+      if (!INV) {
+        if (on) st_run<R, RUN>(p, d + q * RUN);
+      } else {
+        ld_run<R, RUN>(p, d + q * RUN);  // (a line past the last reads the first one's)
+      }
+    }
+    if (INV) {
+      HL::template inv<true>(d, W, k, xc, HL::SJ, 1, 1);
+      if (h == 0) {
+#pragma unroll
+        for (int r = 0; r < V; ++r) x[r] = cmulc(d[r], W[k + G * r]);
+      }
+    }
+  }
+  if (INV) {
+#pragma unroll
+    for (int r = 0; r < V; ++r)
+      if (id[r] >= 0) F.io[id[r]] = line_out(d[r] + x[r]);
+    if (ih >= 0) F.io[ih] = line_out(d[0] - x[0]);
+  }
+}
+
 // --------------------------------------------------------------------------- z passes
 
 // The six P spectra (blocks 00, 11, 22, 01, 02, 12) in the y/z-folded form (Spectrum::yz) and
@@ -433,9 +792,6 @@ __device__ __forceinline__ cx<R> spec_cx(const void* p, size_t i) {
   return mk<R>(R(v.x), R(v.y));
 }
 
-__device__ __forceinline__ int brevn(int v, int n) {
-  return n ? (int)(__brev((unsigned)v) >> (32 - n)) : 0;
-}
 // folded frequency at DIF position p of a length-2^n axis
 __device__ __forceinline__ int fold_pos(int p, int n) {
   const int k = brevn(p, n), L = 1 << n;
@@ -981,7 +1337,7 @@ __global__ void __launch_bounds__(ZTPB, 4) k_zedge_staged(EdgeSet E, int nzs, in
 // What bounds them: FP32 instruction issue and loads, float-float the FP32 pipes; the pruning
 // halves the arithmetic of the padded transforms. z passes of an operator application at
 // 128x128x64, faces + edges: FP32 267 us in the direct and staged forms, 169 here (93 + 72);
-// float-float 2541 us direct, 1491 here. FP64 stays direct (see conv_all_t).
+// float-float 2541 us direct, 1382 here. FP64 stays direct (see conv_all_t).
 template <typename R>
 struct ZPairJob {
   cx<R>* T[3];        // face families (edges: T[0] only)
@@ -1438,6 +1794,9 @@ struct Plans {
 };
 
 template <typename R>
+struct LinePass;
+
+template <typename R>
 struct Launch {
   static cx<R>* buf(const Family& f) { return reinterpret_cast<cx<R>*>(f.T[slot_of<R>()]); }
   // kind 0: forward x, 1: inverse x, 2: forward y, 3: inverse y; io[f]: the compact
@@ -1445,10 +1804,13 @@ struct Launch {
   static int pass(int kind, const Family* F, int nfam, c64* const* io, const cx<R>* tw,
                   int twmax, cudaStream_t st) {
     PassSet<R> s{};
+    bool done[kMaxFam] = {};
+    if constexpr (!std::is_same<R, double>::value)
+      CTX_CHECK(LinePass<R>::run(kind, F, nfam, io, tw, twmax, st, done));
     int ctas = 0;
     size_t sm = 0;
     for (int f = 0; f < nfam; ++f) {
-      if (!F[f].active) continue;
+      if (!F[f].active || done[f]) continue;
       if (s.nf == kMaxFam) return set_error("too many families in one pass"), PEEC_ERR_UNSUPPORTED_INTERNAL;
       const Family& fam = F[f];
       FamPass<R>& d = s.f[s.nf++];
@@ -1525,6 +1887,73 @@ struct Launch {
     CTX_CHECK(smem_optin(kern, sm));
     dim3 g((f.L[0] + TX - 1) / TX, f.L[1]);
     kern<<<g, ZTPB, sm, st>>>(buf(f), f.dims[2], s, f.L[0], f.L[1], p, tw, twmax);
+    return 0;
+  }
+};
+
+// x and y passes as pairs: kinds as in Launch::pass; a launch per circulant length, done[f]:
+// family f was taken (lengths 2 to 512)
+template <typename R>
+struct LinePass {
+  template <int A, int B>
+  static int launch(int kind, LineSet<R>& S, const cx<R>* tw, int twmax, cudaStream_t st) {
+    using HL = HalfLine<R, A, B>;
+    int ctas = 0;
+    const int C = kind < 2 ? HL::CX : HL::CY;
+    for (int i = 0; i < S.nf; ++i) {
+      S.f[i].cta0 = ctas;
+      ctas += (S.f[i].lines + C - 1) / C;
+    }
+    // registers: 80 or 128 (FP32), 128 or 168 (float-float)
+    constexpr int MINX = sizeof(R) == 4 ? (HL::V == 16 ? 4 : 6) : (HL::V == 16 ? 3 : 4);
+    constexpr int MINY = HL::CY > HL::CX ? (MINX / 2 > 0 ? MINX / 2 : 1) : MINX;
+    void (*kern)(LineSet<R>, const cx<R>*, int) =
+        kind == 0   ? k_xpair<R, A, B, false, MINX>
+        : kind == 1 ? k_xpair<R, A, B, true, MINX>
+        : kind == 2 ? k_ypair<R, A, B, false, MINY>
+                    : k_ypair<R, A, B, true, MINY>;
+    const size_t sm = HL::smem(kind < 2);
+    CTX_CHECK(smem_optin(kern, sm));
+    kern<<<ctas, C << B, sm, st>>>(S, tw, twmax);
+    return 0;
+  }
+  static int run(int kind, const Family* F, int nfam, c64* const* io, const cx<R>* tw, int twmax,
+                 cudaStream_t st, bool* done) {
+    const int ax = kind < 2 ? 0 : 1;
+    for (int f = 0; f < nfam; ++f) {
+      if (done[f] || !line_pair_ok(F[f], ax)) continue;
+      LineSet<R> S{};
+      for (int g = f; g < nfam; ++g) {
+        if (done[g] || !line_pair_ok(F[g], ax) || F[g].L[ax] != F[f].L[ax]) continue;
+        LineFam<R>& d = S.f[S.nf++];
+        d.T = Launch<R>::buf(F[g]);
+        d.map = F[g].map;
+        d.io = io ? io[g] : nullptr;
+        d.lx = F[g].logL[0];
+        d.ly = F[g].logL[1];
+        d.n = F[g].dims[ax];
+        d.ny = F[g].dims[1];
+        d.lines = ax == 0 ? F[g].dims[1] * F[g].dims[2] : F[g].dims[2] << F[g].logL[0];
+        done[g] = true;
+      }
+      // H = V G: four entries a thread up to H = 16, then eight, sixteen at H = 256
+      switch (F[f].logL[ax] - 1) {
+        case 0: CTX_CHECK((launch<0, 0>(kind, S, tw, twmax, st))); break;
+        case 1: CTX_CHECK((launch<1, 0>(kind, S, tw, twmax, st))); break;
+        case 2: CTX_CHECK((launch<2, 0>(kind, S, tw, twmax, st))); break;
+        case 3: CTX_CHECK((launch<2, 1>(kind, S, tw, twmax, st))); break;
+        case 4: CTX_CHECK((launch<2, 2>(kind, S, tw, twmax, st))); break;
+        case 5: CTX_CHECK((launch<3, 2>(kind, S, tw, twmax, st))); break;
+        case 6: CTX_CHECK((launch<3, 3>(kind, S, tw, twmax, st))); break;
+        case 7:
+          // FP32 forward y: sixteen entries a thread keep more rows in flight (52 against 60 us at
+          // 128x128x64; inverse y 76 against 67, x 53 against 50)
+          if (sizeof(R) == 4 && kind == 2) CTX_CHECK((launch<4, 3>(kind, S, tw, twmax, st)));
+          else CTX_CHECK((launch<3, 4>(kind, S, tw, twmax, st)));
+          break;
+        default: CTX_CHECK((launch<4, 4>(kind, S, tw, twmax, st))); break;
+      }
+    }
     return 0;
   }
 };
