@@ -97,13 +97,13 @@ void launch_xupdate(const c64*, const cff*, size_t, const c64*, const c64*, int,
                     cudaStream_t);
 int fill_rows_rcc_gpu(const double origin[3], double sx, double sy, double sz, double escal_Lp,
                       double escal_P, int Nx, int Ny, int Nz, double* const d_rows[9],
-                      const int64_t row_len[9], int* d_bad, cudaStream_t st);
+                      const int64_t row_len[9], int* d_bad, cudaMemPool_t pool, cudaStream_t st);
 int rcc_rows_gpu(const double origin[3], double sx, double sy, double sz, int Nx, int Ny, int Nz,
                  double beta, const double* const d_qs[9], double* const d_re[9],
                  double* const d_im[9], const int64_t row_len[9], cudaStream_t st);
 int fill_rows_gpu(const double origin[3], double sx, double sy, double sz, double escal_Lp,
                   double escal_P, int Nx, int Ny, int Nz, double* const d_rows[9],
-                  const int64_t row_len[9], int* d_bad, cudaStream_t st);
+                  const int64_t row_len[9], int* d_bad, cudaMemPool_t pool, cudaStream_t st);
 size_t ris_box_bytes();
 int ris_prep_gpu(int surfaces, const double* d_geom, int64_t count, int64_t mx, int64_t my,
                  void* boxes, double* self, int* nrm, cudaStream_t st);
@@ -131,6 +131,8 @@ struct LevelTri {  // triangular factor without its diagonal (CSR) and its level
   std::vector<int32_t> hptr, hcol;  // host copy of the structure
   bool unit = false;                // the diagonal is one
 };
+
+constexpr uint64_t POOL_KEEP = (uint64_t)1 << 30;
 
 struct peec_ctx {
   int dev = 0;
@@ -180,6 +182,9 @@ struct peec_ctx {
   Spectrum spec[9];
   void* ph64[3] = {nullptr, nullptr, nullptr};  // face-grid phase tables
   void* ph32[3] = {nullptr, nullptr, nullptr};  // their FP32 rounding (FP32 z passes)
+  // scratch of fills and spectra: up to POOL_KEEP bytes stay mapped between calls, given back
+  // with the context
+  cudaMemPool_t pool = nullptr;
   int* zerr = nullptr;  // set by a staged z pass whose copy wait ran into its limit
   int nsm = 0;          // SM count of the device
   ZTune zt;             // FP32 z-pass forms chosen by the tuner for this context's grids
@@ -446,6 +451,14 @@ static int peec_ctx_create_body(peec_ctx** out, int device) {
   if (cudaMalloc(&ctx->zerr, sizeof(int)) != cudaSuccess ||
       cudaMemset(ctx->zerr, 0, sizeof(int)) != cudaSuccess)
     return fail(fail_cuda(cudaErrorMemoryAllocation, "cudaMalloc error word", __FILE__, __LINE__));
+  cudaMemPoolProps pp = {};
+  pp.allocType = cudaMemAllocationTypePinned;
+  pp.location.type = cudaMemLocationTypeDevice;
+  pp.location.id = device;
+  uint64_t keep = POOL_KEEP;
+  if (cudaMemPoolCreate(&ctx->pool, &pp) != cudaSuccess) ctx->pool = nullptr;
+  else cudaMemPoolSetAttribute(ctx->pool, cudaMemPoolAttrReleaseThreshold, &keep);
+  cudaGetLastError();
   cudaMallocHost(&ctx->hsmall, sizeof(c64) * 16 * 4096);
   cudaMallocHost(&ctx->hread, sizeof(c64) * 4096);
   cudaMallocHost(&ctx->hscal, sizeof(double) * 64);
@@ -506,6 +519,7 @@ extern "C" void peec_ctx_destroy(peec_ctx* ctx) {
     if (ctx->ph32[a]) cudaFree(ctx->ph32[a]);
   }
   cudaFree(ctx->zerr);
+  if (ctx->pool) cudaMemPoolDestroy(ctx->pool);
   free_tri(ctx->Lf);
   free_tri(ctx->Uf);
   cudaFree(ctx->sf_ord);
@@ -1095,7 +1109,7 @@ struct ZChoice {
 };
 static std::mutex g_tune_mu;
 static std::map<std::vector<int>, ZChoice> g_tune;
-static int check_solve_errors(peec_ctx* ctx);
+static int check_solve_errors(peec_ctx* ctx, bool staged = false);
 
 static int tune_zpass(peec_ctx* ctx) {
   ctx->zt.err = ctx->zerr;
@@ -1177,7 +1191,7 @@ static int tune_zpass(peec_ctx* ctx) {
     CTX_TRY(timed(z, 1, &ms));
     if (ms < best) c.edge = 3;
   }
-  CTX_TRY(check_solve_errors(ctx));
+  CTX_TRY(check_solve_errors(ctx, true));
   {
     std::lock_guard<std::mutex> lock(g_tune_mu);
     g_tune[key] = c;
@@ -1206,7 +1220,7 @@ static int build_spectrum_set(peec_ctx* ctx, Spectrum* dst, double* const d_rows
     jobs[nj++] = SpecJob{&dst[i], d_rows[srow[i]], ctx->row_dims[srow[i]], ctx->fam[fout[i]].dims,
                          ctx->fam[fin[i]].dims, sdim[i], odim[i], sym ? 1 : 0};
   }
-  CTX_TRY(spectra_build(jobs, nj, ctx->tw64, ctx->twmax, ctx->st));
+  CTX_TRY(spectra_build(jobs, nj, ctx->tw64, ctx->twmax, ctx->pool, ctx->st));
   ctx->launches += nj ? 3 + nj : 0;
   return PEEC_OK;
 }
@@ -1234,16 +1248,16 @@ static int peec_set_rows_body(peec_ctx* ctx, const double* const rows[9]) {
   for (int i = 0; i < 9 && rc == PEEC_OK; ++i) {
     const size_t len = (size_t)ctx->row_dims[i][0] * ctx->row_dims[i][1] * ctx->row_dims[i][2];
     if (len == 0 || !rows[i]) continue;
-    if (cudaMalloc(&d_rows[i], len * sizeof(double)) != cudaSuccess) {
+    if (scratch_alloc((void**)&d_rows[i], len * sizeof(double), ctx->pool, ctx->st) != cudaSuccess) {
       rc = bad(ctx, PEEC_ERR_OOM, "row upload allocation");
       break;
     }
     cudaMemcpyAsync(d_rows[i], rows[i], len * sizeof(double), cudaMemcpyHostToDevice, ctx->st);
   }
   if (rc == PEEC_OK) rc = build_spectra(ctx, d_rows);
-  cudaStreamSynchronize(ctx->st);
   for (auto p : d_rows)
-    if (p) cudaFree(p);
+    if (p) cudaFreeAsync(p, ctx->st);
+  cudaStreamSynchronize(ctx->st);
   return rc;
 }
 
@@ -1258,18 +1272,19 @@ static int peec_fill_body(peec_ctx* ctx, const double origin[3], double sx, doub
   int64_t len[9];
   int rc = PEEC_OK;
   int* d_bad = nullptr;
-  PEEC_CUDA_TRY(cudaMalloc(&d_bad, sizeof(int)));
+  PEEC_CUDA_TRY(scratch_alloc((void**)&d_bad, sizeof(int), ctx->pool, ctx->st));
   PEEC_CUDA_TRY(cudaMemsetAsync(d_bad, 0, sizeof(int), ctx->st));
   for (int i = 0; i < 9; ++i) {
     len[i] = (int64_t)ctx->row_dims[i][0] * ctx->row_dims[i][1] * ctx->row_dims[i][2];
-    if (len[i] > 0 && cudaMalloc(&d_rows[i], len[i] * sizeof(double)) != cudaSuccess) {
+    if (len[i] > 0 && scratch_alloc((void**)&d_rows[i], len[i] * sizeof(double), ctx->pool,
+                                    ctx->st) != cudaSuccess) {
       rc = bad(ctx, PEEC_ERR_OOM, "row allocation");
       break;
     }
   }
   if (rc == PEEC_OK) {
     rc = fill_rows_gpu(origin, sx, sy, sz, escal_Lp, escal_P, ctx->Nx, ctx->Ny, ctx->Nz, d_rows,
-                       len, d_bad, ctx->st);
+                       len, d_bad, ctx->pool, ctx->st);
     ctx->launches += 9;
     if (rc) ctx->err = g_err;
   }
@@ -1289,10 +1304,10 @@ static int peec_fill_body(peec_ctx* ctx, const double origin[3], double sx, doub
                         ctx->st);
   }
   if (rc == PEEC_OK) rc = build_spectra(ctx, d_rows);
-  cudaStreamSynchronize(ctx->st);
   for (auto p : d_rows)
-    if (p) cudaFree(p);
-  cudaFree(d_bad);
+    if (p) cudaFreeAsync(p, ctx->st);
+  cudaFreeAsync(d_bad, ctx->st);
+  cudaStreamSynchronize(ctx->st);
   return rc;
 }
 
@@ -1331,10 +1346,10 @@ static int peec_fill_rcc_body(peec_ctx* ctx, const double origin[3], double sx, 
   ctx->have_rcc_rows = false;
   CTX_TRY(rcc_alloc_rows(ctx, len));
   int* d_bad = nullptr;
-  PEEC_CUDA_TRY(cudaMalloc(&d_bad, sizeof(int)));
+  PEEC_CUDA_TRY(scratch_alloc((void**)&d_bad, sizeof(int), ctx->pool, ctx->st));
   cudaMemsetAsync(d_bad, 0, sizeof(int), ctx->st);
   int rc = fill_rows_rcc_gpu(origin, sx, sy, sz, escal_Lp, escal_P, ctx->Nx, ctx->Ny, ctx->Nz,
-                             ctx->rcc_qs, len, d_bad, ctx->st);
+                             ctx->rcc_qs, len, d_bad, ctx->pool, ctx->st);
   ctx->launches += 9;
   if (rc) ctx->err = g_err;
   int hbad = 0;
@@ -1350,7 +1365,7 @@ static int peec_fill_rcc_body(peec_ctx* ctx, const double origin[3], double sx, 
       rc = bad(ctx, PEEC_ERR_UNSUPPORTED,
                "fill_rcc: a row entry is not finite (degenerate cell sizes?)");
   }
-  cudaFree(d_bad);
+  cudaFreeAsync(d_bad, ctx->st);
   if (rc != PEEC_OK) return rc;
   if (rows_out)
     for (int i = 0; i < 9; ++i)
@@ -1407,8 +1422,8 @@ static int peec_set_rcc_frequency_body(peec_ctx* ctx, double freq_hz) {
   for (int i = 0; i < 9 && rc == PEEC_OK; ++i) {
     len[i] = (int64_t)ctx->row_dims[i][0] * ctx->row_dims[i][1] * ctx->row_dims[i][2];
     if (len[i] == 0) continue;
-    if (cudaMallocAsync(&re[i], len[i] * sizeof(double), ctx->st) != cudaSuccess ||
-        cudaMallocAsync(&im[i], len[i] * sizeof(double), ctx->st) != cudaSuccess)
+    if (scratch_alloc((void**)&re[i], len[i] * sizeof(double), ctx->pool, ctx->st) != cudaSuccess ||
+        scratch_alloc((void**)&im[i], len[i] * sizeof(double), ctx->pool, ctx->st) != cudaSuccess)
       rc = bad(ctx, PEEC_ERR_OOM, "Rcc phased rows");
   }
   drop_graphs(ctx);
@@ -2231,20 +2246,24 @@ static void lu_solve(peec_ctx* ctx, const c64* b, const NodeSums* S, c64* x) {
   ctx->launches += 1;
 }
 
-// A triangular-solve wait that ran into its limit leaves an error word on the device;
-// entry points read it once their work is complete.
-static int check_solve_errors(peec_ctx* ctx) {
-  int e = 0, ez = 0;
-  if (ctx->sf_ctl)
-    PEEC_CUDA_TRY(cudaMemcpyAsync(&e, ctx->sf_ctl + 2, sizeof(int), cudaMemcpyDeviceToHost, ctx->st));
-  if (ctx->zerr)
-    PEEC_CUDA_TRY(cudaMemcpyAsync(&ez, ctx->zerr, sizeof(int), cudaMemcpyDeviceToHost, ctx->st));
+// A wait that ran into its limit leaves an error word on the device; entry points read it once
+// their work is complete. Only the synchronisation-free solves (rows outside the LU groups) and
+// the staged z passes wait, so the words of the others are not fetched; the copies go to pinned
+// memory behind the work, and the stream is synchronised once. staged: staged passes ran that
+// the context's own forms do not name (the tuner's).
+static int check_solve_errors(peec_ctx* ctx, bool staged) {
+  int* h = reinterpret_cast<int*>(ctx->hscal + 62);
+  h[0] = h[1] = 0;
+  if (ctx->sf_ctl && ctx->sf_total > 0)
+    PEEC_CUDA_TRY(cudaMemcpyAsync(h, ctx->sf_ctl + 2, sizeof(int), cudaMemcpyDeviceToHost, ctx->st));
+  if (ctx->zerr && (staged || ctx->zt.face == 2 || ctx->zt.edge == 2))
+    PEEC_CUDA_TRY(cudaMemcpyAsync(h + 1, ctx->zerr, sizeof(int), cudaMemcpyDeviceToHost, ctx->st));
   PEEC_CUDA_TRY(cudaStreamSynchronize(ctx->st));
-  if (e) {
+  if (h[0]) {
     cudaMemsetAsync(ctx->sf_ctl + 2, 0, sizeof(int), ctx->st);
     return bad(ctx, PEEC_ERR_TIMEOUT, "LU solve: a row dependency wait ran into its limit");
   }
-  if (ez) {
+  if (h[1]) {
     cudaMemsetAsync(ctx->zerr, 0, sizeof(int), ctx->st);
     return bad(ctx, PEEC_ERR_TIMEOUT, "z pass: a staged tile copy wait ran into its limit");
   }
@@ -2398,12 +2417,11 @@ static int peec_matvec_dev_body(peec_ctx* ctx, const void* x, void* y, int preci
   if (precision < 0 || precision > 2) return bad(ctx, PEEC_ERR_BADARG, "precision must be 0, 1 or 2");
   PEEC_CUDA_TRY(cudaSetDevice(ctx->dev));
   CTX_TRY(matvec_dev(ctx, (const c64*)x, (c64*)y, precision, true));
-  PEEC_CUDA_TRY(cudaEventSynchronize(ctx->ev[2]));
+  const int rc = check_solve_errors(ctx);  // waits for the stream
   cudaEventElapsedTime(&ctx->t_total, ctx->ev[0], ctx->ev[2]);
   cudaEventElapsedTime(&ctx->t_conv, ctx->ev[0], ctx->ev[1]);
   cudaEventElapsedTime(&ctx->t_sparse, ctx->ev[1], ctx->ev[2]);
-  CTX_TRY(check_solve_errors(ctx));
-  return PEEC_OK;
+  return rc;
 }
 
 static int peec_matvec_body(peec_ctx* ctx, const double* x, double* y, int precision) {

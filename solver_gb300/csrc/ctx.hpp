@@ -150,6 +150,12 @@ size_t gm_part_doubles(size_t N, int k);
 int gm_pre(const GmBody& B);   // returns the kernels launched
 int gm_post(const GmBody& B);
 
+// Stream-ordered scratch from a context's pool (nullptr: the device's default pool, which gives
+// its memory back at every synchronisation and maps it again at the next allocation)
+inline cudaError_t scratch_alloc(void** p, size_t bytes, cudaMemPool_t pool, cudaStream_t st) {
+  return pool ? cudaMallocFromPoolAsync(p, bytes, pool, st) : cudaMallocAsync(p, bytes, st);
+}
+
 #define CTX_CHECK(expr)      \
   do {                       \
     int _r = (expr);         \
@@ -234,6 +240,7 @@ struct SpecJob {
   const int *M, *na, *nb, *sdim, *odim;
   int symmetric;
 };
-int spectra_build(const SpecJob* jobs, int njobs, const void* tw64, int twmax, cudaStream_t st);
+int spectra_build(const SpecJob* jobs, int njobs, const void* tw64, int twmax, cudaMemPool_t pool,
+                  cudaStream_t st);
 
 }  // namespace peec

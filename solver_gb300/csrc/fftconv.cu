@@ -308,7 +308,7 @@ static int spec_axis(SpecSet& S, const c64* tw, int twmax, cudaStream_t st) {
   return spec_pass<AX, 0>(S, ctas, tw, twmax, st);
 }
 
-int spectra_build(const SpecJob* jobs, int njobs, const void* tw64, int twmax, cudaStream_t st) {
+int spectra_build(const SpecJob* jobs, int njobs, const void* tw64, int twmax, cudaMemPool_t pool, cudaStream_t st) {
   if (njobs <= 0) return 0;
   if (njobs > kSpecRows) return set_error("too many spectra"), PEEC_ERR_UNSUPPORTED_INTERNAL;
   SpecSet set{};
@@ -335,7 +335,7 @@ int spectra_build(const SpecJob* jobs, int njobs, const void* tw64, int twmax, c
     no += (size_t)(S.L[0] / 2 + 1) * (S.L[1] / 2 + 1) * (S.L[2] / 2 + 1);
   }
   double* scr = nullptr;
-  PEEC_CUDA_TRY(cudaMallocAsync(&scr, (na + nb + no + 1) * sizeof(double), st));
+  PEEC_CUDA_TRY(scratch_alloc((void**)&scr, (na + nb + no + 1) * sizeof(double), pool, st));
   size_t oa = 0, ob = na, oo = na + nb;
   for (int i = 0; i < njobs; ++i) {
     SpecRow& R = set.r[i];

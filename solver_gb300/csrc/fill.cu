@@ -909,7 +909,7 @@ static int face_normal(int caser, const double s[3]) {
 static int fill_rows_any(const double origin[3], double sx, double sy, double sz,
                          double escal_Lp, double escal_P, int Nx, int Ny, int Nz,
                          double* const d_rows[9], const int64_t row_len[9], int* d_bad,
-                         cudaStream_t st, int rcc) {
+                         cudaMemPool_t pool, cudaStream_t st, int rcc) {
   RowSet S{};
   int maxM = 1, maxz = 1;
   const int lpM[3][3] = {{Nx - 1, Ny, Nz}, {Nx, Ny - 1, Nz}, {Nx, Ny, Nz - 1}};
@@ -980,7 +980,7 @@ static int fill_rows_any(const double origin[3], double sx, double sy, double sz
   int32_t *map = nullptr, *rank = nullptr;
   int* cnt = nullptr;
   const size_t list_bytes = lists * (2 * sizeof(double) + 2 * sizeof(int32_t)) + 27 * sizeof(int);
-  PEEC_CUDA_TRY(cudaMallocAsync((void**)&val, list_bytes, st));
+  PEEC_CUDA_TRY(scratch_alloc((void**)&val, list_bytes, pool, st));
   scr = val + lists;
   map = reinterpret_cast<int32_t*>(scr + lists);
   rank = map + lists;
@@ -1017,7 +1017,7 @@ static int fill_rows_any(const double origin[3], double sx, double sy, double sz
         tab = nullptr;
         tab_cap = std::max(tab_cap, most);
         near_cap = std::max(near_cap, cells);
-        PEEC_CUDA_TRY(cudaMallocAsync((void**)&tab, tab_cap * (sizeof(double) + 1) + near_cap, st));
+        PEEC_CUDA_TRY(scratch_alloc((void**)&tab, tab_cap * (sizeof(double) + 1) + near_cap, pool, st));
         need = reinterpret_cast<uint8_t*>(tab + tab_cap);
         near = need + tab_cap;
       }
@@ -1050,16 +1050,16 @@ static int fill_rows_any(const double origin[3], double sx, double sy, double sz
 
 int fill_rows_gpu(const double origin[3], double sx, double sy, double sz, double escal_Lp,
                   double escal_P, int Nx, int Ny, int Nz, double* const d_rows[9],
-                  const int64_t row_len[9], int* d_bad, cudaStream_t st) {
+                  const int64_t row_len[9], int* d_bad, cudaMemPool_t pool, cudaStream_t st) {
   return fill_rows_any(origin, sx, sy, sz, escal_Lp, escal_P, Nx, Ny, Nz, d_rows, row_len, d_bad,
-                       st, 0);
+                       pool, st, 0);
 }
 
 int fill_rows_rcc_gpu(const double origin[3], double sx, double sy, double sz, double escal_Lp,
                       double escal_P, int Nx, int Ny, int Nz, double* const d_rows[9],
-                      const int64_t row_len[9], int* d_bad, cudaStream_t st) {
+                      const int64_t row_len[9], int* d_bad, cudaMemPool_t pool, cudaStream_t st) {
   return fill_rows_any(origin, sx, sy, sz, escal_Lp, escal_P, Nx, Ny, Nz, d_rows, row_len, d_bad,
-                       st, 1);
+                       pool, st, 1);
 }
 
 // ---------------------------------------------------------------------------------
