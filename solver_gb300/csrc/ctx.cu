@@ -2076,6 +2076,13 @@ static int peec_lu_refactor_setup_body(peec_ctx* ctx, int64_t yle_nnz, const int
   R.nL = nL;
   R.nU = nU;
   R.lvl_off = L.lvl_off;
+  R.lvl_cap.assign(L.lvl_off.size(), 1);
+  for (size_t l = 0; l + 1 < L.lvl_off.size(); ++l)
+    for (int i = L.lvl_off[l]; i < L.lvl_off[l + 1]; ++i) {
+      const int r = L.rows[i];
+      R.lvl_cap[l] = std::max(R.lvl_cap[l], (int)(L.hptr[r + 1] - L.hptr[r] + U.hptr[r + 1] -
+                                                  U.hptr[r] + 1));
+    }
   std::vector<int32_t> lrows(L.rows.begin(), L.rows.end());
   CTX_TRY(upload(&R.asm_ptr, aptr, ctx->st));
   CTX_TRY(upload(&R.asm_src, asrc, ctx->st));

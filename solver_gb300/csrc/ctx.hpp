@@ -97,6 +97,7 @@ struct RefactorPlan {
   uint32_t* asm_src = nullptr;   // contribution codes (type << 30 | index)
   int32_t* rows = nullptr;       // rows grouped by L level
   std::vector<int> lvl_off;      // level offsets into rows (host)
+  std::vector<int> lvl_cap;      // most entries (L, diagonal, U) of a level's rows (host)
   int32_t* upd_off = nullptr;    // per L entry (p, k): its targets in upd_tgt
   int32_t* upd_tgt = nullptr;    // per entry of U(k,:): its slot in row p
   c64* D = nullptr;              // diagonal of U

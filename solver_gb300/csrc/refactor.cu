@@ -10,7 +10,7 @@
 //   assemble: every slot of L (off-diagonal), of the diagonal D and of U (off-diagonal)
 //             is the sum of its SS contributions, in a fixed order per slot (edges'
 //             +-1/DZ, surfaces' jw/P, Yle entries); slots of fill start at zero
-//   rows:     up-looking, one thread per permuted row, rows of one L level per launch
+//   rows:     up-looking, a group of lanes per permuted row, rows of one L level per launch
 //             (a row depends on the rows of its L pattern, all of earlier levels):
 //               for k in L(p,:) in increasing order: L(p,k) = w(k) / D(k);
 //                 w(j) -= L(p,k) U(k,j) for j in U(k,:)   (targets precomputed)
@@ -20,6 +20,8 @@
 namespace peec {
 
 // contribution codes of asm_src: type in the top two bits, index below
+constexpr int RF_TPB = 128;
+constexpr int RF_WIDE = 152 * 32;  // rows of a level that get a warp each at most
 constexpr uint32_t RF_EDGE_DIAG = 0u, RF_EDGE_OFF = 1u, RF_SURF = 2u, RF_YLE = 3u;
 
 __global__ void k_rf_assemble(int64_t nslot, const int64_t* __restrict__ ptr,
@@ -47,37 +49,112 @@ __global__ void k_rf_assemble(int64_t nslot, const int64_t* __restrict__ ptr,
   }
 }
 
+// x / d from r = 1 / d rounded to nearest: the quotient's estimate corrected by its remainder
+// (Markstein, IBM J. Res. Dev. 34, 1990), three dependent operations where a division takes some
+// ten; plain division where the reciprocal leaves the range the correction needs
+__device__ __forceinline__ double rf_quot(double x, double d, double r) {
+  const double q = x * r;
+  const double y = fma(fma(-q, d, x), r, q);
+  return r > 1e-250 && r < 1e250 ? y : x / d;
+}
+
 // upd_tgt codes: -1 the row's own diagonal; bit 30 set: U.val index (low 30 bits); else
 // L.val index
-__global__ void k_rf_rows(const int32_t* __restrict__ rows, int nrows, SfTri L, SfTri U, c64* D,
-                          const int32_t* __restrict__ upd_off, const int32_t* __restrict__ upd_tgt,
-                          int* err) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= nrows) return;
+//
+// LN lanes a row: the L entries in order, each one's updates over the lanes (a row's slots are
+// distinct, and each gets its updates in the order of the L entries, so the sums are those of
+// one thread). The row is worked on in shared memory (SM; cap: its entries at most), and the next
+// entry's pivot and first updates are on their way while one is applied: what is left of an
+// entry's latency is a quotient, a complex product and a difference, some 0.3 us. One thread a row, in
+// global memory, took 25 to 41 us a level (22 levels 0.93 ms at 128x128x64, 18 levels 0.46 ms at
+// 48x48x24); they take 0.72 and 0.31 ms so.
+template <int LN, bool SM>
+__global__ void __launch_bounds__(RF_TPB) k_rf_rows(const int32_t* __restrict__ rows, int nrows,
+                                                    SfTri L, SfTri U, c64* D,
+                                                    const int32_t* __restrict__ upd_off,
+                                                    const int32_t* __restrict__ upd_tgt, int cap,
+                                                    int* err) {
+  extern __shared__ __align__(16) unsigned char rf_smem[];
+  const int g = threadIdx.x / LN, lane = threadIdx.x % LN;
+  const int t = blockIdx.x * (RF_TPB / LN) + g;
+  if (t >= nrows) return;  // whole groups
+  const unsigned mask =
+      LN == 32 ? 0xffffffffu : ((1u << (LN & 31)) - 1u) << ((threadIdx.x & 31) / LN * LN);
   const int p = rows[t];
   c64* Lval = const_cast<c64*>(L.val);
   c64* Uval = const_cast<c64*>(U.val);
-  for (int q = L.ptr[p]; q < L.ptr[p + 1]; ++q) {
-    const int k = L.col[q];
-    const c64 dk = D[k];
-    const double den = dk.x * dk.x + dk.y * dk.y;
-    const c64 w = Lval[q];
-    const c64 l = mk<double>((w.x * dk.x + w.y * dk.y) / den, (w.y * dk.x - w.x * dk.y) / den);
-    Lval[q] = l;
-    const int u0 = U.ptr[k];
-    for (int e = upd_off[q]; e < upd_off[q + 1]; ++e) {
-      const int tg = upd_tgt[e];
-      const c64 v = l * Uval[u0 + (e - upd_off[q])];
-      if (tg < 0) D[p] = D[p] - v;
-      else if (tg & 0x40000000) Uval[tg & 0x3fffffff] = Uval[tg & 0x3fffffff] - v;
-      else Lval[tg] = Lval[tg] - v;
-    }
+  const int l0 = L.ptr[p], nl = L.ptr[p + 1] - l0, u0 = U.ptr[p], nu = U.ptr[p + 1] - u0;
+  c64* w = reinterpret_cast<c64*>(rf_smem) + (size_t)g * cap;
+  // the row's entry i: its L entries, the diagonal, its U entries
+  auto at = [&](int i) -> c64* {
+    if (SM) return w + i;
+    return i < nl ? Lval + l0 + i : (i == nl ? D + p : Uval + u0 + (i - nl - 1));
+  };
+  if (SM) {
+    for (int i = lane; i < nl; i += LN) w[i] = Lval[l0 + i];
+    for (int i = lane; i < nu; i += LN) w[nl + 1 + i] = Uval[u0 + i];
+    if (lane == 0) w[nl] = D[p];
   }
-  const c64 d = D[p];
-  const double den = d.x * d.x + d.y * d.y;
-  if (!(den > 0.0) || !isfinite(den)) atomicExch(err, 1);
-  const_cast<c64*>(U.dinv)[p] = mk<double>(d.x / den, -d.y / den);
-  const_cast<c64*>(L.dinv)[p] = mk<double>(1.0, 0.0);
+  __syncwarp(mask);
+  // of an L entry: its pivot, its updates' range, this lane's first target and factor
+  struct Step {
+    c64 d, u;
+    double den, r;  // |d|^2 and its reciprocal
+    int e0, e1, uk, tg;
+  };
+  auto fetch = [&](int q) {
+    Step s;
+    const int k = L.col[l0 + q];
+    s.e0 = upd_off[l0 + q];
+    s.e1 = upd_off[l0 + q + 1];
+    s.uk = U.ptr[k];
+    s.d = D[k];
+    s.den = s.d.x * s.d.x + s.d.y * s.d.y;
+    s.r = 1.0 / s.den;
+    s.tg = 0;
+    s.u = mk<double>(0, 0);
+    if (s.e0 + lane < s.e1) {
+      s.tg = upd_tgt[s.e0 + lane];
+      s.u = Uval[s.uk + lane];
+    }
+    return s;
+  };
+  auto slot = [&](int tg) {
+    return tg < 0 ? nl : (tg & 0x40000000) ? nl + 1 + (tg & 0x3fffffff) - u0 : tg - l0;
+  };
+  if (nl > 0) {
+    Step s = fetch(0);
+    for (int q = 0; q < nl; ++q) {
+      const Step c = s;
+      if (q + 1 < nl) s = fetch(q + 1);
+      const c64 z = *at(q);
+      const c64 l = mk<double>(rf_quot(z.x * c.d.x + z.y * c.d.y, c.den, c.r),
+                               rf_quot(z.y * c.d.x - z.x * c.d.y, c.den, c.r));
+      if (c.e0 + lane < c.e1) {
+        c64* x = at(slot(c.tg));
+        *x = *x - l * c.u;
+      }
+      for (int e = c.e0 + lane + LN; e < c.e1; e += LN) {
+        c64* x = at(slot(upd_tgt[e]));
+        *x = *x - l * Uval[c.uk + (e - c.e0)];
+      }
+      __syncwarp(mask);
+      if (lane == 0) *at(q) = l;
+    }
+    __syncwarp(mask);
+  }
+  if (SM) {
+    for (int i = lane; i < nl; i += LN) Lval[l0 + i] = w[i];
+    for (int i = lane; i < nu; i += LN) Uval[u0 + i] = w[nl + 1 + i];
+  }
+  if (lane == 0) {
+    const c64 d = *at(nl);
+    if (SM) D[p] = d;
+    const double den = d.x * d.x + d.y * d.y;
+    if (!(den > 0.0) || !isfinite(den)) atomicExch(err, 1);
+    const_cast<c64*>(U.dinv)[p] = mk<double>(d.x / den, -d.y / den);
+    const_cast<c64*>(L.dinv)[p] = mk<double>(1.0, 0.0);
+  }
 }
 
 int refactor_launch(const RefactorPlan& R, const SfTri& L, const SfTri& U, c64* Lval, c64* Uval,
@@ -93,8 +170,15 @@ int refactor_launch(const RefactorPlan& R, const SfTri& L, const SfTri& U, c64* 
   for (size_t l = 0; l + 1 < R.lvl_off.size(); ++l) {
     const int a = R.lvl_off[l], b = R.lvl_off[l + 1];
     if (b <= a) continue;
-    k_rf_rows<<<(b - a + 127) / 128, 128, 0, st>>>(R.rows + a, b - a, L, U, R.D, R.upd_off,
-                                                   R.upd_tgt, err);
+    // a level of few rows (the upper ones, with long rows) gives each a warp, the others eight
+    // lanes; rows beyond 48 KB a CTA stay in global memory
+    const int cap = R.lvl_cap[l], ln = b - a <= RF_WIDE ? 32 : 8, per = RF_TPB / ln;
+    const size_t sm = sizeof(c64) * (size_t)cap * per;
+    const bool in_sm = sm <= 48 * 1024;
+    auto kern = ln == 32 ? (in_sm ? k_rf_rows<32, true> : k_rf_rows<32, false>)
+                         : (in_sm ? k_rf_rows<8, true> : k_rf_rows<8, false>);
+    kern<<<(b - a + per - 1) / per, RF_TPB, in_sm ? sm : 0, st>>>(R.rows + a, b - a, L, U, R.D,
+                                                                  R.upd_off, R.upd_tgt, cap, err);
     ++launches;
   }
   PEEC_CUDA_TRY(cudaGetLastError());

@@ -211,3 +211,44 @@ def test_device_formed_state_matches_the_host_state(case):
             other.set_frequency_device(w, ds.Yle)
     finally:
         other.close()
+
+
+@pytest.mark.parametrize("shape,p,hub", [
+    ((3, 2, 1), 1.0, 0), ((9, 8, 7), 1.0, 0), ((30, 24, 10), 0.3, 0), ((44, 40, 22), 0.4, 0),
+    ((24, 20, 12), 0.6, 1100)], ids=str)
+def test_refactor_rows_by_level(shape, p, hub):
+    """The row kernel's forms (rows of a warp and of eight lanes, in shared and in global memory):
+    a few rows, solid bodies with long dense rows, levels of more and of fewer rows than the
+    SMs' warps, and a node linked to 1100 others, whose row exceeds the shared memory of its
+    CTA. The backward error of the device factors as in test_refactor_backward_error."""
+    import scipy.sparse as sp
+    req = configs.random_mixed(shape, s=5e-5, p=p, seed=3, nports=1, freqs=[1e9], tol=1e-8)
+    (esc, inc, cc, diag, exp, ports, le, _li, Zs), _f, _s, z0, _g = mesher.parse_request(req)
+    op = GpuOperator(inc, exp, diag["P"])
+    try:
+        w = 2 * np.pi * 1e9 * esc["freq"]
+        fs = O.frequency_setup(w, esc, inc, diag, Zs, le, ports, z0)
+        SS, Yle = fs["SS"].tocsc(), sp.csc_matrix(fs["Yle"])
+        if hub:
+            n = SS.shape[0]
+            assert n > hub
+            others = np.random.default_rng(1).choice(n - 1, hub, replace=False) + 1
+            y = 1e-3 * abs(SS.diagonal()).mean() * np.ones(hub)
+            link = sp.coo_matrix((np.concatenate([-y, -y, y, [y.sum()]]),
+                                  (np.concatenate([others, 0 * others, others, [0]]),
+                                   np.concatenate([0 * others, others, others, [0]]))), shape=(n, n))
+            Yle, SS = (Yle + link).tocsc(), (SS + link).tocsc()
+        import scipy.sparse.linalg as spla
+        lu = spla.splu(SS, permc_spec="MMD_AT_PLUS_A", options={"Equil": False})
+        op.set_frequency(w, fs["DZ"], Yle, lu)
+        op.enable_refactor(Yle)
+        op.set_frequency_refactor(w, fs["DZ"], Yle)
+        pn = np.asarray(ports["port_nodes"], dtype=np.int64).reshape(-1, 2)
+        Is = esc["Is"]
+        isv = np.zeros(SS.shape[0])
+        isv[pn[0, 0]], isv[pn[0, 1]] = Is, -Is
+        x3 = op.port_rhs(pn[0, 0], pn[0, 1], Is)[op.m + op.ns:]
+        be = np.max(np.abs(SS @ x3 - isv)) / (abs(SS).max() * np.max(np.abs(x3)) + Is)
+        assert be < 1e-13, be
+    finally:
+        op.close()
