@@ -44,3 +44,15 @@ def test_fill_matches_oracle(shape, cell, origin):
             continue
         assert np.all(np.abs(got[key] - row) <= 64 * eps * scale + 1e-300), key
         assert np.array_equal(got[key], again[key]), key
+
+
+@pytest.mark.parametrize("shape,cell", [((270, 3, 2), (5e-5, 5e-5, 5e-5)),
+                                        ((3, 2, 120), (4e-5, 6e-5, 1.2e-4)),
+                                        ((2, 190, 40), (2e-4, 3e-5, 4e-5)),
+                                        ((40, 30, 3), (1e-3, 1e-3, 1.1e-6)),
+                                        ((40, 30, 3), (1e-3, 1e-3, 1.3e-6))])
+def test_fill_near_far_boundary(shape, cell):
+    """The near-field test by distance (fill.cu, near_for_sure) around its bound, where cells go
+    from one test to the other and then to the far field: rows far longer than 166 cells along
+    each axis, uneven cells, and cells at the shape (1.2e-3) beyond which it is not used."""
+    test_fill_matches_oracle(shape, cell, 0.0)
