@@ -1432,7 +1432,7 @@ static int peec_set_rcc_frequency_body(peec_ctx* ctx, double freq_hz) {
   if (rc == PEEC_OK) {
     rc = rcc_rows_gpu(ctx->rcc_origin, ctx->rcc_s[0], ctx->rcc_s[1], ctx->rcc_s[2], ctx->Nx,
                       ctx->Ny, ctx->Nz, beta, ctx->rcc_qs, re, im, len, ctx->st);
-    ctx->launches += 9;
+    ctx->launches += 1;
     if (rc) ctx->err = g_err;
   }
   if (rc == PEEC_OK) rc = build_spectrum_set(ctx, ctx->spec, re);
