@@ -46,16 +46,39 @@ __device__ __forceinline__ double sgn(int k) { return (k & 1) ? -1.0 : 1.0; }
 // i.e. (-1)^(sum0 + n [+1]) with the 0-based corner bits used here
 // ---------------------------------------------------------------------------------
 
+// x / D for the closed forms' constants 6, 24, 60: the product with 1 / D corrected by its
+// remainder (Markstein, IBM J. Res. Dev. 34, 1990) is the rounded quotient, in three FP64
+// instructions where a division takes some ten; zero is exact, and what is out of the range in
+// which the remainder is exact (or not finite) is divided. With flip for the products by +-1 the
+// dense fill of 24x24x8 bodies takes 21.6 ms instead of 22.9 (bound by the FP64 pipe throughout),
+// the same bits.
+template <int D>
+__device__ __forceinline__ double div_const(double x) {
+  constexpr double r = 1.0 / D;
+  const unsigned h = (unsigned)__double2hiint(x) & 0x7fffffffu;
+  if (h - 0x04000000u < 0x77000000u || (h | (unsigned)__double2loint(x)) == 0) {
+    const double q = x * r;
+    return fma(fma(-q, (double)D, x), r, q);
+  }
+  return x / D;
+}
+// x (-1)^k
+__device__ __forceinline__ double flip(int k, double x) {
+  return __hiloint2double(__double2hiint(x) ^ (k << 31), __double2loint(x));
+}
+
 __device__ __forceinline__ double vol_corner(double X, double Y, double Z) {
   const double X2 = X * X, Y2 = Y * Y, Z2 = Z * Z;
   const double R = sqrt(X2 + Y2 + Z2);
-  const double t1 = (X2 * X2 + Y2 * Y2 + Z2 * Z2 - 3 * X2 * Y2 - 3 * Y2 * Z2 - 3 * X2 * Z2) * R / 60;
-  const double t2 = fin((Y2 * Z2 / 4 - Y2 * Y2 / 24 - Z2 * Z2 / 24) * X * lgc(X + R));
-  const double t3 = fin((Y2 * X2 / 4 - Y2 * Y2 / 24 - X2 * X2 / 24) * Z * lgc(Z + R));
-  const double t4 = fin((Z2 * X2 / 4 - Z2 * Z2 / 24 - X2 * X2 / 24) * Y * lgc(Y + R));
-  const double t5 = -fabs(X) * X2 * Y * Z / 6 * atan2(Y * Z, fabs(X) * R);
-  const double t6 = -X * fabs(Y) * Y2 * Z / 6 * atan2(X * Z, fabs(Y) * R);
-  const double t7 = -X * Y * fabs(Z) * Z2 / 6 * atan2(X * Y, fabs(Z) * R);
+  const double X4 = div_const<24>(X2 * X2), Y4 = div_const<24>(Y2 * Y2), Z4 = div_const<24>(Z2 * Z2);
+  const double t1 =
+      div_const<60>((X2 * X2 + Y2 * Y2 + Z2 * Z2 - 3 * X2 * Y2 - 3 * Y2 * Z2 - 3 * X2 * Z2) * R);
+  const double t2 = fin((Y2 * Z2 / 4 - Y4 - Z4) * X * lgc(X + R));
+  const double t3 = fin((Y2 * X2 / 4 - Y4 - X4) * Z * lgc(Z + R));
+  const double t4 = fin((Z2 * X2 / 4 - Z4 - X4) * Y * lgc(Y + R));
+  const double t5 = div_const<6>(-fabs(X) * X2 * Y * Z) * atan2(Y * Z, fabs(X) * R);
+  const double t6 = div_const<6>(-X * fabs(Y) * Y2 * Z) * atan2(X * Z, fabs(Y) * R);
+  const double t7 = div_const<6>(-X * Y * fabs(Z) * Z2) * atan2(X * Y, fabs(Z) * R);
   return t1 + t2 + t3 + t4 + t5 + t6 + t7;
 }
 
@@ -66,8 +89,8 @@ __device__ double vol_vol(const double* x1v, const double* y1v, const double* z1
   for (int c = 0; c < 64; ++c) {
     const int c1 = (c >> 5) & 1, c2 = (c >> 4) & 1, c3 = (c >> 3) & 1, c4 = (c >> 2) & 1,
               c5 = (c >> 1) & 1, c6 = c & 1;
-    sol += sgn(c1 + c2 + c3 + c4 + c5 + c6 + 1) *
-           vol_corner(x1v[c1] - x2v[c4], y1v[c2] - y2v[c5], z1v[c3] - z2v[c6]);
+    sol += flip(c1 + c2 + c3 + c4 + c5 + c6 + 1,
+                vol_corner(x1v[c1] - x2v[c4], y1v[c2] - y2v[c5], z1v[c3] - z2v[c6]));
   }
   return sol;
 }
@@ -88,7 +111,7 @@ __device__ double ss_para(const double* x1v, const double* y1v, double z1, const
 #pragma unroll 1
   for (int c = 0; c < 16; ++c) {
     const int c1 = (c >> 3) & 1, c2 = (c >> 2) & 1, c3 = (c >> 1) & 1, c4 = c & 1;
-    sol += sgn(c1 + c2 + c3 + c4) * para_corner(x1v[c1] - x2v[c4], y1v[c2] - y2v[c3], z1 - z2);
+    sol += flip(c1 + c2 + c3 + c4, para_corner(x1v[c1] - x2v[c4], y1v[c2] - y2v[c3], z1 - z2));
   }
   return sol;
 }
@@ -118,8 +141,8 @@ __device__ double ss_ortho(const double* x1v, const double* y1v, double z1, cons
 #pragma unroll 1
   for (int c = 0; c < 16; ++c) {
     const int c1 = (c >> 3) & 1, c2 = (c >> 2) & 1, c3 = (c >> 1) & 1, c4 = c & 1;
-    sol += sgn(c1 + c2 + c3 + c4) *
-           ortho_corner(x1v[c1] - x2v[c4], y1v[c2] - y2, z1 - z2v[c3], pform);
+    sol += flip(c1 + c2 + c3 + c4,
+                ortho_corner(x1v[c1] - x2v[c4], y1v[c2] - y2, z1 - z2v[c3], pform));
   }
   return sol;
 }
@@ -743,7 +766,7 @@ __device__ __forceinline__ size_t corner_at(const int U[3], int x, int y, int z)
   return ((size_t)z * U[1] + y) * U[0] + x;
 }
 
-// calls f(sign, index) for a near-field cell's corners in the closed form's order
+// calls f(parity, index) for a near-field cell's corners in the closed form's order
 template <typename F>
 __device__ __forceinline__ void each_corner(const RowSet& S, const RowSpec& s, int r, const int U[3],
                                             const int i[3], F&& f) {
@@ -759,7 +782,7 @@ __device__ __forceinline__ void each_corner(const RowSet& S, const RowSpec& s, i
     for (int k = 0; k < 64; ++k) {
       const int c1 = (k >> 5) & 1, c2 = (k >> 4) & 1, c3 = (k >> 3) & 1, c4 = (k >> 2) & 1,
                 c5 = (k >> 1) & 1, c6 = k & 1;
-      f(sgn(c1 + c2 + c3 + c4 + c5 + c6 + 1),
+      f(c1 + c2 + c3 + c4 + c5 + c6 + 1,
         corner_at(U, id[0][2 * c1 + c4], id[1][2 * c2 + c5], id[2][2 * c3 + c6]));
     }
   } else {
@@ -768,7 +791,7 @@ __device__ __forceinline__ void each_corner(const RowSet& S, const RowSpec& s, i
       const int c1 = (k >> 3) & 1, c2 = (k >> 2) & 1, c3 = (k >> 1) & 1, c4 = k & 1;
       const size_t at = s.kind == 1 ? corner_at(U, id[0][2 * c1 + c4], id[1][2 * c2 + c3], id[2][0])
                                     : corner_at(U, id[0][2 * c1 + c4], id[1][c2], id[2][c3]);
-      f(sgn(c1 + c2 + c3 + c4), at);
+      f(c1 + c2 + c3 + c4, at);
     }
   }
 }
@@ -830,7 +853,7 @@ __global__ void k_fill_mark(RowSet S, int r, int U0, int U1, int U2, uint8_t* ne
       nr = slab_cell(S, s, p, i, A, B);
     }
     near[p] = nr;
-    if (nr) each_corner(S, s, r, U, i, [&](double, size_t at) { need[at] = 1; });
+    if (nr) each_corner(S, s, r, U, i, [&](int, size_t at) { need[at] = 1; });
   }
 }
 
@@ -865,7 +888,7 @@ __global__ void __launch_bounds__(128) k_fill_sum(RowSet S, int r, int U0, int U
       i[1] = (int)((p / s.D[0]) % s.D[1]);
       i[2] = S.k0 + (int)(p / ((int64_t)s.D[0] * s.D[1]));
       double sol = 0.0;
-      each_corner(S, s, r, U, i, [&](double sg, size_t at) { sol += sg * tab[at]; });
+      each_corner(S, s, r, U, i, [&](int k, size_t at) { sol += flip(k, tab[at]); });
       v = sol;  // the faces' normal lengths, a factor of the closed form, are one
     } else {
       Box A, B;
