@@ -2370,9 +2370,8 @@ static int matvec_enqueue(peec_ctx* ctx, const c64* x, c64* y, int prec, bool ev
     launch_add_i(ctx->PQ2, ctx->ns, ctx->PQ, st);
     ctx->launches += 2;
   }
-  // one launch per x / y pass over all families, the shared z pass of the face
-  // families, and the edge families' z passes: one launch over all of them in the staged
-  // FP32 form (ZTune form 2), else one per family
+  // x and y passes: one launch over the families of one length; the shared z pass of the face
+  // families; the edge families' z passes
   const int lines = line_launches(ctx->fam, 6, prec, 0) + line_launches(ctx->fam, 6, prec, 1);
   ctx->launches += (1 + 2 * lines + zedge_launches(ctx->fam, 6, prec, ctx->zt)) * (ctx->rcc ? 2 : 1);
   if (events) cudaEventRecord(ctx->ev[1], st);

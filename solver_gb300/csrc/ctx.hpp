@@ -133,7 +133,8 @@ struct GmDev {
 
 // Buffers of the device loop's Arnoldi body (krylov.cu): the basis is U (complex double)
 // or U32 (complex float-float), whichever is set; T the compact-WY factor (ld ldT); v the
-// iteration's vector, w = A v; kmax the largest column count of the cycle (inner).
+// iteration's vector (not normalised, *scal its inverse norm), w = A v; kmax the largest column
+// count of the cycle (inner).
 struct GmBody {
   c64* U = nullptr;
   cff* U32 = nullptr;

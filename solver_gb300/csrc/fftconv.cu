@@ -12,21 +12,19 @@
 // the edge direction and keep one forward/inverse pair each.
 //
 // Each 3-D transform runs as passes over one axis at a time on a per-family buffer
-// T_f[z][y][kx] (kx fastest, Lx x Ly x nz_f), in place:
-//   k_xfwd   gather the family's compact vector through its lattice map, zero pad,
-//            forward FFT along x (16 pencils per CTA)
-//   k_ypass  forward / inverse FFT along y (16 consecutive kx per CTA)
-//   k_zconv3 forward FFT along z of the three face families, 3x3 spectral product,
-//            inverse FFT along z (one ky, a kx tile per CTA)
-//   k_zconv1 same for one edge family with its real spectrum
-//   k_xinv   inverse FFT along x and plain store into the compact output through the
-//            lattice map (each compact index belongs to exactly one family)
-// Only the occupied lattice octant is transformed in each pass (pruning). Inside a
-// pass the first radix group reads global memory straight into registers and the
-// last group writes straight back (fft_reg.cuh); in the z passes the last forward
-// group, the spectral product and the first inverse group run back to back in
-// registers. Shared-memory tiles keep sequences contiguous (element (pos, seq) at
-// pos*rs + seq), so the middle groups are bank-conflict free.
+// T_f[z][y][kx] (kx fastest, Lx x Ly x nz_f), in place: x forward (gather of the family's
+// compact vector through its lattice map), y forward, z (forward, spectral product, inverse),
+// y inverse, x inverse (plain store into the compact output through the lattice map; each
+// compact index belongs to exactly one family). Only the occupied lattice octant is
+// transformed in each pass (pruning). Two sets of kernels (fftconv_impl.cuh):
+//   pair     k_xpair, k_ypair, k_zpair / k_zpair_wide: the even and the odd frequencies as
+//            transforms of half the length on the occupied entries, in registers (FP32 and
+//            float-float, up to 512 points along x and y and 128 along z)
+//   direct   k_xfwd, k_ypass, k_zconv3 / k_zconv1, k_xinv: the padded lines in radix groups
+//            (fft_reg.cuh), the first and last ones straight from and to global memory, the
+//            middle ones in shared-memory tiles with contiguous sequences (element (pos, seq)
+//            at pos*rs + seq, bank-conflict free); FP64 and longer lines. The staged z passes
+//            are the direct ones with bulk-copied tiles.
 // Spectra carry the 1/(Lx*Ly*Lz) normalisation (Spectrum).
 #include <mutex>
 #include <set>

@@ -1,10 +1,9 @@
 // Vector kernels of the Householder GMRES (compact-WY form).
 //
-// The reflector basis U (N x kmax, column-major, complex double) is applied with
-// two passes per application instead of the reference's one dot+axpy per
-// reflector (gmres_custom.jl:112-127): a multi-dot z = U(:,0:k)^H v, a small
-// triangular product on the host, and a multi-axpy v -= U(:,0:k) c. Reductions
-// are deterministic: warp-shuffle partials per CTA, then a fixed-order sum.
+// The reflector basis U (N x kmax, column-major) is applied whole instead of the reference's
+// one dot and axpy per reflector (gmres_custom.jl:112-127): z = U(:,0:k)^H v, a product with the
+// triangular factor T, v -= U(:,0:k) c. Reductions have a fixed order: partials per CTA, then a
+// fixed-order sum.
 #include <mutex>
 
 #include "ctx.hpp"
