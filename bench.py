@@ -181,12 +181,9 @@ def conv_bytes(info, prec):
     """Algorithmic bytes of the convolution passes per operator application: every
     per-family intermediate written once and read once by the next pass, each
     spectrum read once, lattice maps (int32) once, compact vectors (complex128) read
-    once by the gather and written once by the scatter. Spectra: full form (face
-    families: 3 real + 3 complex on the shared grid; edge families: one real each), or
-    for the staged FP32 z passes (staged = {"faces", "edges"}) the y/z-folded real
-    tables of Lx(Ly/2+1)(Lz/2+1) floats (six for the faces, one per edge family)."""
+    once by the gather and written once by the scatter. Spectra: the y/z-folded real
+    tables of Lx(Ly/2+1)(Lz/2+1) values (six for the faces, one per edge family)."""
     c = 16 if prec == 0 else 8
-    staged = staged or {"faces": False, "edges": False}
     b = {"xfwd": 0, "yfwd": 0, "z": 0, "yinv": 0, "xinv": 0}
     for f in info:
         if not f["active"]:
