@@ -415,8 +415,8 @@ __global__ void __launch_bounds__(TPB) k_ypass(PassSet<R> s, const cx<R>* __rest
 // gathers' latency, float-float the FP32 pipes. The direct kernels (k_xfwd and so on) ran 37M and
 // 52M warp instructions in x and y at 128x128x64, on padding and through three transposes in
 // shared memory with CTA barriers. Operator application at 128x128x64, x / y / inverse y / inverse
-// x: FP32 70 / 78 / 70 / 87 -> 50 / 52 / 67 / 49 us, float-float 262 / 291 / 311 / 258 -> 186 / 234
-// / 252 / 158 us; FP32 at 64x64x32 13.9 / 16.3 / 14.9 / 15.5 -> 8.3 / 6.9 / 8.1 / 8.8 us. FP64
+// x: FP32 70 / 78 / 70 / 87 -> 51 / 53 / 65 / 47 us, float-float 262 / 291 / 311 / 258 -> 186 / 234
+// / 252 / 158 us; FP32 at 64x64x32 13.9 / 16.3 / 14.9 / 15.5 -> 8.3 / 6.8 / 7.5 / 8.9 us. FP64
 // stays direct, like its z passes (its pipe is the bound in either form).
 __device__ __forceinline__ int brevn(int v, int n) {
   return n ? (int)(__brev((unsigned)v) >> (32 - n)) : 0;
@@ -659,6 +659,20 @@ k_ypair(LineSet<R> S, const cx<R>* __restrict__ twm, int twmax) {
       x[r] = on && k + G * r < n ? ld_stream(T + (k + G * r) * rs) : mk<R>(0, 0);
     if (on && k == 0 && n > H) xh = ld_stream(T + H * rs);
   }
+  // inverse, FP32: both halves' loads in flight before the first is worked on (x holds the even
+  // half until its turn; 67 -> 65 us in y, 49 -> 47 in x at 128x128x64, 8.1 -> 7.5 in y at 64x64x32)
+  constexpr bool AHEAD = INV && sizeof(R) == 4 && V <= 8;
+  if (AHEAD) {
+#pragma unroll
+    for (int q = 0; q < HL::NRUN; ++q) {
+#pragma unroll
+      for (int t = 0; t < HL::RUN; ++t) {
+        const cx<R>* p = T + (HL::pos(q, k) + t) * rs;
+        d[q * HL::RUN + t] = on ? ld_stream(p + H * rs) : mk<R>(0, 0);
+        x[q * HL::RUN + t] = on ? ld_stream(p) : mk<R>(0, 0);
+      }
+    }
+  }
   __syncthreads();
 #pragma unroll 1
   for (int h = 0; h < 2; ++h) {
@@ -677,7 +691,7 @@ k_ypair(LineSet<R> S, const cx<R>* __restrict__ twm, int twmax) {
       for (int t = 0; t < RUN; ++t) {
         if (!INV) {
           if (on) st_stream(p + t * rs, d[q * RUN + t]);
-        } else {
+        } else if (!AHEAD) {
           d[q * RUN + t] = on ? ld_stream(p + t * rs) : mk<R>(0, 0);
         }
       }
@@ -686,7 +700,11 @@ k_ypair(LineSet<R> S, const cx<R>* __restrict__ twm, int twmax) {
       HL::template inv<false>(d, W, k, xb, G * C, C, C & 31);
       if (h == 0) {
 #pragma unroll
-        for (int r = 0; r < V; ++r) x[r] = cmulc(d[r], W[k + G * r]);
+        for (int r = 0; r < V; ++r) {
+          const cx<R> o = cmulc(d[r], W[k + G * r]);
+          if (AHEAD) d[r] = x[r];
+          x[r] = o;
+        }
       }
     }
   }
@@ -724,6 +742,15 @@ __global__ void __launch_bounds__(XP_TPB, MINB) k_xpair(LineSet<R> S, const cx<R
     for (int r = 0; r < V; ++r) x[r] = id[r] >= 0 ? line_in(F.io[id[r]], R()) : mk<R>(0, 0);
     if (ih >= 0) xh = line_in(F.io[ih], R());
   }
+  constexpr bool AHEAD = INV && sizeof(R) == 4 && V <= 8;  // as in k_ypair
+  if (AHEAD) {
+#pragma unroll
+    for (int q = 0; q < HL::NRUN; ++q) {
+      const cx<R>* p = T + HL::pos(q, k);
+      ld_run<R, HL::RUN>(p + H, d + q * HL::RUN);
+      ld_run<R, HL::RUN>(p, x + q * HL::RUN);
+    }
+  }
   __syncthreads();
 #pragma unroll 1
   for (int h = 0; h < 2; ++h) {
@@ -738,7 +765,7 @@ __global__ void __launch_bounds__(XP_TPB, MINB) k_xpair(LineSet<R> S, const cx<R
       cx<R>* p = T + par * H + HL::pos(q, k);
       if (!INV) {
         if (on) st_run<R, RUN>(p, d + q * RUN);
-      } else {
+      } else if (!AHEAD) {
         ld_run<R, RUN>(p, d + q * RUN);  // (a line past the last reads the first one's)
       }
     }
@@ -746,7 +773,11 @@ __global__ void __launch_bounds__(XP_TPB, MINB) k_xpair(LineSet<R> S, const cx<R
       HL::template inv<true>(d, W, k, xc, HL::SJ, 1, 1);
       if (h == 0) {
 #pragma unroll
-        for (int r = 0; r < V; ++r) x[r] = cmulc(d[r], W[k + G * r]);
+        for (int r = 0; r < V; ++r) {
+          const cx<R> o = cmulc(d[r], W[k + G * r]);
+          if (AHEAD) d[r] = x[r];
+          x[r] = o;
+        }
       }
     }
   }
