@@ -277,9 +277,15 @@ static int spec_pass(SpecSet& S, int ctas, const c64* tw, int twmax, cudaStream_
   size_t sm = 0;
   for (int i = 0; i < S.n; ++i)
     sm = std::max(sm, sizeof(c64) * (size_t)S.r[i].ax[AX].L * ((1 << LC) + 2));
-  if (sm > 48 * 1024)
+  if (sm > 48 * 1024) {
+    // the device's limit, the same for every context (the attribute is the function's, and
+    // contexts of other sizes may launch it from other threads)
+    int dev = 0, lim = 0;
+    PEEC_CUDA_TRY(cudaGetDevice(&dev));
+    PEEC_CUDA_TRY(cudaDeviceGetAttribute(&lim, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
     PEEC_CUDA_TRY(cudaFuncSetAttribute(k_spec_pass<AX, LC>,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+                                       cudaFuncAttributeMaxDynamicSharedMemorySize, lim));
+  }
   k_spec_pass<AX, LC><<<ctas, 256, sm, st>>>(S, tw, twmax);
   return 0;
 }

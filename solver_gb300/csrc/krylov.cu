@@ -925,10 +925,10 @@ static int gm_launch(const GmBody& B, UT* U, const GmGrid& g, bool pre) {
                                                                         B.part, B.scal);
     return 1;
   }
-  // up to 24 KB of rows and sums and 32 KB of coefficients
+  // up to 24 KB of rows and sums and 32 KB of coefficients; the limit is one for all contexts
+  // (the attribute is the function's, and contexts of other sizes launch it from other threads)
   const size_t sm2 = g.sm + sizeof(c64) * (B.kmax + 1);
-  cudaFuncSetAttribute(k_gm_dot<WR, UT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)g.sm);
-  cudaFuncSetAttribute(k_gm_orth<WR, UT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm2);
+  cudaFuncSetAttribute(k_gm_orth<WR, UT>, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024);
   k_gm_dot<WR, UT><<<g.nb + 1, GM_TPB, g.sm, B.st>>>(U, B.N, g.rows, B.w, B.T, B.ldT, B.gs, B.part,
                                                      B.scal, B.coef);
   k_gm_orth<WR, UT><<<g.nb, GM_TPB, sm2, B.st>>>(U, B.N, g.rows, B.w, B.T, B.ldT, B.gs, B.part,
