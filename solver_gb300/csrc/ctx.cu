@@ -1848,23 +1848,13 @@ static int peec_set_frequency_body(peec_ctx* ctx, double w, const double* DZ, in
   if (!ctx->have_topo) return bad(ctx, PEEC_ERR_STATE, "topology not set");
   PEEC_CUDA_TRY(cudaSetDevice(ctx->dev));
   const int64_t n = ctx->n, m = ctx->m;
-  ctx->w = w;
-  std::vector<c64> dz(m);
-  for (int64_t e = 0; e < m; ++e) dz[e] = mk<double>(DZ[2 * e], DZ[2 * e + 1]);
-  CTX_TRY(upload(&ctx->DZ, dz, ctx->st));
-  launch_inv_dz(ctx->DZ, m, ctx->invZ, ctx->st);
-  ctx->launches++;
+  // A failure from here on leaves no frequency state: the arrays are replaced one by one, and
+  // the groups' plan (GrpRow: rows of Yle, entries of the factors) belongs to the ones before.
+  ctx->have_freq = false;
   // Yle COO -> CSR (duplicates summed, as sparse() does)
   std::vector<int32_t> yp, yc;
   std::vector<c64> yv;
   CTX_TRY(yle_csr(ctx, n, yle_nnz, yle_row, yle_col, yle_val, yp, yc, yv));
-  CTX_TRY(upload(&ctx->yle_ptr, yp, ctx->st));
-  ctx->h_yp = yp;
-  CTX_TRY(upload(&ctx->yle_col, yc, ctx->st));
-  CTX_TRY(upload(&ctx->yle_val, yv, ctx->st));
-  ctx->yle_cap = yv.size();
-  if (!ctx->d_w) CTX_TRY(dalloc(&ctx->d_w, 1));
-  launch_set_scalar(ctx->d_w, w, ctx->st);
   // LU: b' = b[iperm_r]; x = z[perm_c]
   std::vector<int32_t> gin(n), gout(n);
   for (int64_t i = 0; i < n; ++i) {
@@ -1873,11 +1863,24 @@ static int peec_set_frequency_body(peec_ctx* ctx, double w, const double* DZ, in
     gin[perm_r[i]] = (int32_t)i;
     gout[i] = (int32_t)perm_c[i];
   }
-  CTX_TRY(upload(&ctx->g_in, gin, ctx->st));
-  CTX_TRY(upload(&ctx->g_out, gout, ctx->st));
   // new factors: a refactorisation plan of the old ones no longer applies
   free_refactor(ctx->rf);
   ctx->have_rf = false;
+  ctx->w = w;
+  std::vector<c64> dz(m);
+  for (int64_t e = 0; e < m; ++e) dz[e] = mk<double>(DZ[2 * e], DZ[2 * e + 1]);
+  CTX_TRY(upload(&ctx->DZ, dz, ctx->st));
+  launch_inv_dz(ctx->DZ, m, ctx->invZ, ctx->st);
+  ctx->launches++;
+  CTX_TRY(upload(&ctx->yle_ptr, yp, ctx->st));
+  ctx->h_yp = yp;
+  CTX_TRY(upload(&ctx->yle_col, yc, ctx->st));
+  CTX_TRY(upload(&ctx->yle_val, yv, ctx->st));
+  ctx->yle_cap = yv.size();
+  if (!ctx->d_w) CTX_TRY(dalloc(&ctx->d_w, 1));
+  launch_set_scalar(ctx->d_w, w, ctx->st);
+  CTX_TRY(upload(&ctx->g_in, gin, ctx->st));
+  CTX_TRY(upload(&ctx->g_out, gout, ctx->st));
   ctx->h_gin = gin;
   ctx->h_gout = gout;
   if (row_scale) {

@@ -1,0 +1,83 @@
+"""GPU: a frequency state that could not be installed is not used. peec_set_frequency replaces
+the context's arrays one by one, and the LU groups' plan holds positions in the ones before, so a
+refused upload has to leave a context that refuses applications and solves (PEEC_ERR_STATE, by the
+host's check, before anything is launched) until a whole state is installed; what then comes out is
+what came out before, bit for bit (the same kernels on the same values)."""
+import numpy as np
+import pytest
+import scipy.sparse as sp
+
+from solver_gb300 import _lib, configs, frequency, mesher
+from solver_gb300.operator import GpuOperator
+
+pytestmark = pytest.mark.gpu
+
+BADARG, STATE = -5, -7  # PEEC_ERR_*
+
+
+@pytest.fixture(scope="module")
+def geom():
+    req = configs.random_mixed((9, 8, 5), s=5e-5, p=0.6, seed=5, nports=1, freqs=[1e9], tol=1e-8)
+    out, freqs, _s, z0, _grid = mesher.parse_request(req)
+    esc, inc, cc, diag, exp, ports, le, _li, Zs = out
+    fs = frequency.FrequencyState(2 * np.pi * freqs[0] * esc["freq"], esc, inc, diag, Zs, le, ports,
+                                  z0)
+    op = GpuOperator(inc, exp, diag["P"])
+    op.fill(cc["origin"], cc["sx"], cc["sy"], cc["sz"], esc["Lp"], esc["P"])
+    yield op, fs
+    op.close()
+
+
+def _refused(op, fs, fault):
+    """set_frequency with an empty Yle and one fault; the code it returns"""
+    (Lp, Lc, Lv), (Up, Uc, Uv), pr, pc = [
+        tuple(np.array(v) for v in t) if isinstance(t, tuple) else np.array(t)
+        for t in frequency.export_lu(fs.lu)]
+    yr, yc, yv = np.zeros(1, np.int64), np.zeros(1, np.int64), np.zeros(2)
+    nnz = 0
+    r = op.n // 2
+    if fault == "yle":
+        nnz, yr[0] = 1, op.n
+    elif fault == "permutation":
+        pc[r] = op.n
+    elif fault == "pivot":
+        at = Up[r] + int(np.flatnonzero(Uc[Up[r]:Up[r + 1]] == r)[0])
+        Uv[2 * at:2 * at + 2] = 0.0
+    elif fault == "side":
+        Lc[Lp[0]] = op.n - 1
+    DZ = np.ascontiguousarray(np.asarray(fs.DZ, dtype=np.complex128).ravel())
+    p = _lib.ptr
+    return op.L.peec_set_frequency(op.h, fs.w, p(DZ.view(np.float64)), nnz, p(yr), p(yc), p(yv), p(Lp),
+                                   p(Lc), p(Lv), p(Up), p(Uc), p(Uv), p(pr), p(pc), None)
+
+
+def _is_refused(call):
+    with pytest.raises(_lib.PeecError) as e:
+        call()
+    assert e.value.code == STATE
+
+
+@pytest.mark.parametrize("fault", ["yle", "permutation", "pivot", "side"])
+def test_refused_frequency_is_not_used(geom, fault):
+    op, fs = geom
+    rng = np.random.default_rng(1)
+    x = rng.standard_normal(op.N) + 1j * rng.standard_normal(op.N)
+    op.set_frequency(fs.w, fs.DZ, fs.Yle, fs.lu)
+    op.enable_refactor(fs.Yle)
+    y = op.matvec(x, 0)
+    assert sp.coo_matrix(fs.Yle).nnz > 0
+    assert _refused(op, fs, fault) == BADARG
+    for call in (lambda: op.matvec(x, 0), lambda: op.matvec(x, 1), lambda: op.port_rhs(0, 1, 1.0),
+                 lambda: op.gmres(x, None, 1e-6, 5), lambda: op.solve_mixed(x, None, 1e-6),
+                 lambda: op.enable_refactor(fs.Yle)):
+        _is_refused(call)
+    op.set_lu_component_max(512)  # no plan is built for factors that are not there
+    _is_refused(lambda: op.matvec(x, 0))
+    if fault in ("yle", "permutation"):  # refused before anything was replaced: the plan stands
+        op.set_frequency_refactor(fs.w, fs.DZ, fs.Yle)
+        assert np.array_equal(op.matvec(x, 0), y)
+    else:
+        _is_refused(lambda: op.set_frequency_refactor(fs.w, fs.DZ, fs.Yle))
+    op.set_frequency(fs.w, fs.DZ, fs.Yle, fs.lu)
+    op.enable_refactor(fs.Yle)
+    assert np.array_equal(op.matvec(x, 0), y)
