@@ -1540,7 +1540,11 @@ static int make_tri(peec_ctx* ctx, LevelTri& T, int64_t n, const int64_t* ptr, c
 // ones packed into groups in order of their level depth (so that a group's levels are
 // mostly full), larger ones one per group; the rows of components above comp_max (or too
 // large for a CTA's shared memory) go to the synchronisation-free global scheme.
+//
+// The plan's arrays are replaced one by one: from here on neither a frequency state nor a
+// refactorisation plan is installed, until the caller says so.
 static int build_solve_plan(peec_ctx* ctx, int64_t n) {
+  ctx->have_freq = ctx->have_rf = false;
   const LevelTri &L = ctx->Lf, &U = ctx->Uf;
   // union-find over the factor entries
   std::vector<int32_t> parent(n);
@@ -1983,6 +1987,7 @@ static int peec_lu_refactor_setup_body(peec_ctx* ctx, int64_t yle_nnz, const int
       return bad(ctx, PEEC_ERR_UNSUPPORTED, "factors too large for the device factorisation");
   }
   // install the pattern (diagonal included, placeholder values) with its levels and plan
+  ctx->have_freq = false;
   {
     auto tri = [&](const std::vector<int64_t>& op, const std::vector<int32_t>& oc, bool lower,
                    LevelTri& T) {
@@ -3367,7 +3372,11 @@ static int peec_set_lu_component_max_body(peec_ctx* ctx, int max_rows) {
   PEEC_CUDA_TRY(cudaSetDevice(ctx->dev));
   drop_graphs(ctx);
   ctx->comp_max = max_rows;
-  if (ctx->have_freq) CTX_TRY(build_solve_plan(ctx, ctx->n));
+  if (!ctx->have_freq) return PEEC_OK;
+  const bool rf = ctx->have_rf;  // the factors' pattern does not change
+  CTX_TRY(build_solve_plan(ctx, ctx->n));
+  ctx->have_freq = true;
+  ctx->have_rf = rf;
   return PEEC_OK;
 }
 

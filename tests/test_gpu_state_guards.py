@@ -81,3 +81,28 @@ def test_refused_frequency_is_not_used(geom, fault):
     op.set_frequency(fs.w, fs.DZ, fs.Yle, fs.lu)
     op.enable_refactor(fs.Yle)
     assert np.array_equal(op.matvec(x, 0), y)
+
+
+def test_new_plan_keeps_the_state(geom):
+    """Another component limit rebuilds the plan: the frequency state and the refactorisation
+    plan stay installed. The rows of the global scheme sum in another order than the groups:
+    the operator's bound of 1e-10, and 20 times its response to inputs changed in the last bit."""
+    op, fs = geom
+    rng = np.random.default_rng(2)
+    x = rng.standard_normal(op.N) + 1j * rng.standard_normal(op.N)
+    op.set_frequency(fs.w, fs.DZ, fs.Yle, fs.lu)
+    op.enable_refactor(fs.Yle)
+    y = op.matvec(x, 0)
+    peak = np.max(np.abs(y))
+    eps = np.finfo(float).eps
+    noise = np.max(np.abs(op.matvec(x * (1 + eps * rng.choice([-1, 1], op.N)), 0) - y))
+    bound = max(1e-10 * peak, 20 * noise)
+    try:
+        for limit in (0, 8):
+            op.set_lu_component_max(limit)
+            assert np.max(np.abs(op.matvec(x, 0) - y)) <= bound
+            op.set_frequency_refactor(fs.w, fs.DZ, fs.Yle)
+            assert np.max(np.abs(op.matvec(x, 0) - y)) <= bound
+    finally:
+        op.set_lu_component_max(512)
+    assert np.array_equal(op.matvec(x, 0), y)
