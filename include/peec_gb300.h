@@ -249,7 +249,8 @@ int peec_set_frequency(peec_ctx* ctx, double w, const double* DZ, int64_t yle_nn
  * depend on the frequency, so the factors of one host factorisation (installed by
  * peec_set_frequency) fix the pattern and the pivot order:
  * peec_lu_refactor_setup: builds the plan from the installed factors and the Yle pattern
- * (COO, values not read).
+ * (COO, values not read). A pattern with more entries than the installed Yle is taken over
+ * for it too (the added entries zero); one that lacks a nonzero entry of it is PEEC_ERR_BADARG.
  * peec_set_frequency_refactor: DZ and Yle as for peec_set_frequency (Yle with the same
  * pattern), then SS assembled and factorised on the device (one launch per level of L),
  * no host factors. A zero or non-finite pivot returns PEEC_ERR_UNSUPPORTED (factorise that

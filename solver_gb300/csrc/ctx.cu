@@ -219,7 +219,7 @@ struct peec_ctx {
   int32_t *grp_rec = nullptr, *grp_esrc = nullptr, *grp_eij = nullptr, *grp_gsrc = nullptr;
   // host copies of the node -> edge / surface lists, for the groups' gather lists
   std::vector<int32_t> h_ne_ptr, h_ne_idx, h_nsn_ptr, h_nsn_idx;
-  std::vector<int32_t> h_yp;  // host copy of the installed Yle's row offsets
+  std::vector<int32_t> h_yp, h_yc;  // host copies of the installed Yle's row offsets and columns
   GrpRow* grp_rows = nullptr;
   c64 *ir_b = nullptr, *ir_x = nullptr, *ir_r = nullptr, *ir_d = nullptr;  // refinement vectors
   // the frequency w on the device (the row kernels read it there, so captured graphs of
@@ -1878,6 +1878,7 @@ static int peec_set_frequency_body(peec_ctx* ctx, double w, const double* DZ, in
   ctx->launches++;
   CTX_TRY(upload(&ctx->yle_ptr, yp, ctx->st));
   ctx->h_yp = yp;
+  ctx->h_yc = yc;
   CTX_TRY(upload(&ctx->yle_col, yc, ctx->st));
   CTX_TRY(upload(&ctx->yle_val, yv, ctx->st));
   ctx->yle_cap = yv.size();
@@ -1936,6 +1937,22 @@ static int peec_lu_refactor_setup_body(peec_ctx* ctx, int64_t yle_nnz, const int
   std::vector<int32_t> yp, yc;
   std::vector<c64> yv;
   CTX_TRY(yle_csr(ctx, n, yle_nnz, yle_row, yle_col, zeros.data(), yp, yc, yv));
+  // a pattern with more entries than the installed Yle: its values move there (yv), the added
+  // entries are zero, and the row kernels, the groups and the factors share the new pattern
+  const bool repattern = yp != ctx->h_yp || yc != ctx->h_yc;
+  if (repattern) {
+    std::vector<c64> old(ctx->h_yc.size());
+    if (!old.empty())
+      PEEC_CUDA_TRY(cudaMemcpy(old.data(), ctx->yle_val, sizeof(c64) * old.size(),
+                               cudaMemcpyDeviceToHost));
+    for (int64_t r = 0; r < n; ++r)
+      for (int32_t q = ctx->h_yp[r]; q < ctx->h_yp[r + 1]; ++q) {
+        const int64_t at = find_col(yc, yp[r], yp[r + 1], ctx->h_yc[q]);
+        if (at >= 0) yv[at] = old[q];
+        else if (old[q].x != 0.0 || old[q].y != 0.0)
+          return bad(ctx, PEEC_ERR_BADARG, "the Yle pattern lacks an entry of the installed Yle");
+      }
+  }
   // topology on the host
   std::vector<int32_t> e1(m), e2(m), sn(ns);
   cudaMemcpy(e1.data(), ctx->n1, sizeof(int32_t) * m, cudaMemcpyDeviceToHost);
@@ -1988,6 +2005,14 @@ static int peec_lu_refactor_setup_body(peec_ctx* ctx, int64_t yle_nnz, const int
   }
   // install the pattern (diagonal included, placeholder values) with its levels and plan
   ctx->have_freq = false;
+  if (repattern) {
+    CTX_TRY(upload(&ctx->yle_ptr, yp, ctx->st));
+    CTX_TRY(upload(&ctx->yle_col, yc, ctx->st));
+    CTX_TRY(upload(&ctx->yle_val, yv, ctx->st));
+    ctx->yle_cap = yv.size();
+    ctx->h_yp = yp;
+    ctx->h_yc = yc;
+  }
   {
     auto tri = [&](const std::vector<int64_t>& op, const std::vector<int32_t>& oc, bool lower,
                    LevelTri& T) {

@@ -6,6 +6,7 @@ what came out before, bit for bit (the same kernels on the same values)."""
 import numpy as np
 import pytest
 import scipy.sparse as sp
+from scipy.sparse.linalg import splu
 
 from solver_gb300 import _lib, configs, frequency, mesher
 from solver_gb300.operator import GpuOperator
@@ -106,3 +107,40 @@ def test_new_plan_keeps_the_state(geom):
     finally:
         op.set_lu_component_max(512)
     assert np.array_equal(op.matvec(x, 0), y)
+
+
+def test_wider_yle_pattern_at_the_set_up(geom):
+    """enable_refactor with a pattern that has an admittance more than the installed Yle: the
+    operator does not change by its zero, and a later frequency with that admittance is the one
+    that host factors of the same SS give. Bounds: two factorisations of one SS agree to 1e-10 (as
+    in test_gpu_refactor) or 20 times the operator's response to inputs changed in the last bit. A
+    pattern without the installed admittances is refused and changes nothing."""
+    op, fs = geom
+    rng = np.random.default_rng(3)
+    x = rng.standard_normal(op.N) + 1j * rng.standard_normal(op.N)
+    op.set_frequency(fs.w, fs.DZ, fs.Yle, fs.lu)
+    y = op.matvec(x, 0)
+    peak, eps = np.max(np.abs(y)), np.finfo(float).eps
+    noise = np.max(np.abs(op.matvec(x * (1 + eps * rng.choice([-1, 1], op.N)), 0) - y))
+    bound = max(1e-10 * peak, 20 * noise)
+    with pytest.raises(_lib.PeecError) as e:
+        op.enable_refactor(sp.csr_matrix((op.n, op.n), dtype=complex))
+    assert e.value.code == BADARG
+    assert np.array_equal(op.matvec(x, 0), y)
+    a, b = 1, op.n - 2
+    g = 0.02 + 0.01j
+    wide = (sp.csr_matrix(fs.Yle) +
+            sp.csr_matrix(([g, g, -g, -g], ([a, b, a, b], [a, b, b, a])), shape=(op.n, op.n))).tocsr()
+    assert wide.nnz > sp.coo_matrix(fs.Yle).nnz
+    op.enable_refactor(wide)
+    assert np.max(np.abs(op.matvec(x, 0) - y)) <= bound
+    op.set_frequency_refactor(fs.w, fs.DZ, wide)
+    got = op.matvec(x, 0)
+    inc, _exp, diagP = op._init_args[:3]
+    A, G = inc["A"], inc["Gamma"]
+    SS = (A.T @ sp.diags(1 / np.asarray(fs.DZ).ravel()) @ A +
+          1j * fs.w * (G @ sp.diags(1 / np.asarray(diagP).ravel()) @ G.T) + wide)
+    op.set_frequency(fs.w, fs.DZ, wide, splu(sp.csc_matrix(SS), options={"Equil": False}))
+    ref = op.matvec(x, 0)
+    assert np.max(np.abs(got - ref)) <= max(bound, 1e-10 * np.max(np.abs(ref)))
+    assert np.max(np.abs(ref - y)) > 10 * bound  # the admittance is seen
