@@ -630,6 +630,17 @@ static int set_incidence_lists(peec_ctx* ctx, int64_t m, int64_t ns, int64_t n,
   return PEEC_OK;
 }
 
+// A new topology replaces the context's sizes and lists step by step: what was installed for the
+// one before (frequency state, factors and their plan, per-edge data, spectra, 1/P) is gone from
+// here on, and so is the topology itself until all of it stands (alloc_work).
+static void drop_topology(peec_ctx* ctx) {
+  ctx->have_topo = ctx->have_spec = ctx->have_freq = ctx->have_pdiag = false;
+  ctx->have_rf = ctx->have_es = false;
+  ctx->have_rcc_rows = ctx->rcc = false;
+  ctx->dense = ctx->dense_rcc = ctx->dense_rcc_ready = false;
+  for (int b = 0; b < 4; ++b) ctx->dn_set[b] = ctx->dnR_set[b] = false;
+}
+
 // work vectors and staging of an operator with the context's sizes
 static int alloc_work(peec_ctx* ctx) {
   const int64_t m = ctx->m, ns = ctx->ns, n = ctx->n;
@@ -656,12 +667,12 @@ static int alloc_work(peec_ctx* ctx) {
   ctx->cc_prec = -1;
   if (ctx->hx) cudaFreeHost(ctx->hx);
   if (ctx->hy) cudaFreeHost(ctx->hy);
+  ctx->hx = ctx->hy = nullptr;
   PEEC_CUDA_TRY(cudaMallocHost(&ctx->hx, sizeof(c64) * ctx->N));
   PEEC_CUDA_TRY(cudaMallocHost(&ctx->hy, sizeof(c64) * ctx->N));
   ctx->kcap = 0;
-  ctx->have_topo = true;
-  ctx->have_spec = ctx->have_freq = ctx->have_pdiag = false;
   PEEC_CUDA_TRY(cudaStreamSynchronize(ctx->st));
+  ctx->have_topo = true;
   return PEEC_OK;
 }
 
@@ -683,6 +694,7 @@ static int peec_set_topology_body(peec_ctx* ctx, int Nx, int Ny, int Nz, int64_t
   if (Nx > (1 << 20) || Ny > (1 << 20) || Nz > (1 << 20))
     return bad(ctx, PEEC_ERR_UNSUPPORTED, "grid axis longer than 2^20 cells");
   PEEC_CUDA_TRY(cudaSetDevice(ctx->dev));
+  drop_topology(ctx);
   ctx->Nx = Nx; ctx->Ny = Ny; ctx->Nz = Nz;
   ctx->mx = mx; ctx->my = my; ctx->mz = mz; ctx->m = m; ctx->ns = ns; ctx->n = n;
   ctx->N = m + ns + n;
@@ -758,11 +770,9 @@ static int peec_set_topology_body(peec_ctx* ctx, int Nx, int Ny, int Nz, int64_t
     if (p) cudaFree(p);
     p = nullptr;
   }
-  ctx->have_rcc_rows = ctx->rcc = false;
   ctx->rcc_freq = -1.0;
   CTX_TRY(phase_tables(LP, ctx->ph64, ctx->ph32, ctx->st));
   ctx->lattice = true;
-  ctx->dense = false;
   return alloc_work(ctx);
 }
 
@@ -781,6 +791,7 @@ static int peec_set_incidence_body(peec_ctx* ctx, int64_t mx, int64_t my, int64_
   if (m + ns + n > INT32_MAX || 2 * m + 1 > INT32_MAX)
     return bad(ctx, PEEC_ERR_UNSUPPORTED, "problem too large for int32 indexing");
   PEEC_CUDA_TRY(cudaSetDevice(ctx->dev));
+  drop_topology(ctx);
   ctx->Nx = ctx->Ny = ctx->Nz = 0;
   ctx->mx = mx; ctx->my = my; ctx->mz = mz; ctx->m = m; ctx->ns = ns; ctx->n = n;
   ctx->N = m + ns + n;
@@ -792,11 +803,8 @@ static int peec_set_incidence_body(peec_ctx* ctx, int64_t mx, int64_t my, int64_
     }
     F.active = false;
   }
-  ctx->have_rcc_rows = ctx->rcc = false;
   ctx->rcc_freq = -1.0;
   ctx->lattice = false;
-  ctx->dense = false;
-  for (int b = 0; b < 4; ++b) ctx->dn_set[b] = ctx->dnR_set[b] = false;
   return alloc_work(ctx);
 }
 

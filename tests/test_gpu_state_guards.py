@@ -16,8 +16,7 @@ pytestmark = pytest.mark.gpu
 BADARG, STATE = -5, -7  # PEEC_ERR_*
 
 
-@pytest.fixture(scope="module")
-def geom():
+def _geometry():
     req = configs.random_mixed((9, 8, 5), s=5e-5, p=0.6, seed=5, nports=1, freqs=[1e9], tol=1e-8)
     out, freqs, _s, z0, _grid = mesher.parse_request(req)
     esc, inc, cc, diag, exp, ports, le, _li, Zs = out
@@ -25,6 +24,12 @@ def geom():
                                   z0)
     op = GpuOperator(inc, exp, diag["P"])
     op.fill(cc["origin"], cc["sx"], cc["sy"], cc["sz"], esc["Lp"], esc["P"])
+    return op, fs, (diag, Zs, esc)
+
+
+@pytest.fixture(scope="module")
+def geom():
+    op, fs, _data = _geometry()
     yield op, fs
     op.close()
 
@@ -144,3 +149,30 @@ def test_wider_yle_pattern_at_the_set_up(geom):
     ref = op.matvec(x, 0)
     assert np.max(np.abs(got - ref)) <= max(bound, 1e-10 * np.max(np.abs(ref)))
     assert np.max(np.abs(ref - y)) > 10 * bound  # the admittance is seen
+
+
+@pytest.mark.parametrize("valid", [False, True])
+def test_new_topology_drops_what_was_installed(valid):
+    """A second topology on a context, refused or not: nothing of the first one is used with it
+    (its factors, refactorisation plan and edge data have other sizes)."""
+    op, fs, data = _geometry()
+    try:
+        x = np.ones(op.N, dtype=complex)
+        op.set_frequency(fs.w, fs.DZ, fs.Yle, fs.lu)
+        op.enable_refactor(fs.Yle)
+        op.set_edge_state(data[0], data[1], data[2])
+        op.matvec(x, 0)
+        n1, n2 = np.zeros(op.m, np.int64), np.ones(op.m, np.int64)
+        n2[-1] = 1 if valid else op.n
+        node = np.zeros(op.ns, np.int64)
+        rc = op.L.peec_set_incidence(op.h, op.m, 0, 0, _lib.ptr(n1), _lib.ptr(n2), op.ns,
+                                     _lib.ptr(node), op.n)
+        assert rc == (0 if valid else BADARG)
+        for call in (lambda: op.matvec(x, 0), lambda: op.port_rhs(0, 1, 1.0),
+                     lambda: op.gmres(x, None, 1e-6, 5), lambda: op.solve_mixed(x, None, 1e-6),
+                     lambda: op.set_frequency_refactor(fs.w, fs.DZ, fs.Yle),
+                     lambda: op.set_frequency_device(fs.w, fs.Yle),
+                     lambda: op.enable_refactor(fs.Yle)):
+            _is_refused(call)
+    finally:
+        op.close()
