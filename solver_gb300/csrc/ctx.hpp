@@ -152,11 +152,11 @@ size_t gm_part_doubles(size_t N, int k);
 int gm_pre(const GmBody& B);   // returns the kernels launched
 int gm_post(const GmBody& B);
 
-// Stream-ordered scratch from a context's pool (nullptr: the device's default pool, which gives
-// its memory back at every synchronisation and maps it again at the next allocation)
-inline cudaError_t scratch_alloc(void** p, size_t bytes, cudaMemPool_t pool, cudaStream_t st) {
-  return pool ? cudaMallocFromPoolAsync(p, bytes, pool, st) : cudaMallocAsync(p, bytes, st);
-}
+// cudaMalloc, and stream-ordered scratch from a context's pool (nullptr: the device's default
+// pool). Where the device is full, both take back what the contexts' pools on it keep unused and
+// try once more, so that a kept pool refuses no allocation.
+cudaError_t dev_alloc(void** p, size_t bytes);
+cudaError_t scratch_alloc(void** p, size_t bytes, cudaMemPool_t pool, cudaStream_t st);
 
 #define CTX_CHECK(expr)      \
   do {                       \

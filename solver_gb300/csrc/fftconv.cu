@@ -264,8 +264,8 @@ int phase_tables(const int L[3], void* e64[3], void* e32[3], cudaStream_t st) {
     if (e64[a]) cudaFree(e64[a]);
     if (e32[a]) cudaFree(e32[a]);
     e64[a] = e32[a] = nullptr;
-    PEEC_CUDA_TRY(cudaMalloc(&e64[a], sizeof(c64) * L[a]));
-    PEEC_CUDA_TRY(cudaMalloc(&e32[a], sizeof(c32) * L[a]));
+    PEEC_CUDA_TRY(dev_alloc(&e64[a], sizeof(c64) * L[a]));
+    PEEC_CUDA_TRY(dev_alloc(&e32[a], sizeof(c32) * L[a]));
     k_phase_table<<<(L[a] + 255) / 256, 256, 0, st>>>(L[a], (c64*)e64[a], (c32*)e32[a]);
   }
   PEEC_CUDA_TRY(cudaGetLastError());
@@ -330,8 +330,8 @@ int spectra_build(const SpecJob* jobs, int njobs, const void* tw64, int twmax, c
                          J.M[a], J.sdim[a] == 2 ? J.M[a] / 2 : J.M[a]};
     }
     const size_t ny = (size_t)S.L[0] * (S.L[1] / 2 + 1) * (S.L[2] / 2 + 1);
-    if (!S.yz[0]) PEEC_CUDA_TRY(cudaMalloc(&S.yz[0], ny * sizeof(double)));
-    if (!S.yz[1]) PEEC_CUDA_TRY(cudaMalloc(&S.yz[1], ny * sizeof(float)));
+    if (!S.yz[0]) PEEC_CUDA_TRY(dev_alloc(&S.yz[0], ny * sizeof(double)));
+    if (!S.yz[1]) PEEC_CUDA_TRY(dev_alloc(&S.yz[1], ny * sizeof(float)));
     R.row = J.row;
     R.scale = 1.0 / ((double)S.L[0] * S.L[1] * S.L[2]);
     na += (size_t)R.ax[2].U * R.ax[1].U * (S.L[0] / 2 + 1);

@@ -25,6 +25,10 @@
 #include <string>
 #include <vector>
 
+namespace peec {
+cudaError_t dev_alloc(void** p, size_t bytes);  // ctx.cu
+}
+
 namespace {
 
 // cudaSuccess and this file's success are both 0
@@ -605,7 +609,7 @@ struct DevPool {
   int alloc(T** out, int64_t n) {
     *out = nullptr;
     const size_t bytes = sizeof(T) * (size_t)(n > 0 ? n : 1);
-    MG_TRY(cudaMalloc((void**)out, bytes));
+    MG_TRY(peec::dev_alloc((void**)out, bytes));
     p.push_back(*out);
     return 0;
   }

@@ -3,6 +3,8 @@ the context's arrays one by one, and the LU groups' plan holds positions in the 
 refused upload has to leave a context that refuses applications and solves (PEEC_ERR_STATE, by the
 host's check, before anything is launched) until a whole state is installed; what then comes out is
 what came out before, bit for bit (the same kernels on the same values)."""
+import ctypes
+
 import numpy as np
 import pytest
 import scipy.sparse as sp
@@ -13,7 +15,7 @@ from solver_gb300.operator import GpuOperator
 
 pytestmark = pytest.mark.gpu
 
-BADARG, STATE = -5, -7  # PEEC_ERR_*
+OOM, BADARG, STATE = -2, -5, -7  # PEEC_ERR_*
 
 
 def _geometry():
@@ -174,5 +176,29 @@ def test_new_topology_drops_what_was_installed(valid):
                      lambda: op.set_frequency_device(fs.w, fs.Yle),
                      lambda: op.enable_refactor(fs.Yle)):
             _is_refused(call)
+    finally:
+        op.close()
+
+
+def test_kept_scratch_is_given_back_to_a_full_device():
+    """The scratch a fill leaves mapped (here some 40 MB of rows and transforms) goes back to the
+    device when an allocation finds it full -- a reduction scratch of 5 TB, which the device refuses
+    at once -- and the next fill maps it again, with the same rows."""
+    import torch
+    req = configs.random_mixed((48, 48, 24), s=5e-5, p=0.02, seed=5, nports=1, freqs=[1e9], tol=1e-8)
+    out = mesher.parse_request(req)[0]
+    esc, inc, cc, diag, exp = out[:5]
+    op = GpuOperator(inc, exp, diag["P"])
+    try:
+        args = (cc["origin"], cc["sx"], cc["sy"], cc["sz"], esc["Lp"], esc["P"])
+        rows = op.fill(*args, return_rows=True)
+        v = torch.zeros(16, dtype=torch.complex128, device="cuda")
+        torch.cuda.synchronize()
+        free = torch.cuda.mem_get_info()[0]
+        p = ctypes.c_void_p(v.data_ptr())
+        assert op.L.peec_multidot(op.h, p, 10**6, p, 10**6, 1 << 30, p) == OOM
+        assert torch.cuda.mem_get_info()[0] >= free + (16 << 20)
+        again = op.fill(*args, return_rows=True)
+        assert all(np.array_equal(rows[k], again[k]) for k in rows)
     finally:
         op.close()
