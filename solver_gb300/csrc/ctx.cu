@@ -8,7 +8,6 @@
 #include <array>
 #include <map>
 #include <queue>
-#include <set>
 #include <mutex>
 #include <new>
 #include <stdexcept>
@@ -50,38 +49,17 @@ int fail_cuda(cudaError_t e, const char* expr, const char* file, int line) {
   return e == cudaErrorMemoryAllocation ? PEEC_ERR_OOM : PEEC_ERR_CUDA;
 }
 
-// the contexts' pools, with their devices
-static std::mutex g_pool_mu;
-static std::set<std::pair<int, cudaMemPool_t>> g_pools;
-
-static void trim_pools() {
-  cudaGetLastError();
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess) return;
-  std::lock_guard<std::mutex> lock(g_pool_mu);
-  for (const auto& p : g_pools)
-    if (p.first == dev) cudaMemPoolTrimTo(p.second, 0);
-}
-cudaError_t dev_alloc(void** p, size_t bytes) {
-  cudaError_t e = cudaMalloc(p, bytes);
-  if (e != cudaErrorMemoryAllocation) return e;
-  trim_pools();
-  e = cudaMalloc(p, bytes);
-  if (e != cudaSuccess) *p = nullptr;
-  if (e == cudaErrorMemoryAllocation) cudaGetLastError();  // reported by its code, not by a later launch
-  return e;
-}
-cudaError_t scratch_alloc(void** p, size_t bytes, cudaMemPool_t pool, cudaStream_t st) {
-  auto get = [&] {
-    return pool ? cudaMallocFromPoolAsync(p, bytes, pool, st) : cudaMallocAsync(p, bytes, st);
-  };
-  cudaError_t e = get();
-  if (e != cudaErrorMemoryAllocation) return e;
-  trim_pools();
-  e = get();
-  if (e != cudaSuccess) *p = nullptr;
+// a refused allocation is reported by its code; the runtime's last-error word, which launch checks
+// read, is cleared
+static cudaError_t refused(cudaError_t e, void** p) {
+  if (e == cudaSuccess) return e;
+  *p = nullptr;
   if (e == cudaErrorMemoryAllocation) cudaGetLastError();
   return e;
+}
+cudaError_t dev_alloc(void** p, size_t bytes) { return refused(cudaMalloc(p, bytes), p); }
+cudaError_t scratch_alloc(void** p, size_t bytes, cudaMemPool_t pool, cudaStream_t st) {
+  return refused(pool ? cudaMallocFromPoolAsync(p, bytes, pool, st) : cudaMallocAsync(p, bytes, st), p);
 }
 
 // launchers defined in the other translation units
@@ -221,7 +199,8 @@ struct peec_ctx {
   void* ph64[3] = {nullptr, nullptr, nullptr};  // face-grid phase tables
   void* ph32[3] = {nullptr, nullptr, nullptr};  // their FP32 rounding (FP32 z passes)
   // scratch of fills and spectra: up to POOL_KEEP bytes stay mapped between calls, given back
-  // with the context, or where an allocation of any context finds the device full (dev_alloc)
+  // with the context; the driver takes them back by itself where an allocation of the process
+  // finds the device full
   cudaMemPool_t pool = nullptr;
   int* zerr = nullptr;  // set by a staged z pass whose copy wait ran into its limit
   int nsm = 0;          // SM count of the device
@@ -494,13 +473,8 @@ static int peec_ctx_create_body(peec_ctx** out, int device) {
   pp.location.type = cudaMemLocationTypeDevice;
   pp.location.id = device;
   uint64_t keep = POOL_KEEP;
-  if (cudaMemPoolCreate(&ctx->pool, &pp) != cudaSuccess) {
-    ctx->pool = nullptr;
-  } else {
-    cudaMemPoolSetAttribute(ctx->pool, cudaMemPoolAttrReleaseThreshold, &keep);
-    std::lock_guard<std::mutex> lock(g_pool_mu);
-    g_pools.insert({device, ctx->pool});
-  }
+  if (cudaMemPoolCreate(&ctx->pool, &pp) != cudaSuccess) ctx->pool = nullptr;
+  else cudaMemPoolSetAttribute(ctx->pool, cudaMemPoolAttrReleaseThreshold, &keep);
   cudaGetLastError();
   cudaMallocHost(&ctx->hsmall, sizeof(c64) * 16 * 4096);
   cudaMallocHost(&ctx->hread, sizeof(c64) * 4096);
@@ -562,11 +536,7 @@ extern "C" void peec_ctx_destroy(peec_ctx* ctx) {
     if (ctx->ph32[a]) cudaFree(ctx->ph32[a]);
   }
   cudaFree(ctx->zerr);
-  if (ctx->pool) {
-    std::lock_guard<std::mutex> lock(g_pool_mu);
-    g_pools.erase({ctx->dev, ctx->pool});
-    cudaMemPoolDestroy(ctx->pool);
-  }
+  if (ctx->pool) cudaMemPoolDestroy(ctx->pool);
   free_tri(ctx->Lf);
   free_tri(ctx->Uf);
   cudaFree(ctx->sf_ord);

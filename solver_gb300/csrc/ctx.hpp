@@ -153,8 +153,8 @@ int gm_pre(const GmBody& B);   // returns the kernels launched
 int gm_post(const GmBody& B);
 
 // cudaMalloc, and stream-ordered scratch from a context's pool (nullptr: the device's default
-// pool). Where the device is full, both take back what the contexts' pools on it keep unused and
-// try once more, so that a kept pool refuses no allocation.
+// pool, which gives its memory back at every synchronisation and maps it again at the next
+// allocation). A refusal for lack of memory leaves nothing for later error checks to find.
 cudaError_t dev_alloc(void** p, size_t bytes);
 cudaError_t scratch_alloc(void** p, size_t bytes, cudaMemPool_t pool, cudaStream_t st);
 

@@ -180,10 +180,11 @@ def test_new_topology_drops_what_was_installed(valid):
         op.close()
 
 
-def test_kept_scratch_is_given_back_to_a_full_device():
-    """The scratch a fill leaves mapped (here some 40 MB of rows and transforms) goes back to the
-    device when an allocation finds it full -- a reduction scratch of 5 TB, which the device refuses
-    at once -- and the next fill maps it again, with the same rows."""
+def test_refused_allocation_leaves_the_context_usable():
+    """An allocation the device refuses (a reduction scratch of 5 TB, at once) is reported as such
+    and not a second time by the next call's launch checks; the scratch a fill leaves mapped (here
+    some 33 MB of rows and transforms) is free again for others by then, and the next fill maps it
+    once more, with the same rows."""
     import torch
     req = configs.random_mixed((48, 48, 24), s=5e-5, p=0.02, seed=5, nports=1, freqs=[1e9], tol=1e-8)
     out = mesher.parse_request(req)[0]
