@@ -846,23 +846,28 @@ __device__ __forceinline__ YzIdx make_yzidx(int Lx, int Ly, int Lz, int kx0, int
   return y;
 }
 
-// The phases of a frequency relative to family 0: S_fg = phi_f conj(phi_g) R_fg with phi =
-// (E_y, E_x, E_z), so with psi_1 = E_x conj(E_y) (constant along a column) and psi_2 =
-// E_z conj(E_y) the product is psi_f sum_g R_fg conj(psi_g) X_g, R real and symmetric.
-// Y_f = sum_g S_fg X_g at the frequency of (column col, z position pz) of the CTA; p1 = psi_1,
-// ey the CTA's y phase
+// Y_f = sum_g S_fg X_g at the frequency of (column col, z position pz) of the CTA; ex the column's
+// x phase, ey the CTA's y phase. FP64, bound by its pipe, rotates families 1 and 2 to family 0's
+// phase and back (psi_1 = E_x conj(E_y), psi_2 = E_z conj(E_y)): there the operator's error, against
+// a reference with 64-bit significands, is that of complex tables either way.
 template <typename R>
 __device__ __forceinline__ void pspec_apply(const PSpec& S, const YzIdx& Y, int col, int pz,
-                                            const cx<R>& p1, const cx<R>& ey, cx<R>& a0,
+                                            const cx<R>& ex, const cx<R>& ey, cx<R>& a0,
                                             cx<R>& a1, cx<R>& a2) {
   const size_t i = Y.at(col, pz);
-  const cx<R> p2 = cmulc(spec_cx<R>(S.ez, pz), ey);
-  const R r00 = spec_re<R>(S.y[0], i), r11 = spec_re<R>(S.y[1], i), r22 = spec_re<R>(S.y[2], i);
-  const R r01 = spec_re<R>(S.y[3], i), r02 = spec_re<R>(S.y[4], i), r12 = spec_re<R>(S.y[5], i);
-  const cx<R> x0 = a0, x1 = cmulc(a1, p1), x2 = cmulc(a2, p2);
-  a0 = cscale(x0, r00) + cscale(x1, r01) + cscale(x2, r02);
-  a1 = (cscale(x0, r01) + cscale(x1, r11) + cscale(x2, r12)) * p1;
-  a2 = (cscale(x0, r02) + cscale(x1, r12) + cscale(x2, r22)) * p2;
+  const cx<R> ez = spec_cx<R>(S.ez, pz);
+  R r[6];
+#pragma unroll
+  for (int b = 0; b < 6; ++b) r[b] = spec_re<R>(S.y[b], i);
+  if constexpr (std::is_same<R, double>::value) {
+    const cx<R> p1 = cmulc(ex, ey), p2 = cmulc(ez, ey);
+    const cx<R> x0 = a0, x1 = cmulc(a1, p1), x2 = cmulc(a2, p2);
+    a0 = cscale(x0, r[0]) + cscale(x1, r[3]) + cscale(x2, r[4]);
+    a1 = (cscale(x0, r[3]) + cscale(x1, r[1]) + cscale(x2, r[5])) * p1;
+    a2 = (cscale(x0, r[4]) + cscale(x1, r[5]) + cscale(x2, r[2])) * p2;
+  } else {
+    pspec_product<R>(r, cmulc(ey, ex), cmulc(ey, ez), cmulc(ex, ez), a0, a1, a2);
+  }
 }
 
 // single-group z transform of all three face families in registers
@@ -873,7 +878,7 @@ __device__ __forceinline__ void z3_single(cx<R>* T0, cx<R>* T1, cx<R>* T2, int n
   constexpr int N = 1 << Q;
   for (int col = threadIdx.x; col < TX; col += blockDim.x) {
     if (col >= ncols) continue;
-    const cx<R> p1 = cmulc(spec_cx<R>(S.ex, kx0 + col), ey);
+    const cx<R> ex = spec_cx<R>(S.ex, kx0 + col);
     cx<R> v[3][N];
 #pragma unroll
     for (int r = 0; r < N; ++r) {
@@ -884,7 +889,7 @@ __device__ __forceinline__ void z3_single(cx<R>* T0, cx<R>* T1, cx<R>* T2, int n
 #pragma unroll
     for (int f = 0; f < 3; ++f) dft_dif<R, Q>(v[f]);
 #pragma unroll
-    for (int r = 0; r < N; ++r) pspec_apply<R>(S, O, col, r, p1, ey, v[0][r], v[1][r], v[2][r]);
+    for (int r = 0; r < N; ++r) pspec_apply<R>(S, O, col, r, ex, ey, v[0][r], v[1][r], v[2][r]);
 #pragma unroll
     for (int f = 0; f < 3; ++f) dft_dit<R, Q>(v[f]);
 #pragma unroll
@@ -915,10 +920,10 @@ __device__ __forceinline__ void z3_fused(cx<R>* buf, size_t tsz, const AxPlan& p
       dft_dif<R, Q>(v[f]);
     }
     if (col < ncols) {
-      const cx<R> p1 = cmulc(spec_cx<R>(S.ex, kx0 + col), ey);
+      const cx<R> ex = spec_cx<R>(S.ex, kx0 + col);
 #pragma unroll
       for (int r = 0; r < N; ++r)
-        pspec_apply<R>(S, O, col, start + r, p1, ey, v[0][r], v[1][r], v[2][r]);
+        pspec_apply<R>(S, O, col, start + r, ex, ey, v[0][r], v[1][r], v[2][r]);
     }
 #pragma unroll
     for (int f = 0; f < 3; ++f) {
@@ -1123,9 +1128,9 @@ __device__ __forceinline__ void z3_fused_yz(c32* buf, size_t tsz, const AxPlan& 
       for (int r = 0; r < N; ++r) v[f][r] = buf[f * tsz + ((start + r) << LTX) + col];
       dft_dif<float, Q>(v[f]);
     }
-    const c32 p1 = cmulc(spec_cx<float>(S.ex, kx0 + col), ey);
+    const c32 ex = spec_cx<float>(S.ex, kx0 + col);
 #pragma unroll
-    for (int r = 0; r < N; ++r) pspec_apply<float>(S, Y, col, start + r, p1, ey, v[0][r], v[1][r], v[2][r]);
+    for (int r = 0; r < N; ++r) pspec_apply<float>(S, Y, col, start + r, ex, ey, v[0][r], v[1][r], v[2][r]);
 #pragma unroll
     for (int f = 0; f < 3; ++f) {
       dft_dit<float, Q>(v[f]);
@@ -1360,9 +1365,7 @@ __global__ void __launch_bounds__(ZTPB, 4) k_zedge_staged(EdgeSet E, int nzs, in
 // the inverse of a half run between two barriers. The three face families share the threads.
 // Spectra: the y/z-folded tables of the half's frequencies go to shared memory by asynchronous
 // copies while the rows load and the forward transform runs; both kz and Lz - kz read them.
-// The cross blocks' phases factor, S_fg = phi_f conj(phi_g) R_fg with R real: the phases of x
-// and y are constant along a column and multiply the rows before and after, those of z
-// multiply one family's points (relative to family 0), and the product is a real 3 x 3.
+// The cross blocks' coefficients are formed from the phases of x, y and z (pspec_product).
 // FP32 keeps the rows in registers for the second half; the wider types read them again and
 // leave the odd half's rows in their place until the even half's are there.
 // What bounds them: FP32 instruction issue and loads, float-float the FP32 pipes; the pruning
@@ -1419,7 +1422,7 @@ struct ZPairCta {
   int c, k, col0, px, py;
   bool on;
   size_t pl, at0;
-  cx<R> ph1, ph2, xh[NF];
+  cx<R> ex, ey, q01, xh[NF];
 
   // the CTA's job and columns; shared memory, the twiddles and the first spectra on their way
   template <typename Set>
@@ -1451,12 +1454,12 @@ struct ZPairCta {
       W[e] = twm[e * (twmax / L)];
       if (NF == 3) Ez[e] = spec_cx<R>(P->ez, brevn(e, A + B + 1));
     }
-    // the columns' x and y phases of families 1 and 2 (relative to family 0)
-    ph1 = ph2 = mk<R>(1, 0);
+    // the column's x and y phases
+    ex = ey = q01 = mk<R>(1, 0);
     if (NF == 3 && on) {
-      const cx<R> ex = spec_cx<R>(P->ex, px), ey = spec_cx<R>(P->ey, py);
-      ph1 = cmulc(ex, ey);  // psi_1; psi_2 = ez conj(ey)
-      ph2 = cconj(ey);
+      ex = spec_cx<R>(P->ex, px);
+      ey = spec_cx<R>(P->ey, py);
+      q01 = cmulc(ey, ex);
     }
   }
 
@@ -1496,15 +1499,6 @@ struct ZPairCta {
         x.d[f][r] = on && n < nz ? ld_stream(T + n * pl) : mk<R>(0, 0);
       }
       xh[f] = on && k == 0 && nz > H ? ld_stream(T + H * pl) : mk<R>(0, 0);
-    }
-    if constexpr (NF == 3) {
-#pragma unroll
-      for (int r = 0; r < V; ++r) {
-        x.d[1][r] = cmulc(x.d[1][r], ph1);
-        x.d[2][r] = cmulc(x.d[2][r], ph2);
-      }
-      xh[1] = cmulc(xh[1], ph1);
-      xh[2] = cmulc(xh[2], ph2);
     }
   }
 
@@ -1547,12 +1541,10 @@ struct ZPairCta {
       } else {
         constexpr size_t TS = (size_t)NS * C;
         const cx<R> e = Ez[kz];
-        const cx<R> x0 = x.d[0][i], x1 = x.d[1][i], x2 = cmulc(x.d[2][i], e);
-        const R r00 = R(s[0]), r11 = R(s[TS]), r22 = R(s[2 * TS]);
-        const R r01 = R(s[3 * TS]), r02 = R(s[4 * TS]), r12 = R(s[5 * TS]);
-        x.d[0][i] = cscale(x0, r00) + cscale(x1, r01) + cscale(x2, r02);
-        x.d[1][i] = cscale(x0, r01) + cscale(x1, r11) + cscale(x2, r12);
-        x.d[2][i] = (cscale(x0, r02) + cscale(x1, r12) + cscale(x2, r22)) * e;
+        R rr[6];
+#pragma unroll
+        for (int b = 0; b < 6; ++b) rr[b] = R(s[b * TS]);
+        pspec_product<R>(rr, q01, cmulc(ey, e), cmulc(ex, e), x.d[0][i], x.d[1][i], x.d[2][i]);
       }
     }
     if constexpr (B > 0) {
@@ -1589,14 +1581,8 @@ struct ZPairCta {
   __device__ __forceinline__ void store(int f, int r, const cx<R>& e, const cx<R>& o) const {
     const int n = k + G * r;
     cx<R>* T = P->T[f] + at0;
-    cx<R> y = e + o;
-    if (NF == 3 && f > 0) y = y * (f == 1 ? ph1 : ph2);
-    if (on && n < P->nz[f]) st_stream(T + n * pl, y);
-    if (r == 0 && on && k == 0 && P->nz[f] > H) {
-      cx<R> yh = e - o;
-      if (NF == 3 && f > 0) yh = yh * (f == 1 ? ph1 : ph2);
-      st_stream(T + H * pl, yh);
-    }
+    if (on && n < P->nz[f]) st_stream(T + n * pl, e + o);
+    if (r == 0 && on && k == 0 && P->nz[f] > H) st_stream(T + H * pl, e - o);
   }
 };
 
@@ -1666,7 +1652,6 @@ __global__ void __launch_bounds__(ZP_TPB, MINB) k_zpair_wide(ZPairSet<R, NF == 3
       cx<R>* T = t.P->T[f] + t.at0;
       const int nz = t.P->nz[f];
       cx<R>* xf = t.xch + (size_t)f * H * C + c;
-      const cx<R> ph = f == 1 ? t.ph1 : t.ph2;
       cx<R> d[V], x[V], xh = mk<R>(0, 0);
       if (stage < 2 && t.on && k == 0 && nz > H) xh = ld_stream(T + H * t.pl);
       if (stage > 0) {
@@ -1684,14 +1669,8 @@ __global__ void __launch_bounds__(ZP_TPB, MINB) k_zpair_wide(ZPairSet<R, NF == 3
 #pragma unroll
         for (int r = 0; r < V; ++r) {
           const int n = k + G * r;
-          cx<R> y = d[r] + x[r];
-          if (NF == 3 && f > 0) y = y * ph;
-          if (t.on && n < nz) st_stream(T + n * t.pl, y);
-          if (r == 0 && t.on && k == 0 && nz > H) {
-            cx<R> yh = d[0] - x[0];
-            if (NF == 3 && f > 0) yh = yh * ph;
-            st_stream(T + H * t.pl, yh);
-          }
+          if (t.on && n < nz) st_stream(T + n * t.pl, d[r] + x[r]);
+          if (r == 0 && t.on && k == 0 && nz > H) st_stream(T + H * t.pl, d[0] - x[0]);
         }
         continue;
       }
@@ -1702,11 +1681,6 @@ __global__ void __launch_bounds__(ZP_TPB, MINB) k_zpair_wide(ZPairSet<R, NF == 3
           const cx<R> o = cmulc(d[r], t.W[n]);
           if (t.on && n < nz) st_stream(T + n * t.pl, o);
         }
-      }
-      if (NF == 3 && f > 0) {
-#pragma unroll
-        for (int r = 0; r < V; ++r) x[r] = cmulc(x[r], ph);
-        xh = cmulc(xh, ph);
       }
       x[0] = stage == 0 ? x[0] - xh : x[0] + xh;
       if (stage == 0) {
@@ -1752,12 +1726,10 @@ __global__ void __launch_bounds__(ZP_TPB, MINB) k_zpair_wide(ZPairSet<R, NF == 3
       } else {
         constexpr size_t TS = (size_t)NS * C, XS = (size_t)H * C;
         const cx<R> e = t.Ez[kz];
-        const cx<R> x0 = x[0], x1 = x[XS], x2 = cmulc(x[2 * XS], e);
-        const R r00 = R(s[0]), r11 = R(s[TS]), r22 = R(s[2 * TS]);
-        const R r01 = R(s[3 * TS]), r02 = R(s[4 * TS]), r12 = R(s[5 * TS]);
-        x[0] = cscale(x0, r00) + cscale(x1, r01) + cscale(x2, r02);
-        x[XS] = cscale(x0, r01) + cscale(x1, r11) + cscale(x2, r12);
-        x[2 * XS] = (cscale(x0, r02) + cscale(x1, r12) + cscale(x2, r22)) * e;
+        R rr[6];
+#pragma unroll
+        for (int b = 0; b < 6; ++b) rr[b] = R(s[b * TS]);
+        pspec_product<R>(rr, t.q01, cmulc(t.ey, e), cmulc(t.ex, e), x[0], x[XS], x[2 * XS]);
       }
     }
     if constexpr (B > 0) {
