@@ -152,24 +152,3 @@ __device__ __forceinline__ double ff_join(ff a) {
   return (double)a;
 }
 using cff = cx<ff>;
-
-// a b + c d: exact high products and their two-sum, the errors and cross terms in FP32, one
-// normalisation: 19 operations where the two products and their sum take 25, and no rounding
-// of the products on the way
-__host__ __device__ __forceinline__ ff ff_dot2(ff a, ff b, ff c, ff d) {
-  const float p = PEEC_FMUL(a.hi, b.hi), q = PEEC_FMUL(c.hi, d.hi);
-  float e = PEEC_FMA(a.hi, b.hi, -p);
-  e = PEEC_FMA(a.hi, b.lo, e);
-  e = PEEC_FMA(a.lo, b.hi, e);
-  float f = PEEC_FMA(c.hi, d.hi, -q);
-  f = PEEC_FMA(c.hi, d.lo, f);
-  f = PEEC_FMA(c.lo, d.hi, f);
-  const ff s = ff_two_sum(p, q);
-  return ff_fast_two_sum(s.hi, PEEC_FADD(s.lo, PEEC_FADD(e, f)));
-}
-__host__ __device__ __forceinline__ cff operator*(const cff& a, const cff& b) {
-  return mk<ff>(ff_dot2(a.x, b.x, -a.y, b.y), ff_dot2(a.x, b.y, a.y, b.x));
-}
-__host__ __device__ __forceinline__ cff cmulc(const cff& a, const cff& b) {
-  return mk<ff>(ff_dot2(a.x, b.x, a.y, b.y), ff_dot2(a.y, b.x, -a.x, b.y));
-}

@@ -238,8 +238,8 @@ __device__ __forceinline__ void load_twiddles(cx<R>* W, const cx<R>* __restrict_
 // error is 1.25 times that of complex coefficients rounded once. Rotating the families to one phase
 // and back (psi_f sum_g R_fg conj(psi_g) a_g) takes ten operations less a frequency, but it is
 // 1.56 times; the FP32 operator's error was 3 % larger with it over 56 grids than with complex
-// tables, and is 2 % smaller so. z passes at 128x128x64: FP32 170 -> 176 us, float-float 1382 ->
-// 1346 us (there the rotations of the rows cost more).
+// tables, and is 2 % smaller so. z passes at 128x128x64: FP32 170 -> 176 us, float-float 3 % faster
+// (there the rotations of the rows cost more).
 template <typename R>
 __host__ __device__ __forceinline__ void pspec_product(const R* r, const cx<R>& q01,
                                                        const cx<R>& q02, const cx<R>& q12,

@@ -1371,7 +1371,7 @@ __global__ void __launch_bounds__(ZTPB, 4) k_zedge_staged(EdgeSet E, int nzs, in
 // What bounds them: FP32 instruction issue and loads, float-float the FP32 pipes; the pruning
 // halves the arithmetic of the padded transforms. z passes of an operator application at
 // 128x128x64, faces + edges: FP32 267 us in the direct and staged forms, 169 here (93 + 72);
-// float-float 2541 us direct, 1382 here. FP64 stays direct (see conv_all_t).
+// float-float 2541 us direct, 1443 here. FP64 stays direct (see conv_all_t).
 template <typename R>
 struct ZPairJob {
   cx<R>* T[3];        // face families (edges: T[0] only)

@@ -61,8 +61,32 @@ static void product() {
   printf("product %.17g\n", sqrt(e[1] / e[0]));
 }
 
+static long double value(ff a) { return (long double)a.hi + (long double)a.lo; }
+
+static void complex_products() {
+  double e[2] = {0, 0};
+  for (int i = 0; i < 500000; ++i) {
+    const c64 w = unit();
+    const cff a = mk<ff>(ff(normal()), ff(normal())), b = mk<ff>(ff(w.x), ff(w.y));
+    const cff p[2] = {a * b, cmulc(a, b)};
+    for (int conj = 0; conj < 2; ++conj) {
+      const ff by = conj ? -b.y : b.y;
+      const ff plain[2] = {a.x * b.x - a.y * by, a.x * by + a.y * b.x};
+      const ff got[2] = {p[conj].x, p[conj].y};
+      const long double ex[2] = {value(a.x) * value(b.x) - value(a.y) * value(by),
+                                 value(a.x) * value(by) + value(a.y) * value(b.x)};
+      for (int k = 0; k < 2; ++k) {
+        e[0] += powl(value(plain[k]) - ex[k], 2);
+        e[1] += powl(value(got[k]) - ex[k], 2);
+      }
+    }
+  }
+  printf("ff_product %.17g\n", sqrt(e[1] / e[0]));
+}
+
 int main() {
   product();
+  complex_products();
   return 0;
 }
 """
@@ -84,3 +108,7 @@ def measured(tmp_path_factory):
 
 def test_block_product(measured):
     assert measured["product"] <= 2 ** 0.5, measured
+
+
+def test_float_float_complex_product(measured):
+    assert measured["ff_product"] <= 1.05, measured
