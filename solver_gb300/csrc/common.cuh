@@ -152,3 +152,17 @@ __device__ __forceinline__ double ff_join(ff a) {
   return (double)a;
 }
 using cff = cx<ff>;
+
+// acc += u x and acc += conj(u) x, products and sums one after the other: in float-float, 72
+// operations. Adding the high parts of both products and of the sum exactly and all error terms
+// before one normalisation takes 54, but a chain of 8 to 512 such sums rounds 1.5 times worse.
+template <typename A>
+__host__ __device__ __forceinline__ void cmac(cx<A>& acc, const cx<A>& u, const cx<A>& x) {
+  acc.x = acc.x + (u.x * x.x - u.y * x.y);
+  acc.y = acc.y + (u.x * x.y + u.y * x.x);
+}
+template <typename A>
+__host__ __device__ __forceinline__ void cmac_conj(cx<A>& acc, const cx<A>& u, const cx<A>& x) {
+  acc.x = acc.x + (u.x * x.x + u.y * x.y);
+  acc.y = acc.y + (u.x * x.y - u.y * x.x);
+}

@@ -253,7 +253,7 @@ __device__ __forceinline__ c64 csign(c64 d) {
 // would take a second pass over the column). Each kernel ends in its last CTA, so the small
 // products over T need no launch of their own; every sum has a fixed order, whichever CTA comes
 // last.
-// What bounds them: float-float's FP32 pipes (54 instructions a complex product and sum) and
+// What bounds them: float-float's FP32 pipes (72 instructions a complex product and sum) and
 // the basis, read once for v, once for z and twice (then from L1 or L2) for x and t; below some
 // 100k rows the latency of the last CTA. FP64 instructions hold their pipe 64 cycles, so
 // conversions are integer code, lanes' sums are exchanged in halves (16 additions a warp for
@@ -301,28 +301,6 @@ size_t gm_part_doubles(size_t N, int k) {
   return std::max<size_t>(2 * (size_t)(k + 1) * (g.nb + (g.nb + GM_FAN - 1) / GM_FAN), g.vb);
 }
 
-// acc += a b + c d, the products and sums of the high parts exact (two-products, two-sums),
-// their errors and the cross terms in FP32: closer than the two rounded sums of acc + (ab + cd)
-__device__ __forceinline__ void mac2(ff& acc, ff a, ff b, ff c, ff d) {
-  const float p = __fmul_rn(a.hi, b.hi), q = __fmul_rn(c.hi, d.hi);
-  const float pe = __fmaf_rn(a.lo, b.hi, __fmaf_rn(a.hi, b.lo, __fmaf_rn(a.hi, b.hi, -p)));
-  const float qe = __fmaf_rn(c.lo, d.hi, __fmaf_rn(c.hi, d.lo, __fmaf_rn(c.hi, d.hi, -q)));
-  const ff s = ff_two_sum(acc.hi, p), t = ff_two_sum(s.hi, q);
-  acc = ff_fast_two_sum(t.hi, __fadd_rn(acc.lo, __fadd_rn(__fadd_rn(s.lo, pe), __fadd_rn(t.lo, qe))));
-}
-__device__ __forceinline__ void mac2(double& acc, double a, double b, double c, double d) {
-  acc += a * b + c * d;
-}
-template <typename A>
-__device__ __forceinline__ void cmac(cx<A>& acc, const cx<A>& u, const cx<A>& x) {  // += u x
-  mac2(acc.x, u.x, x.x, -u.y, x.y);
-  mac2(acc.y, u.x, x.y, u.y, x.x);
-}
-template <typename A>
-__device__ __forceinline__ void cmac_conj(cx<A>& acc, const cx<A>& u, const cx<A>& x) {
-  mac2(acc.x, u.x, x.x, u.y, x.y);
-  mac2(acc.y, u.x, x.y, -u.y, x.x);
-}
 __device__ __forceinline__ double shfl_xor(double v, int m) {
   return __shfl_xor_sync(0xffffffffu, v, m);
 }

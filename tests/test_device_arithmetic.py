@@ -84,8 +84,36 @@ static void complex_products() {
   printf("ff_product %.17g\n", sqrt(e[1] / e[0]));
 }
 
+static void sums(int terms) {
+  double e[2] = {0, 0};
+  for (int i = 0; i < 400000 / terms; ++i) {
+    const cff zero = mk<ff>(ff(0.f, 0.f), ff(0.f, 0.f));
+    cff got[2] = {zero, zero}, plain[2] = {zero, zero};
+    long double ex[2][2] = {{0, 0}, {0, 0}};
+    for (int t = 0; t < terms; ++t) {
+      const cff u = mk<ff>(ff(normal()), ff(normal())), x = mk<ff>(ff(normal()), ff(normal()));
+      cmac(got[0], u, x);
+      cmac_conj(got[1], u, x);
+      for (int conj = 0; conj < 2; ++conj) {
+        const ff uy = conj ? -u.y : u.y;
+        plain[conj].x = plain[conj].x + (u.x * x.x - uy * x.y);
+        plain[conj].y = plain[conj].y + (u.x * x.y + uy * x.x);
+        ex[conj][0] += value(u.x) * value(x.x) - value(uy) * value(x.y);
+        ex[conj][1] += value(u.x) * value(x.y) + value(uy) * value(x.x);
+      }
+    }
+    for (int c = 0; c < 2; ++c) {
+      e[0] += powl(value(plain[c].x) - ex[c][0], 2) + powl(value(plain[c].y) - ex[c][1], 2);
+      e[1] += powl(value(got[c].x) - ex[c][0], 2) + powl(value(got[c].y) - ex[c][1], 2);
+    }
+  }
+  printf("ff_sums_%d %.17g\n", terms, sqrt(e[1] / e[0]));
+}
+
 int main() {
   product();
+  sums(8);
+  sums(64);
   complex_products();
   return 0;
 }
@@ -112,3 +140,8 @@ def test_block_product(measured):
 
 def test_float_float_complex_product(measured):
     assert measured["ff_product"] <= 1.05, measured
+
+
+@pytest.mark.parametrize("terms", [8, 64])
+def test_float_float_sums_of_products(measured, terms):
+    assert measured[f"ff_sums_{terms}"] <= 1.05, measured
