@@ -153,6 +153,37 @@ __device__ __forceinline__ double ff_join(ff a) {
 }
 using cff = cx<ff>;
 
+// Sums of float-float values with the precision of an FP64 sum of them, in FP32 instructions: the
+// high and the low parts are added exactly, what is below them gathers in a third part. An
+// addition is 21 FP32 instructions (an FP64 one holds its pipe as long as 64 of them).
+struct ffsum {
+  float hi, lo, c;
+};
+__host__ __device__ __forceinline__ ffsum ffsum_of(ff a) { return ffsum{a.hi, a.lo, 0.f}; }
+__host__ __device__ __forceinline__ ffsum operator+(const ffsum& a, const ffsum& b) {
+  const ff s = ff_two_sum(a.hi, b.hi), t = ff_two_sum(a.lo, b.lo), u = ff_two_sum(s.lo, t.hi);
+  return ffsum{s.hi, u.hi, PEEC_FADD(PEEC_FADD(a.c, b.c), PEEC_FADD(t.lo, u.lo))};
+}
+__host__ __device__ __forceinline__ double ffsum_double(const ffsum& a) {
+  const ff s = ff_two_sum(a.hi, a.lo), t = ff_two_sum(s.lo, a.c);
+#ifdef __CUDA_ARCH__
+  // as ff_join, with the third part in units of the double's last place
+  const unsigned h = __float_as_uint(s.hi);
+  const int e = (int)(h >> 23) & 0xff;
+  if (e >= 60 && e < 255) {
+    const float unit = __uint_as_float((unsigned)(306 - e) << 23);
+    const float u = __fmul_rn(t.hi, unit);
+    int r = __float2int_rn(u) + __float2int_rn(__fmul_rn(t.lo, unit));
+    if ((int)h < 0) r = -r;
+    if (fabsf(u) <= 268435456.f && ((h & 0x7fffffu) != 0 || r >= 0)) {
+      const long long b = (((long long)(h & 0x7fffffffu) + (896ll << 23)) << 29) + r;
+      return __longlong_as_double(b | (long long)((unsigned long long)(h & 0x80000000u) << 32));
+    }
+  }
+#endif
+  return (double)s.hi + ((double)t.hi + (double)t.lo);
+}
+
 // acc += u x and acc += conj(u) x, products and sums one after the other: in float-float, 72
 // operations. Adding the high parts of both products and of the sum exactly and all error terms
 // before one normalisation takes 54, but a chain of 8 to 512 such sums rounds 1.5 times worse.

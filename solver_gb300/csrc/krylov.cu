@@ -22,10 +22,12 @@ struct BasisArith;
 template <>
 struct BasisArith<c64> {
   using A = double;
+  using S = double;  // sums over the lanes
 };
 template <>
 struct BasisArith<cff> {
   using A = ff;
+  using S = ffsum;
 };
 template <typename A, typename T>
 __device__ __forceinline__ cx<A> as(const T& v) {
@@ -257,7 +259,8 @@ __device__ __forceinline__ c64 csign(c64 d) {
 // the basis, read once for v, once for z and twice (then from L1 or L2) for x and t; below some
 // 100k rows the latency of the last CTA. FP64 instructions hold their pipe 64 cycles, so
 // conversions are integer code, lanes' sums are exchanged in halves (16 additions a warp for
-// eight columns instead of 80, float-float ones for a float-float basis), and small systems
+// eight columns instead of 80; of a float-float basis in three FP32 parts, ffsum: in FP64 they
+// cost 5.6 % of a mixed solve at 64x64x32, so 1.0 %), and small systems
 // spread over CTAs of 32 or 128 rows whose warps share out the columns.
 // An iteration outside the operator, mean of a solve: 155 -> 66 us at 64x64x32 (N = 87k), 315 ->
 // 170 us at 128x128x64 (N = 750k), where the basis is read from DRAM at 4 TB/s; the FP64 solve of
@@ -304,9 +307,20 @@ size_t gm_part_doubles(size_t N, int k) {
 __device__ __forceinline__ double shfl_xor(double v, int m) {
   return __shfl_xor_sync(0xffffffffu, v, m);
 }
-__device__ __forceinline__ ff shfl_xor(ff v, int m) {
-  return ff(__shfl_xor_sync(0xffffffffu, v.hi, m), __shfl_xor_sync(0xffffffffu, v.lo, m));
+
+__device__ __forceinline__ ffsum shfl_xor(const ffsum& v, int m) {
+  return ffsum{__shfl_xor_sync(0xffffffffu, v.hi, m), __shfl_xor_sync(0xffffffffu, v.lo, m),
+               __shfl_xor_sync(0xffffffffu, v.c, m)};
 }
+// t ? a : b by value: a choice between array elements would put the array in memory
+__device__ __forceinline__ double lane_pick(bool t, double a, double b) { return t ? a : b; }
+__device__ __forceinline__ ffsum lane_pick(bool t, ffsum a, ffsum b) {
+  return ffsum{t ? a.hi : b.hi, t ? a.lo : b.lo, t ? a.c : b.c};
+}
+__device__ __forceinline__ double lane_sum(double v) { return v; }
+__device__ __forceinline__ ffsum lane_sum(ff v) { return ffsum_of(v); }
+__device__ __forceinline__ double lane_double(double v) { return v; }
+__device__ __forceinline__ double lane_double(const ffsum& v) { return ffsum_double(v); }
 
 // counts the CTA in; true for every thread of the last one, which then sees the others' writes
 __device__ __forceinline__ bool gm_last(unsigned* tick, unsigned cnt) {
@@ -435,24 +449,25 @@ __device__ void gm_dots(const UT* __restrict__ U, size_t N, size_t r0, int rows,
         for (int c = 0; c < KB; ++c)
           if (c < nc) cmac_conj(acc[c], u[c], x);
       }
-      // lanes' sums: halves change hands, so a lane ends with the sum of one of the 16 values
-      A d[2 * KB];
+      // lanes' sums, with the precision of FP64: halves change hands, so a lane ends with the sum
+      // of one of the 16 values
+      typename BasisArith<UT>::S d[2 * KB];
 #pragma unroll
       for (int c = 0; c < KB; ++c) {
-        d[2 * c] = acc[c].x;
-        d[2 * c + 1] = acc[c].y;
+        d[2 * c] = lane_sum(acc[c].x);
+        d[2 * c + 1] = lane_sum(acc[c].y);
       }
 #pragma unroll
       for (int s = KB; s >= 1; s >>= 1) {
         const bool up = lane & (2 * s);
 #pragma unroll
         for (int i = 0; i < s; ++i) {
-          const A o = shfl_xor(up ? d[i] : d[i + s], 2 * s);
-          d[i] = (up ? d[i + s] : d[i]) + o;
+          const auto o = shfl_xor(lane_pick(up, d[i], d[i + s]), 2 * s);
+          d[i] = lane_pick(up, d[i + s], d[i]) + o;
         }
       }
       d[0] = d[0] + shfl_xor(d[0], 1);
-      if (!(lane & 1)) red[buf][wc][wr][lane >> 1] = as_double(d[0]);
+      if (!(lane & 1)) red[buf][wc][wr][lane >> 1] = lane_double(d[0]);
     }
     __syncthreads();
     if (tid < WC * 2 * KB) {

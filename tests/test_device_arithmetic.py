@@ -110,8 +110,33 @@ static void sums(int terms) {
   printf("ff_sums_%d %.17g\n", terms, sqrt(e[1] / e[0]));
 }
 
+static void lanes() {
+  double e[2] = {0, 0};
+  for (int i = 0; i < 100000; ++i) {
+    ffsum f[32];
+    double d[32];
+    long double ex = 0;
+    for (int l = 0; l < 32; ++l) {
+      const ff v(normal() * pow(2.0, 8 * normal()));
+      f[l] = ffsum_of(v);
+      d[l] = (double)v;
+      ex += value(v);
+    }
+    for (int s = 16; s >= 1; s >>= 1)
+      for (int l = 0; l < s; ++l) {
+        f[l] = f[l] + f[l + s];
+        d[l] = d[l] + d[l + s];
+      }
+    const double scale = fabs((double)ex);
+    e[0] += powl((d[0] - ex) / scale, 2);
+    e[1] += powl((ffsum_double(f[0]) - ex) / scale, 2);
+  }
+  printf("lanes %.17g\n", sqrt(e[1] / e[0]));
+}
+
 int main() {
   product();
+  lanes();
   sums(8);
   sums(64);
   complex_products();
@@ -145,3 +170,7 @@ def test_float_float_complex_product(measured):
 @pytest.mark.parametrize("terms", [8, 64])
 def test_float_float_sums_of_products(measured, terms):
     assert measured[f"ff_sums_{terms}"] <= 1.05, measured
+
+
+def test_lane_sums(measured):
+    assert measured["lanes"] <= 1.05, measured
