@@ -35,14 +35,6 @@ __device__ __forceinline__ cx<A> as(const T& v) {
 }
 __device__ __forceinline__ double as_double(double v) { return v; }
 __device__ __forceinline__ double as_double(ff v) { return ff_join(v); }
-template <typename A>
-__device__ __forceinline__ A as_arith(double v) {
-  return v;
-}
-template <>
-__device__ __forceinline__ ff as_arith<ff>(double v) {
-  return ff_split(v);
-}
 template <>
 __device__ __forceinline__ cff as<ff, c64>(const c64& v) {
   return mk<ff>(ff_split(v.x), ff_split(v.y));
@@ -771,7 +763,7 @@ __global__ void __launch_bounds__(GM_TPB, 2) k_gm_orth(UT* U, size_t N, unsigned
   cx<A>* sx = reinterpret_cast<cx<A>*>(gm_smem);
   cx<A>* coef = sx + min(rows, (unsigned)GM_ROWS);
   for (int c = tid; c < k; c += GM_TPB) coef[c] = as<A>(coef_g[c]);
-  const A inv = as_arith<A>(*rnorm);
+  const double inv = *rnorm;
   const size_t head = gs->headlen, initer = (size_t)k;
   c64* headv = gs->head;
   UT* Uk = U + (size_t)k * N;
@@ -781,11 +773,12 @@ __global__ void __launch_bounds__(GM_TPB, 2) k_gm_orth(UT* U, size_t N, unsigned
     const int nr = (int)min((size_t)GM_ROWS, row1 - r0);
     __syncthreads();
     gm_rows<WR, UT, A>(U, N, r0, nr, coef, k, [&](int r, size_t i, const cx<A>& s) {
-      const cx<A> x = cscale(as<A>(w[i]), inv) - s;
-      const c64 xd = as<double>(x);
+      // one FP64 subtraction per part; the basis takes its rounding
+      const c64 wi = w[i], sd = as<double>(s);
+      const c64 xd = mk<double>(fma(wi.x, inv, -sd.x), fma(wi.y, inv, -sd.y));
       if (i < head) headv[i] = xd;
       if (i >= initer) acc += xd.x * xd.x + xd.y * xd.y;
-      const cx<A> u = i > initer ? x : mk<A>(0, 0);
+      const cx<A> u = i > initer ? as<A>(xd) : mk<A>(0, 0);
       if (i != initer) Uk[i] = u;
       sx[r] = u;
     });
