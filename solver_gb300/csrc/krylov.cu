@@ -936,15 +936,23 @@ int gm_post(const GmBody& B) {
   return B.U32 ? gm_kernels(B, B.U32, false) : gm_kernels(B, B.U, false);
 }
 
+// the coefficients and the head in shared memory: 64 KB at the longest cycle (2,047 columns). The
+// limit beyond 48 KB is one for all contexts, as in gm_launch.
+template <typename UT>
+static void xupdate(const c64* x, const UT* U, size_t ldu, const c64* coef, const c64* ypad, int k,
+                    size_t N, c64* out, cudaStream_t st) {
+  const size_t sm = (sizeof(c64) + sizeof(UT)) * (size_t)(k > 0 ? k : 1);
+  if (sm > 48 * 1024)
+    cudaFuncSetAttribute(k_xupdate<UT>, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024);
+  k_xupdate<UT><<<g_stream(N), 256, sm, st>>>(x, U, ldu, coef, ypad, k, N, out);
+}
 void launch_xupdate(const c64* x, const c64* U, size_t ldu, const c64* coef, const c64* ypad,
                     int k, size_t N, c64* out, cudaStream_t st) {
-  k_xupdate<c64><<<g_stream(N), 256, 2 * sizeof(c64) * (k > 0 ? k : 1), st>>>(x, U, ldu, coef,
-                                                                             ypad, k, N, out);
+  xupdate(x, U, ldu, coef, ypad, k, N, out, st);
 }
 void launch_xupdate(const c64* x, const cff* U, size_t ldu, const c64* coef, const c64* ypad,
                     int k, size_t N, c64* out, cudaStream_t st) {
-  k_xupdate<cff><<<g_stream(N), 256, (sizeof(c64) + sizeof(cff)) * (k > 0 ? k : 1), st>>>(
-      x, U, ldu, coef, ypad, k, N, out);
+  xupdate(x, U, ldu, coef, ypad, k, N, out, st);
 }
 
 // ------------------------------------------------------------------------------------
