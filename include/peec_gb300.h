@@ -412,12 +412,12 @@ int peec_conv_info(const peec_ctx* ctx, int i, int* L, int* dims, int* active, i
  * Profiling: the FP32 z-pass forms the autotuner picked for this context's grids, and the
  * times it measured (ms per z pass, mean of three after a warm-up; -1 where a form was not
  * a candidate). Forms, all on y/z-folded spectra (Lx(Ly/2+1)(Lz/2+1) values per block): 0
- * register-direct kernels (1 is another name for them), 2 staged (persistent CTAs, each
+ * register-direct kernels (1 is another name for them, never timed or picked), 2 staged (persistent CTAs, each
  * tile's pencils brought into shared memory by bulk asynchronous copies while the previous
  * tile computes; the edge families in one launch), 3 pair (half-length transforms of the
  * even and the odd z frequencies; measured too, its time is not in the arrays). choice =
- * {face form, edge form, edge radix plan}; face_ms[form]; edge_ms[plan * 3 + form]. The tuner runs when the spectra are built (peec_fill,
- * peec_set_rows) and caches its choice per device and grids. No counterpart in the
+ * {face form, edge form, edge radix plan}; face_ms[form]; edge_ms[plan * 3 + form]. The tuner
+ * runs when the spectra are built (peec_fill, peec_set_rows) and caches its choice per device and grids. No counterpart in the
  * reference (it plans FFTW with MEASURE, FFT_solver_QS_S_type.jl:17-53).
  */
 int peec_zpass_tuning(const peec_ctx* ctx, int choice[3], double face_ms[3], double edge_ms[6]);

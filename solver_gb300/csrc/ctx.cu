@@ -1182,7 +1182,7 @@ static int tune_zpass(peec_ctx* ctx) {
   ZTune z = ctx->zt;
   if (faces) {
     const int nform = zpass_yz_faces(ctx->fam, 6) ? 3 : 1;
-    for (int form = 0; form < nform; ++form) {
+    for (int form = 0; form < nform; form += 2) {  // (form 1 is form 0)
       z.face = form;
       CTX_TRY(timed(z, 0, &c.fms[form]));
       if (c.fms[form] < c.fms[c.face]) c.face = form;
@@ -1198,7 +1198,7 @@ static int tune_zpass(peec_ctx* ctx) {
     const int nform = zpass_yz_edges(ctx->fam, 6) ? 3 : 1;
     double best = -1;
     for (int plan = 0; plan < 2; ++plan) {
-      for (int form = 0; form < nform; ++form) {
+      for (int form = 0; form < nform; form += 2) {
         z.edge = form;
         z.edge_plan = plan;
         double& ms = c.ems[plan * 3 + form];

@@ -1082,7 +1082,7 @@ __global__ void __launch_bounds__(ZTPB, 4) k_zconv1(cx<R>* T0, int nz0, const vo
 // mbarrier completion) while the CTA computes the current tile, so HBM reads overlap the
 // FFT arithmetic instead of stalling it. The first group reads the staged rows; the
 // middle, fused and last groups are those of k_zconv3 / k_zconv1. Spectra come from the
-// y/z-folded FP32 tables (Spectrum::yz32), which stay largely resident in L2.
+// y/z-folded FP32 tables (Spectrum::yz[1]), which stay largely resident in L2.
 // Bounded waits: a copy wait that runs out sets *err, waits once more (bounded) for the
 // copies in flight and ends the CTA.
 
