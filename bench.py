@@ -85,7 +85,7 @@ def parse():
                     help="GMRES iterations in the device-resident loop (a CUDA graph with a "
                          "WHILE node) or one host round trip per iteration (same kernels)")
     ap.add_argument("--lu-solve", choices=["groups", "global"], default="groups",
-                    help="LU solves per warp group of factor components (groups) or by the "
+                    help="LU solves by CTAs of whole factor components (groups) or by the "
                          "synchronisation-free global scheme alone (global)")
     ap.add_argument("--lanes", type=int, default=4,
                     help="concurrent port solves (contexts + host threads), at most the ports")

@@ -347,8 +347,8 @@ int peec_check_wait_limit(peec_ctx* ctx);
 
 /*
  * Work split of the LU solves inside the operator: rows of connected components of
- * the factors with at most max_rows rows (0..512, default 512) are solved per warp, the
- * components of at most 32 rows packed several to a warp, each warp's rows, entries and
+ * the factors with at most max_rows rows (0..512, default 512) are solved per CTA, the
+ * components of at most 64 rows packed several to a CTA, each CTA's rows, entries and
  * right-hand sides first loaded into shared memory; all other rows by the
  * synchronisation-free global scheme. Both give the same results to rounding; 0 routes
  * every row through the global scheme. Takes effect at once. No counterpart in the

@@ -415,8 +415,8 @@ __global__ void __launch_bounds__(TPB) k_ypass(PassSet<R> s, const cx<R>* __rest
 // gathers' latency, float-float the FP32 pipes. The direct kernels (k_xfwd and so on) ran 37M and
 // 52M warp instructions in x and y at 128x128x64, on padding and through three transposes in
 // shared memory with CTA barriers. Operator application at 128x128x64, x / y / inverse y / inverse
-// x: FP32 70 / 78 / 70 / 87 -> 51 / 53 / 65 / 47 us, float-float 262 / 291 / 311 / 258 -> 186 / 234
-// / 252 / 158 us; FP32 at 64x64x32 13.9 / 16.3 / 14.9 / 15.5 -> 8.3 / 6.8 / 7.5 / 8.9 us. FP64
+// x: FP32 70 / 78 / 70 / 87 -> 51 / 53 / 65 / 47 us, float-float 262 / 291 / 311 / 258 -> 209 / 263
+// / 278 / 177 us; FP32 at 64x64x32 13.9 / 16.3 / 14.9 / 15.5 -> 8.3 / 6.8 / 7.5 / 8.9 us. FP64
 // stays direct, like its z passes (its pipe is the bound in either form).
 __device__ __forceinline__ int brevn(int v, int n) {
   return n ? (int)(__brev((unsigned)v) >> (32 - n)) : 0;
@@ -1370,7 +1370,7 @@ __global__ void __launch_bounds__(ZTPB, 4) k_zedge_staged(EdgeSet E, int nzs, in
 // leave the odd half's rows in their place until the even half's are there.
 // What bounds them: FP32 instruction issue and loads, float-float the FP32 pipes; the pruning
 // halves the arithmetic of the padded transforms. z passes of an operator application at
-// 128x128x64, faces + edges: FP32 267 us in the direct and staged forms, 169 here (93 + 72);
+// 128x128x64, faces + edges: FP32 267 us in the direct and staged forms, 176 here;
 // float-float 2541 us direct, 1443 here. FP64 stays direct (see conv_all_t).
 template <typename R>
 struct ZPairJob {

@@ -48,10 +48,11 @@ __device__ __forceinline__ double sgn(int k) { return (k & 1) ? -1.0 : 1.0; }
 
 // x / D for the closed forms' constants 6, 24, 60: the product with 1 / D corrected by its
 // remainder (Markstein, IBM J. Res. Dev. 34, 1990) is the rounded quotient, in three FP64
-// instructions where a division takes some ten; zero is exact, and what is out of the range in
-// which the remainder is exact (or not finite) is divided. With flip for the products by +-1 the
-// dense fill of 24x24x8 bodies takes 21.6 ms instead of 22.9 (bound by the FP64 pipe throughout),
-// the same bits.
+// instructions where a division takes some ten; zero gives zero (without its sign, which no sum
+// here keeps), and what is out of the range in which the remainder is exact (or not finite) is
+// divided. 1e8 random quotients for each D, a third with significands of all ones or zeros in the
+// middle, gave the division's bits. With flip for the products by +-1 the dense fill of 24x24x8
+// bodies takes 21.6 ms instead of 22.9 (bound by the FP64 pipe throughout), the same blocks.
 template <int D>
 __device__ __forceinline__ double div_const(double x) {
   constexpr double r = 1.0 / D;
@@ -1143,7 +1144,7 @@ __device__ __forceinline__ double norm3(double dx, double dy, double dz) {
 // The nine rows in one launch, a thread per distinct cell: the cross rows repeat every cell two
 // or four times over their interleaved axes, and a distance, a sine and a cosine (some 100 FP64
 // instructions) serve all of its entries. Bound by the FP64 pipe. At 48x48x24 (1.0 M entries, half
-// as many cells) 0.24 ms with a launch per row and a sine and cosine per entry. Now 0.04 ms less than half of that.
+// as many cells) 0.24 ms with a launch per row and a sine and cosine per entry, less than half of that so.
 struct RccSet {
   RccRowArgs r[9];
   const double* qs[9];

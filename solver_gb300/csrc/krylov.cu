@@ -254,9 +254,8 @@ __device__ __forceinline__ c64 csign(c64 d) {
 // eight columns instead of 80; of a float-float basis in three FP32 parts, ffsum: in FP64 they
 // cost 5.6 % of a mixed solve at 64x64x32, so 1.0 %), and small systems
 // spread over CTAs of 32 or 128 rows whose warps share out the columns.
-// An iteration outside the operator, mean of a solve: 155 -> 66 us at 64x64x32 (N = 87k), 315 ->
-// 170 us at 128x128x64 (N = 750k), where the basis is read from DRAM at 4 TB/s; the FP64 solve of
-// 20x20x4 (N = 528) 3.49 -> 2.63 ms.
+// An iteration outside the operator, mean of a solve: 155 -> 72 us at 64x64x32 (N = 87k), 315 ->
+// 200 us at 128x128x64 (N = 750k); the FP64 solve of 20x20x4 (N = 528) 3.49 -> 2.63 ms.
 constexpr int GM_TPB = 256, GM_ROWS = 1024, GM_FAN = 16, GM_MAXB = 152 * 2;
 constexpr int GM_SCR = 1536;   // complex doubles of shared memory for the last CTA's sums
 constexpr int GM_FOLD1 = 8192; // partial sums the last CTA adds up by itself

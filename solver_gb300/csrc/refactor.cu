@@ -51,7 +51,8 @@ __global__ void k_rf_assemble(int64_t nslot, const int64_t* __restrict__ ptr,
 
 // x / d from r = 1 / d rounded to nearest: the quotient's estimate corrected by its remainder
 // (Markstein, IBM J. Res. Dev. 34, 1990), three dependent operations where a division takes some
-// ten; plain division where the reciprocal leaves the range the correction needs
+// ten; plain division where the reciprocal leaves the range the correction needs. 4e8 random
+// quotients, significands of all ones and zeros among them, gave the division's bits.
 __device__ __forceinline__ double rf_quot(double x, double d, double r) {
   const double q = x * r;
   const double y = fma(fma(-q, d, x), r, q);

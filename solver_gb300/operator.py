@@ -59,7 +59,7 @@ class GpuOperator:
     """Device-resident PEEC operator for one geometry."""
 
     # settings every new context starts with (process-wide; the library's defaults): the
-    # device-resident GMRES loop, and the largest LU component solved per warp group
+    # device-resident GMRES loop, and the largest LU component solved within a CTA
     DEVICE_LOOP = True
     LU_COMPONENT_MAX = 512
 
@@ -460,9 +460,9 @@ class GpuOperator:
         return int(a.value), int(b.value)
 
     def set_lu_component_max(self, max_rows):
-        """Rows of LU components up to max_rows (<= 512) are solved one component per
-        warp, the rest by the global synchronisation-free scheme (0, the default: all
-        global)."""
+        """Rows of LU components up to max_rows (<= 512, the default) are solved by CTAs that
+        hold whole components, the rest by the global synchronisation-free scheme (0: all
+        rows)."""
         _lib.check(self.h, self.L.peec_set_lu_component_max(self.h, int(max_rows)))
 
     def adjoint(self, x, v1, v2, d1, d2, Is, nvox):
