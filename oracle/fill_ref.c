@@ -1,7 +1,7 @@
 /*
  * ORACLE -- test infrastructure only. CPU restatement of the reference's voxel
- * Lp / P generating-row fill, used by tests/ and bench.py's cpu_baseline leg as
- * the checker; never linked into the product.
+ * Lp / P generating-row fill, used by tests/ and bench.py's cpu_baseline leg to
+ * check against; never linked into the product.
  *
  * Parity unpinned: the reference (Julia) cannot run here and ships no outputs for
  * this path; the rows are held to closed forms (coincident-cell self terms, the

@@ -1,7 +1,7 @@
 """ORACLE -- test infrastructure only.
 
 CPU restatement of the reference FFT-PEEC hot path, used by tests/ (and the
-cpu_baseline leg of bench.py) as the checker. It is never imported by the product
+cpu_baseline leg of bench.py) to check against. It is never imported by the product
 package. Every function follows the reference at the cited lines and keeps its
 algorithm as written: 2N-extent circulant embeddings (store_circulant_fft), the
 per-call zero-padded FFT convolutions, three separate sparse-LU solves in the

@@ -1,5 +1,5 @@
 """ORACLE -- test infrastructure only. CPU restatement of the reference's retarded
-("Rcc", QS_Rcc_FW == 2) operator set-up, used by tests/ as the checker; never imported by
+("Rcc", QS_Rcc_FW == 2) operator set-up, used by tests/ to check against; never imported by
 the product.
 
 Parity unpinned: the reference (Julia) cannot run here and ships no outputs for this

@@ -1,6 +1,6 @@
 """ORACLE -- test infrastructure only. Python access to the dense RIS fill of
 oracle/fill_ref.c (calcola_Lp.jl / calcola_P.jl restated in C, double and long double),
-used by tests/ and by bench.py's cpu_baseline leg as the checker; never by the product."""
+used by tests/ and by bench.py's cpu_baseline leg to check against; never by the product."""
 import ctypes
 
 import numpy as np

@@ -1,5 +1,5 @@
 """ORACLE -- test infrastructure only. CPU restatement of the reference's dense RIS solver
-(src/lib/solverRis), used by tests/ as the checker; never imported by the product.
+(src/lib/solverRis), used by tests/ to check against; never imported by the product.
 
 Parity unpinned: the reference (Julia) cannot run here and ships no outputs for this
 path (its only numeric test is the unrelated electric-field solver). The restatement is

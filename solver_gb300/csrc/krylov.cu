@@ -211,16 +211,12 @@ __global__ void k_add(const c64* __restrict__ a, const c64* __restrict__ b, size
 
 // Small dense triangular products of the compact-WY representation (T upper
 // triangular, column-major with leading dimension ld), one CTA.
-// mode 0: out = T(0:k,0:k) * in;  mode 1: out = T(0:k,0:k)^H * in;
+// mode 0: out = T(0:k,0:k) * in;
 // mode 2: T(0:k, k) = -2 T(0:k,0:k) * in, T(k,k) = 2 (append a reflector)
 __global__ void k_tri(c64* T, int ld, int k, const c64* __restrict__ in, c64* out, int mode) {
   for (int i = threadIdx.x; i < k; i += blockDim.x) {
     c64 s = mk<double>(0, 0);
-    if (mode == 1) {
-      for (int j = 0; j <= i; ++j) s = s + cconj(T[(size_t)i * ld + j]) * in[j];
-    } else {
-      for (int j = i; j < k; ++j) s = s + T[(size_t)j * ld + i] * in[j];
-    }
+    for (int j = i; j < k; ++j) s = s + T[(size_t)j * ld + i] * in[j];
     if (mode == 2) out[i] = cscale(s, -2.0);
     else out[i] = s;
   }

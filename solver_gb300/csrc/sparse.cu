@@ -132,12 +132,6 @@ __global__ void k_perm_gather(const c64* __restrict__ b, const int32_t* __restri
   }
 }
 
-__global__ void k_perm_scatter(const c64* __restrict__ z, const int32_t* __restrict__ perm, int n,
-                               c64* out) {
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-    out[perm[i]] = z[i];
-}
-
 // L2-coherent loads and stores of values other SMs publish during the same launch
 __device__ __forceinline__ c64 ld_cg(const c64* p) {
   const double2 v = __ldcg(reinterpret_cast<const double2*>(p));
@@ -467,9 +461,6 @@ void launch_scale_u(const int32_t* ptr, const c64* val, const c64* dinv, int64_t
 void launch_perm_gather(const c64* b, const int32_t* perm, const double* rs, int n, c64* out,
                         cudaStream_t st) {
   k_perm_gather<<<grid_for(n), 256, 0, st>>>(b, perm, rs, n, out);
-}
-void launch_perm_scatter(const c64* z, const int32_t* perm, int n, c64* out, cudaStream_t st) {
-  k_perm_scatter<<<grid_for(n), 256, 0, st>>>(z, perm, n, out);
 }
 // Raises the shared memory the group kernel may be launched with on the current device
 // to at least smem_bytes (the default limit is 48 KB per block). The limit belongs to the
