@@ -235,7 +235,8 @@ int peec_set_rcc_frequency(peec_ctx* ctx, double freq_hz);
  * factors of SS with Pr*diag(row_scale)*SS*Pc = L*U in CSR form (L lower, U upper;
  * both include their diagonal), perm_r / perm_c as in SuperLU (row i goes to row
  * perm_r[i]; column i to column perm_c[i]). row_scale may be NULL (no scaling; for
- * UMFPACK factors pass F.Rs).
+ * UMFPACK factors pass F.Rs). A refused call leaves no frequency state: applications and
+ * solves return PEEC_ERR_STATE until one is installed whole.
  */
 int peec_set_frequency(peec_ctx* ctx, double w, const double* DZ, int64_t yle_nnz,
                        const int64_t* yle_row, const int64_t* yle_col, const double* yle_val,
